@@ -49,6 +49,17 @@ __device__ __forceinline__ uint64_t tc_operand_desc(uint32_t smem_addr) {
     return d;
 }
 
+// The same for the 64-byte swizzle: rows of 64 bytes, groups of 8 rows 512 bytes apart.
+__device__ __forceinline__ uint64_t tc_operand_desc_64(uint32_t smem_addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(512 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)4 << 61;                                   // 64-byte swizzle
+    return d;
+}
+
 // D (float32, tensor memory) (+)= A (bfloat16, K-major) x B^T (bfloat16, K-major), M 128, N 256, K 16.
 __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(

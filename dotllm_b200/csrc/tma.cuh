@@ -13,11 +13,11 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-enum DlTmapSwizzle { DL_TMAP_SWIZZLE_NONE = 0, DL_TMAP_SWIZZLE_128B = 1 };
+enum DlTmapSwizzle { DL_TMAP_SWIZZLE_NONE = 0, DL_TMAP_SWIZZLE_128B = 1, DL_TMAP_SWIZZLE_64B = 2 };
 
 // Encode a map over `rows` x `cols` bfloat16 with `pitch_bytes` between rows; each copy moves a
 // box of box_rows x box_cols (box_cols * 2 bytes a multiple of 16, at most 256 elements per side;
-// with the 128-byte swizzle box_cols * 2 == 128).  Out-of-range parts of a box read as zero.
+// with the 128-byte swizzle box_cols * 2 == 128, with the 64-byte one 64).  Out-of-range parts of a box read as zero.
 // Returns 0 or a negative code (-1: no driver entry point, -2: the encoder refused).
 int dl_tmap_encode_2d_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch_bytes,
                            uint32_t box_rows, uint32_t box_cols, int swizzle);
@@ -26,6 +26,9 @@ int dl_tmap_encode_2d_bf16(CUtensorMap* out, const void* base, uint64_t rows, ui
 // driver call, and a model's matrices and step buffers come back launch after launch.  Thread-safe.
 int dl_tmap_cached_2d_bf16(CUtensorMap* out, const void* base, unsigned long long rows, unsigned long long cols,
                            unsigned long long pitch_bytes, uint32_t box_rows, uint32_t box_cols, int swizzle);
+// ... and over float32 elements (the 128-byte swizzle then wants boxes of 32 columns).
+int dl_tmap_cached_2d_f32(CUtensorMap* out, const void* base, unsigned long long rows, unsigned long long cols,
+                          unsigned long long pitch_bytes, uint32_t box_rows, uint32_t box_cols, int swizzle);
 
 #ifdef __CUDACC__
 // Copy the box whose first element is (row, col) into shared memory; `bar` receives the bytes.

@@ -11,7 +11,7 @@ import ctypes
 import torch
 
 from ..errors import KernelError
-from . import attention_fast, gemm_skinny, gemm_tc
+from . import attention_fast, gemm_f32_tc, gemm_skinny, gemm_tc
 from . import library as _library
 
 PAGE = 64                      # tokens per cache page (DL_PAGE in csrc/common.cuh)
@@ -1298,7 +1298,8 @@ def linear(x, w, out_dtype=None, resident=False, lazy=False):
     PendingProduct, for a caller whose result goes to ``add_rmsnorm`` as the delta.  x may be a
     ScaledRows.
 
-    float32: the library's own FFMA kernel (true 32-bit, the same bits for any number of rows).
+    float32: the library's own kernels (32-bit accuracy, the same bits for any number of rows): the tensor cores on values
+    split three ways where the matrix is large enough (``gemm_f32_tc.takes``), else FFMA.
     bfloat16: cuBLAS through torch with float32 accumulation, the library product that the
     reference also uses for its projections (src/DotLLM.Cuda/CudaGemm.cs:29-40)."""
     given, rows = x, None
@@ -1323,6 +1324,8 @@ def linear(x, w, out_dtype=None, resident=False, lazy=False):
         if out_dtype != torch.float32:
             raise KernelError("linear: the float32 product writes float32")
         xs = _rows_view(x, "linear x")
+        if gemm_f32_tc.takes(w):
+            return gemm_f32_tc.run(x, xs, w, resident)
         y = torch.empty((M, N), dtype=torch.float32, device=x.device)
         _library.call("dl_gemm_f32", _ptr(x), xs, _ptr(w), _ptr(y), N, M, N, K, _stream())
         return y
