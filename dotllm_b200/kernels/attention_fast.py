@@ -19,6 +19,8 @@ _library.register_signatures({
                                        _I, _F, _I, _I, _P, _P, _I, _P, _I, _P, _P],
     "dl_attention_decode_gated_bf16": [_P, _I, _P, _I, _P, _I, _P, _P, _I, _I, _P, _P, _P, _P, _I, _P, _F, _P, _I, _P, _I, _P, _P, _I, _P, _P, _I, _I,
                                        _I, _I, _I, _F, _I, _I, _P, _P, _I, _P, _I, _P, _P],
+    "dl_attention_f32_tile": [_P, _I, _P, _I, _P, _P, _I, _P, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _F, _P, _P, _I, _I, _P, _P],
+    "dl_attention_f32_split": [_P, _I, _P, _I, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _F, _P, _P, _I, _I, _P, _P, _P, _P],
     "dl_attention_prefill_bf16": [_P, _I, _P, _I, _P, _P, _I, _P, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I,
                                   _F, _I, _I, _P, _F, _P, _P, _I, _P, _P],
     "dl_attention_prefill_tc_bf16": [_P, _I, _I, _P, _I, _P, _P, _I, _P, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I,
@@ -160,11 +162,8 @@ def decode_fresh(q, k, v, cos, sin, rotary_dim, block_table, k_pool, v_pool, n_h
     return out
 
 
-def _prefill(q, q_stride, out, k_pool, v_pool, n_pages, block_table, n_heads, n_kv_heads, head_dim,
-             scale, window, plan, keep_first=0, sinks=None, softcap=0.0, slopes=None, gate=None):
-    tc = PREFILL_TC and head_dim in PREFILL_TC_HEAD_DIMS and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 \
-        and (PREFILL_TC_SPECIAL or (not keep_first and sinks is None)) and (slopes is None or softcap <= 0)
-    rows = PREFILL_TC_ROWS if tc else PREFILL_ROWS
+def _prompt_tiles(plan, rows, device):
+    """(sequence, first row) of every tile of ``rows`` new tokens, and how many; made once per step."""
     if ("prefill_tiles", rows) not in plan.scratch:
         # tiles that see the most keys first: the kernels start blocks in this order, and the short
         # ones at the end fill the multiprocessors' last gaps
@@ -172,10 +171,17 @@ def _prefill(q, q_stride, out, k_pool, v_pool, n_pages, block_table, n_heads, n_
         tiles.sort(key=lambda t: -((plan.starts[t[0]] if plan.starts else 0) + min(plan.news[t[0]], t[1] + rows)))
         tile_seq, tile_row0 = [t[0] for t in tiles], [t[1] for t in tiles]
         host = torch.tensor(tile_seq + tile_row0, dtype=torch.int32).pin_memory()
-        dev = host.to(q.device, non_blocking=True)
+        dev = host.to(device, non_blocking=True)
         # the pinned list stays with the plan: a captured step copies it again, from this memory, at every replay
         plan.scratch[("prefill_tiles", rows)] = (dev[:len(tile_seq)], dev[len(tile_seq):], len(tile_seq), host)
-    tile_seq, tile_row0, n_tiles, _ = plan.scratch[("prefill_tiles", rows)]
+    return plan.scratch[("prefill_tiles", rows)][:3]
+
+
+def _prefill(q, q_stride, out, k_pool, v_pool, n_pages, block_table, n_heads, n_kv_heads, head_dim,
+             scale, window, plan, keep_first=0, sinks=None, softcap=0.0, slopes=None, gate=None):
+    tc = PREFILL_TC and head_dim in PREFILL_TC_HEAD_DIMS and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 \
+        and (PREFILL_TC_SPECIAL or (not keep_first and sinks is None)) and (slopes is None or softcap <= 0)
+    tile_seq, tile_row0, n_tiles = _prompt_tiles(plan, PREFILL_TC_ROWS if tc else PREFILL_ROWS, q.device)
     if tc:
         _library.call("dl_attention_prefill_tc_bf16", q.data_ptr(), q_stride, q.shape[0], out.data_ptr(), out.stride(0),
                       k_pool.data_ptr(), v_pool.data_ptr(), n_pages, tile_seq.data_ptr(), tile_row0.data_ptr(),
@@ -217,3 +223,43 @@ def run(q, q_stride, out, k_pool, v_pool, n_pages, token_seq, token_pos, block_t
         return _prefill(q, q_stride, out, k_pool, v_pool, n_pages, block_table, n_heads, n_kv_heads,
                         head_dim, scale, window, plan, keep_first, sinks, softcap, slopes, gate)
     return False
+
+
+F32_HEAD_DIMS = (64, 128)            # head sizes of the float32 kernels (keys and values of one width); others take the generic kernel
+F32_MAX_GROUP = 16                   # AF_MAX_GROUP in csrc/attention_f32.cu
+F32_TILE_ROWS = 64                   # AF_ROWS
+# Steps whose sequences bring at most SPLIT_TOKENS new tokens go token by token to the kernel that cuts the keys into pages; longer
+# ones to the kernel over tiles of 64 rows, unless those are too few to fill the machine.  Both give a query the same bits.  Measured
+# (32 heads of 64, one sequence, kernels alone; a tile's time does not depend on how full it is): 8 new tokens after 1,500 25 against
+# 208 us, 32 after 1,500 60 against 208, 32 after 200 20 against 40; a token's pages are read again for every token, so where tiles
+# fill the machine the line is lower.
+F32_SPLIT_TOKENS, F32_SPLIT_TOKENS_FEW, F32_FULL_BLOCKS = 8, 32, 148
+
+
+def run_f32(q, q_stride, out, k_pool, v_pool, n_pages, token_seq, token_pos, block_table, n_heads, n_kv_heads, head_dim, scale, window, plan,
+            keep_first=0, sinks=None, softcap=0.0, slopes=None, gate=None):
+    """The float32 kernels of csrc/attention_f32.cu into ``out``; False where the generic kernel has to take the call.  What decides
+    is the same for a model's steps of any size (the two give different bits), alignment apart."""
+    if head_dim not in F32_HEAD_DIMS or n_heads // n_kv_heads > F32_MAX_GROUP or q_stride % 4 or q.data_ptr() % 16 or k_pool.data_ptr() % 16 \
+            or v_pool.data_ptr() % 16 or not plan.news or q.shape[0] != sum(plan.news):
+        return False
+    tail = (n_heads, n_kv_heads, head_dim, scale, window, float(softcap), None if slopes is None else slopes.data_ptr(), *_gate_args(gate),
+            int(keep_first), None if sinks is None else sinks.data_ptr())
+    head = (q.data_ptr(), q_stride, out.data_ptr(), out.stride(0), k_pool.data_ptr(), v_pool.data_ptr(), n_pages)
+    T = q.shape[0]
+    few = sum(-(-n // F32_TILE_ROWS) for n in plan.news) * n_heads <= F32_FULL_BLOCKS
+    if plan.max_new <= (F32_SPLIT_TOKENS_FEW if few else F32_SPLIT_TOKENS) and T <= 65535:
+        n = T * n_heads * block_table.shape[1]
+        key = ("f32_parts", n, head_dim)
+        if key not in plan.scratch:                        # the layers of a step run one after another on one stream
+            plan.scratch[key] = torch.empty(n * (head_dim + 2), dtype=torch.float32, device=q.device)
+        parts = (plan.scratch[key].data_ptr(), plan.scratch[key].data_ptr() + 4 * n * head_dim)
+        _library.call("dl_attention_f32_split", *head, token_seq.data_ptr(), token_pos.data_ptr(), block_table.data_ptr(), block_table.shape[1], T,
+                      *tail, *parts, _library.current_stream())
+        return True
+    tile_seq, tile_row0, n_tiles = _prompt_tiles(plan, F32_TILE_ROWS, q.device)
+    if n_tiles > 65535:
+        return False
+    _library.call("dl_attention_f32_tile", *head, tile_seq.data_ptr(), tile_row0.data_ptr(), n_tiles, plan.seq_start.data_ptr(),
+                  plan.seq_new.data_ptr(), plan.cu_new.data_ptr(), block_table.data_ptr(), block_table.shape[1], *tail, _library.current_stream())
+    return True

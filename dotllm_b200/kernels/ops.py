@@ -716,6 +716,10 @@ def attention(q, k_pool, v_pool, token_seq, token_pos, block_table, n_heads, n_k
                               n_heads, n_kv_heads, head_dim, float(scale), int(window), plan,
                               keep_first=int(keep_first), sinks=sinks, softcap=softcap, split=split, slopes=slopes, gate=gate):
             return out
+    if plan is not None and q.dtype == torch.float32 and vd == head_dim:
+        if attention_fast.run_f32(q, qs, out, k_pool, v_pool, n_pages, token_seq, token_pos, block_table, n_heads, n_kv_heads, head_dim,
+                                  float(scale), int(window), plan, int(keep_first), sinks, softcap, slopes, gate):
+            return out
     _library.call("dl_attention_generic", _ptr(q), qs, _ptr(out), out.stride(0), _code(q.dtype),
                   _ptr(k_pool), _ptr(v_pool), n_pages, _ptr(token_seq), _ptr(token_pos),
                   _ptr(block_table), block_table.shape[1], T, n_heads, n_kv_heads, head_dim, vd,
