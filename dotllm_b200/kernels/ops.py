@@ -38,7 +38,10 @@ _library.register_signatures({
     "dl_per_head_rows": [_P, _I, _I, _P, _I, _I, _I, _P, _I, _I, _P, _I, _I, _I, _P, _P, _I, _P, _I, _P],
     "dl_channel_gate": [_P, _I, _I, _P, _I, _P, _I, _I, _I, _I, _I, _F, _P],
     "dl_delta_rule": [_P, _I, _P, _I, _I, _P, _I, _P, _I, _P, _P, _P, _P, _P, _P, _P, ctypes.c_long, _I,
-                      _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _I, _P],
+                      _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _I, _P, _I, _P],
+    "dl_gla_chunk": [_P, _P, _P, _I, _P, _I, _P, _P, _P, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _F, _F, _I, _P],
+    "dl_gla_chunk_scratch": [_I, _I, _I, _I, _P],
+    "dl_delta_chunk_scratch": [_I, _I, _I, _P],
     "dl_expert_gate_up": [_P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P],
     "dl_expert_down": [_P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _I, _P, _I, _I, _P],
     "dl_expert_sort": [_P, _I, _I, _P, _P, _I, _P],
@@ -816,12 +819,33 @@ def gated_activation(gate_up, kind, limit=0.0, alpha=1.0, bias=None):
 
 
 # ------------------------------------------------------- gated linear attention
-def gla_scan(q, k, v, z, z_bias, cu_new, slots, state, n_heads, dim, vdim, q_scale, tau=1.0):
+CHUNK = 32                       # CK_L in csrc/chunk_scan.cu
+CHUNK_MAX_DIM = 64               # CK_DIM
+CHUNK_SCRATCH_BYTES = 4 << 30    # most scratch the chunks' operands may take (1.2 KB a token and head); more: token by token
+# Steps whose longest sequence brings fewer tokens walk them one by one: a scan takes 0.11 (gated linear attention) to 0.19 us (delta rule)
+# a token, whatever else is in the batch, the chunks' launches 25 to 45 us (16 heads of 64 x 128, one sequence of 300 tokens: 33 and 58 us by
+# the scans, 20 and 59 by chunks; of 2,048: 227 and 320 against 95 and 199).
+CHUNK_MIN_TOKENS = 256
+
+
+def _chunk_scratch(device, name, n_seqs, max_new, n_heads, *more):
+    """(scratch, chunks of the longest sequence) of a recurrence's chunked form, or (None, 0) where it would take too much."""
+    chunks = (int(max_new) + CHUNK - 1) // CHUNK
+    need = ctypes.c_longlong(0)
+    getattr(_library.library(), name)(n_seqs, chunks, n_heads, *more, ctypes.byref(need))
+    if 4 * need.value > CHUNK_SCRATCH_BYTES or n_seqs > 65535 or n_heads > 65535:
+        return None, 0
+    return torch.empty(need.value, dtype=torch.float32, device=device), chunks
+
+
+def gla_scan(q, k, v, z, z_bias, cu_new, slots, state, n_heads, dim, vdim, q_scale, tau=1.0, max_new=1):
     """The recurrence S_t = diag(alpha_t) S_(t-1) + k_t v_t^T, o_t = S_t^T (q_t q_scale) with
     alpha_t = sigmoid(z_t + z_bias)^(1/tau), over each sequence's new rows in order, from and into
     ``state`` float32 [slots, H, dim, vdim].  q, k [T, H*dim] and v [T, H*vdim] are column views of one
     matrix (a common row stride) and of one dtype, z float32 [T, H*dim].  With ``z`` None the decay is one constant
     per head, ``z_bias`` float32 [H] holding it, and q, k and v pass through silu on their way into the recurrence.
+    ``max_new``: the most tokens a sequence brings - prompts of a bfloat16 run go a chunk of tokens at a time (csrc/chunk_scan.cu,
+    float32 as the scan, another order of its sums).
     Returns o float32 [T, H*vdim]."""
     _need_cuda(q, k, v, z, z_bias, cu_new, slots, state)
     T = q.shape[0]
@@ -840,6 +864,14 @@ def gla_scan(q, k, v, z, z_bias, cu_new, slots, state, n_heads, dim, vdim, q_sca
     _int32(cu_new, "gla cu_new")
     _int32(slots, "gla slots")
     out = torch.empty((T, n_heads * vdim), dtype=torch.float32, device=q.device)
+    if q.dtype == torch.bfloat16 and max_new >= CHUNK_MIN_TOKENS and dim <= CHUNK_MAX_DIM and vdim % 4 == 0 and ld % 4 == 0 and v.data_ptr() % 8 == 0 \
+            and state.data_ptr() % 16 == 0:
+        scratch, chunks = _chunk_scratch(q.device, "dl_gla_chunk_scratch", slots.numel(), max_new, n_heads, vdim)
+        if scratch is not None:
+            _library.call("dl_gla_chunk", _ptr(q), _ptr(k), _ptr(v), ld, _ptr(z), zs, _ptr(z_bias), _ptr(cu_new), _ptr(slots), _ptr(state),
+                          state.shape[0], _ptr(out), out.stride(0), _ptr(scratch), slots.numel(), T, n_heads, dim, vdim, float(q_scale), float(tau),
+                          chunks, _stream())
+            return out
     _library.call("dl_gla_scan", _ptr(q), _ptr(k), _ptr(v), ld, _ptr(z), zs, _ptr(z_bias), _code(q.dtype), _ptr(cu_new),
                   _ptr(slots), _ptr(state), state.shape[0], _ptr(out), out.stride(0), slots.numel(), T, n_heads, dim, vdim,
                   float(q_scale), float(tau), _stream())
@@ -1049,7 +1081,7 @@ def channel_gate(o, gate, heads, width, lay=None, scale=1.0, out=None):
 
 # ------------------------------------------------------------------ delta rule
 def delta_rule(x, taps, b_logit, z, dt_bias, a_log, token_seq, cu_new, slots, memory, n_heads, n_kv_heads, dim, vdim,
-               q_scale, unit_eps, head_decay=False):
+               q_scale, unit_eps, head_decay=False, max_new=1):
     """The gated delta rule with a decay per key channel over each sequence's new rows in order.
 
     x [T, >= C]: the stacked projection, its first C = 2*G*dim + H*vdim columns the channels of q, k (G = ``n_kv_heads``
@@ -1059,6 +1091,7 @@ def delta_rule(x, taps, b_logit, z, dt_bias, a_log, token_seq, cu_new, slots, me
     (query/key head h // (H/G)): S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q.
     ``memory`` float32 [slots, H*dim*vdim + (K-1)*C]: per slot the states and behind them the convolution's last K - 1
     inputs; read and updated.  ``head_decay``: one decay for all key channels of a head, z float32 [T, H] and dt_bias [H].
+    ``max_new``: the most tokens a sequence brings - prompts of a bfloat16 run go a chunk of tokens at a time, as in ``gla_scan``.
     Returns o float32 [T, H*vdim]."""
     _need_cuda(x, taps, b_logit, z, dt_bias, a_log, token_seq, cu_new, slots, memory)
     T = x.shape[0]
@@ -1083,11 +1116,14 @@ def delta_rule(x, taps, b_logit, z, dt_bias, a_log, token_seq, cu_new, slots, me
     qo, ko = torch.empty((T, G * dim), **f32), torch.empty((T, G * dim), **f32)
     vo, go = torch.empty((T, H * vdim), **f32), torch.empty((T, H * dim), **f32)
     bo, out = torch.empty((T, H), **f32), torch.empty((T, H * vdim), **f32)
+    scratch, chunks = None, 0
+    if x.dtype == torch.bfloat16 and max_new >= CHUNK_MIN_TOKENS and dim <= CHUNK_MAX_DIM and vdim % 4 == 0:
+        scratch, chunks = _chunk_scratch(x.device, "dl_delta_chunk_scratch", slots.numel(), max_new, H)
     _library.call("dl_delta_rule", _ptr(x), ld, _ptr(taps), K, _code(x.dtype), _ptr(b_logit), _rows_view(b_logit, "delta_rule b"),
                   _ptr(z), _rows_view(z, "delta_rule z"), _ptr(dt_bias), _ptr(a_log), _ptr(token_seq), _ptr(cu_new), _ptr(slots),
                   memory.data_ptr(), memory.data_ptr() + 4 * n_state, memory.stride(0), memory.shape[0],
                   _ptr(qo), _ptr(ko), _ptr(vo), _ptr(go), _ptr(bo), _ptr(out), slots.numel(), T, H, G, int(dim), int(vdim),
-                  float(q_scale), float(unit_eps), 1 if head_decay else 0, _stream())
+                  float(q_scale), float(unit_eps), 1 if head_decay else 0, _ptr(scratch), chunks, _stream())
     return out
 
 

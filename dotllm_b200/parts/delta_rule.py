@@ -147,7 +147,7 @@ class ChannelDeltaMixer(Mixer):
         gate = ops.linear(low_gate, self.w_gate, resident=True) if self.gate_low_rank else low_gate
         o = ops.delta_rule(proj, self.conv, b, z, self.decay_bias, self.rate, step.token_seq, step.cu_new, cache_view.slots,
                            cache_view.state, self.n_heads, self.n_kv_heads, self.key_dim, self.value_dim,
-                           self.key_dim ** -0.5, self.unit_eps, head_decay=self.head_decay)
+                           self.key_dim ** -0.5, self.unit_eps, head_decay=self.head_decay, max_new=step.attention_plan.max_new)
         y = ops.head_norm_gate(o, gate, self.norm_gain, self.n_heads, self.value_dim, self.eps, self.runtime.dtype,
                                gate=self.gate_activation)
         return ops.linear(y, self.w_o, out_dtype=BRANCH_DTYPE, resident=True, lazy=True)

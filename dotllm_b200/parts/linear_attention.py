@@ -83,7 +83,8 @@ class GatedLinearAttentionMixer(Mixer):
         gate, low = proj[:, 2 * kw + vw:2 * kw + 2 * vw], proj[:, 2 * kw + 2 * vw:]
         z = ops.linear(low, self.w_decay, out_dtype=torch.float32, resident=True)
         o = ops.gla_scan(q, k, v, z, self.decay_bias, step.cu_new, cache_view.slots, cache_view.state,
-                         self.n_heads, self.key_dim, self.value_dim, self.key_dim ** -0.5, self.tau)
+                         self.n_heads, self.key_dim, self.value_dim, self.key_dim ** -0.5, self.tau,
+                         max_new=step.attention_plan.max_new)
         y = ops.head_norm_gate(o, gate, self.norm_gain, self.n_heads, self.value_dim, self.eps, self.runtime.dtype)
         return ops.linear(y, self.w_o, out_dtype=BRANCH_DTYPE, resident=True, lazy=True)
 
@@ -150,7 +151,7 @@ class DecayedLinearAttentionMixer(Mixer):
         proj = ops.linear(x, self.w_in, resident=True)
         q, k, v, gate = proj[:, :kw], proj[:, kw:2 * kw], proj[:, 2 * kw:2 * kw + vw], proj[:, 2 * kw + vw:2 * kw + 2 * vw]
         o = ops.gla_scan(q, k, v, None, self.decay, step.cu_new, cache_view.slots, cache_view.state, self.n_heads, self.key_dim,
-                         self.value_dim, 1.0)
+                         self.value_dim, 1.0, max_new=step.attention_plan.max_new)
         y = ops.head_norm_gate(o, gate, self.norm_gain, 1, vw, self.eps, self.runtime.dtype, gate="sigmoid")
         return ops.linear(y, self.w_o, out_dtype=BRANCH_DTYPE, resident=True, lazy=True)
 

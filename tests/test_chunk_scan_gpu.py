@@ -1,0 +1,105 @@
+"""The chunked form of the two recurrences with a decay per key channel, against float64 and against the token-by-token scans."""
+import numpy as np
+import pytest
+import torch
+
+import kernel_refs
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def g64(*shape, seed=0, scale=1.0):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed), dtype=torch.float64) * scale
+
+
+def i32(v):
+    return torch.tensor([int(x) for x in v], dtype=torch.int32, device=DEV)
+
+
+# A sum of up to 64 state channels plus 32 tokens, each term rounded once or twice: some hundred roundings of terms no larger than the
+# results' scale (values of about 10 here).
+TOL = 2e-5
+
+
+@pytest.mark.parametrize("lens", [[2], [64], [1, 96, 31, 32, 33, 2], [257, 100]])
+@pytest.mark.parametrize("H,dim,vdim", [(2, 64, 128), (2, 40, 24), (2, 1, 4), (2, 24, 68)])
+@pytest.mark.parametrize("form", ["logits", "steep", "constant"])
+def test_gated_linear_attention(lens, H, dim, vdim, form, monkeypatch):
+    from dotllm_b200.kernels import ops
+    monkeypatch.setattr(ops, "CHUNK_MIN_TOKENS", 2)
+    T, tau = sum(lens), 5.0
+    proj = g64(T, 2 * H * dim + H * vdim + 4, seed=1).to(torch.bfloat16).to(DEV)
+    q, k, v = proj[:, :H * dim], proj[:, H * dim:2 * H * dim], proj[:, 2 * H * dim:2 * H * dim + H * vdim]
+    z = None if form == "constant" else (g64(T, H * dim, seed=3) * (80.0 if form == "steep" else 2.0)).float().to(DEV)
+    bias = (torch.linspace(0.3, 1.0, H) if z is None else g64(H * dim, seed=5)).float().to(DEV)
+    slots = [4, 0, 3, 1, 5, 2][:len(lens)]
+    state0 = g64(7, H, dim, vdim, seed=6).float().to(DEV)
+    cu = i32([0] + list(np.cumsum(lens)))
+
+    def run(most):
+        s = state0.clone()
+        return ops.gla_scan(q, k, v, z, bias, cu, i32(slots), s, H, dim, vdim, 0.3, tau, max_new=most), s
+
+    got, state = run(max(lens))
+    scan, _ = run(1)
+    act = (lambda t: t * torch.sigmoid(t)) if z is None else (lambda t: t)
+    at = 0
+    for n, slot in zip(lens, slots):
+        rows = slice(at, at + n)
+        qd, kd = act(q[rows].double()).view(n, H, dim) * 0.3, act(k[rows].double()).view(n, H, dim)
+        vd, s = act(v[rows].double()).view(n, H, vdim), state0[slot].double()
+        alpha = bias.double().view(1, H, 1).expand(n, H, dim) if z is None else \
+            (torch.nn.functional.logsigmoid((z[rows] + bias).double()) / tau).exp().view(n, H, dim)
+        want = torch.empty(n, H, vdim, dtype=torch.float64, device=DEV)
+        for t in range(n):
+            s = alpha[t].unsqueeze(-1) * s + kd[t].unsqueeze(-1) * vd[t].unsqueeze(1)
+            want[t] = (s * qd[t].unsqueeze(-1)).sum(1)
+        scale = 1.0 + float(want.abs().max())
+        assert float((got[rows].view(n, H, vdim) - want).abs().max()) < TOL * scale
+        assert float((state[slot] - s).abs().max()) < TOL * (1 + float(s.abs().max()))
+        # no further off than the scan, beyond the last bits
+        far = lambda x: float((x[rows].view(n, H, vdim) - want).norm() / want.norm())
+        assert far(got) < 1.5 * far(scan) + 1e-7
+        at += n
+    others = [i for i in range(7) if i not in slots]
+    assert torch.equal(state[others], state0[others])
+
+
+@pytest.mark.parametrize("H,G,dim,vdim", [(4, 2, 64, 128), (2, 2, 24, 20), (1, 1, 8, 4), (6, 2, 40, 68), (40, 40, 64, 128)])
+@pytest.mark.parametrize("head_decay", [False, True])
+def test_delta_rule(H, G, dim, vdim, head_decay, monkeypatch):
+    """(Forty heads of 128 value channels: the walk over 32 columns a block; the others: over 16.)"""
+    from dotllm_b200.kernels import ops
+    monkeypatch.setattr(ops, "CHUNK_MIN_TOKENS", 2)
+    K, lens = 4, [70, 1, 97, 32, 5]
+    C, T, n_state = 2 * G * dim + H * vdim, sum(lens), H * dim * vdim
+    taps = g64(C, K, seed=1, scale=0.5).to(torch.bfloat16)
+    decays = H if head_decay else H * dim
+    dt_bias, a_log = g64(decays, seed=2).float(), g64(H, seed=3, scale=0.5).float()
+    x = g64(T, C + H, seed=10).to(torch.bfloat16)
+    z = g64(T, decays, seed=20).float()
+    memory = g64(6, n_state + (K - 1) * C, seed=4).float()
+    slots = [4, 1, 5, 0, 2]
+    seq, cu = [i for i, n in enumerate(lens) for _ in range(n)], [0] + list(np.cumsum(lens))
+    gx = x.to(DEV)
+
+    def run(most):
+        m = memory.clone().to(DEV)
+        return ops.delta_rule(gx, taps.to(DEV), gx[:, C:], z.to(DEV), dt_bias.to(DEV), a_log.to(DEV), i32(seq), i32(cu), i32(slots), m, H, G, dim, vdim,
+                              dim ** -0.5, 1e-6, head_decay=head_decay, max_new=most), m
+
+    got, mem = run(max(lens))
+    scan, scan_mem = run(1)
+    if H > 6:                                              # the oracle takes too long: the scan, which it has been held to at other sizes
+        want, want_mem = scan.cpu(), scan_mem.cpu()
+    else:
+        want_mem = memory.clone()
+        want = kernel_refs.delta_rule(x, taps, x[:, C:], z.repeat_interleave(dim, 1) if head_decay else z,
+                                      dt_bias.repeat_interleave(dim) if head_decay else dt_bias, a_log, torch.tensor(seq), torch.tensor(cu),
+                                      torch.tensor(slots), want_mem, H, G, dim, vdim, dim ** -0.5, 1e-6)
+    scale = 1.0 + float(want.abs().max())
+    assert float((got.cpu() - want).abs().max()) < 3 * TOL * scale
+    assert float((mem.cpu() - want_mem).abs().max()) < 3 * TOL * (1 + float(want_mem.abs().max()))
+    assert float((got - scan).abs().max()) < 3 * TOL * scale
+    assert torch.equal(mem[3], memory[3].to(DEV)) and torch.equal(mem[:, n_state:], scan_mem[:, n_state:])
