@@ -145,6 +145,110 @@ delta_prepare_kernel(const T* __restrict__ x, int ld, const T* __restrict__ taps
     }
 }
 
+// The same for prompts that go chunk by chunk, bfloat16 rows, at most four taps and heads of 16, 32, 64 or 128 key channels: a thread
+// takes four neighbouring channels of four tokens in a row, so that its seven 8-byte rows are asked for at once (the kernel above
+// waits for one row after the other: 3,743 tokens of 8,192 channels in 205 us, this one in 105; the bytes alone are 37).  Tiles of
+// 256 channels along grid.y, then tiles of 256 decays (the step sizes with them).
+#define DP_VEC_TILE 256
+#define DP_VEC_TOKENS 8                                   // tokens a block: two runs of four
+__device__ __forceinline__ float4 dp_load4(const __nv_bfloat16* p) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), b = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+    return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
+}
+__device__ __forceinline__ float dp_silu(float v) { return v / (1.0f + expf(-v)); }
+
+__global__ void __launch_bounds__(DP_THREADS)
+delta_prepare_vec_kernel(const __nv_bfloat16* __restrict__ x, int ld, const __nv_bfloat16* __restrict__ taps, int K, const float* __restrict__ hist,
+                         long slot_stride, int n_slots, const int32_t* __restrict__ token_seq, const int32_t* __restrict__ cu_new,
+                         const int32_t* __restrict__ slots, const __nv_bfloat16* __restrict__ b_logit, int b_stride, const float* __restrict__ z,
+                         int z_stride, const float* __restrict__ dt_bias, const float* __restrict__ a_log, float* __restrict__ qo, float* __restrict__ ko,
+                         float* __restrict__ vo, float* __restrict__ go, float* __restrict__ bo, int H, int G, int dim, int vdim, float q_scale,
+                         float unit_eps, int n_tokens, int head_decay, int channel_tiles) {
+    dl_launch_dependents();
+    dl_grid_dependency_wait();
+    const int qk = 2 * G * dim, C = qk + H * vdim;
+    const int t0 = blockIdx.x * DP_VEC_TOKENS + (threadIdx.x >> 6) * 4, sub = (threadIdx.x & 63) * 4;
+    if ((int)blockIdx.y >= channel_tiles) {                // decays and step sizes
+        const int c = ((int)blockIdx.y - channel_tiles) * DP_VEC_TILE + sub, h = c / dim;     // dim is a multiple of 4: one head
+        if (c >= H * dim) return;
+        const float rate = expf(a_log[h]);
+        float4 zs[4];
+        const float4 bias = head_decay ? make_float4(dt_bias[h], dt_bias[h], dt_bias[h], dt_bias[h]) : *reinterpret_cast<const float4*>(dt_bias + c);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const long row = min(t0 + i, n_tokens - 1);
+            if (head_decay) zs[i].x = z[row * z_stride + h];
+            else zs[i] = *reinterpret_cast<const float4*>(z + row * z_stride + c);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = t0 + i;
+            if (t >= n_tokens) break;
+            float4 g;
+            g.x = expf(-rate * dr_softplus(zs[i].x + bias.x));
+            if (head_decay) g.y = g.z = g.w = g.x;
+            else {
+                g.y = expf(-rate * dr_softplus(zs[i].y + bias.y));
+                g.z = expf(-rate * dr_softplus(zs[i].z + bias.z));
+                g.w = expf(-rate * dr_softplus(zs[i].w + bias.w));
+            }
+            *reinterpret_cast<float4*>(go + (long)t * H * dim + c) = g;
+            if (c % dim == 0) bo[(long)t * H + h] = 1.0f / (1.0f + expf(-__bfloat162float(b_logit[(long)t * b_stride + h])));
+        }
+        return;
+    }
+    const int c = blockIdx.y * DP_VEC_TILE + sub;
+    const bool live = c < C;
+    const int cc = live ? c : 0;
+    float4 in[7], tap[4];                                  // rows t0 - 3 .. t0 + 3; taps, place 3 - lag meets the input `lag` tokens back
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+        const int t = t0 - 3 + i;
+        in[i] = dp_load4(x + (long)min(max(t, 0), n_tokens - 1) * ld + cc);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int lag = 3 - i;
+        float e[4];
+#pragma unroll
+        for (int d = 0; d < 4; ++d) e[d] = lag < K ? __bfloat162float(taps[(long)(cc + d) * K + (K - 1 - lag)]) : 0.f;
+        tap[i] = make_float4(e[0], e[1], e[2], e[3]);
+    }
+    const int lanes = dim / 4;                             // lanes of a head: 4, 8, 16 or 32, aligned (a tile starts at a whole head)
+    const bool is_v = c >= qk;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = t0 + i, row = min(t, n_tokens - 1), b = token_seq[row], slot = slots[b], j = row - cu_new[b];
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {                      // oldest first; a place in front of the taps adds 0 * 0
+            const int lag = 3 - p;
+            float4 v = in[i + p];
+            if (lag >= K) v = make_float4(0.f, 0.f, 0.f, 0.f);
+            else if (lag > j)                              // before the sequence's new tokens: its history, whose row K - 2 is the newest
+                v = slot >= 0 && slot < n_slots ? *reinterpret_cast<const float4*>(hist + (long)slot * slot_stride + (long)(K - 1 - (lag - j)) * C + cc)
+                                                : make_float4(0.f, 0.f, 0.f, 0.f);
+            acc.x = fmaf(tap[p].x, v.x, acc.x);
+            acc.y = fmaf(tap[p].y, v.y, acc.y);
+            acc.z = fmaf(tap[p].z, v.z, acc.z);
+            acc.w = fmaf(tap[p].w, v.w, acc.w);
+        }
+        float4 y = make_float4(dp_silu(acc.x), dp_silu(acc.y), dp_silu(acc.z), dp_silu(acc.w));
+        float ss = (y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w);
+        for (int o = lanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (!live || t >= n_tokens || slot < 0 || slot >= n_slots) continue;
+        if (is_v) {
+            *reinterpret_cast<float4*>(vo + (long)t * H * vdim + (c - qk)) = y;
+            continue;
+        }
+        const bool query = c < G * dim;
+        const float r = (1.0f / sqrtf(ss + unit_eps)) * (query ? q_scale : 1.0f);
+        float* dst = query ? qo + (long)t * G * dim + c : ko + (long)t * G * dim + (c - G * dim);
+        *reinterpret_cast<float4*>(dst) = make_float4(y.x * r, y.y * r, y.z * r, y.w * r);
+    }
+}
+
 // The history after a step of any shape: the last K - 1 inputs of each sequence, oldest first.  One thread per (sequence,
 // channel); runs behind delta_prepare (which read the old history).
 template <typename T>
@@ -336,6 +440,9 @@ extern "C" int dl_delta_rule(const void* x, int ld, const void* taps, int K, int
     if (n_seqs == 0 || n_tokens == 0) return DL_OK;
     cudaStream_t s = (cudaStream_t)stream;
     const bool single = n_tokens == n_seqs;               // every sequence brings exactly one token
+    const bool vec = chunk_scratch != nullptr && dtype == DL_BF16 && K <= 4 && !single && (dim == 16 || dim == 32 || dim == 64 || dim == 128) && vdim % 4 == 0 &&
+                     ld % 4 == 0 && ((uintptr_t)x % 8) == 0 && slot_stride % 4 == 0 && ((uintptr_t)hist % 16) == 0 &&
+                     (head_decay || (z_stride % 4 == 0 && ((uintptr_t)z % 16) == 0 && ((uintptr_t)dt_bias % 16) == 0));
     // enough blocks for a few rounds over the machine; beyond that a block walks a run of tokens
     const long rounds = (long)n_tokens * (2 * G + H) / 4096;
     const int per_block = rounds < 1 ? 1 : rounds > DP_RUN ? DP_RUN : (int)rounds;
@@ -347,7 +454,13 @@ extern "C" int dl_delta_rule(const void* x, int ld, const void* taps, int K, int
                             K, hist, slot_stride, n_slots, token_seq, cu_new, slots, (const T*)b_logit, b_stride, z,          \
                             z_stride, dt_bias, a_log, qo, ko, vo, go, bo, H, G, dim, vdim, q_scale, unit_eps,                 \
                             single ? 1 : 0, n_tokens, per_block, head_decay)
-    if (dtype == DL_F32) {
+    if (vec) {
+        const int channel_tiles = (C + DP_VEC_TILE - 1) / DP_VEC_TILE, decay_tiles = (H * dim + DP_VEC_TILE - 1) / DP_VEC_TILE;
+        e = dl_launch_dependent(delta_prepare_vec_kernel, dim3((n_tokens + DP_VEC_TOKENS - 1) / DP_VEC_TOKENS, channel_tiles + decay_tiles), dim3(DP_THREADS), 0, s,
+                                (const __nv_bfloat16*)x, ld, (const __nv_bfloat16*)taps, K, (const float*)hist, slot_stride, n_slots, token_seq, cu_new, slots,
+                                (const __nv_bfloat16*)b_logit, b_stride, z, z_stride, dt_bias, a_log, qo, ko, vo, go, bo, H, G, dim, vdim, q_scale, unit_eps,
+                                n_tokens, head_decay, channel_tiles);
+    } else if (dtype == DL_F32) {
         if (K <= 4) { DP_LAUNCH(float, 4); } else if (K <= 8) { DP_LAUNCH(float, 8); } else if (K <= 16) { DP_LAUNCH(float, 16); } else { DP_LAUNCH(float, DP_MAX_TAPS); }
     } else {
         if (K <= 4) { DP_LAUNCH(__nv_bfloat16, 4); } else if (K <= 8) { DP_LAUNCH(__nv_bfloat16, 8); } else if (K <= 16) { DP_LAUNCH(__nv_bfloat16, 16); }

@@ -237,6 +237,54 @@ head_norm_gate_kernel(const float* __restrict__ o, int o_stride, const T* __rest
     }
 }
 
+// The same with four neighbouring channels a lane (heads of up to 128 channels, a multiple of four, aligned rows) and HNG_ITEMS (token, head)
+// pairs a warp, whose rows are asked for together: at 3,743 tokens of 32 heads of 128 the kernel above takes 59 us, this one 45 (the bytes:
+// 19).  A decode step's few rows get one pair a warp: as many warps as there are pairs.
+#define HNG_ITEMS 4
+__device__ __forceinline__ float4 hng_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 hng_load4(const __nv_bfloat16* p) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), b = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+    return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
+}
+__device__ __forceinline__ void hng_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void hng_store4(__nv_bfloat16* p, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+template <typename T, int ITEMS>
+__global__ void __launch_bounds__(128)
+head_norm_gate_vec_kernel(const float* __restrict__ o, int o_stride, const T* __restrict__ g, int g_stride, const float* __restrict__ gain,
+                          T* __restrict__ out, int out_stride, int rows, int H, int vdim, float eps, int gate_kind) {
+    dl_launch_dependents();
+    dl_grid_dependency_wait();
+    const int lane = threadIdx.x & 31, j = 4 * lane;
+    const long first = ((long)blockIdx.x * 4 + (threadIdx.x >> 5)) * ITEMS, n = (long)rows * H;
+    const bool live = j < vdim;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), w = live ? hng_load4(gain + j) : zero;
+    float4 v[ITEMS], gt[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const long idx = min(first + i, n - 1), t = idx / H, h = idx % H;
+        v[i] = live ? hng_load4(o + t * o_stride + h * vdim + j) : zero;
+        gt[i] = live ? hng_load4(g + t * g_stride + h * vdim + j) : zero;
+    }
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const float ss = dl_warp_sum((v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w));
+        if (first + i >= n) break;
+        const float scale = 1.0f / sqrtf(ss / (float)vdim + eps);
+        const long idx = first + i, t = idx / H, h = idx % H;
+        auto one = [&](float value, float gate, float gain_j) {
+            const float sig = 1.0f / (1.0f + expf(-gate));
+            return value * scale * gain_j * (gate_kind == 1 ? sig : gate * sig);
+        };
+        if (live)
+            hng_store4(out + t * out_stride + h * vdim + j,
+                       make_float4(one(v[i].x, gt[i].x, w.x), one(v[i].y, gt[i].y, w.y), one(v[i].z, gt[i].z, w.z), one(v[i].w, gt[i].w, w.w)));
+    }
+}
+
 // The same for heads wider than a warp walks well (a norm over all heads' outputs at once is one head as wide as all): a
 // block per (token, head), the row's values waiting in registers across the reduction.
 #define HNG_WIDE_THREADS 256
@@ -292,6 +340,20 @@ extern "C" int dl_head_norm_gate(const float* o, int o_stride, const void* g, in
         else
             e = dl_launch_dependent(head_norm_gate_wide_kernel<__nv_bfloat16>, wide, threads, 0, s, o, o_stride, (const __nv_bfloat16*)g,
                                     g_stride, gain, (__nv_bfloat16*)out, out_stride, H, vdim, eps, gate_kind);
+        if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "head_norm_gate: %s", cudaGetErrorString(e));
+        return DL_OK;
+    }
+    const size_t size = dtype == DL_F32 ? 4 : 2;
+    if (vdim <= 128 && vdim % 4 == 0 && o_stride % 4 == 0 && g_stride % 4 == 0 && out_stride % 4 == 0 && ((uintptr_t)o % 16) == 0 &&
+        ((uintptr_t)gain % 16) == 0 && ((uintptr_t)g % (4 * size)) == 0 && ((uintptr_t)out % (4 * size)) == 0 && (dtype == DL_F32 || dtype == DL_BF16)) {
+        const bool many = warps >= 4L * HNG_ITEMS * 4 * dl_sm_count();        // every multiprocessor still gets its blocks
+        const dim3 vgrid((unsigned)((warps + (many ? 4 * HNG_ITEMS : 4) - 1) / (many ? 4 * HNG_ITEMS : 4)));
+#define HNG_VEC(T, N)                                                                                                                   \
+    e = dl_launch_dependent(head_norm_gate_vec_kernel<T, N>, vgrid, block, 0, s, o, o_stride, (const T*)g, g_stride, gain, (T*)out, out_stride, rows, H, \
+                            vdim, eps, gate_kind)
+        if (dtype == DL_F32) { if (many) HNG_VEC(float, HNG_ITEMS); else HNG_VEC(float, 1); }
+        else { if (many) HNG_VEC(__nv_bfloat16, HNG_ITEMS); else HNG_VEC(__nv_bfloat16, 1); }
+#undef HNG_VEC
         if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "head_norm_gate: %s", cudaGetErrorString(e));
         return DL_OK;
     }
