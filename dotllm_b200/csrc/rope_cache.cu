@@ -186,53 +186,124 @@ rope_cache_write_tile_kernel(T* __restrict__ q, int q_stride, const T* __restric
     }
 }
 
-// The tile kernel for bfloat16 rows that can be moved 16 bytes at a time (hd a multiple of 8, the rotated part a multiple
-// of 16 channels, 16-byte aligned rows, values as wide as keys): a thread moves eight rotation pairs of Q or K, or eight
-// channels beyond the rotation, or eight values of V, instead of one element.  Biases (float32, NULL for none) are added
+// The tile kernel for rows that can be moved 16 bytes at a time: E = 8 bfloat16 or 4 float32 elements (hd a multiple of E, the
+// rotated part a multiple of 2 E channels, 16-byte aligned rows, values as wide as keys).  A thread moves E rotation pairs of Q
+// or K, or E channels beyond the rotation, or E values of V, instead of one element.  Biases (float32, NULL for none) are added
 // before the rotation.
-__device__ __forceinline__ void rope_add8(uint4& x, const float* b) {
-    __nv_bfloat16* a = reinterpret_cast<__nv_bfloat16*>(&x);
+//
+// The work is a read and a write of every row.  What bounds it is how many loads are in flight: a multiprocessor's blocks of
+// float32 prompts are few, with a handful of units a thread, so a thread loads BATCH units (rows, cosines and sines) before it
+// rotates and stores the first; stores to Q in place would otherwise hold the next unit's loads back.  bfloat16 rows are half as
+// long and come with more tokens (blocks), and a second unit's registers cost more blocks than its loads bring.  Measured: float32,
+// 1,000 tokens of 32 + 8 heads of 128, 59 us one element a thread, 14 us here; bfloat16, 11,922 tokens of 32 + 8 heads of 64,
+// 33 us with a batch of one (4.5 TB/s of rows read and written), 54 us with two.
+template <typename T>
+struct RopeUnit {
+    static constexpr int E = 16 / (int)sizeof(T);
+    static constexpr int BATCH = sizeof(T) == 4 ? 4 : 1;
+    alignas(16) T x[E];
+};
+template <typename T>
+__device__ __forceinline__ RopeUnit<T> rope_load(const T* p) {
+    RopeUnit<T> u;
+    *reinterpret_cast<uint4*>(u.x) = *reinterpret_cast<const uint4*>(p);
+    return u;
+}
+template <typename T>
+__device__ __forceinline__ void rope_store(T* p, const RopeUnit<T>& u) { *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(u.x); }
+
+template <typename T>
+__device__ __forceinline__ void rope_add(RopeUnit<T>& u, const float* b) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) a[e] = __float2bfloat16_rn(__bfloat162float(a[e]) + b[e]);
+    for (int e = 0; e < RopeUnit<T>::E; ++e) u.x[e] = dl_from_f32<T>(dl_to_f32<T>(u.x[e]) + b[e]);
 }
 
-__device__ __forceinline__ void rope_rotate8(uint4& x0, uint4& x1, const float* cs, const float* sn, const float* b0, const float* b1) {
-    const float4 c0 = *reinterpret_cast<const float4*>(cs), c1 = *reinterpret_cast<const float4*>(cs + 4);
-    const float4 s0 = *reinterpret_cast<const float4*>(sn), s1 = *reinterpret_cast<const float4*>(sn + 4);
-    const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-    const float s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-    __nv_bfloat16* a = reinterpret_cast<__nv_bfloat16*>(&x0);
-    __nv_bfloat16* b = reinterpret_cast<__nv_bfloat16*>(&x1);
+template <typename T>
+__device__ __forceinline__ void rope_rotate(RopeUnit<T>& u0, RopeUnit<T>& u1, const float4* c4, const float4* s4, const float* b0, const float* b1) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        float f0 = __bfloat162float(a[e]), f1 = __bfloat162float(b[e]);
+    for (int e = 0; e < RopeUnit<T>::E; ++e) {
+        const float4 cv = c4[e / 4], sv = s4[e / 4];
+        const float c = e % 4 == 0 ? cv.x : e % 4 == 1 ? cv.y : e % 4 == 2 ? cv.z : cv.w;
+        const float s = e % 4 == 0 ? sv.x : e % 4 == 1 ? sv.y : e % 4 == 2 ? sv.z : sv.w;
+        float f0 = dl_to_f32<T>(u0.x[e]), f1 = dl_to_f32<T>(u1.x[e]);
         if (b0 != nullptr) f0 += b0[e], f1 += b1[e];
-        a[e] = __float2bfloat16_rn(rope_lo(f0, f1, c[e], s[e]));
-        b[e] = __float2bfloat16_rn(rope_hi(f0, f1, c[e], s[e]));
+        u0.x[e] = dl_from_f32<T>(rope_lo(f0, f1, c, s));
+        u1.x[e] = dl_from_f32<T>(rope_hi(f0, f1, c, s));
     }
 }
 
+// The units of one head's rows in a tile, from `src` to where `dst_of(row)` says (NULL: the row is left out).  `rest` units a row
+// beyond the rotation are moved too.
+template <typename T, typename Dst>
+__device__ __forceinline__ void rope_units(const T* src, int stride, int nt, int pairs, int rest, int half, const int* s_pos, const float* cos_t,
+                                           const float* sin_t, const float* bias, Dst dst_of) {
+    constexpr int E = RopeUnit<T>::E, BATCH = RopeUnit<T>::BATCH;
+    const int per = pairs + rest, n = nt * per;
+    for (int base = threadIdx.x; base < n; base += BATCH * RT_THREADS) {
+        RopeUnit<T> x0[BATCH], x1[BATCH];
+        float4 c[BATCH][E / 4], s[BATCH][E / 4];
+        T* dst[BATCH];
+        int at[BATCH];
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+            const int idx = base + u * RT_THREADS;
+            const int i = min(idx, n - 1) / per, g = min(idx, n - 1) - i * per;
+            dst[u] = idx < n ? dst_of(i) : nullptr;
+            if (dst[u] == nullptr) continue;
+            const T* row = src + (size_t)i * stride;
+            if (g < pairs) {
+                at[u] = g * E;
+                const size_t angle = (size_t)s_pos[i] * half + g * E;
+                x0[u] = rope_load(row + at[u]);
+                x1[u] = rope_load(row + half + at[u]);
+#pragma unroll
+                for (int e = 0; e < E / 4; ++e) {
+                    c[u][e] = *reinterpret_cast<const float4*>(cos_t + angle + 4 * e);
+                    s[u][e] = *reinterpret_cast<const float4*>(sin_t + angle + 4 * e);
+                }
+            } else {
+                at[u] = 2 * half + (g - pairs) * E;
+                x0[u] = rope_load(row + at[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+            if (dst[u] == nullptr) continue;
+            if (at[u] < half) {
+                rope_rotate(x0[u], x1[u], c[u], s[u], bias ? bias + at[u] : nullptr, bias ? bias + half + at[u] : nullptr);
+                rope_store(dst[u] + at[u], x0[u]);
+                rope_store(dst[u] + half + at[u], x1[u]);
+            } else {
+                if (bias != nullptr) rope_add(x0[u], bias + at[u]);
+                rope_store(dst[u] + at[u], x0[u]);
+            }
+        }
+    }
+}
+
+template <typename T>
 __global__ void __launch_bounds__(RT_THREADS)
-rope_cache_write_tile_vec_kernel(__nv_bfloat16* __restrict__ q, int q_stride, const __nv_bfloat16* __restrict__ k, int k_stride,
-                                 const __nv_bfloat16* __restrict__ v, int v_stride, const float* __restrict__ cos_t,
+rope_cache_write_tile_vec_kernel(T* __restrict__ q, int q_stride, const T* __restrict__ k, int k_stride,
+                                 const T* __restrict__ v, int v_stride, const float* __restrict__ cos_t,
                                  const float* __restrict__ sin_t, int rotary_dim, int table_rows, const int32_t* __restrict__ token_seq,
                                  const int32_t* __restrict__ token_pos, const int32_t* __restrict__ block_table, int bt_stride,
-                                 __nv_bfloat16* __restrict__ k_pool, __nv_bfloat16* __restrict__ v_pool, int n_pages,
+                                 T* __restrict__ k_pool, T* __restrict__ v_pool, int n_pages,
                                  int n_tokens, int nh, int nkv, int hd, const float* __restrict__ q_bias,
                                  const float* __restrict__ k_bias, const float* __restrict__ v_bias, int write_cache) {
+    constexpr int E = RopeUnit<T>::E;
     extern __shared__ __align__(16) unsigned char rt_raw[];
-    __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(rt_raw);      // [64 tokens][hd + 2]: V rows of one KV head
+    T* tile = reinterpret_cast<T*>(rt_raw);                  // [64 tokens][hd + a 32-bit word]: V rows of one KV head
     __shared__ int s_pos[RT_TOKENS], s_page[RT_TOKENS];
     dl_launch_dependents();
     dl_grid_dependency_wait();
     const int t0 = blockIdx.x * RT_TOKENS;
     const int nt = min(RT_TOKENS, n_tokens - t0);
     const int half = rotary_dim / 2;
-    const int pairs = half / 8, rest = (hd - rotary_dim) / 8;   // groups of eight rotation pairs, and of eight channels beyond them, per head
+    const int pairs = half / E, rest = (hd - rotary_dim) / E;   // groups of E rotation pairs, and of E channels beyond them, per head
     // KV heads first: their blocks do more (K to its page, V through the transposing tile) and should not start last
     const int kv_first = write_cache ? nkv : 0;
     const bool is_q = (int)blockIdx.y >= kv_first;
-    const int pitch = hd + 2;
+    const int pitch = hd + 4 / (int)sizeof(T);
     if (threadIdx.x < RT_TOKENS) {
         int pos = -1, page = -1;
         if ((int)threadIdx.x < nt) {
@@ -249,62 +320,31 @@ rope_cache_write_tile_vec_kernel(__nv_bfloat16* __restrict__ q, int q_stride, co
     __syncthreads();
     if (is_q) {                                              // a query head: rotate in place
         const int qh = (int)blockIdx.y - kv_first;
-        const float* qb = q_bias != nullptr ? q_bias + (size_t)qh * hd : nullptr;
-        const int per = pairs + (qb != nullptr ? rest : 0);  // without a bias the channels beyond the rotation stay as they are
-        for (int idx = threadIdx.x; idx < nt * per; idx += RT_THREADS) {
-            const int i = idx / per, g = idx - i * per;
-            const int pos = s_pos[i];
-            if (pos < 0) continue;
-            __nv_bfloat16* row = q + (size_t)(t0 + i) * q_stride + (size_t)qh * hd;
-            if (g < pairs) {
-                const int u = g * 8;
-                uint4 x0 = *reinterpret_cast<const uint4*>(row + u), x1 = *reinterpret_cast<const uint4*>(row + half + u);
-                rope_rotate8(x0, x1, cos_t + (size_t)pos * half + u, sin_t + (size_t)pos * half + u, qb ? qb + u : nullptr,
-                             qb ? qb + half + u : nullptr);
-                *reinterpret_cast<uint4*>(row + u) = x0;
-                *reinterpret_cast<uint4*>(row + half + u) = x1;
-            } else {
-                const int d = rotary_dim + (g - pairs) * 8;
-                uint4 x = *reinterpret_cast<const uint4*>(row + d);
-                rope_add8(x, qb + d);
-                *reinterpret_cast<uint4*>(row + d) = x;
-            }
-        }
+        T* rows = q + (size_t)t0 * q_stride + (size_t)qh * hd;
+        // without a bias the channels beyond the rotation stay as they are
+        rope_units<T>(rows, q_stride, nt, pairs, q_bias != nullptr ? rest : 0, half, s_pos, cos_t, sin_t,
+                      q_bias != nullptr ? q_bias + (size_t)qh * hd : nullptr,
+                      [&](int i) { return s_pos[i] < 0 ? nullptr : rows + (size_t)i * q_stride; });
         return;
     }
     if (!write_cache) return;
     const int h = blockIdx.y;                                // a KV head: rotate K on its way to the page, stage V
-    const float* kb = k_bias != nullptr ? k_bias + (size_t)h * hd : nullptr;
     const float* vb = v_bias != nullptr ? v_bias + (size_t)h * hd : nullptr;
-    const int per = pairs + rest, units = hd / 8;
+    const int units = hd / E;
+#pragma unroll 4
     for (int idx = threadIdx.x; idx < nt * units; idx += RT_THREADS) {
-        const int i = idx / units, d = (idx - i * units) * 8;
-        uint4 x = *reinterpret_cast<const uint4*>(v + (size_t)(t0 + i) * v_stride + (size_t)h * hd + d);
-        if (vb != nullptr) rope_add8(x, vb + d);
-        uint32_t* dst = reinterpret_cast<uint32_t*>(tile + i * pitch + d);          // 4-byte aligned: pitch and d are even
-        dst[0] = x.x; dst[1] = x.y; dst[2] = x.z; dst[3] = x.w;
+        const int i = idx / units, d = (idx - i * units) * E;
+        RopeUnit<T> x = rope_load(v + (size_t)(t0 + i) * v_stride + (size_t)h * hd + d);
+        if (vb != nullptr) rope_add(x, vb + d);
+        uint32_t* dst = reinterpret_cast<uint32_t*>(tile + i * pitch + d);          // 4-byte aligned: so are the pitch and d
+        const uint32_t* words = reinterpret_cast<const uint32_t*>(x.x);
+        dst[0] = words[0]; dst[1] = words[1]; dst[2] = words[2]; dst[3] = words[3];
     }
-    for (int idx = threadIdx.x; idx < nt * per; idx += RT_THREADS) {
-        const int i = idx / per, g = idx - i * per;
-        const int page = s_page[i], pos = s_pos[i];
-        if (page < 0) continue;
-        const __nv_bfloat16* krow = k + (size_t)(t0 + i) * k_stride + (size_t)h * hd;
-        __nv_bfloat16* kdst = k_pool + dl_k_offset(page, nkv, h, pos % DL_PAGE, hd);
-        if (g < pairs) {
-            const int u = g * 8;
-            uint4 x0 = *reinterpret_cast<const uint4*>(krow + u), x1 = *reinterpret_cast<const uint4*>(krow + half + u);
-            rope_rotate8(x0, x1, cos_t + (size_t)pos * half + u, sin_t + (size_t)pos * half + u, kb ? kb + u : nullptr,
-                         kb ? kb + half + u : nullptr);
-            *reinterpret_cast<uint4*>(kdst + u) = x0;
-            *reinterpret_cast<uint4*>(kdst + half + u) = x1;
-        } else {
-            const int d = rotary_dim + (g - pairs) * 8;
-            uint4 x = *reinterpret_cast<const uint4*>(krow + d);
-            if (kb != nullptr) rope_add8(x, kb + d);
-            *reinterpret_cast<uint4*>(kdst + d) = x;
-        }
-    }
+    rope_units<T>(k + (size_t)t0 * k_stride + (size_t)h * hd, k_stride, nt, pairs, rest, half, s_pos, cos_t, sin_t,
+                  k_bias != nullptr ? k_bias + (size_t)h * hd : nullptr,
+                  [&](int i) { return s_page[i] < 0 ? nullptr : k_pool + dl_k_offset(s_page[i], nkv, h, s_pos[i] % DL_PAGE, hd); });
     __syncthreads();
+#pragma unroll 4
     for (int idx = threadIdx.x; idx < RT_TOKENS * hd; idx += RT_THREADS) {    // token fastest
         const int i = idx % RT_TOKENS, d = idx / RT_TOKENS;
         if (i >= nt) continue;
@@ -340,15 +380,23 @@ extern "C" int dl_rope_cache_write(void* q, int q_stride, const void* k, int k_s
         const int q_blocks = (rotary_dim > 0 || q_bias != nullptr) ? nh : 0;
         if (q_blocks == 0 && !write_cache) return DL_OK;
         dim3 tgrid((n_tokens + RT_TOKENS - 1) / RT_TOKENS, (write_cache ? nkv : 0) + q_blocks);
-        const bool aligned = ((uintptr_t)q % 16) == 0 && q_stride % 8 == 0 && ((uintptr_t)cos_t % 16) == 0 &&
+        const int unit = 16 / (int)elem;                     // elements of 16 bytes
+        const bool aligned = ((uintptr_t)q % 16) == 0 && q_stride % unit == 0 && ((uintptr_t)cos_t % 16) == 0 &&
                              ((uintptr_t)sin_t % 16) == 0 &&
-                             (!write_cache || (((uintptr_t)k % 16) == 0 && ((uintptr_t)v % 16) == 0 && k_stride % 8 == 0 &&
-                                               v_stride % 8 == 0 && ((uintptr_t)k_pool % 16) == 0));
-        if (dtype == DL_BF16 && vd == hd && hd % 8 == 0 && rotary_dim % 16 == 0 && aligned && biases_aligned) {
-            e = dl_launch_dependent(rope_cache_write_tile_vec_kernel, tgrid, dim3(RT_THREADS), tile_smem, s, (__nv_bfloat16*)q,
-                                    q_stride, (const __nv_bfloat16*)k, k_stride, (const __nv_bfloat16*)v, v_stride, cos_t, sin_t,
-                                    rotary_dim, table_rows, token_seq, token_pos, block_table, bt_stride, (__nv_bfloat16*)k_pool,
-                                    (__nv_bfloat16*)v_pool, n_pages, n_tokens, nh, nkv, hd, q_bias, k_bias, v_bias, write_cache);
+                             (!write_cache || (((uintptr_t)k % 16) == 0 && ((uintptr_t)v % 16) == 0 && k_stride % unit == 0 &&
+                                               v_stride % unit == 0 && ((uintptr_t)k_pool % 16) == 0));
+        if (vd == hd && hd % unit == 0 && rotary_dim % (2 * unit) == 0 && aligned && biases_aligned) {
+            if (dtype == DL_F32)
+                e = dl_launch_dependent(rope_cache_write_tile_vec_kernel<float>, tgrid, dim3(RT_THREADS), tile_smem, s, (float*)q,
+                                        q_stride, (const float*)k, k_stride, (const float*)v, v_stride, cos_t, sin_t, rotary_dim,
+                                        table_rows, token_seq, token_pos, block_table, bt_stride, (float*)k_pool, (float*)v_pool,
+                                        n_pages, n_tokens, nh, nkv, hd, q_bias, k_bias, v_bias, write_cache);
+            else
+                e = dl_launch_dependent(rope_cache_write_tile_vec_kernel<__nv_bfloat16>, tgrid, dim3(RT_THREADS), tile_smem, s,
+                                        (__nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)k, k_stride, (const __nv_bfloat16*)v,
+                                        v_stride, cos_t, sin_t, rotary_dim, table_rows, token_seq, token_pos, block_table, bt_stride,
+                                        (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, n_pages, n_tokens, nh, nkv, hd, q_bias,
+                                        k_bias, v_bias, write_cache);
             if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "rope_cache_write: %s", cudaGetErrorString(e));
             return DL_OK;
         }
