@@ -26,8 +26,19 @@
 //                divided by the row's sum at the end.
 // The tensor core takes about as long for an MMA of 64 or 128 columns as for one of 256 (measured),
 // so the kernel is bound by the number of MMAs: two tiles keep that pipe fed while each tile's
-// softmax threads work through their page.  Tensor memory: 4 x 64 columns of scores, 2 x 128 of
-// outputs - all 512, which one block per SM (its shared memory) makes safe.
+// softmax threads work through their page.  Tensor memory: for heads of 128, 4 x 64 columns of scores
+// and 2 x 128 of outputs - all 512, which one block per SM (its shared memory) makes safe.
+// Heads of 64 have half the MMAs a page (16 of about 86 cycles for the two tiles) under the same chain of a
+// softmax thread (about 2,000 cycles a page), so two tiles leave the tensor core idle a third of the time.  There a
+// block keeps one buffer for a tile's scores and one for its weights instead of two, and two blocks share
+// a multiprocessor: 256 columns each, half of the shared memory each to the byte, 16 softmax warps instead of 8.
+// Registers decide whether that pays: with 80 a thread (what two blocks leave) the row's 64 scores spill and a prompt of 8,192
+// tokens takes 0.83 ms; with 40 for the issuing warps and 96 for the softmax threads nothing spills.  The mask
+// compares with constants and has no branches: element by element with short-circuit conditions, a tile with fewer than
+// 128 rows, which took it on every page, ran three times as long as its neighbours and with it the whole of a short prompt.
+// 32 query over 8 KV heads, before -> now: heads of 64, 1,987 tokens 0.079 -> 0.058 ms, six of them in one call
+// 0.230 -> 0.140, 8,192 tokens 0.558 -> 0.422; heads of 128 (the mask alone) 700 tokens 0.037 -> 0.027, 1,987 tokens
+// 0.086 -> 0.060, 8,192 tokens 0.607 -> 0.598 ms.
 // Keys that no query of the tile may see are never used: masked scores are replaced, not
 // multiplied, and the slots of the last page beyond the sequence's length (which may hold
 // anything) are zeroed in the V stage before the product.
@@ -42,9 +53,11 @@
 
 #define PT_ROWS 128                          // query rows of a tile
 #define PT_TILES 2                           // tiles of a block: it covers PT_TILES * PT_ROWS consecutive rows
-#define PT_STAGES(hd) ((hd) > 64 ? 3 : 4)    // K/V pages in flight: what 227 KB of shared memory leave room for
+#define PT_STAGES 3                          // K/V pages in flight: what shared memory leaves room for
 #define PT_THREADS 384
-#define PT_TMEM_COLS 512
+#define PT_BLOCKS(hd) ((hd) > 64 ? 1 : 2)    // blocks of a multiprocessor
+#define PT_BUFS(hd) ((hd) > 64 ? 2 : 1)      // buffers a tile has for its scores, and for its weights
+#define PT_TMEM_COLS(hd) (PT_TILES * (PT_BUFS(hd) * DL_PAGE + (hd)))    // 512 for heads of 128, 256 for heads of 64
 #define PT_RESCALE_STEP 8.0f                 // log2 units a row's maximum may grow before O is rescaled
 
 __device__ __forceinline__ float pt_ex2(float x) {             // 2^x, 2 ulp; ex2(-inf) = 0
@@ -90,17 +103,18 @@ struct PtTile {
 enum { PT_PLAIN = 0, PT_CAP = 1, PT_SLOPE = 2 };
 
 template <int HD, int SHAPE>
-__global__ void __launch_bounds__(PT_THREADS, 1)
+__global__ void __launch_bounds__(PT_THREADS, PT_BLOCKS(HD))
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                             const __grid_constant__ CUtensorMap tmap_v, __nv_bfloat16* __restrict__ out, int out_stride,
                             int n_pages, const int32_t* __restrict__ tile_seq, const int32_t* __restrict__ tile_row0,
                             const int32_t* __restrict__ seq_start, const int32_t* __restrict__ seq_new,
                             const int32_t* __restrict__ cu_new, const int32_t* __restrict__ block_table, int bt_stride,
                             int nkv, int group, float scale, int window, int keep_first, const float* __restrict__ sinks, const DlScoreCap cap,
-                            const float* __restrict__ slopes, const __nv_bfloat16* __restrict__ gate, int gate_stride, int* __restrict__ status) {
+                            const float* __restrict__ slopes, const __nv_bfloat16* __restrict__ gate, int gate_stride, int smem_bytes,
+                            int* __restrict__ status) {
     constexpr bool CAP = SHAPE == PT_CAP;
     constexpr int ATOMS = HD / 64;                           // 64-dim (128-byte) slices of a head
-    constexpr int STAGES = PT_STAGES(HD);
+    constexpr int STAGES = PT_STAGES, BUFS = PT_BUFS(HD);
     constexpr uint32_t Q_BYTES = PT_ROWS * HD * 2;
     constexpr uint32_t K_BYTES = DL_PAGE * HD * 2, V_BYTES = HD * DL_PAGE * 2;
     constexpr uint32_t STAGE_BYTES = K_BYTES + V_BYTES;
@@ -109,9 +123,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
     unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)pt_smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* q_smem = base;                            // [tile][atom][128 rows][64 dims]
     unsigned char* kv_smem = q_smem + PT_TILES * Q_BYTES;    // [stage][K: [atom][64 keys][64 dims] | V: [hd][64 keys]]
-    unsigned char* p_smem = kv_smem + STAGES * STAGE_BYTES;  // [tile][2][128 rows][64 keys]
+    unsigned char* p_smem = kv_smem + STAGES * STAGE_BYTES;  // [tile][buffer][128 rows][64 keys]
+    // the host leaves out what the barriers below take of the alignment's slack: never write past what it asked for
+    if (p_smem + PT_TILES * BUFS * P_BYTES > pt_smem_raw + smem_bytes) {
+        if (threadIdx.x == 0) atomicExch(status, 38);
+        return;
+    }
     __shared__ uint64_t q_full[PT_TILES], kv_full[STAGES], kv_empty[STAGES];
-    __shared__ uint64_t s_full[PT_TILES][2], s_empty[PT_TILES][2], p_ready[PT_TILES][2], pv_done[PT_TILES][2];
+    __shared__ uint64_t s_full[PT_TILES][BUFS], s_empty[PT_TILES][BUFS], p_ready[PT_TILES][BUFS], pv_done[PT_TILES][BUFS];
     __shared__ uint32_t tmem_base_holder;
     __shared__ volatile int gave_up;
 
@@ -159,7 +178,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
         }
         for (int t = 0; t < PT_TILES; ++t) {
             tc_mbar_init(&q_full[t], 1);
-            for (int i = 0; i < 2; ++i) {
+            for (int i = 0; i < BUFS; ++i) {
                 tc_mbar_init(&s_full[t][i], 1);
                 tc_mbar_init(&s_empty[t][i], 4);              // one arrival per softmax warp of the tile
                 tc_mbar_init(&p_ready[t][i], 4);
@@ -168,139 +187,145 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) tc_tmem_alloc(&tmem_base_holder, PT_TMEM_COLS);
+    if (warp == 1) tc_tmem_alloc(&tmem_base_holder, PT_TMEM_COLS(HD));
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_holder;
-    // scores: tile t, buffer i at column (2 t + i) * 64; outputs: tile t at column 256 + 128 t
-    const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 2 * PT_TILES * DL_PAGE;
+    // scores: tile t, buffer i at column (BUFS t + i) * 64; the tiles' outputs, HD columns each, after them
+    const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + BUFS * PT_TILES * DL_PAGE;
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ copies
-        bool stop = false;
-        int issued = 0;
-        if (lane == 0) {
-#pragma unroll
-            for (int t = 0; t < PT_TILES; ++t) {
-                if (tiles[t].rows <= 0) continue;
-                tc_mbar_expect(&q_full[t], Q_BYTES);
-#pragma unroll
-                for (int a = 0; a < ATOMS; ++a)
-                    dl_tma_load_2d(q_smem + t * Q_BYTES + a * (PT_ROWS * 128), &tmap_q, head * HD + a * 64,
-                                   cu_new[b] + row0 + t * PT_ROWS, &q_full[t]);
-            }
-        }
-        const int32_t* pages = block_table + (size_t)b * bt_stride;
-        for (int j0 = 0; j0 < n_kv && !stop; j0 += 32) {
-            const int mine = (j0 + lane < n_kv) ? pages[page_of(j0 + lane)] : 0;
-            const int count = min(32, n_kv - j0);
-            for (int jj = 0; jj < count; ++jj) {
-                const int page = __shfl_sync(0xffffffffu, mine, jj);
-                const int j = j0 + jj, s = j % STAGES;
-                int bad = 0;
-                if (lane == 0) {
-                    if (page < 0 || page >= n_pages) {
-                        bad = 2;
-                    } else if (j >= STAGES && !tc_mbar_wait(&kv_empty[s], ((j / STAGES) - 1) & 1, &gave_up)) {
-                        bad = 31;
-                    } else {
-                        unsigned char* k_dst = kv_smem + (size_t)s * STAGE_BYTES;
-                        tc_mbar_expect(&kv_full[s], STAGE_BYTES);
-#pragma unroll
-                        for (int a = 0; a < ATOMS; ++a)
-                            dl_tma_load_2d(k_dst + a * (DL_PAGE * 128), &tmap_k, a * 64, (page * nkv + kvh) * DL_PAGE, &kv_full[s]);
-                        dl_tma_load_2d(k_dst + K_BYTES, &tmap_v, 0, (page * nkv + kvh) * HD, &kv_full[s]);
-                        issued = j + 1;
-                    }
-                }
-                bad = __shfl_sync(0xffffffffu, bad, 0);
-                if (bad) {
-                    if (lane == 0) {
-                        if (!gave_up) atomicExch(status, bad);
-                        gave_up = 1;
-                    }
-                    stop = true;
-                    break;
-                }
-            }
-        }
-        if (stop && lane == 0) {
-            // copies already issued must land before the block's shared memory is released
-            for (int t = 0; t < PT_TILES; ++t) {
-                if (tiles[t].rows <= 0) continue;
-                const long long t0 = clock64();
-                while (!tc_mbar_try(&q_full[t], 0) && clock64() - t0 < TC_WAIT_CYCLES) {}
-            }
-            for (int i = max(0, issued - STAGES); i < issued; ++i) {
-                const long long t0 = clock64();
-                while (!tc_mbar_try(&kv_full[i % STAGES], (i / STAGES) & 1) && clock64() - t0 < TC_WAIT_CYCLES) {}
-            }
-        }
-    } else if (warp == 1 || warp == 2) {
-        // ------------------------------------------------------------ tensor-core issue: the scores of tile `t`
-        const int t = warp - 1;
-        const PtTile T = tiles[t];
-        if (lane == 0 && T.rows > 0) {
-            const uint32_t idesc_qk = tc_idesc_bf16(PT_ROWS, DL_PAGE);
-            const uint32_t q_addr = tc_smem(q_smem + t * Q_BYTES);
-            bool ok = tc_mbar_wait(&q_full[t], 0, &gave_up);
-            if (!ok && !gave_up) atomicExch(status, 32);
-            for (int j = T.j_lo; j <= T.j_hi && ok; ++j) {
-                const int c = j - T.j_lo, s = j % STAGES, sb = c & 1;
-                if (t == 0) PT_STAMP(0, j);                     // issuing thread: top of page j
-                ok = tc_mbar_wait(&kv_full[s], (j / STAGES) & 1, &gave_up) &&
-                     (c < 2 || tc_mbar_wait(&s_empty[t][sb], ((c >> 1) - 1) & 1, &gave_up));
-                if (!ok) {
-                    if (!gave_up) atomicExch(status, 33);
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t k_addr = tc_smem(kv_smem + (size_t)s * STAGE_BYTES);
-#pragma unroll
-                for (int k = 0; k < HD / 16; ++k) {
-                    const int a = k / 4, kk = k % 4;            // 64-dim slice, 16-dim step inside it (32 bytes)
-                    tc_mma(tmem_s + (uint32_t)((2 * t + sb) * DL_PAGE), tc_operand_desc(q_addr + a * (PT_ROWS * 128)) + (uint64_t)(kk * 2),
-                           tc_operand_desc(k_addr + a * (DL_PAGE * 128)) + (uint64_t)(kk * 2), idesc_qk, k != 0 ? 1u : 0u);
-                }
-                tc_commit(&s_full[t][sb]);
-                if (t == 0) PT_STAMP(1, j);                     // scores of page j issued and committed
-            }
-            if (!ok) gave_up = 1;
-        }
-    } else if (warp == 3) {
-        // ------------------------------------------------------------ tensor-core issue: the products with V
-        if (lane == 0) {
-            const uint32_t idesc_pv = tc_idesc_bf16(PT_ROWS, HD);
-            bool ok = true;
-            for (int j = 0; j < n_kv && ok; ++j) {
-                const int s = j % STAGES;
-                const uint32_t v_addr = tc_smem(kv_smem + (size_t)s * STAGE_BYTES + K_BYTES);
-#pragma unroll
+    // Two blocks a multiprocessor leave 80 registers a thread, 30,720 a block: the four issuing warps give some up for the
+    // threads that hold a row's scores (40 x 128 + 96 x 256 = 29,696)
+    if (warp < 4) {
+        if (BUFS == 1) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (warp == 0) {
+            // ------------------------------------------------------------ copies
+            bool stop = false;
+            int issued = 0;
+            if (lane == 0) {
+    #pragma unroll
                 for (int t = 0; t < PT_TILES; ++t) {
-                    if (j < tiles[t].j_lo || j > tiles[t].j_hi) continue;
-                    const int c = j - tiles[t].j_lo, pb = c & 1;
-                    if (t == 0) PT_STAMP(2, j);                 // waiting for the weights of page j
-                    ok = tc_mbar_wait(&p_ready[t][pb], (c >> 1) & 1, &gave_up) && tc_mbar_wait(&kv_full[s], (j / STAGES) & 1, &gave_up);
-                    if (t == 0) PT_STAMP(3, j);                 // weights of page j seen
+                    if (tiles[t].rows <= 0) continue;
+                    tc_mbar_expect(&q_full[t], Q_BYTES);
+    #pragma unroll
+                    for (int a = 0; a < ATOMS; ++a)
+                        dl_tma_load_2d(q_smem + t * Q_BYTES + a * (PT_ROWS * 128), &tmap_q, head * HD + a * 64,
+                                       cu_new[b] + row0 + t * PT_ROWS, &q_full[t]);
+                }
+            }
+            const int32_t* pages = block_table + (size_t)b * bt_stride;
+            for (int j0 = 0; j0 < n_kv && !stop; j0 += 32) {
+                const int mine = (j0 + lane < n_kv) ? pages[page_of(j0 + lane)] : 0;
+                const int count = min(32, n_kv - j0);
+                for (int jj = 0; jj < count; ++jj) {
+                    const int page = __shfl_sync(0xffffffffu, mine, jj);
+                    const int j = j0 + jj, s = j % STAGES;
+                    int bad = 0;
+                    if (lane == 0) {
+                        if (page < 0 || page >= n_pages) {
+                            bad = 2;
+                        } else if (j >= STAGES && !tc_mbar_wait(&kv_empty[s], ((j / STAGES) - 1) & 1, &gave_up)) {
+                            bad = 31;
+                        } else {
+                            unsigned char* k_dst = kv_smem + (size_t)s * STAGE_BYTES;
+                            tc_mbar_expect(&kv_full[s], STAGE_BYTES);
+    #pragma unroll
+                            for (int a = 0; a < ATOMS; ++a)
+                                dl_tma_load_2d(k_dst + a * (DL_PAGE * 128), &tmap_k, a * 64, (page * nkv + kvh) * DL_PAGE, &kv_full[s]);
+                            dl_tma_load_2d(k_dst + K_BYTES, &tmap_v, 0, (page * nkv + kvh) * HD, &kv_full[s]);
+                            issued = j + 1;
+                        }
+                    }
+                    bad = __shfl_sync(0xffffffffu, bad, 0);
+                    if (bad) {
+                        if (lane == 0) {
+                            if (!gave_up) atomicExch(status, bad);
+                            gave_up = 1;
+                        }
+                        stop = true;
+                        break;
+                    }
+                }
+            }
+            if (stop && lane == 0) {
+                // copies already issued must land before the block's shared memory is released
+                for (int t = 0; t < PT_TILES; ++t) {
+                    if (tiles[t].rows <= 0) continue;
+                    const long long t0 = clock64();
+                    while (!tc_mbar_try(&q_full[t], 0) && clock64() - t0 < TC_WAIT_CYCLES) {}
+                }
+                for (int i = max(0, issued - STAGES); i < issued; ++i) {
+                    const long long t0 = clock64();
+                    while (!tc_mbar_try(&kv_full[i % STAGES], (i / STAGES) & 1) && clock64() - t0 < TC_WAIT_CYCLES) {}
+                }
+            }
+        } else if (warp == 1 || warp == 2) {
+            // ------------------------------------------------------------ tensor-core issue: the scores of tile `t`
+            const int t = warp - 1;
+            const PtTile T = tiles[t];
+            if (lane == 0 && T.rows > 0) {
+                const uint32_t idesc_qk = tc_idesc_bf16(PT_ROWS, DL_PAGE);
+                const uint32_t q_addr = tc_smem(q_smem + t * Q_BYTES);
+                bool ok = tc_mbar_wait(&q_full[t], 0, &gave_up);
+                if (!ok && !gave_up) atomicExch(status, 32);
+                for (int j = T.j_lo; j <= T.j_hi && ok; ++j) {
+                    const int c = j - T.j_lo, s = j % STAGES, sb = c % BUFS;
+                    if (t == 0) PT_STAMP(0, j);                     // issuing thread: top of page j
+                    ok = tc_mbar_wait(&kv_full[s], (j / STAGES) & 1, &gave_up) &&
+                         (c < BUFS || tc_mbar_wait(&s_empty[t][sb], (c / BUFS - 1) & 1, &gave_up));
                     if (!ok) {
-                        if (!gave_up) atomicExch(status, 34);
+                        if (!gave_up) atomicExch(status, 33);
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t p_addr = tc_smem(p_smem + (2 * t + pb) * P_BYTES);
-#pragma unroll
-                    for (int k = 0; k < DL_PAGE / 16; ++k)
-                        tc_mma(tmem_o + (uint32_t)(t * HD), tc_operand_desc(p_addr) + (uint64_t)(k * 2), tc_operand_desc(v_addr) + (uint64_t)(k * 2),
-                               idesc_pv, (c | k) != 0 ? 1u : 0u);
-                    tc_commit(&pv_done[t][pb]);
-                    if (t == 0) PT_STAMP(4, j);                 // product of page j issued and committed
+                    const uint32_t k_addr = tc_smem(kv_smem + (size_t)s * STAGE_BYTES);
+    #pragma unroll
+                    for (int k = 0; k < HD / 16; ++k) {
+                        const int a = k / 4, kk = k % 4;            // 64-dim slice, 16-dim step inside it (32 bytes)
+                        tc_mma(tmem_s + (uint32_t)((BUFS * t + sb) * DL_PAGE), tc_operand_desc(q_addr + a * (PT_ROWS * 128)) + (uint64_t)(kk * 2),
+                               tc_operand_desc(k_addr + a * (DL_PAGE * 128)) + (uint64_t)(kk * 2), idesc_qk, k != 0 ? 1u : 0u);
+                    }
+                    tc_commit(&s_full[t][sb]);
+                    if (t == 0) PT_STAMP(1, j);                     // scores of page j issued and committed
                 }
-                if (ok) tc_commit(&kv_empty[s]);                // every tile that reads this page has issued its product
+                if (!ok) gave_up = 1;
             }
-            if (!ok) gave_up = 1;
+        } else if (warp == 3) {
+            // ------------------------------------------------------------ tensor-core issue: the products with V
+            if (lane == 0) {
+                const uint32_t idesc_pv = tc_idesc_bf16(PT_ROWS, HD);
+                bool ok = true;
+                for (int j = 0; j < n_kv && ok; ++j) {
+                    const int s = j % STAGES;
+                    const uint32_t v_addr = tc_smem(kv_smem + (size_t)s * STAGE_BYTES + K_BYTES);
+    #pragma unroll
+                    for (int t = 0; t < PT_TILES; ++t) {
+                        if (j < tiles[t].j_lo || j > tiles[t].j_hi) continue;
+                        const int c = j - tiles[t].j_lo, pb = c % BUFS;
+                        if (t == 0) PT_STAMP(2, j);                 // waiting for the weights of page j
+                        ok = tc_mbar_wait(&p_ready[t][pb], (c / BUFS) & 1, &gave_up) && tc_mbar_wait(&kv_full[s], (j / STAGES) & 1, &gave_up);
+                        if (t == 0) PT_STAMP(3, j);                 // weights of page j seen
+                        if (!ok) {
+                            if (!gave_up) atomicExch(status, 34);
+                            break;
+                        }
+                        tc_fence_after();
+                        const uint32_t p_addr = tc_smem(p_smem + (BUFS * t + pb) * P_BYTES);
+    #pragma unroll
+                        for (int k = 0; k < DL_PAGE / 16; ++k)
+                            tc_mma(tmem_o + (uint32_t)(t * HD), tc_operand_desc(p_addr) + (uint64_t)(k * 2), tc_operand_desc(v_addr) + (uint64_t)(k * 2),
+                                   idesc_pv, (c | k) != 0 ? 1u : 0u);
+                        tc_commit(&pv_done[t][pb]);
+                        if (t == 0) PT_STAMP(4, j);                 // product of page j issued and committed
+                    }
+                    if (ok) tc_commit(&kv_empty[s]);                // every tile that reads this page has issued its product
+                }
+                if (!ok) gave_up = 1;
+            }
         }
     } else {
+        if (BUFS == 1) asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
         // ------------------------------------------------------------ softmax: thread -> row of tile `t`
         const int t = (warp - 4) >> 2, quarter = warp & 3;
         const PtTile T = tiles[t];
@@ -309,16 +334,16 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
         const bool live = r < T.rows;
         const bool stamps = (warp == 4 && lane == 0);
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-        const uint32_t my_s = tmem_s + lane_base + (uint32_t)(2 * t * DL_PAGE), my_o = tmem_o + lane_base + (uint32_t)(t * HD);
+        const uint32_t my_s = tmem_s + lane_base + (uint32_t)(BUFS * t * DL_PAGE), my_o = tmem_o + lane_base + (uint32_t)(t * HD);
         const float scale2 = SHAPE != PT_PLAIN ? 1.f : scale * 1.4426950408889634f;    // scores in units of log2 (the others come in them)
         const float to_log2 = scale * 1.4426950408889634f, slope2 = SHAPE == PT_SLOPE ? slopes[head] * 1.4426950408889634f : 0.f;
         float m_ref = -INFINITY, l = 0.f;                    // reference maximum (log2 units), sum of weights
         bool ok = true;
         const int n_mine = T.j_hi - T.j_lo + 1;
         for (int c = 0; c < n_mine; ++c) {
-            const int j = T.j_lo + c, sb = c & 1;
+            const int j = T.j_lo + c, sb = c % BUFS;
             if (stamps) PT_STAMP(5, j);                         // softmax warp: waiting for the scores of page j
-            ok = __all_sync(0xffffffffu, tc_mbar_wait(&s_full[t][sb], (c >> 1) & 1, &gave_up));
+            ok = __all_sync(0xffffffffu, tc_mbar_wait(&s_full[t][sb], (c / BUFS) & 1, &gave_up));
             if (stamps) PT_STAMP(6, j);                         // scores seen
             if (!ok) {
                 if (lane == 0 && !gave_up) atomicExch(status, 35);
@@ -337,7 +362,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) tc_mbar_arrive(&s_empty[t][sb]);     // the score buffer may take the tile's page after next
+            if (lane == 0) tc_mbar_arrive(&s_empty[t][sb]);     // the score buffer may take the next page that uses it
             if (stamps) PT_STAMP(7, j);                         // scores read into registers
 
             if (CAP) {                                          // before the mask: a hidden key's score is replaced, not capped
@@ -350,22 +375,24 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
 #pragma unroll
                 for (int i = 0; i < 64; ++i) sc[i] = fmaf(sc[i], to_log2, fmaf(slope2, (float)i, from));
             }
-            // pages wholly visible to every row of the tile need no mask
-            const bool ragged = T.rows < PT_ROWS || key0 + DL_PAGE - 1 > T.pos0 || key0 < T.first_key ||
-                                (window > 0 && key0 <= T.pos_last - window);
-            if (ragged) {
+            // Pages wholly visible to every row of the tile need no mask.  Rows beyond the tile's last take none: nothing of them
+            // is stored, and they have no say in when the warp's rows rescale.  Comparisons with constants, no branches: a page
+            // in front of the diagonal and one on it then cost about the same.
+            if (key0 + DL_PAGE - 1 > T.pos0) {                  // keys behind the query
+                const int ahead = pos - key0;
 #pragma unroll
-                for (int i = 0; i < 64; ++i) {
-                    const int key = key0 + i;
-                    const bool seen = live && key <= pos && (window == 0 || key > pos - window || key < keep_first);
-                    if (!seen) sc[i] = -INFINITY;
-                }
+                for (int i = 0; i < 64; ++i) sc[i] = i > ahead ? -INFINITY : sc[i];
+            }
+            if (window > 0 && key0 <= T.pos_last - window) {    // keys in front of the window that are not kept
+                const int behind = pos - window - key0, kept = keep_first - key0;
+#pragma unroll
+                for (int i = 0; i < 64; ++i) sc[i] = (i <= behind) & (i >= kept) ? -INFINITY : sc[i];
             }
             float mx4[4] = {sc[0], sc[1], sc[2], sc[3]};     // four chains: a single one is 64 dependent steps
 #pragma unroll
             for (int i = 4; i < 64; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], sc[i]);
             const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale2;   // scale > 0: the maximum of the scaled scores
-            const bool grow = mx > m_ref + PT_RESCALE_STEP || (m_ref == -INFINITY && mx > -INFINITY);
+            const bool grow = live && (mx > m_ref + PT_RESCALE_STEP || (m_ref == -INFINITY && mx > -INFINITY));
             const bool rescale = __any_sync(0xffffffffu, grow);   // the warp decides: tensor-memory accesses are warp-wide
             float corr = 1.f;
             if (rescale) {
@@ -375,10 +402,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
                 l *= corr;
             }
             if (stamps) PT_STAMP(8, j);                         // maximum done
-            // the P buffer is free once the product of the tile's page before last has finished
-            if (c >= 2) ok = tc_mbar_wait(&pv_done[t][sb], ((c >> 1) - 1) & 1, &gave_up);
-            // rescaling O needs the product of the page before finished too (it is the other buffer's barrier)
-            if (ok && rescale && c >= 1) ok = tc_mbar_wait(&pv_done[t][sb ^ 1], ((c - 1) >> 1) & 1, &gave_up);
+            // the P buffer is free once the product of the page that used it before has finished
+            if (c >= BUFS) ok = tc_mbar_wait(&pv_done[t][sb], (c / BUFS - 1) & 1, &gave_up);
+            // rescaling O needs the product of the page before finished too (with two buffers it is the other one's barrier)
+            if (BUFS > 1 && ok && rescale && c >= 1) ok = tc_mbar_wait(&pv_done[t][(c - 1) % BUFS], ((c - 1) / BUFS) & 1, &gave_up);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
                 if (lane == 0 && !gave_up) atomicExch(status, 36);
@@ -388,18 +415,18 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
             if (rescale && c >= 1) {
                 tc_fence_after();
 #pragma unroll 1
-                for (int c0 = 0; c0 < HD; c0 += 32) {
-                    float o[32];
-                    tc_tmem_load32(my_o + (uint32_t)c0, o);
+                for (int c0 = 0; c0 < HD; c0 += 8) {            // few columns at a time: the row's 64 scores stay in registers
+                    float o[8];
+                    tc_tmem_load8(my_o + (uint32_t)c0, o);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) o[i] *= corr;
-                    tc_tmem_store32(my_o + (uint32_t)c0, o);
+                    for (int i = 0; i < 8; ++i) o[i] *= corr;
+                    tc_tmem_store8(my_o + (uint32_t)c0, o);
                 }
                 tc_fence_before();
             }
             // weights of this page, as the A operand of P V: row r is 128 bytes, its 16-byte chunk c at c ^ (r & 7)
             const float sub = (m_ref == -INFINITY) ? 0.f : m_ref;
-            const uint32_t p_row = tc_smem(p_smem + (2 * t + sb) * P_BYTES) + (uint32_t)r * 128u;
+            const uint32_t p_row = tc_smem(p_smem + (BUFS * t + sb) * P_BYTES) + (uint32_t)r * 128u;
             // all exponentials first, in place: the special-function unit takes them back to back, and the
             // sums, the packing and the stores follow in its shadow
 #pragma unroll
@@ -434,7 +461,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
         // ---- O / l -> out
         if (ok && n_mine > 0) {
             const int last = n_mine - 1;
-            ok = __all_sync(0xffffffffu, tc_mbar_wait(&pv_done[t][last & 1], (last >> 1) & 1, &gave_up));
+            ok = __all_sync(0xffffffffu, tc_mbar_wait(&pv_done[t][last % BUFS], (last / BUFS) & 1, &gave_up));
             if (!ok && lane == 0 && !gave_up) atomicExch(status, 37);
         }
         if (!ok) gave_up = 1;
@@ -465,7 +492,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
     __syncthreads();                                         // nobody leaves while copies or MMAs may be in flight
     if (warp == 1) {
         tc_fence_after();
-        tc_tmem_free(tmem_base, PT_TMEM_COLS);
+        tc_tmem_free(tmem_base, PT_TMEM_COLS(HD));
     }
 }
 
@@ -508,13 +535,19 @@ static int pt_launch(dim3 grid, cudaStream_t s, const void* q, int q_stride, int
                      const int32_t* seq_start, const int32_t* seq_new, const int32_t* cu_new, const int32_t* block_table,
                      int bt_stride, int nh, int nkv, float scale, int window, int keep_first, const float* sinks, float softcap,
                      const float* slopes, const void* gate, int gate_stride, int* status) {
-    const size_t smem = (size_t)PT_TILES * PT_ROWS * HD * 2 + (size_t)PT_STAGES(HD) * 2 * DL_PAGE * HD * 2 +
-                        (size_t)PT_TILES * 2 * PT_ROWS * DL_PAGE * 2 + 1024;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD, SHAPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "attention_prefill_tc: shared memory %zu: %s", smem, cudaGetErrorString(e));
-        configured = true;
+    const size_t data = (size_t)PT_TILES * PT_ROWS * HD * 2 + (size_t)PT_STAGES * 2 * DL_PAGE * HD * 2 +
+                        (size_t)PT_TILES * PT_BUFS(HD) * PT_ROWS * DL_PAGE * 2;
+    static size_t smem = 0;
+    if (smem == 0) {
+        // 1,024 bytes to align the data by, of which the kernel's barriers (in front of it) already are a part: two blocks of
+        // heads of 64 then fill a multiprocessor's shared memory to the byte
+        cudaFuncAttributes attr;
+        cudaError_t e = cudaFuncGetAttributes(&attr, attention_prefill_tc_kernel<HD, SHAPE>);
+        if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "attention_prefill_tc: %s", cudaGetErrorString(e));
+        const size_t ask = data + 1024 - (attr.sharedSizeBytes < 1024 ? attr.sharedSizeBytes : 0);
+        e = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD, SHAPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ask);
+        if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "attention_prefill_tc: shared memory %zu: %s", ask, cudaGetErrorString(e));
+        smem = ask;
     }
     CUtensorMap tmap_q, tmap_k, tmap_v;
     int rc = pt_tensor_map(&tmap_q, q, n_tokens, (long long)nh * HD, (long long)q_stride * 2, PT_ROWS);
@@ -527,7 +560,7 @@ static int pt_launch(dim3 grid, cudaStream_t s, const void* q, int q_stride, int
                                                                   tile_seq, tile_row0, seq_start, seq_new, cu_new, block_table,
                                                                   bt_stride, nkv, nh / nkv, scale, window, keep_first, sinks,
                                                                   dl_score_cap(softcap, scale), slopes, (const __nv_bfloat16*)gate,
-                                                                  gate_stride, status);
+                                                                  gate_stride, (int)smem, status);
     DL_CHECK_LAUNCH("attention_prefill_tc");
     return DL_OK;
 }

@@ -107,6 +107,15 @@ __device__ __forceinline__ void tc_tmem_load8(uint32_t taddr, float (&v)[8]) {
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Write 8 consecutive float32 columns of this thread's lane of tensor memory.
+__device__ __forceinline__ void tc_tmem_store8(uint32_t taddr, const float (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(__float_as_uint(v[0])),
+                 "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])),
+                 "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+                 : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 // Write 32 consecutive float32 columns of this thread's lane of tensor memory.
 __device__ __forceinline__ void tc_tmem_store32(uint32_t taddr, const float (&v)[32]) {
     asm volatile(
