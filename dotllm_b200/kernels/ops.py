@@ -828,6 +828,14 @@ CHUNK_SCRATCH_BYTES = 4 << 30    # most scratch the chunks' operands may take (1
 CHUNK_MIN_TOKENS = 256
 
 
+def chunk_hint(rows, plan):
+    """What a mixer adds to its ``gla_scan`` or ``delta_rule`` call: ``max_new``, the most tokens that a sequence of the step brings, where
+    the chunked form may take them; nothing where the tokens are walked one by one whatever their number."""
+    if plan is None or not rows.is_cuda or rows.dtype != torch.bfloat16 or plan.max_new < CHUNK_MIN_TOKENS:
+        return {}
+    return {"max_new": plan.max_new}
+
+
 def _chunk_scratch(device, name, n_seqs, max_new, n_heads, *more):
     """(scratch, chunks of the longest sequence) of a recurrence's chunked form, or (None, 0) where it would take too much."""
     chunks = (int(max_new) + CHUNK - 1) // CHUNK

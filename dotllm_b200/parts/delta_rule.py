@@ -12,8 +12,9 @@ x (q, k, v, the two low-rank first factors and the step size) are one stacked ma
 two second factors are one product each (the decay's leaves its result in float32).  What a sequence carries - every
 head's state and the convolutions' last taps - 1 inputs - is the layer execution's fixed-size cache entry, one float32
 vector per slot, zero when a sequence opens; convolution sums, unit lengths, step sizes, decays, the recurrence and the
-per-head norm are float32 in either run dtype.  The kernels walk a sequence's new tokens in order from that entry, so
-prompts, parts of prompts and decoded tokens are one code path.
+per-head norm are float32 in either run dtype.  The kernels walk a sequence's new tokens in order from that entry; in a
+float32 run prompts, parts of prompts and decoded tokens are that one code path (the same bits however a sequence is
+cut), in a bfloat16 run the recurrence of prompts of 256 tokens and more goes a chunk of tokens at a time.
 
 Two simpler forms, each a parameter: ``decay`` "head" - one decay per head, g = exp(-exp(A_h) softplus(a_h . x + dt_h)),
 from a projection of its own with one row per head (no low-rank pair), the same for all key channels of the head; and
@@ -147,7 +148,7 @@ class ChannelDeltaMixer(Mixer):
         gate = ops.linear(low_gate, self.w_gate, resident=True) if self.gate_low_rank else low_gate
         o = ops.delta_rule(proj, self.conv, b, z, self.decay_bias, self.rate, step.token_seq, step.cu_new, cache_view.slots,
                            cache_view.state, self.n_heads, self.n_kv_heads, self.key_dim, self.value_dim,
-                           self.key_dim ** -0.5, self.unit_eps, head_decay=self.head_decay, max_new=step.attention_plan.max_new)
+                           self.key_dim ** -0.5, self.unit_eps, head_decay=self.head_decay, **ops.chunk_hint(proj, step.attention_plan))
         y = ops.head_norm_gate(o, gate, self.norm_gain, self.n_heads, self.value_dim, self.eps, self.runtime.dtype,
                                gate=self.gate_activation)
         return ops.linear(y, self.w_o, out_dtype=BRANCH_DTYPE, resident=True, lazy=True)

@@ -8,8 +8,9 @@ The five projections that read x (q, k, v, the output gate and the low-rank deca
 stacked matrix, so one product feeds the scan.  The state is the layer execution's fixed-size cache entry
 (float32, zero when a sequence opens, carried from step to step); the decay logits leave their product in
 float32, and decays, recurrence and the per-head norm are float32 in either run dtype.  The scan walks a
-sequence's new tokens in order from the cached state, so prompts, parts of prompts and decoded tokens
-are one code path.
+sequence's new tokens in order from the cached state; in a float32 run prompts, parts of prompts and decoded
+tokens are that one code path (the same bits however a sequence is cut), in a bfloat16 run prompts of 256 tokens
+and more go a chunk of tokens at a time, equal to float32 rounding.
 """
 from __future__ import annotations
 
@@ -84,7 +85,7 @@ class GatedLinearAttentionMixer(Mixer):
         z = ops.linear(low, self.w_decay, out_dtype=torch.float32, resident=True)
         o = ops.gla_scan(q, k, v, z, self.decay_bias, step.cu_new, cache_view.slots, cache_view.state,
                          self.n_heads, self.key_dim, self.value_dim, self.key_dim ** -0.5, self.tau,
-                         max_new=step.attention_plan.max_new)
+                         **ops.chunk_hint(proj, step.attention_plan))
         y = ops.head_norm_gate(o, gate, self.norm_gain, self.n_heads, self.value_dim, self.eps, self.runtime.dtype)
         return ops.linear(y, self.w_o, out_dtype=BRANCH_DTYPE, resident=True, lazy=True)
 
@@ -151,7 +152,7 @@ class DecayedLinearAttentionMixer(Mixer):
         proj = ops.linear(x, self.w_in, resident=True)
         q, k, v, gate = proj[:, :kw], proj[:, kw:2 * kw], proj[:, 2 * kw:2 * kw + vw], proj[:, 2 * kw + vw:2 * kw + 2 * vw]
         o = ops.gla_scan(q, k, v, None, self.decay, step.cu_new, cache_view.slots, cache_view.state, self.n_heads, self.key_dim,
-                         self.value_dim, 1.0, max_new=step.attention_plan.max_new)
+                         self.value_dim, 1.0, **ops.chunk_hint(proj, step.attention_plan))
         y = ops.head_norm_gate(o, gate, self.norm_gain, 1, vw, self.eps, self.runtime.dtype, gate="sigmoid")
         return ops.linear(y, self.w_o, out_dtype=BRANCH_DTYPE, resident=True, lazy=True)
 
