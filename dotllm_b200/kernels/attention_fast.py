@@ -234,6 +234,7 @@ F32_TILE_ROWS = 64                   # AF_ROWS
 # 208 us, 32 after 1,500 60 against 208, 32 after 200 20 against 40; a token's pages are read again for every token, so where tiles
 # fill the machine the line is lower.
 F32_SPLIT_TOKENS, F32_SPLIT_TOKENS_FEW, F32_FULL_BLOCKS = 8, 32, 148
+F32_PARTS_BYTES = 1 << 30            # most room the pages' parts of a launch may take (head_dim + 2 floats a token, head and page); more tokens: more launches
 
 
 def run_f32(q, q_stride, out, k_pool, v_pool, n_pages, token_seq, token_pos, block_table, n_heads, n_kv_heads, head_dim, scale, window, plan,
@@ -243,23 +244,30 @@ def run_f32(q, q_stride, out, k_pool, v_pool, n_pages, token_seq, token_pos, blo
     if head_dim not in F32_HEAD_DIMS or n_heads // n_kv_heads > F32_MAX_GROUP or q_stride % 4 or q.data_ptr() % 16 or k_pool.data_ptr() % 16 \
             or v_pool.data_ptr() % 16 or not plan.news or q.shape[0] != sum(plan.news):
         return False
-    tail = (n_heads, n_kv_heads, head_dim, scale, window, float(softcap), None if slopes is None else slopes.data_ptr(), *_gate_args(gate),
-            int(keep_first), None if sinks is None else sinks.data_ptr())
-    head = (q.data_ptr(), q_stride, out.data_ptr(), out.stride(0), k_pool.data_ptr(), v_pool.data_ptr(), n_pages)
+    def tail(gate):
+        return (n_heads, n_kv_heads, head_dim, scale, window, float(softcap), None if slopes is None else slopes.data_ptr(), *_gate_args(gate),
+                int(keep_first), None if sinks is None else sinks.data_ptr())
+
+    pools = (k_pool.data_ptr(), v_pool.data_ptr(), n_pages)
     T = q.shape[0]
     few = sum(-(-n // F32_TILE_ROWS) for n in plan.news) * n_heads <= F32_FULL_BLOCKS
-    if plan.max_new <= (F32_SPLIT_TOKENS_FEW if few else F32_SPLIT_TOKENS) and T <= 65535:
-        n = T * n_heads * block_table.shape[1]
+    if plan.max_new <= (F32_SPLIT_TOKENS_FEW if few else F32_SPLIT_TOKENS):
+        a_token = n_heads * block_table.shape[1]           # parts
+        at_once = max(1, min(T, 65535, F32_PARTS_BYTES // (4 * a_token * (head_dim + 2))))
+        n = at_once * a_token
         key = ("f32_parts", n, head_dim)
         if key not in plan.scratch:                        # the layers of a step run one after another on one stream
             plan.scratch[key] = torch.empty(n * (head_dim + 2), dtype=torch.float32, device=q.device)
         parts = (plan.scratch[key].data_ptr(), plan.scratch[key].data_ptr() + 4 * n * head_dim)
-        _library.call("dl_attention_f32_split", *head, token_seq.data_ptr(), token_pos.data_ptr(), block_table.data_ptr(), block_table.shape[1], T,
-                      *tail, *parts, _library.current_stream())
+        for lo in range(0, T, at_once):
+            _library.call("dl_attention_f32_split", q.data_ptr() + 4 * lo * q_stride, q_stride, out.data_ptr() + 4 * lo * out.stride(0), out.stride(0),
+                          *pools, token_seq.data_ptr() + 4 * lo, token_pos.data_ptr() + 4 * lo, block_table.data_ptr(), block_table.shape[1],
+                          min(at_once, T - lo), *tail(None if gate is None else gate[lo:]), *parts, _library.current_stream())
         return True
     tile_seq, tile_row0, n_tiles = _prompt_tiles(plan, F32_TILE_ROWS, q.device)
     if n_tiles > 65535:
         return False
-    _library.call("dl_attention_f32_tile", *head, tile_seq.data_ptr(), tile_row0.data_ptr(), n_tiles, plan.seq_start.data_ptr(),
-                  plan.seq_new.data_ptr(), plan.cu_new.data_ptr(), block_table.data_ptr(), block_table.shape[1], *tail, _library.current_stream())
+    _library.call("dl_attention_f32_tile", q.data_ptr(), q_stride, out.data_ptr(), out.stride(0), *pools, tile_seq.data_ptr(), tile_row0.data_ptr(), n_tiles, plan.seq_start.data_ptr(),
+                  plan.seq_new.data_ptr(), plan.cu_new.data_ptr(), block_table.data_ptr(), block_table.shape[1], *tail(gate),
+                  _library.current_stream())
     return True

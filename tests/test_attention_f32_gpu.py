@@ -131,3 +131,17 @@ def test_longer_tables():
     short = case.run([99, 29], [1, 1])
     case.table = torch.cat([case.table, torch.full((2, 30), -1, dtype=torch.int32, device=DEV)], dim=1).contiguous()
     assert all(torch.equal(a, b) for a, b in zip(short, case.run([99, 29], [1, 1])))
+
+
+@pytest.mark.parametrize("tokens_at_once", [1, 2, 5])
+def test_a_few_tokens_in_several_launches(monkeypatch, tokens_at_once):
+    """Where the pages' parts of all tokens would take too much room, a launch takes as many tokens as fit: the same bits."""
+    from dotllm_b200.kernels import attention_fast
+    nh, hd = 8, 64
+    lens, news = [100, 300, 64, 7], [3, 2, 1, 1]
+    starts = [n - m for n, m in zip(lens, news)]
+    case = Case(lens, nh, 2, hd, seed=5)
+    gates = [torch.randn(n, nh, generator=torch.Generator().manual_seed(n)).to(DEV) for n in lens]
+    whole = case.run(starts, news, gates=gates)
+    monkeypatch.setattr(attention_fast, "F32_PARTS_BYTES", tokens_at_once * 4 * nh * case.table.shape[1] * (hd + 2) + 3)
+    assert all(torch.equal(a, b) for a, b in zip(whole, case.run(starts, news, gates=gates)))
