@@ -10,7 +10,8 @@
 // positions, one key per lane for the scores and one output dimension per lane for the
 // weighted sum, with exact expf.  The order of operations for a query therefore depends
 // only on its position, never on how the tokens were cut into steps or batched: this is
-// the kernel of the float32 path and the fallback of the bfloat16 path for sizes that the
+// the kernel of the float32 path for the heads that attention_f32.cu does not take (it takes
+// 64 and 128 channels), and the fallback of the bfloat16 path for sizes that the
 // tensor-core kernels do not take.
 //
 // It also honours every change of the scores before the softmax (as the tensor-core kernels do), the place where

@@ -36,8 +36,8 @@
 // tokens takes 0.83 ms; with 40 for the issuing warps and 96 for the softmax threads nothing spills.  The mask
 // compares with constants and has no branches: element by element with short-circuit conditions, a tile with fewer than
 // 128 rows, which took it on every page, ran three times as long as its neighbours and with it the whole of a short prompt.
-// 32 query over 8 KV heads, before -> now: heads of 64, 1,987 tokens 0.079 -> 0.058 ms, six of them in one call
-// 0.230 -> 0.140, 8,192 tokens 0.558 -> 0.422; heads of 128 (the mask alone) 700 tokens 0.037 -> 0.027, 1,987 tokens
+// 32 query over 8 KV heads, before -> now: heads of 64, 1,987 tokens 0.079 -> 0.058 ms, six prompts of 1,160 to 1,987
+// in one call 0.230 -> 0.140 (its tensor-core instructions are 0.085), 8,192 tokens 0.558 -> 0.422; heads of 128 (the mask alone) 700 tokens 0.037 -> 0.027, 1,987 tokens
 // 0.086 -> 0.060, 8,192 tokens 0.607 -> 0.598 ms.
 // Keys that no query of the tile may see are never used: masked scores are replaced, not
 // multiplied, and the slots of the last page beyond the sequence's length (which may hold

@@ -15,7 +15,8 @@
 // What a sequence carries from step to step lies in one float32 vector per slot: the state S of every head
 // [H, dim, vdim], and behind it the convolution's last K - 1 inputs [K - 1, channels] (oldest first).  A prompt, a
 // part of a prompt and one decoded token are the same code, so a position's result does not depend on how the
-// sequence was cut into steps.
+// sequence was cut into steps.  (In a bfloat16 run the recurrence of prompts of 256 tokens and more goes 32 tokens at a
+// time instead of through `delta_scan`: chunk_scan.cu, equal to float32 rounding.)
 //
 // The scan: columns of S never mix, so a block owns DR_COLS value channels of one (sequence, head).  DR_SPLIT
 // lanes of one warp share a column, each with a run of ROWS key channels in registers; per token they take the

@@ -2,7 +2,8 @@
 //
 // The reference's 32-bit model runs its projections as per-row dot products
 // (src/DotLLM.Cpu/Kernels/MatMul.cs:1121-1134, GemmF32 over GemvF32 :55-64).  This kernel is
-// the same contraction tiled through shared memory.  Each output element is accumulated over k
+// the same contraction tiled through shared memory.  Matrices of 256 columns and more go to gemm_f32_tc.cu
+// (the tensor cores on values split three ways); this kernel takes the smaller and the unaligned ones.  Each output element is accumulated over k
 // in ascending order by one thread, so its value does not depend on how many rows x has or on
 // which rows share the launch: the 32-bit path gives the same bits however the tokens are cut
 // into steps.

@@ -15,7 +15,9 @@
 //
 // The scan walks a sequence's new tokens in order, starting from the state that the sequence's slot
 // holds and leaving the new state there: a prompt, a part of a prompt and a single decoded token are
-// the same loop, so a position's result does not depend on how its sequence was cut into steps.  A
+// the same loop, so a position's result does not depend on how its sequence was cut into steps.  (In a
+// bfloat16 run, prompts of 256 tokens and more go 32 tokens at a time instead: chunk_scan.cu, equal to
+// float32 rounding.)  A
 // block owns GLA_COLS value channels of one (sequence, head): columns of S never mix, so blocks need
 // nothing from each other.  GLA_SPLIT threads share a column, each holding a run of ROWS
 // key channels of it in registers.  Tokens are staged in shared memory a batch at a time (two

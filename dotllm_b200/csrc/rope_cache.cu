@@ -195,8 +195,8 @@ rope_cache_write_tile_kernel(T* __restrict__ q, int q_stride, const T* __restric
 // float32 prompts are few, with a handful of units a thread, so a thread loads BATCH units (rows, cosines and sines) before it
 // rotates and stores the first; stores to Q in place would otherwise hold the next unit's loads back.  bfloat16 rows are half as
 // long and come with more tokens (blocks), and a second unit's registers cost more blocks than its loads bring.  Measured: float32,
-// 1,000 tokens of 32 + 8 heads of 128, 59 us one element a thread, 14 us here; bfloat16, 11,922 tokens of 32 + 8 heads of 64,
-// 33 us with a batch of one (4.5 TB/s of rows read and written), 54 us with two.
+// 1,000 tokens of 32 + 8 heads of 128, 59 us one element a thread, 14 us here; bfloat16, 9,431 tokens of 32 + 8 heads of 64,
+// 33 us with a batch of one (3.5 TB/s of rows read and written), 54 us with two.
 template <typename T>
 struct RopeUnit {
     static constexpr int E = 16 / (int)sizeof(T);
