@@ -10,8 +10,9 @@
 //     tree (keys x, x + 16, x + 32, x + 48 in order, then the sixteen sums in a butterfly) and per channel again two chains, over
 //     the page's even and odd keys;
 //   * pages are merged in ascending order: M' = max(M, m), both sides scaled by exp(. - M').
-// A key that a query does not see has weight 0 and changes no sum, so pages that hold none may be skipped or not; keys beyond the
-// query are read (as finite numbers) only where a neighbour in the tile sees them.
+// A key that a query does not see has weight 0 and changes no sum; a page is left out where the query sees none of its keys, and
+// only there: whether it does follows from positions, never from a score, so that a score that is no number (which a maximum
+// ignores) reaches the sums and the result.  Keys beyond the query are read only where a neighbour in the tile sees them.
 //
 // What bounds it.  Prompts: the FFMA pipes (74 TFLOP/s) and, about as much, the reads of shared memory that feed them; the generic
 // kernel ran a warp per (token, head) and brought every tile of keys into shared memory once per token.  Here 64 rows share a
@@ -39,6 +40,10 @@ struct AfScore {
 __device__ __forceinline__ void af_range(const AfScore& sc, int pos, int& first, int& kept) {
     first = (sc.window > 0 && pos - sc.window + 1 > 0) ? pos - sc.window + 1 : 0;
     kept = min(sc.keep_first, first);
+}
+// Does the query see some key of the page at key0?
+__device__ __forceinline__ bool af_sees(int key0, int pos, int first, int kept) {
+    return key0 <= pos && (key0 < kept || key0 + DL_PAGE > first);
 }
 // The score of the key at j from the raw dot product; explicit roundings, so that both kernels get the same bits.
 __device__ __forceinline__ float af_score(float dot, const AfScore& sc, float slope, int j, int pos) {
@@ -183,7 +188,8 @@ attention_f32_tile_kernel(const float* __restrict__ q, int q_stride, float* __re
         float e1[R], e2[R];                                // factors of the running output and of the page's
         // a page that every row sees whole needs no mask
         const int key0 = page * DL_PAGE;
-        const bool whole = key0 + DL_PAGE - 1 <= pos0 && n_rows == AF_ROWS && (key0 >= first1 || key0 + DL_PAGE <= kept0);
+        const bool there = page_id(page) >= 0;
+        const bool whole = there && key0 + DL_PAGE - 1 <= pos0 && n_rows == AF_ROWS && (key0 >= first1 || key0 + DL_PAGE <= kept0);
 #pragma unroll
         for (int i = 0; i < R; ++i) {
             const int row = ty + TY * i, pos = pos0 + row;
@@ -193,7 +199,7 @@ attention_f32_tile_kernel(const float* __restrict__ q, int q_stride, float* __re
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int key = key0 + tx + 16 * j;
-                const bool seen = whole || (row < n_rows && key <= pos && (key >= first || key < kept));
+                const bool seen = whole || (there && row < n_rows && key <= pos && (key >= first || key < kept));
                 s[i][j] = seen ? af_score(s[i][j], sc, slope, key, pos) : -INFINITY;
                 top = fmaxf(top, s[i][j]);
             }
@@ -210,7 +216,7 @@ attention_f32_tile_kernel(const float* __restrict__ q, int q_stride, float* __re
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, o));
             e1[i] = 1.f, e2[i] = 0.f;                          // a page without a visible key changes nothing
-            if (top != -INFINITY) af_merge(M[i], L[i], top, sum, e1[i], e2[i]);
+            if (there && af_sees(key0, pos, first, kept)) af_merge(M[i], L[i], top, sum, e1[i], e2[i]);
         }
         af_wait<1>();                                      // this page's values have landed
         __syncthreads();
@@ -285,7 +291,7 @@ attention_f32_tile_kernel(const float* __restrict__ q, int q_stride, float* __re
 
 // ------------------------------------------------------- a few new tokens
 // Grid (page, KV head, token): the token's queries of all G heads of the KV head over one page.  part_o, part_ml: per (token, head, page)
-// the output [HD], m and l (m -inf: the token sees nothing of the page).  PAIRS: (head, channel) pairs a thread keeps.
+// the output [HD], m and l (l -1: the token sees nothing of the page).  PAIRS: (head, channel) pairs a thread keeps.
 template <int HD, int PAIRS>
 __global__ void __launch_bounds__(AF_SPLIT_THREADS)
 attention_f32_split_kernel(const float* __restrict__ q, int q_stride, const float* __restrict__ k_pool, const float* __restrict__ v_pool,
@@ -308,8 +314,8 @@ attention_f32_split_kernel(const float* __restrict__ q, int q_stride, const floa
     af_range(sc, pos, first, kept);
     const size_t part0 = ((size_t)t * nh + kvh * G) * bt_stride + page;      // head g's: + g * bt_stride
     const int id = block_table[(size_t)token_seq[t] * bt_stride + page];
-    if (key0 > pos || (key0 >= kept && key0 + DL_PAGE <= first) || id < 0 || id >= n_pages) {      // nothing here for this token
-        for (int g = tid; g < G; g += AF_SPLIT_THREADS) part_ml[(part0 + (size_t)g * bt_stride) * 2] = -INFINITY;
+    if (!af_sees(key0, pos, first, kept) || id < 0 || id >= n_pages) {      // nothing here for this token
+        for (int g = tid; g < G; g += AF_SPLIT_THREADS) part_ml[(part0 + (size_t)g * bt_stride) * 2 + 1] = -1.f;
         return;
     }
     auto visible = [&](int key) { return key <= pos && (key >= first || key < kept); };
@@ -412,7 +418,7 @@ attention_f32_merge_kernel(float* __restrict__ out, int out_stride, const float*
         }
 #pragma unroll
         for (int i = 0; i < AF_MERGE_AHEAD; ++i) {
-            if (p0 + i >= end || x[i].x == -INFINITY) continue;
+            if (p0 + i >= end || x[i].y < 0.f) continue;
             float e1, e2;
             af_merge(M, L, x[i].x, x[i].y, e1, e2);
             A = af_blend(A, e1, o[i], e2);

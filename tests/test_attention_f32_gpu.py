@@ -125,6 +125,50 @@ def test_a_later_value_that_is_no_number_stays_unseen():
     assert torch.equal(case.run([139], [1])[0], clean[139:140]) and torch.equal(case.run([130], [70])[0], got[130:])
 
 
+@pytest.mark.parametrize("what", ["newest key", "page of keys", "first page of keys", "query", "page beyond the window", "scores of -inf", "first scores of -inf"])
+@pytest.mark.parametrize("with_sinks", [False, True])
+def test_keys_and_queries_that_are_no_numbers(what, with_sinks):
+    """A NaN among the visible scores makes the output NaN, through either kernel, and nothing else does: exactly where float64 says so.
+    A page whose scores are all -inf has no weight beside others."""
+    nan, inf = float("nan"), float("inf")
+    case = Case([193, 260], 8, 2, 64, seed=8)                  # the first one's newest key is a page's only one
+    kw = dict(sinks=torch.linspace(-1, 1, 8, device=DEV)) if with_sinks else {}
+    if what == "page beyond the window":
+        kw["window"] = 70
+
+    def put(b, lo, hi, channels, value):                       # keys of the first KV head
+        case.k[b][lo:hi, 0, channels] = value
+        for at in range(lo, hi):
+            case.k_pool[int(case.table[b, at // PAGE]), 0, at % PAGE, channels] = value
+
+    if what == "newest key":
+        put(0, 192, 193, slice(None), nan)
+        put(1, 256, 257, slice(None), nan)
+    elif what == "page of keys":
+        put(0, 64, 128, slice(5, 6), nan)
+        put(1, 128, 192, slice(None), nan)
+    elif what in ("first page of keys", "page beyond the window"):
+        put(0, 0, 64, slice(None), nan)
+        put(1, 0, 64, slice(None), nan)
+    elif what == "query":
+        case.q[0][192, 3] = nan
+        case.q[1][258, 0, 7] = nan
+    else:
+        page = 0 if what.startswith("first") else 64
+        for b in (0, 1):
+            case.q[b][:, :, 0] = 1.0
+            put(b, page, page + 64, slice(0, 1), -inf)
+    whole = case.run([0, 0], [193, 260], **kw)
+    few = case.run([192, 257], [1, 3], **kw)
+    for b in (0, 1):
+        want = case.exact(b, kw.get("window", 0), sinks=kw.get("sinks"))
+        assert bool(torch.isnan(want).any()) == (what != "scores of -inf" and (what != "first scores of -inf" or not with_sinks))
+        assert torch.equal(torch.isnan(whole[b]), torch.isnan(want)), b
+        fine = ~torch.isnan(want)
+        assert float((whole[b].double() - want)[fine].abs().max()) < bound(260, None)
+        assert torch.equal(few[b].nan_to_num(nan=9.0), whole[b][-few[b].shape[0]:].nan_to_num(nan=9.0)), b
+
+
 def test_longer_tables():
     """Columns of a table beyond a sequence's pages change nothing."""
     case = Case([100, 30], 8, 2, 64, seed=4)
