@@ -29,6 +29,10 @@
 // 734 -> 489 us (208 for G, 281 the walk); one of 2,048, 16 heads: 320 -> 199.  What bounds them now is the FFMA pipes' issue
 // (18 and 50 million multiply-adds a thousand tokens and head).
 //
+// A token that is no number (an infinity or a NaN among its inputs) must not reach the outputs of the tokens before it, and 0 times it
+// is a NaN: A and T hold nothing but zeros above their diagonals, and an output that is not finite is summed again over its own and
+// earlier tokens only (the same sums in the same order, so the bits of the tokens before do not change).
+//
 // The sums run in another order than the scans': the results agree to float32 rounding, not to the bit.  A float32 run therefore
 // keeps the scans (there a sequence may be cut anywhere), and so do steps of few tokens.
 #include "common.cuh"
@@ -41,6 +45,7 @@
 #define CK_LDT (CK_L + 4)                // rows along tokens, in floats: 16-byte aligned, eight rows' reads meet different banks
 #define CK_LDX (CK_X + 4)
 
+__device__ __forceinline__ bool ck_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
 __device__ __forceinline__ float ck_silu(float v) { return v / (1.0f + expf(-v)); }
 __device__ __forceinline__ void ck_copy16(float* dst, const float* src, bool live) {      // 16 bytes, zeros where not live
     const int bytes = live ? 16 : 0;
@@ -86,6 +91,28 @@ __device__ __forceinline__ void ck_product(float (&acc)[RN][N], const float* a, 
                 acc[i][e] = fmaf(av.w, bv[3][e], fmaf(av.z, bv[2][e], fmaf(av.y, bv[1][e], fmaf(av.x, bv[0][e], acc[i][e]))));
         }
     }
+}
+
+// One row of a product once more, over its first n values k alone (in ck_product's order), from the sum `from`: for an output that is not finite.
+template <int N, int LDB>
+__device__ __noinline__ void ck_row_again(float* dst, const float* a, const float* b, int n, typename CkVec<N>::type from) {
+    float acc[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e) acc[e] = reinterpret_cast<const float*>(&from)[e];
+    for (int k = 0; k < n; ++k) {
+        float bv[N];
+        ck_load<N>(b + k * LDB, bv);
+#pragma unroll
+        for (int e = 0; e < N; ++e) acc[e] = fmaf(a[k], bv[e], acc[e]);
+    }
+    ck_store<N>(dst, acc);
+}
+template <int N>
+__device__ __forceinline__ bool ck_all_finite(const float (&v)[N]) {
+    bool ok = true;
+#pragma unroll
+    for (int e = 0; e < N; ++e) ok = ok && ck_finite(v[e]);
+    return ok;
 }
 
 // What the kernels have of a chunk.
@@ -193,7 +220,10 @@ delta_chunk_prepare_kernel(const float* __restrict__ q, const float* __restrict_
 #pragma unroll
         for (int t = 0; t < CK_L; ++t) part[(warp * CK_L + t) * CK_L + lane] = aq[t];
         __syncthreads();
-        for (int e = tid; e < W; e += CK_THREADS) sA[(e / CK_L) * CK_LDT + e % CK_L] = (part[e] + part[W + e]) + (part[2 * W + e] + part[3 * W + e]);
+        for (int e = tid; e < W; e += CK_THREADS) {
+            const int t = e / CK_L, j = e % CK_L;
+            sA[t * CK_LDT + j] = j <= t ? (part[e] + part[W + e]) + (part[2 * W + e] + part[3 * W + e]) : 0.f;
+        }
         __syncthreads();
 #pragma unroll
         for (int t = 0; t < CK_L; ++t) part[(warp * CK_L + t) * CK_L + lane] = ak[t];
@@ -252,7 +282,16 @@ delta_chunk_prepare_kernel(const float* __restrict__ q, const float* __restrict_
 #pragma unroll
         for (int i = 0; i < 4; ++i) ck_store<4>(out + (rg + 16 * i) * CK_X + col, top[i]);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) ck_store<4>(out + (CK_DIM + rg + 16 * i) * CK_X + col, low[i]);
+        for (int i = 0; i < 2; ++i) {
+            const int t = rg + 16 * i;
+            float* dst = out + (CK_DIM + t) * CK_X + col;
+            ck_store<4>(dst, low[i]);
+            if (!ck_all_finite(low[i])) {
+                const float* from = sq + col * CK_LDT + t;
+                ck_row_again<4, CK_LDX>(dst, sA + t * CK_LDT, part + col, t + 1,
+                                        col < CK_DIM ? make_float4(from[0], from[CK_LDT], from[2 * CK_LDT], from[3 * CK_LDT]) : make_float4(0.f, 0.f, 0.f, 0.f));
+            }
+        }
     }
 }
 
@@ -326,11 +365,18 @@ delta_chunk_walk_kernel(const float* __restrict__ v, const float* __restrict__ G
         ck_commit();
         ck_wait<1>();
         __syncthreads();                                   // its second half is there
+        typename CkVec<N>::type half_o[2];                 // the outputs so far
+#pragma unroll
+        for (int i = 0; i < 2; ++i) ck_store<N>(reinterpret_cast<float*>(&half_o[i]), acc[4 + i]);
         ck_product<6, N, HALF / 4, CK_LDX, CW>(acc, s_g + rg * CK_LDX + HALF, x + HALF * CW + N * cg);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const int t = chunk * CK_L + rg + 16 * i;
-            if (t < n && col_ok) ck_store<N>(o_at + t * step, acc[4 + i]);
+            const int t = rg + 16 * i;
+            if (chunk * CK_L + t >= n || !col_ok) continue;
+            float* dst = o_at + (chunk * CK_L + t) * step;
+            ck_store<N>(dst, acc[4 + i]);
+            if (!ck_all_finite(acc[4 + i]))
+                ck_row_again<N, CW>(dst, s_g + (CK_DIM + t) * CK_LDX + HALF, x + HALF * CW + N * cg, CK_DIM - HALF + t + 1, half_o[i]);
         }
         __syncthreads();                                   // and has been used
         if (chunk + 1 < chunks) bring(chunk + 1, 1);
@@ -414,7 +460,8 @@ gla_chunk_states_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
     float* qa = out.qa + piece * (CK_L * CK_X);
     constexpr int W = CK_L * CK_L;
     for (int e = tid; e < W; e += CK_GLA_THREADS)
-        qa[(e / CK_L) * CK_X + CK_DIM + e % CK_L] = (part[e] + part[W + e]) + (part[2 * W + e] + part[3 * W + e]);
+        qa[(e / CK_L) * CK_X + CK_DIM + e % CK_L] =
+            e % CK_L <= e / CK_L ? (part[e] + part[W + e]) + (part[2 * W + e] + part[3 * W + e]) : 0.f;
     if (tid < CK_DIM) out.end[piece * CK_DIM + tid] = ck_keys_to_end(sk + tid * CK_LDT, sa + tid * CK_LDT);
     else if (tid < 2 * CK_DIM) ck_queries_from_start(sq + (tid - CK_DIM) * CK_LDT, sa + (tid - CK_DIM) * CK_LDT);
     __syncthreads();
@@ -503,7 +550,12 @@ gla_chunk_out_kernel(const T* __restrict__ v, long v_ld, int v_silu, CkGla in, c
         const int col = col0 + 4 * cg;
 #pragma unroll
         for (int i = 0; i < 2; ++i)
-            if (rg + 16 * i < r.count && col < vdim) ck_store<4>(out + (long)(r.t0 + r.first + rg + 16 * i) * out_ld + (long)h * vdim + col, acc[i]);
+            if (rg + 16 * i < r.count && col < vdim) {
+                float* dst = out + (long)(r.t0 + r.first + rg + 16 * i) * out_ld + (long)h * vdim + col;
+                ck_store<4>(dst, acc[i]);
+                if (!ck_all_finite(acc[i]))
+                    ck_row_again<4, CK_GLA_COLS>(dst, s_qa + (rg + 16 * i) * CK_LDX, s_x + 4 * cg, CK_DIM + rg + 16 * i + 1, make_float4(0.f, 0.f, 0.f, 0.f));
+            }
         __syncthreads();
     }
 }

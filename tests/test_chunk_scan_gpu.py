@@ -103,3 +103,72 @@ def test_delta_rule(H, G, dim, vdim, head_decay, monkeypatch):
     assert float((mem.cpu() - want_mem).abs().max()) < 3 * TOL * (1 + float(want_mem.abs().max()))
     assert float((got - scan).abs().max()) < 3 * TOL * scale
     assert torch.equal(mem[3], memory[3].to(DEV)) and torch.equal(mem[:, n_state:], scan_mem[:, n_state:])
+
+
+def no_worse(got, state, clean, scan, scan_state, before):
+    """Rows of the tokens before keep their bits; what is no number is so exactly where the scan has it, the rest agrees with the scan."""
+    assert torch.equal(got[before], clean[before])
+    for a, b in ((got, scan), (state, scan_state)):
+        fine = torch.isfinite(b)
+        assert torch.equal(torch.isfinite(a), fine) and not bool(fine.all())
+        assert float((a - b)[fine].abs().max()) < TOL * (1 + float(b[fine].abs().max()))
+
+
+@pytest.mark.parametrize("what", ["v", "k", "q", "z"])
+@pytest.mark.parametrize("token", [0, 45, 63, 64])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_linear_attention_of_a_token_that_is_no_number(what, token, value, monkeypatch):
+    from dotllm_b200.kernels import ops
+    monkeypatch.setattr(ops, "CHUNK_MIN_TOKENS", 2)
+    H, dim, vdim, lens = 2, 40, 72, [100, 70]
+    T = sum(lens)
+    proj = g64(T, 2 * H * dim + H * vdim, seed=1).to(torch.bfloat16).to(DEV)
+    z, bias = (g64(T, H * dim, seed=3) * 2).float().to(DEV), g64(H * dim, seed=5).float().to(DEV)
+    state0 = g64(2, H, dim, vdim, seed=6).float().to(DEV)
+
+    def run(most):
+        s = state0.clone()
+        q, k, v = proj[:, :H * dim], proj[:, H * dim:2 * H * dim], proj[:, 2 * H * dim:]
+        return ops.gla_scan(q, k, v, z, bias, i32([0, 100, 170]), i32([1, 0]), s, H, dim, vdim, 0.3, 5.0, max_new=most), s
+
+    clean, clean_state = run(100)
+    if what == "z":
+        z[token, 3] = float("nan")                         # (an infinite logit is a decay of 0 or 1)
+    else:
+        proj[token, {"q": 0, "k": H * dim, "v": 2 * H * dim}[what] + 5] = value
+    got, state = run(100)
+    scan, scan_state = run(1)
+    if what == "q":                                        # only its own row
+        assert torch.equal(state, clean_state) and torch.equal(torch.isfinite(got), torch.isfinite(scan))
+        assert torch.equal(got[[t for t in range(T) if t != token]], clean[[t for t in range(T) if t != token]])
+        return
+    no_worse(got, state, clean, scan, scan_state, list(range(token)) + list(range(100, T)))
+
+
+@pytest.mark.parametrize("what", ["v", "k", "b", "z"])
+@pytest.mark.parametrize("token", [0, 45, 63, 64])
+@pytest.mark.parametrize("H,G", [(4, 2), (40, 40)])
+def test_delta_rule_of_a_token_that_is_no_number(what, token, H, G, monkeypatch):
+    """(Forty heads: the walk over 32 columns a block.)"""
+    from dotllm_b200.kernels import ops
+    monkeypatch.setattr(ops, "CHUNK_MIN_TOKENS", 2)
+    dim, vdim, K, lens = 64, 128, 4, [100, 70]
+    C, T, n_state = 2 * G * dim + H * vdim, sum(lens), H * dim * vdim
+    taps, dt_bias, a_log = g64(C, K, seed=1, scale=0.5).to(torch.bfloat16).to(DEV), g64(H * dim, seed=2).float().to(DEV), g64(H, seed=3, scale=0.5).float().to(DEV)
+    x, z = g64(T, C + H, seed=10).to(torch.bfloat16).to(DEV), g64(T, H * dim, seed=20).float().to(DEV)
+    memory = g64(2, n_state + (K - 1) * C, seed=4).float().to(DEV)
+    seq = i32([0] * 100 + [1] * 70)
+
+    def run(most):
+        m = memory.clone()
+        o = ops.delta_rule(x, taps, x[:, C:], z, dt_bias, a_log, seq, i32([0, 100, 170]), i32([1, 0]), m, H, G, dim, vdim, dim ** -0.5, 1e-6, max_new=most)
+        return o, m[:, :n_state].contiguous()
+
+    clean, _ = run(100)
+    if what == "z":
+        z[token, 3] = float("nan")
+    else:
+        x[token, {"v": 2 * G * dim, "k": G * dim, "b": C}[what] + 1] = float("inf") if what == "v" else float("nan")
+    got, state = run(100)
+    scan, scan_state = run(1)
+    no_worse(got, state, clean, scan, scan_state, list(range(token)) + list(range(100, T)))
