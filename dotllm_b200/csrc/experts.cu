@@ -441,9 +441,10 @@ expert_combine_kernel(const float* __restrict__ y, int y_stride, const int32_t* 
     }
 }
 
-// ids int32 [rows] (rows = tokens * top); place int32 [rows]; tile_expert int32 [max_tiles], max_tiles >= rows / 128 + E.
+// ids int32 [rows] (rows = tokens * top); place int32 [rows]; tile_expert int32 [max_tiles]: as many as the experts that have rows
+// (at most min(rows, E)) can need, each with a last tile that is not full.
 extern "C" int dl_expert_sort(const int32_t* ids, int rows, int E, int32_t* place, int32_t* tile_expert, int max_tiles, void* stream) {
-    DL_REQUIRE(rows >= 0 && E > 0 && max_tiles >= (rows + EX_TILE - 1) / EX_TILE + E - 1, "expert_sort: %d tiles do not hold %d rows of %d experts",
+    DL_REQUIRE(rows >= 0 && E > 0 && max_tiles >= ((long long)rows + (EX_TILE - 1) * (long long)(E < rows ? E : rows)) / EX_TILE, "expert_sort: %d tiles do not hold %d rows of %d experts",
                max_tiles, rows, E);
     DL_REQUIRE((size_t)2 * E * sizeof(int) <= 48 * 1024, "expert_sort: too many experts");
     cudaError_t e = dl_launch_dependent(expert_sort_kernel, dim3(1), dim3(EX_SORT_THREADS), (size_t)2 * E * sizeof(int),

@@ -1256,22 +1256,41 @@ def expert_down(h, ids, weights, w_down, addend=None, addend_gate=None, identity
     return out
 
 
-# (token, choice) rows from which the experts' products run as tensor-core tiles.  Row by row a matrix is read once per row that chose
-# it, as tiles once per expert, behind a sort and a gather.  The whole part, by row / as tiles, us: 16 experts of 2,048 (width 2,048, two
-# chosen): 16 rows 114 / 137, 24 rows 169 / 148, 64 rows 303 / 176, 126 rows 452 / 177; 32 experts (width 4,096, four chosen): 16 rows
-# 222 / 255, 24 rows 298 / 280, 64 rows 589 / 371, 128 rows 929 / 434.
-GROUPED_MIN_ROWS = 24
+# (token, choice) rows from which the experts' products always run as tensor-core tiles, and the fewest that they are open to.
+GROUPED_ALWAYS_ROWS, GROUPED_MIN_ROWS = 128, 24
 EXPERT_TILE = 128              # rows of a tile (EX_TILE in csrc/experts.cu, GT_BM in csrc/gemm_tc.cu)
 
 
 def experts_grouped_takes(x, ids, w_gate_up, w_down):
-    """Do the sorted, tensor-core products take this step's experts?  bfloat16, enough rows to fill tiles, and
-    widths and addresses that the copy engine takes (multiples of 8 values, 16-byte aligned)."""
+    """Are the sorted, tensor-core products open to this step's experts?  bfloat16, a number of rows at which they may pay
+    (`experts_as_tiles` says whether they do), and widths and addresses that the copy engine takes (multiples of 8 values, 16-byte aligned)."""
     T, top = ids.shape
     K, ff = w_gate_up.shape[2], w_down.shape[2]
     return (x.dtype == torch.bfloat16 and T * top >= GROUPED_MIN_ROWS and K % 8 == 0 and ff % 8 == 0
             and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
             and w_gate_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0)
+
+
+def experts_as_tiles(x, ids, w_gate_up, w_down, row_scale=None):
+    """Should this step's experts run as tensor-core tiles (``experts_grouped``) and not row by row?
+
+    From 128 rows always.  Below, row by row a matrix is read once per row that chose it, as tiles once per expert that any row chose, behind
+    a sort and a gather: with b megabytes of matrices an expert, about 8 + rows b / 4.4 us against 65 + experts (b / 5 + 0.6) us, the
+    experts' number taken as uniform choices would have it.  Measured, row by row / as tiles, us (the line's answer in capitals): 16
+    experts of 25 MB: 16 rows 98 / 117, 24 rows 150 / 125 TILES, 64 rows 260 / 133 TILES; of 13 MB: 24 rows 84 / 88 ROWS, 48 rows
+    143 / 92 TILES; of 3 MB: 24 rows 33 / 61 ROWS, 64 rows 55 / 63 ROWS; 32 of 50 MB: 24 rows 254 / 246 TILES; of 9 MB: 24 rows 70 /
+    111 ROWS, 48 rows 113 / 121 ROWS, 96 rows 184 / 125 TILES; 64 of 17 MB: 24 rows 141 / 168 ROWS, 48 rows 219 / 217 ROWS, 96 rows
+    367 / 285 TILES; 128 of 9 MB: 64 rows 162 / 190 ROWS, 96 rows 213 / 229 ROWS, 120 rows 266 / 268 TILES; 256 of 88 MB: 24 rows
+    623 / 543 TILES.  A ``row_scale`` is multiplied into bfloat16 rows for the tiles, where the kernels row by row keep the
+    product in float32: such steps stay row by row below 128 rows."""
+    if not experts_grouped_takes(x, ids, w_gate_up, w_down):
+        return False
+    rows, E = ids.numel(), w_gate_up.shape[0]
+    if rows >= GROUPED_ALWAYS_ROWS:
+        return True
+    mb = 2e-6 * (w_gate_up[0].numel() + w_down[0].numel())
+    distinct = E * (1.0 - (1.0 - 1.0 / E) ** rows)
+    return row_scale is None and 8 + rows * mb / 4.4 > 65 + distinct * (mb / 5 + 0.6)
 
 
 def experts_grouped(x, ids, weights, w_gate_up, w_down, kind, limit=0.0, alpha=1.0, addend=None, row_scale=None,
@@ -1289,7 +1308,8 @@ def experts_grouped(x, ids, weights, w_gate_up, w_down, kind, limit=0.0, alpha=1
     E, rows_w, K = w_gate_up.shape
     ff, N = (rows_w // 2 if gated else rows_w), w_down.shape[1]
     rows = T * top
-    tiles = (rows + EXPERT_TILE - 1) // EXPERT_TILE + E - 1          # every expert may end in a tile that is not full
+    # every expert that has rows may end in a tile that is not full
+    tiles = (rows + (EXPERT_TILE - 1) * min(E, rows)) // EXPERT_TILE
     dev = x.device
     place = torch.empty(rows, dtype=torch.int32, device=dev)
     tile_expert = torch.empty(tiles, dtype=torch.int32, device=dev)
