@@ -73,7 +73,7 @@ def test_tiles_for_the_experts_that_have_rows(tokens, top, E):
     # both round the same intermediate rows to bfloat16; a sum that lies near a rounding's edge may fall to either side (2^-9 of one of 256)
     assert float((tiles - rows).norm() / rows.norm()) < 2.0 ** -8
     n = (tokens * top + 127 * min(E, tokens * top)) // 128
-    assert peak < n * 128 * (2 * 512 + 2 * 256 + 4 * 512) + 4 * tokens * 512 + (1 << 20)
+    assert peak < n * 128 * (2 * 512 + 2 * 256 + 4 * 512) + 4 * tokens * 512 + (2 << 20)          # (small buffers share segments of 2 MB)
 
 
 @pytest.mark.parametrize("tokens", [32, 63, 64])
