@@ -290,10 +290,12 @@ attention_f32_tile_kernel(const float* __restrict__ q, int q_stride, float* __re
 }
 
 // ------------------------------------------------------- a few new tokens
-// Grid (page, KV head, token): the token's queries of all G heads of the KV head over one page.  part_o, part_ml: per (token, head, page)
+// Grid (pages, KV head, token): the token's queries of all G heads of the KV head over page x, then x + the grid's width and so on up to
+// the token's own page.  The width is the table's up to the machine filled several times over (a captured step's table is as wide as
+// its longest sequence may become: a block for every column would be blocks that find nothing to do).  part_o, part_ml: per (token, head, page)
 // the output [HD], m and l (l -1: the token sees nothing of the page).  PAIRS: (head, channel) pairs a thread keeps.
 template <int HD, int PAIRS>
-__global__ void __launch_bounds__(AF_SPLIT_THREADS)
+__global__ void __launch_bounds__(AF_SPLIT_THREADS, HD == 64 ? 6 : 3)
 attention_f32_split_kernel(const float* __restrict__ q, int q_stride, const float* __restrict__ k_pool, const float* __restrict__ v_pool,
                            int n_pages, const int32_t* __restrict__ token_seq, const int32_t* __restrict__ token_pos,
                            const int32_t* __restrict__ block_table, int bt_stride, int nh, int nkv, const AfScore sc,
@@ -307,89 +309,95 @@ attention_f32_split_kernel(const float* __restrict__ q, int q_stride, const floa
     float* ps = qs + G * HD;                               // [G][64]
     dl_launch_dependents();
     dl_grid_dependency_wait();
-    const int page = blockIdx.x, kvh = blockIdx.y, t = blockIdx.z;
+    const int kvh = blockIdx.y, t = blockIdx.z;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int pos = token_pos[t], key0 = page * DL_PAGE;
+    const int pos = token_pos[t], end = min(pos / DL_PAGE + 1, bt_stride);
     int first, kept;
     af_range(sc, pos, first, kept);
-    const size_t part0 = ((size_t)t * nh + kvh * G) * bt_stride + page;      // head g's: + g * bt_stride
-    const int id = block_table[(size_t)token_seq[t] * bt_stride + page];
-    if (!af_sees(key0, pos, first, kept) || id < 0 || id >= n_pages) {      // nothing here for this token
-        for (int g = tid; g < G; g += AF_SPLIT_THREADS) part_ml[(part0 + (size_t)g * bt_stride) * 2 + 1] = -1.f;
-        return;
-    }
-    auto visible = [&](int key) { return key <= pos && (key >= first || key < kept); };
-    const float* ksrc = k_pool + dl_k_offset(id, nkv, kvh, 0, HD);
-    for (int e = tid; e < DL_PAGE * CH; e += AF_SPLIT_THREADS) af_copy16(ks + af_at<CH>(e / CH, e % CH), ksrc + 4 * e, visible(key0 + e / CH));
-    af_commit();
-    const float* vsrc = v_pool + dl_v_offset(id, nkv, kvh, 0, HD);
-    for (int e = tid; e < HD * 16; e += AF_SPLIT_THREADS) af_copy16(vs + af_at<16>(e / 16, e % 16), vsrc + 4 * e, key0 + 4 * (e % 16) <= pos);
-    af_commit();
-    for (int e = tid; e < G * HD; e += AF_SPLIT_THREADS) qs[e] = q[(size_t)t * q_stride + (size_t)kvh * G * HD + e];
-    af_wait<1>();
-    __syncthreads();
-    for (int e = tid; e < G * DL_PAGE; e += AF_SPLIT_THREADS) {
-        const int g = e / DL_PAGE, kk = e % DL_PAGE, key = key0 + kk;
-        float2 pair = make_float2(0.f, 0.f);
-#pragma unroll 8
-        for (int c = 0; c < CH; ++c)
-            af_dot4(pair, *reinterpret_cast<const float4*>(qs + g * HD + 4 * c), *reinterpret_cast<const float4*>(ks + af_at<CH>(kk, c)));
-        const float dot = __fadd_rn(pair.x, pair.y);
-        const float slope = sc.slopes != nullptr ? sc.slopes[kvh * G + g] : 0.f;
-        ps[e] = visible(key) ? af_score(dot, sc, slope, key, pos) : -INFINITY;
-    }
-    __syncthreads();
-    // a half warp per head: sixteen lanes with four keys each
-    for (int g = warp * 2 + (lane >> 4); g < ((G + 1) & ~1); g += AF_SPLIT_THREADS / 16) {
-        const int x = lane & 15, row = min(g, G - 1);
-        float s[4], top = -INFINITY;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) s[j] = ps[row * DL_PAGE + x + 16 * j], top = fmaxf(top, s[j]);
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-        const float base = af_base(top);
-        float sum = 0.f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            s[j] = expf(__fsub_rn(s[j], base));
-            sum = __fadd_rn(sum, s[j]);
+    bool asked = false;                                    // the queries are asked for behind the first page
+    for (int page = blockIdx.x; page < end; page += gridDim.x) {
+        const int key0 = page * DL_PAGE;
+        const size_t part0 = ((size_t)t * nh + kvh * G) * bt_stride + page;      // head g's: + g * bt_stride
+        const int id = block_table[(size_t)token_seq[t] * bt_stride + page];
+        if (!af_sees(key0, pos, first, kept) || id < 0 || id >= n_pages) {      // nothing here for this token
+            for (int g = tid; g < G; g += AF_SPLIT_THREADS) part_ml[(part0 + (size_t)g * bt_stride) * 2 + 1] = -1.f;
+            continue;
         }
+        auto visible = [&](int key) { return key <= pos && (key >= first || key < kept); };
+        const float* ksrc = k_pool + dl_k_offset(id, nkv, kvh, 0, HD);
+        for (int e = tid; e < DL_PAGE * CH; e += AF_SPLIT_THREADS) af_copy16(ks + af_at<CH>(e / CH, e % CH), ksrc + 4 * e, visible(key0 + e / CH));
+        af_commit();
+        const float* vsrc = v_pool + dl_v_offset(id, nkv, kvh, 0, HD);
+        for (int e = tid; e < HD * 16; e += AF_SPLIT_THREADS) af_copy16(vs + af_at<16>(e / 16, e % 16), vsrc + 4 * e, key0 + 4 * (e % 16) <= pos);
+        af_commit();
+        for (int e = asked ? G * HD : tid; e < G * HD; e += AF_SPLIT_THREADS) qs[e] = q[(size_t)t * q_stride + (size_t)kvh * G * HD + e];
+        asked = true;
+        af_wait<1>();
+        __syncthreads();
+        for (int e = tid; e < G * DL_PAGE; e += AF_SPLIT_THREADS) {
+            const int g = e / DL_PAGE, kk = e % DL_PAGE, key = key0 + kk;
+            float2 pair = make_float2(0.f, 0.f);
+#pragma unroll 8
+            for (int c = 0; c < CH; ++c)
+                af_dot4(pair, *reinterpret_cast<const float4*>(qs + g * HD + 4 * c), *reinterpret_cast<const float4*>(ks + af_at<CH>(kk, c)));
+            const float dot = __fadd_rn(pair.x, pair.y);
+            const float slope = sc.slopes != nullptr ? sc.slopes[kvh * G + g] : 0.f;
+            ps[e] = visible(key) ? af_score(dot, sc, slope, key, pos) : -INFINITY;
+        }
+        __syncthreads();
+        // a half warp per head: sixteen lanes with four keys each
+        for (int g = warp * 2 + (lane >> 4); g < ((G + 1) & ~1); g += AF_SPLIT_THREADS / 16) {
+            const int x = lane & 15, row = min(g, G - 1);
+            float s[4], top = -INFINITY;
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, o));
-        __syncwarp();
-        if (g < G) {
+            for (int j = 0; j < 4; ++j) s[j] = ps[row * DL_PAGE + x + 16 * j], top = fmaxf(top, s[j]);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) ps[g * DL_PAGE + x + 16 * j] = s[j];
-            if (x == 0) {
-                float* ml = part_ml + (part0 + (size_t)g * bt_stride) * 2;
-                ml[0] = top, ml[1] = sum;
+            for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+            const float base = af_base(top);
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                s[j] = expf(__fsub_rn(s[j], base));
+                sum = __fadd_rn(sum, s[j]);
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, o));
+            __syncwarp();
+            if (g < G) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) ps[g * DL_PAGE + x + 16 * j] = s[j];
+                if (x == 0) {
+                    float* ml = part_ml + (part0 + (size_t)g * bt_stride) * 2;
+                    ml[0] = top, ml[1] = sum;
+                }
             }
         }
-    }
-    af_wait<0>();
-    __syncthreads();
-    const bool whole = key0 + DL_PAGE - 1 <= pos && (key0 >= first || key0 + DL_PAGE <= kept);
+        af_wait<0>();
+        __syncthreads();
+        const bool whole = key0 + DL_PAGE - 1 <= pos && (key0 >= first || key0 + DL_PAGE <= kept);
 #pragma unroll
-    for (int a = 0; a < PAIRS; ++a) {
-        const int e = tid + a * AF_SPLIT_THREADS;
-        if (e >= G * HD) continue;
-        const int g = e / HD, d = e % HD;
-        float2 o = make_float2(0.f, 0.f);
+        for (int a = 0; a < PAIRS; ++a) {
+            const int e = tid + a * AF_SPLIT_THREADS;
+            if (e >= G * HD) continue;
+            const int g = e / HD, d = e % HD;
+            float2 o = make_float2(0.f, 0.f);
 #pragma unroll 8
-        for (int kc = 0; kc < 16; ++kc) {
-            const float4 vv = *reinterpret_cast<const float4*>(vs + af_at<16>(d, kc));
-            const float4 pp = *reinterpret_cast<const float4*>(ps + g * DL_PAGE + 4 * kc);
-            if (whole) {
-                af_dot4(o, pp, vv);
-            } else {                                       // a value nobody may see may hold anything
-                const int key = key0 + 4 * kc;
-                if (visible(key)) o.x = fmaf(pp.x, vv.x, o.x);
-                if (visible(key + 1)) o.y = fmaf(pp.y, vv.y, o.y);
-                if (visible(key + 2)) o.x = fmaf(pp.z, vv.z, o.x);
-                if (visible(key + 3)) o.y = fmaf(pp.w, vv.w, o.y);
+            for (int kc = 0; kc < 16; ++kc) {
+                const float4 vv = *reinterpret_cast<const float4*>(vs + af_at<16>(d, kc));
+                const float4 pp = *reinterpret_cast<const float4*>(ps + g * DL_PAGE + 4 * kc);
+                if (whole) {
+                    af_dot4(o, pp, vv);
+                } else {                                       // a value nobody may see may hold anything
+                    const int key = key0 + 4 * kc;
+                    if (visible(key)) o.x = fmaf(pp.x, vv.x, o.x);
+                    if (visible(key + 1)) o.y = fmaf(pp.y, vv.y, o.y);
+                    if (visible(key + 2)) o.x = fmaf(pp.z, vv.z, o.x);
+                    if (visible(key + 3)) o.y = fmaf(pp.w, vv.w, o.y);
+                }
             }
+            part_o[(part0 + (size_t)g * bt_stride) * HD + d] = __fadd_rn(o.x, o.y);
         }
-        part_o[(part0 + (size_t)g * bt_stride) * HD + d] = __fadd_rn(o.x, o.y);
+        __syncthreads();                                       // the page has been used
     }
 }
 
@@ -490,7 +498,8 @@ extern "C" int dl_attention_f32_split(const float* q, int q_stride, float* out, 
     DL_REQUIRE(part_o != nullptr && part_ml != nullptr && ((uintptr_t)part_ml % 8) == 0, "attention_f32_split: no room for the pages' parts");
     if (n_tokens == 0) return DL_OK;
     const AfScore sc = {scale, softcap, slopes, window, keep_first};
-    const dim3 grid(bt_stride, nkv, n_tokens), block(AF_SPLIT_THREADS);
+    const long fill = (16L * dl_sm_count() + (long)nkv * n_tokens - 1) / ((long)nkv * n_tokens);     // some three times what the machine holds at once
+    const dim3 grid(bt_stride < fill ? bt_stride : (unsigned)(fill > 1 ? fill : 1), nkv, n_tokens), block(AF_SPLIT_THREADS);
     const int smem = (2 * DL_PAGE * hd + G * hd + G * DL_PAGE) * 4, most = (2 * DL_PAGE * hd + AF_MAX_GROUP * (hd + DL_PAGE)) * 4;
     cudaStream_t s = (cudaStream_t)stream;
     const int pairs = (G * hd + AF_SPLIT_THREADS - 1) / AF_SPLIT_THREADS;

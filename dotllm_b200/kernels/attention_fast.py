@@ -234,7 +234,7 @@ F32_TILE_ROWS = 64                   # AF_ROWS
 # 208 us, 32 after 1,500 60 against 208, 32 after 200 20 against 40; a token's pages are read again for every token, so where tiles
 # fill the machine the line is lower.
 F32_SPLIT_TOKENS, F32_SPLIT_TOKENS_FEW, F32_FULL_BLOCKS = 8, 32, 148
-F32_PARTS_BYTES = 1 << 30            # most room the pages' parts of a launch may take (head_dim + 2 floats a token, head and page); more tokens: more launches
+F32_PARTS_BYTES = 256 << 20          # most room the pages' parts of a launch may take (head_dim + 2 floats a token, head and page); more tokens: more launches
 
 
 def run_f32(q, q_stride, out, k_pool, v_pool, n_pages, token_seq, token_pos, block_table, n_heads, n_kv_heads, head_dim, scale, window, plan,

@@ -189,3 +189,38 @@ def test_a_few_tokens_in_several_launches(monkeypatch, tokens_at_once):
     whole = case.run(starts, news, gates=gates)
     monkeypatch.setattr(attention_fast, "F32_PARTS_BYTES", tokens_at_once * 4 * nh * case.table.shape[1] * (hd + 2) + 3)
     assert all(torch.equal(a, b) for a, b in zip(whole, case.run(starts, news, gates=gates)))
+
+
+def test_blocks_that_walk_several_pages():
+    """So many tokens and pages that a block takes more than one: the bits of the whole prompts."""
+    case = Case([2500, 2450, 70, 2500, 1900], 4, 2, 64, seed=6)
+    for kw in ({}, dict(window=700, keep_first=70)):
+        whole = case.run([0] * 5, case.lens, **kw)
+        starts = [n - 8 for n in case.lens]
+        assert 2 * 40 * case.table.shape[1] > 16 * 148
+        assert all(torch.equal(a, b[-8:]) for a, b in zip(case.run(starts, [8] * 5, **kw), whole))
+
+
+def test_a_wide_table_costs_nothing():
+    """Short sequences in a step whose tables are as wide as a long one's (a captured step keeps its width): the columns beyond cost no time."""
+    n = 64
+    case = Case([30] * n, 8, 8, 64, seed=7)
+
+    def time():
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            a.record()
+            out = case.run([29] * n, [1] * n)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return sorted(times)[2], out
+
+    narrow, out = time()
+    case.table = torch.cat([case.table, torch.full((n, 2500), -1, dtype=torch.int32, device=DEV)], dim=1).contiguous()
+    wide, got = time()
+    print(f"observed: {narrow * 1e3:.0f} us, a table of 2,500 columns more {wide * 1e3:.0f} us")
+    assert all(torch.equal(a, b) for a, b in zip(out, got))
+    assert wide < narrow + 0.4                                 # (blocks for 1.3 million columns: some 2 ms)
