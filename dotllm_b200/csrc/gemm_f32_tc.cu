@@ -16,9 +16,11 @@
 // blocks of 32), segments in ascending order.  Any number of rows, any tile of tokens and any cut of the segments between blocks
 // gives the same bits; the 32-bit path relies on that (a prompt in one step, in portions or token by token).
 //
-// A result that is not finite - an infinity or a NaN went in, a piece or a sum overflowed - is computed again as one chain of
-// fused multiply-adds, so those outputs are the FFMA kernels'.  Values below about 1e-33 lose low bits (their last piece would
-// be smaller than any bfloat16).
+// Values are multiplied by 2^24 as they are split and the sums by 2^-48 at the end, all of it exact: without it the last piece of a
+// value below about 1e-33 would be smaller than any bfloat16, now even the smallest float32 keeps its bits.
+//
+// A result that is not finite - an infinity or a NaN went in, a piece (of a value above 2e31) or a sum (above 1e24) overflowed - is
+// computed again as one chain of fused multiply-adds, so those outputs are the FFMA kernels'.
 //
 // Shape: 128 rows of W are the MMA's M and up to 128 tokens its N, so that a step of any number of rows runs the same
 // arithmetic and W, four bytes a value, is read once per tile of tokens.  The three pieces of x lie behind one another in shared
@@ -98,8 +100,12 @@ __device__ __noinline__ float ft_chain(const FtWork& wk, int m, int n) {
 }
 __device__ __forceinline__ bool ft_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
 
-// Two values into their three pieces, packed as bfloat16 pairs (first value in the low half).
+#define FT_SCALE 16777216.f              // 2^24: of every value that is split
+#define FT_UNSCALE 3.5527136788005009e-15f   // 2^-48: of a sum of products of two such values
+
+// Two values (times FT_SCALE) into their three pieces, packed as bfloat16 pairs (first value in the low half).
 __device__ __forceinline__ void ft_split2(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    asm("{\n\t.reg .b64 v, s;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 s, {%2, %2};\n\tmul.rn.f32x2 v, v, s;\n\tmov.b64 {%0, %1}, v;\n\t}" : "+f"(a), "+f"(b) : "f"(FT_SCALE));
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     hi = *reinterpret_cast<const uint32_t*>(&h);
     a -= __uint_as_float(hi << 16);
@@ -155,8 +161,7 @@ __global__ void __launch_bounds__(256) ft_reduce_kernel(const FtWork wk) {
 #pragma unroll
     for (int j = 1; j < FT_SEGMENTS; ++j)
         if (j < wk.segments) total += v[j];
-    if (!ft_finite(total)) total = ft_chain(wk, m, n);
-    wk.y[(size_t)m * wk.y_stride + n] = total;
+    wk.y[(size_t)m * wk.y_stride + n] = ft_finite(total) ? total * FT_UNSCALE : ft_chain(wk, m, n);
 }
 
 // 8 values of a row: read from two 16-byte pieces of a raw tile (128-byte swizzle), written as one 16-byte piece of each operand tile.
@@ -458,7 +463,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 #pragma unroll
                     for (int i = 0; i < COLS; ++i) {
                         fine = fine && ft_finite(sum[i]);
-                        if (n < wk.N && m0 + i < wk.M) dst[(size_t)i * wk.y_stride] = sum[i];
+                        if (n < wk.N && m0 + i < wk.M) dst[(size_t)i * wk.y_stride] = sum[i] * FT_UNSCALE;
                     }
                     if (!fine && n < wk.N) {                  // (columns beyond M may hold anything: their rows are not written)
 #pragma unroll 1

@@ -76,3 +76,16 @@ def test_small_and_large_values_keep_their_digits():
         xs, ws = x * sx, w * sw
         err = (ops.linear(xs, ws).double() - xs.double() @ ws.double().T).abs()
         assert bool((err <= bound(xs, ws)).all())
+
+
+@pytest.mark.parametrize("M", [1, 24, 50, 200])
+@pytest.mark.parametrize("sx,sw", [(1e-36, 1.0), (1.0, 1e-35), (1.0, 2e-37), (1e-18, 1e-17), (1e-34, 1e3), (3e30, 1e-34), (2e-38, 2e4)])
+def test_the_smallest_values_keep_their_digits(M, sx, sw):
+    """Down to numbers below the normal ones: every bit of a value counts (the result's own rounding may be that of such a number)."""
+    from dotllm_b200.kernels import ops
+    x, w = make(M, 144, 1024, seed=7)
+    xs, ws = x * sx, w * sw
+    want = xs.double() @ ws.double().T
+    err = (ops.linear(xs, ws).double() - want).abs()
+    assert bool((err <= bound(xs, ws) + 2.0 ** -149).all())
+    assert float(err.norm() / want.norm()) < 5e-7
