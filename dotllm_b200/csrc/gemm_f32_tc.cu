@@ -20,7 +20,8 @@
 // value below about 1e-33 would be smaller than any bfloat16, now even the smallest float32 keeps its bits.
 //
 // A result that is not finite - an infinity or a NaN went in, a piece (of a value above 2e31) or a sum (above 1e24) overflowed - is
-// computed again as one chain of fused multiply-adds, so those outputs are the FFMA kernels'.
+// computed again as one chain of fused multiply-adds, so those outputs are the FFMA kernels'.  A block does that with all its
+// threads, tile by tile through shared memory, once its pipeline has ended (of cut tiles, the blocks that sum them).
 //
 // Shape: 128 rows of W are the MMA's M and up to 128 tokens its N, so that a step of any number of rows runs the same
 // arithmetic and W, four bytes a value, is read once per tile of tokens.  The three pieces of x lie behind one another in shared
@@ -91,13 +92,6 @@ struct FtWork {
     int units;                          // row_tiles * token_tiles * parts
 };
 
-__device__ __noinline__ float ft_chain(const FtWork& wk, int m, int n) {
-    const float* a = wk.x + (size_t)m * wk.x_stride;
-    const float* b = wk.w + (size_t)n * wk.K;
-    float acc = 0.f;
-    for (int k = 0; k < wk.K; ++k) acc = fmaf(a[k], b[k], acc);
-    return acc;
-}
 __device__ __forceinline__ bool ft_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
 
 #define FT_SCALE 16777216.f              // 2^24: of every value that is split
@@ -146,22 +140,115 @@ ft_split_kernel(const float* __restrict__ x, int x_stride, __nv_bfloat16* __rest
         *reinterpret_cast<uint4*>(planes + ((size_t)s * M + m) * Kp + k) = make_uint4(p[s][0], p[s][1], p[s][2], p[s][3]);
 }
 
-// y = the segments' sums in ascending order (the order in which an uncut tile adds them).
-__global__ void __launch_bounds__(256) ft_reduce_kernel(const FtWork wk) {
+// Rows of `src` (at most `rows` of them, `ld` apart), values k0 .. k0 + 4 `vecs` - 1, into shared memory `pitch` floats apart.
+__device__ __forceinline__ void ft_stage(float* dst, int pitch, const float* src, size_t ld, bool aligned, int rows, int live, int k0, int vecs, int tid,
+                                         int threads) {
+    for (int e = tid; e < rows * vecs; e += threads) {
+        const int r = e / vecs, c = 4 * (e - r * vecs);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < live) {
+            const float* p = src + r * ld + k0 + c;
+            v = aligned ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+        }
+        *reinterpret_cast<float4*>(dst + r * pitch + c) = v;
+    }
+}
+__device__ __forceinline__ float ft_chain4(float acc, const float4& a, const float4& b) {
+    return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
+}
+
+// The outputs of a unit's tile (128 rows of W from row0, NT tokens from token0) that are not finite, as chains over k in ascending order.
+// All threads of the block; `smem`: 128 rows of 36 floats.
+template <int NT>
+__device__ __noinline__ void ft_tile_again(const FtWork& wk, float* smem, int row0, int token0, int tid, int threads) {
+    constexpr int TM = NT < 64 ? NT : 64, TN = 64, PER = TM / 16, PITCH = FT_BK + 4;       // a thread: 4 x PER outputs
+    float* ws = smem;
+    float* xs = ws + TN * PITCH;
+    const int tx = tid & 15, ty = tid >> 4;                // (256 of the threads multiply, all of them stage)
+    const bool aligned = wk.x_stride % 4 == 0 && ((uintptr_t)wk.x % 16) == 0;
+#pragma unroll 1
+    for (int part = 0; part < (FT_BM / TN) * (NT / TM); ++part) {
+        const int n0 = row0 + (part % (FT_BM / TN)) * TN, m0 = token0 + (part / (FT_BM / TN)) * TM;
+        auto place = [&](int i, int j, float*& y) {        // the thread's output (i, j), if there is one
+            const int n = n0 + tx + 16 * i, m = m0 + ty + 16 * j;
+            y = wk.y + (size_t)m * wk.y_stride + n;
+            return tid < 256 && n < wk.N && m < wk.M;
+        };
+        bool fine = true;
+        float* y;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < PER; ++j)
+                if (place(i, j, y)) fine = fine && ft_finite(*y);
+        if (!__syncthreads_or(!fine)) continue;
+        float acc[4][PER];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < PER; ++j) acc[i][j] = 0.f;
+        for (int k0 = 0; k0 < wk.K; k0 += FT_BK) {         // K is a multiple of 4
+            const int vecs = min(FT_BK, wk.K - k0) / 4;
+            ft_stage(ws, PITCH, wk.w + (size_t)n0 * wk.K, wk.K, true, TN, wk.N - n0, k0, vecs, tid, threads);
+            ft_stage(xs, PITCH, wk.x + (size_t)m0 * wk.x_stride, wk.x_stride, aligned, TM, wk.M - m0, k0, vecs, tid, threads);
+            __syncthreads();
+            if (tid < 256) {
+                for (int c = 0; c < vecs; ++c) {
+                    float4 xv[PER];
+#pragma unroll
+                    for (int j = 0; j < PER; ++j) xv[j] = *reinterpret_cast<const float4*>(xs + (ty + 16 * j) * PITCH + 4 * c);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float4 wv = *reinterpret_cast<const float4*>(ws + (tx + 16 * i) * PITCH + 4 * c);
+#pragma unroll
+                        for (int j = 0; j < PER; ++j) acc[i][j] = ft_chain4(acc[i][j], xv[j], wv);
+                    }
+                }
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < PER; ++j)
+                if (place(i, j, y) && !ft_finite(*y)) *y = acc[i][j];
+    }
+}
+
+// One output as a chain over k in ascending order, four values at a time (K is a multiple of 4).  No shared memory: the kernel that calls it
+// starts beside the product's blocks, which leave none.
+__device__ __noinline__ float ft_chain(const FtWork& wk, int m, int n) {
+    const float* a = wk.x + (size_t)m * wk.x_stride;
+    const float* b = wk.w + (size_t)n * wk.K;
+    float acc = 0.f;
+    if (((uintptr_t)a % 16) == 0) {
+#pragma unroll 8
+        for (int k = 0; k < wk.K; k += 4) acc = ft_chain4(acc, __ldg(reinterpret_cast<const float4*>(a + k)), __ldg(reinterpret_cast<const float4*>(b + k)));
+    } else {
+        for (int k = 0; k < wk.K; k += 4) acc = ft_chain4(acc, make_float4(a[k], a[k + 1], a[k + 2], a[k + 3]), __ldg(reinterpret_cast<const float4*>(b + k)));
+    }
+    return acc;
+}
+
+// y = the segments' sums in ascending order (the order in which an uncut tile adds them).  A block: 256 / tm outputs of each of tm = 2^log_tm tokens
+// (chains of neighbours share the rows they read).
+#define FT_REDUCE_THREADS 256
+__global__ void __launch_bounds__(FT_REDUCE_THREADS) ft_reduce_kernel(const FtWork wk, int log_tm) {
     dl_launch_dependents();
     dl_grid_dependency_wait();
-    const long idx = (long)blockIdx.x * 256 + threadIdx.x;
-    if (idx >= (long)wk.M * wk.N) return;
-    const int m = (int)(idx / wk.N), n = (int)(idx % wk.N);
-    const size_t step = (size_t)wk.M * wk.N;
-    float v[FT_SEGMENTS];
+    const int tid = threadIdx.x, log_tn = 8 - log_tm;      // 256 threads
+    const int n = (blockIdx.x << log_tn) + (tid & ((1 << log_tn) - 1));
+    for (long m = ((long)blockIdx.y << log_tm) + (tid >> log_tn); m < wk.M && n < wk.N; m += (long)gridDim.y << log_tm) {
+        const size_t step = (size_t)wk.M * wk.N, at = (size_t)m * wk.N + n;
+        float v[FT_SEGMENTS];
 #pragma unroll
-    for (int j = 0; j < FT_SEGMENTS; ++j) v[j] = j < wk.segments ? __ldcg(wk.sums + j * step + idx) : 0.f;
-    float total = v[0];
+        for (int j = 0; j < FT_SEGMENTS; ++j) v[j] = j < wk.segments ? __ldcg(wk.sums + j * step + at) : 0.f;
+        float total = v[0];
 #pragma unroll
-    for (int j = 1; j < FT_SEGMENTS; ++j)
-        if (j < wk.segments) total += v[j];
-    wk.y[(size_t)m * wk.y_stride + n] = ft_finite(total) ? total * FT_UNSCALE : ft_chain(wk, m, n);
+        for (int j = 1; j < FT_SEGMENTS; ++j)
+            if (j < wk.segments) total += v[j];
+        wk.y[(size_t)m * wk.y_stride + n] = ft_finite(total) ? total * FT_UNSCALE : ft_chain(wk, (int)m, n);
+    }
 }
 
 // 8 values of a row: read from two 16-byte pieces of a raw tile (128-byte swizzle), written as one 16-byte piece of each operand tile.
@@ -217,11 +304,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     __shared__ uint64_t raw_full[FT_MAX_RING], raw_empty[FT_MAX_RING], x_full[FT_MAX_RING], x_empty[FT_MAX_RING];
     __shared__ uint64_t split_full[3], split_empty[3], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_holder;
-    __shared__ volatile int gave_up;
+    __shared__ volatile int gave_up, odd;                     // odd: an output is not finite
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
-        gave_up = 0;
+        gave_up = 0, odd = 0;
         for (int s = 0; s < RAW; ++s) tc_mbar_init(&raw_full[s], 1), tc_mbar_init(&raw_empty[s], FT_GROUP_WARPS);
         for (int s = 0; s < XR; ++s) tc_mbar_init(&x_full[s], 1), tc_mbar_init(&x_empty[s], 1);
         for (int s = 0; s < GROUPS; ++s) tc_mbar_init(&split_full[s], FT_GROUP_WARPS), tc_mbar_init(&split_empty[s], 1);
@@ -465,11 +552,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                         fine = fine && ft_finite(sum[i]);
                         if (n < wk.N && m0 + i < wk.M) dst[(size_t)i * wk.y_stride] = sum[i] * FT_UNSCALE;
                     }
-                    if (!fine && n < wk.N) {                  // (columns beyond M may hold anything: their rows are not written)
-#pragma unroll 1
-                        for (int i = 0; i < COLS; ++i)
-                            if (m0 + i < wk.M && !ft_finite(dst[(size_t)i * wk.y_stride])) dst[(size_t)i * wk.y_stride] = ft_chain(wk, m0 + i, n);
-                    }
+                    if (!fine) odd = 1;                       // (or a column beyond M, which may hold anything: then nothing is found)
                 }
             }
         }
@@ -478,6 +561,15 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     __syncthreads();
     tc_fence_after();
     if (warp == 1) tc_tmem_free(tmem, TMEM_COLS);
+    if (odd && !gave_up) {
+        static_assert(RAW * RAW_STAGE >= 128 * (FT_BK + 4) * 4, "ft_tile_again's rows lie where the copies' ring was");
+#pragma unroll 1
+        for (int u = blockIdx.x; u < wk.units; u += gridDim.x) {
+            int row0, token0, s0, s1, b0, b1;
+            unit_of(u, row0, token0, s0, s1, b0, b1);
+            ft_tile_again<NT>(wk, reinterpret_cast<float*>(base), row0, token0, threadIdx.x, FtShape<NT>::THREADS);
+        }
+    }
 }
 
 static int ft_tokens(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128; }
@@ -567,8 +659,9 @@ extern "C" int dl_gemm_f32_tc(const float* x, int x_stride, const float* w, floa
     else e = ft_launch<128>(mw, mx, wk, resident, grid, status, s);
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "gemm_f32_tc: %s", cudaGetErrorString(e));
     if (wk.parts > 1) {
-        const long n = (long)M * N;
-        e = dl_launch_dependent(ft_reduce_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, wk);
+        const int log_tm = M >= 16 ? 4 : M >= 8 ? 3 : M >= 4 ? 2 : M >= 2 ? 1 : 0, tm = 1 << log_tm, tn = FT_REDUCE_THREADS / tm;
+        const int rows = (M + tm - 1) / tm;
+        e = dl_launch_dependent(ft_reduce_kernel, dim3((N + tn - 1) / tn, rows < 65535 ? rows : 65535), dim3(FT_REDUCE_THREADS), 0, s, wk, log_tm);
         if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "gemm_f32_tc: %s", cudaGetErrorString(e));
     }
     return DL_OK;

@@ -89,3 +89,36 @@ def test_the_smallest_values_keep_their_digits(M, sx, sw):
     err = (ops.linear(xs, ws).double() - want).abs()
     assert bool((err <= bound(xs, ws) + 2.0 ** -149).all())
     assert float(err.norm() / want.norm()) < 5e-7
+
+
+@pytest.mark.parametrize("M,N,K", [(700, 2048, 2048), (700, 2500, 516), (300, 1024, 8192), (40, 4096, 2048), (8, 2048, 2048), (1, 2048, 1024)])
+def test_results_that_are_not_finite_cost_an_ffma_product(M, N, K):
+    """Every output infinite: the bits of the FFMA kernel, and a few of its times on top of this one's (not thousands of loads one after the other)."""
+    from dotllm_b200.kernels import library, ops
+    x, w = make(M, N, K, seed=9)
+    bad = x.clone()
+    bad[:, K - 3] = float("inf")
+    chain = torch.empty(M, N, device=DEV)
+
+    def ffma(x):
+        library.call("dl_gemm_f32", x.data_ptr(), K, w.data_ptr(), chain.data_ptr(), N, M, N, K, library.current_stream())
+
+    def time(f):
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            a.record()
+            f()
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return sorted(times[3:])[2]
+
+    y = ops.linear(bad, w)
+    ffma(bad)
+    assert torch.equal(y.nan_to_num(nan=1.25), chain.nan_to_num(nan=1.25)) and not bool(torch.isfinite(y).any())
+    library.check_status()
+    finite, infinite, product = time(lambda: ops.linear(x, w)), time(lambda: ops.linear(bad, w)), time(lambda: ffma(x))
+    print(f"observed {M} x {N} x {K}: finite {finite * 1e3:.0f} us, not finite {infinite * 1e3:.0f}, FFMA {product * 1e3:.0f}")
+    assert infinite < finite + 10 * product                    # (8 rows: 7.8 times; a cut tile's chains are single lanes' and read rows of W side by side)
