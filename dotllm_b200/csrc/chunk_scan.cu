@@ -93,19 +93,17 @@ __device__ __forceinline__ void ck_product(float (&acc)[RN][N], const float* a, 
     }
 }
 
-// One row of a product once more, over its first n values k alone (in ck_product's order), from the sum `from`: for an output that is not finite.
+// One row of a product once more, over its first n values k alone (in ck_product's order), from the sums at `from` (distance `apart`; NULL:
+// from 0): for an output that is not finite.  Rare, so one value after the other: it must not cost the kernels registers.
 template <int N, int LDB>
-__device__ __noinline__ void ck_row_again(float* dst, const float* a, const float* b, int n, typename CkVec<N>::type from) {
-    float acc[N];
-#pragma unroll
-    for (int e = 0; e < N; ++e) acc[e] = reinterpret_cast<const float*>(&from)[e];
-    for (int k = 0; k < n; ++k) {
-        float bv[N];
-        ck_load<N>(b + k * LDB, bv);
-#pragma unroll
-        for (int e = 0; e < N; ++e) acc[e] = fmaf(a[k], bv[e], acc[e]);
+__device__ __forceinline__ void ck_row_again(float* dst, const float* a, const float* b, int n, const float* from, int apart) {
+#pragma unroll 1
+    for (int e = 0; e < N; ++e) {
+        float acc = from != nullptr ? from[e * apart] : 0.f;
+#pragma unroll 1
+        for (int k = 0; k < n; ++k) acc = fmaf(a[k], b[k * LDB + e], acc);
+        dst[e] = acc;
     }
-    ck_store<N>(dst, acc);
 }
 template <int N>
 __device__ __forceinline__ bool ck_all_finite(const float (&v)[N]) {
@@ -116,13 +114,36 @@ __device__ __forceinline__ bool ck_all_finite(const float (&v)[N]) {
 }
 
 // What the kernels have of a chunk.
+//
+// Chunks of all sequences lie one behind the other: chunk c of sequence b is piece ck_piece0(b) + c.  With ck_piece0(b) = floor((cu_new[b] +
+// 31 b) / 32) a sequence of n tokens has at least ceil(n / 32) pieces before the next one's, and all have at most floor((tokens +
+// 31 sequences) / 32) in all, which the host knows without reading cu_new.  The operands of a window of pieces (`lo` .. `lo` + n - 1)
+// lie in the scratch at a time: what it holds follows the tokens, whatever the sequences' lengths.
 struct CkRange {
     int t0, n, first, count, slot;       // the sequence's first row, its tokens, the chunk's first of them and how many, the slot
 };
-__device__ __forceinline__ bool ck_range(CkRange& r, const int32_t* cu_new, const int32_t* slots, int n_slots, int b, int chunk) {
-    r.t0 = cu_new[b], r.n = cu_new[b + 1] - r.t0, r.first = chunk * CK_L, r.slot = slots[b];
-    r.count = min(CK_L, r.n - r.first);
-    return r.first < r.n && r.slot >= 0 && r.slot < n_slots;
+__device__ __forceinline__ bool ck_sequence(CkRange& r, const int32_t* cu_new, const int32_t* slots, int n_slots, int b) {
+    r.t0 = cu_new[b], r.n = cu_new[b + 1] - r.t0, r.first = 0, r.count = min(CK_L, r.n), r.slot = slots[b];
+    return r.n > 0 && r.slot >= 0 && r.slot < n_slots;
+}
+__device__ __forceinline__ int ck_piece0(int cu, int b) { return (int)(((unsigned)cu + (CK_L - 1) * (unsigned)b) / CK_L); }
+// The chunk of a piece (every warp searches for itself: 32 sequences at a time, what it needs of them asked for at once); false where the
+// piece holds none.
+__device__ __forceinline__ bool ck_find(CkRange& r, const int32_t* cu_new, const int32_t* slots, int n_slots, int n_seqs, int piece, int lane) {
+    int b = 0, step = 1;
+    while (step * 32 < n_seqs) step *= 32;
+    for (;;) {                                             // the last sequence whose first piece is not behind this one
+        const int i = b + lane * step, at = min(i, n_seqs - 1);
+        const int cu = cu_new[at], cu1 = cu_new[at + 1], slot = slots[at];
+        const int w = __popc(__ballot_sync(0xffffffffu, i < n_seqs && ck_piece0(cu, i) <= piece)) - 1;
+        b += w * step;
+        if (step == 1) {
+            r.t0 = __shfl_sync(0xffffffffu, cu, w), r.n = __shfl_sync(0xffffffffu, cu1, w) - r.t0, r.slot = __shfl_sync(0xffffffffu, slot, w);
+            r.first = (piece - ck_piece0(r.t0, b)) * CK_L, r.count = min(CK_L, r.n - r.first);
+            return r.first < r.n && r.slot >= 0 && r.slot < n_slots;
+        }
+        step /= 32;
+    }
 }
 
 // Lane j of a warp: its key, decayed step by step, against every later token's query (aq) and key (ak): sixteen channels a warp.
@@ -181,12 +202,12 @@ __device__ __forceinline__ void ck_queries_from_start(float* q, const float* a) 
 }
 
 // ------------------------------------------------------------ the delta rule
-// A block per (chunk, head, sequence): G.  q, k [tokens, G*dim] (unit vectors, q scaled), g [tokens, H*dim] the decays, beta [tokens, H].
+// A block per (piece of the window, head): G.  q, k [tokens, G*dim] (unit vectors, q scaled), g [tokens, H*dim] the decays, beta [tokens, H].
 #define CK_DELTA_SMEM ((3 * CK_DIM * CK_LDT + 4 * CK_L * CK_L + 2 * CK_L * CK_LDT + CK_L + CK_DIM) * 4)
 __global__ void __launch_bounds__(CK_THREADS, 4)
 delta_chunk_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ g, const float* __restrict__ beta,
-                           const int32_t* __restrict__ cu_new, const int32_t* __restrict__ slots, int n_slots, float* __restrict__ G, int H, int group,
-                           int dim, int n_chunks) {
+                           const int32_t* __restrict__ cu_new, const int32_t* __restrict__ slots, int n_slots, int n_seqs, float* __restrict__ G, int H,
+                           int group, int dim, int lo) {
     extern __shared__ __align__(16) float ck_smem[];
     float* sq = ck_smem;                                   // [64][LDT]: q, then Q+, by channel
     float* sk = sq + CK_DIM * CK_LDT;                      // k, then K'
@@ -199,9 +220,9 @@ delta_chunk_prepare_kernel(const float* __restrict__ q, const float* __restrict_
     static_assert(CK_L * CK_LDX <= 4 * CK_L * CK_L, "W and T lie where the shares were");
     dl_launch_dependents();
     dl_grid_dependency_wait();
-    const int chunk = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kvh = h / group;
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kvh = h / group;
     CkRange r;
-    if (!ck_range(r, cu_new, slots, n_slots, b, chunk)) return;
+    if (!ck_find(r, cu_new, slots, n_slots, n_seqs, lo + blockIdx.x, lane)) return;
     for (int e = tid; e < CK_L * CK_DIM; e += CK_THREADS) {
         const int t = e / CK_DIM, c = e % CK_DIM;
         float qv = 0.f, kv = 0.f, av = t < r.count ? 0.f : 1.f;    // a token that is not there decays nothing and adds nothing
@@ -263,7 +284,7 @@ delta_chunk_prepare_kernel(const float* __restrict__ q, const float* __restrict_
     else ck_queries_from_start(sq + (tid - CK_DIM) * CK_LDT, sa + (tid - CK_DIM) * CK_LDT);
     __syncthreads();
     // G = [diag(P_L) | 0; Q+ | 0] + [K'^T; A] [-W | T]: thread (rg, cg) of 16 x 8 takes rows rg + 16 i, columns 4 cg + 32 p
-    float* out = G + (((long)b * n_chunks + chunk) * H + h) * (CK_X * CK_X);
+    float* out = G + ((long)blockIdx.x * H + h) * (CK_X * CK_X);
     const int rg = tid >> 3, cg = tid & 7;
 #pragma unroll 1
     for (int p = 0; p < 3; ++p) {
@@ -286,22 +307,19 @@ delta_chunk_prepare_kernel(const float* __restrict__ q, const float* __restrict_
             const int t = rg + 16 * i;
             float* dst = out + (CK_DIM + t) * CK_X + col;
             ck_store<4>(dst, low[i]);
-            if (!ck_all_finite(low[i])) {
-                const float* from = sq + col * CK_LDT + t;
-                ck_row_again<4, CK_LDX>(dst, sA + t * CK_LDT, part + col, t + 1,
-                                        col < CK_DIM ? make_float4(from[0], from[CK_LDT], from[2 * CK_LDT], from[3 * CK_LDT]) : make_float4(0.f, 0.f, 0.f, 0.f));
-            }
+            if (!ck_all_finite(low[i]))
+                ck_row_again<4, CK_LDX>(dst, sA + t * CK_LDT, part + col, t + 1, col < CK_DIM ? sq + col * CK_LDT + t : nullptr, CK_LDT);
         }
     }
 }
 
-// The walk: thread (rg, cg) of 16 x 8, rows rg + 16 i of G, columns N cg .. of [S_0; V] (N = CW / 8).  G comes in two halves of its
+// The walk over the window's chunks of a sequence: thread (rg, cg) of 16 x 8, rows rg + 16 i of G, columns N cg .. of [S_0; V] (N = CW / 8).  G comes in two halves of its
 // columns: while one is used the other, or the next chunk's, is under way.
 template <int CW>
 __global__ void __launch_bounds__(CK_THREADS, 3)
 delta_chunk_walk_kernel(const float* __restrict__ v, const float* __restrict__ G, const int32_t* __restrict__ cu_new,
                         const int32_t* __restrict__ slots, float* __restrict__ state, long slot_stride, int n_slots, float* __restrict__ out, int H,
-                        int dim, int vdim, int n_chunks) {
+                        int dim, int vdim, int lo, int n_pieces) {
     constexpr int N = CW / 8, HALF = CK_X / 2;
     extern __shared__ __align__(16) float ck_smem[];
     float* s_g = ck_smem;                                  // [96][LDX]
@@ -310,27 +328,30 @@ delta_chunk_walk_kernel(const float* __restrict__ v, const float* __restrict__ G
     dl_grid_dependency_wait();
     const int tid = threadIdx.x, rg = tid >> 3, cg = tid & 7, h = blockIdx.y, b = blockIdx.z;
     CkRange r;
-    if (!ck_range(r, cu_new, slots, n_slots, b, 0)) return;
+    if (!ck_sequence(r, cu_new, slots, n_slots, b)) return;
+    const int first = ck_piece0(r.t0, b) - lo;             // the sequence's first piece, from the window's
+    const int begin = max(0, -first), end = min((r.n + CK_L - 1) / CK_L, n_pieces - first);      // its chunks in the window
+    if (begin >= end) return;
     const int n = r.n, col = blockIdx.x * CW + N * cg;     // vdim is a multiple of 4: a thread's columns are all there or all beyond
     const bool col_ok = col < vdim;
     float* S = state + (long)r.slot * slot_stride + (long)h * dim * vdim;
     auto bring = [&](int chunk, int half) {
-        const float* src = G + (((long)b * n_chunks + chunk) * H + h) * (CK_X * CK_X) + half * HALF;
+        const float* src = G + ((long)(first + chunk) * H + h) * (CK_X * CK_X) + half * HALF;
         for (int e = tid; e < CK_X * (HALF / 4); e += CK_THREADS)
             ck_copy16(s_g + (e / (HALF / 4)) * CK_LDX + half * HALF + 4 * (e % (HALF / 4)), src + (e / (HALF / 4)) * CK_X + 4 * (e % (HALF / 4)), true);
     };
-    bring(0, 0);
+    bring(begin, 0);
     ck_commit();
-    bring(0, 1);
+    bring(begin, 1);
     ck_commit();
     const float* v_at = v + ((long)r.t0 * H + h) * vdim + col;
     float* o_at = out + ((long)r.t0 * H + h) * vdim + col;
     const long step = (long)H * vdim;
     float vv[2][N], acc[6][N];
-    auto fetch_v = [&](int first) {
+    auto fetch_v = [&](int chunk) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const int t = first + rg + 16 * i;
+            const int t = chunk * CK_L + rg + 16 * i;
             if (t < n && col_ok) ck_load<N>(v_at + t * step, vv[i]);
             else {
 #pragma unroll
@@ -338,21 +359,20 @@ delta_chunk_walk_kernel(const float* __restrict__ v, const float* __restrict__ G
             }
         }
     };
-    fetch_v(0);
+    fetch_v(begin);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int c = rg + 16 * i;
 #pragma unroll
         for (int e = 0; e < N; ++e) acc[i][e] = c < dim && col_ok ? S[(long)c * vdim + col + e] : 0.f;
     }
-    const int chunks = (n + CK_L - 1) / CK_L;
-    for (int chunk = 0; chunk < chunks; ++chunk) {
+    for (int chunk = begin; chunk < end; ++chunk) {
         float* x = s_x + (chunk & 1) * CK_X * CW;
 #pragma unroll
         for (int i = 0; i < 4; ++i) ck_store<N>(x + (rg + 16 * i) * CW + N * cg, acc[i]);
 #pragma unroll
         for (int i = 0; i < 2; ++i) ck_store<N>(x + (CK_DIM + rg + 16 * i) * CW + N * cg, vv[i]);
-        fetch_v((chunk + 1) * CK_L);
+        fetch_v(chunk + 1);
 #pragma unroll
         for (int i = 0; i < 6; ++i)
 #pragma unroll
@@ -361,13 +381,15 @@ delta_chunk_walk_kernel(const float* __restrict__ v, const float* __restrict__ G
         __syncthreads();                                   // G's first half, the state and the values are there
         ck_product<6, N, HALF / 4, CK_LDX, CW>(acc, s_g + rg * CK_LDX, x + N * cg);
         __syncthreads();                                   // G's first half has been used
-        if (chunk + 1 < chunks) bring(chunk + 1, 0);
+        if (chunk + 1 < end) bring(chunk + 1, 0);
         ck_commit();
         ck_wait<1>();
         __syncthreads();                                   // its second half is there
-        typename CkVec<N>::type half_o[2];                 // the outputs so far
+        float half_o[2][N];                                // the outputs so far
 #pragma unroll
-        for (int i = 0; i < 2; ++i) ck_store<N>(reinterpret_cast<float*>(&half_o[i]), acc[4 + i]);
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int e = 0; e < N; ++e) half_o[i][e] = acc[4 + i][e];
         ck_product<6, N, HALF / 4, CK_LDX, CW>(acc, s_g + rg * CK_LDX + HALF, x + HALF * CW + N * cg);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -375,11 +397,13 @@ delta_chunk_walk_kernel(const float* __restrict__ v, const float* __restrict__ G
             if (chunk * CK_L + t >= n || !col_ok) continue;
             float* dst = o_at + (chunk * CK_L + t) * step;
             ck_store<N>(dst, acc[4 + i]);
-            if (!ck_all_finite(acc[4 + i]))
-                ck_row_again<N, CW>(dst, s_g + (CK_DIM + t) * CK_LDX + HALF, x + HALF * CW + N * cg, CK_DIM - HALF + t + 1, half_o[i]);
+            if (!ck_all_finite(acc[4 + i])) {
+                ck_store<N>(dst, half_o[i]);
+                ck_row_again<N, CW>(dst, s_g + (CK_DIM + t) * CK_LDX + HALF, x + HALF * CW + N * cg, CK_DIM - HALF + t + 1, dst, 1);
+            }
         }
         __syncthreads();                                   // and has been used
-        if (chunk + 1 < chunks) bring(chunk + 1, 1);
+        if (chunk + 1 < end) bring(chunk + 1, 1);
         ck_commit();
     }
     ck_wait<0>();
@@ -396,7 +420,7 @@ delta_chunk_walk_kernel(const float* __restrict__ v, const float* __restrict__ G
 // --------------------------------------------------- gated linear attention
 #define CK_GLA_COLS 64                   // value channels that a block's threads take at a time: (rg, cg) of 16 x 16, four columns each
 #define CK_GLA_THREADS 256
-struct CkGla {                           // per (sequence, chunk, head), float32
+struct CkGla {                           // per (piece of the window, head), float32
     float* qa;                           // [L][96]: Q+, then A
     float* end;                          // [64]: P_L
     float* states;                       // [64][vdim]: K'^T V, then the state before the chunk
@@ -419,20 +443,20 @@ __device__ __forceinline__ void ck_bring_v(float* s_v, const T* v, long v_ld, in
     }
 }
 
-// A block per (chunk, head, sequence): Q+, A, P_L and K'^T V.  z, z_bias as in dl_gla_scan.
+// A block per (piece, head): Q+, A, P_L and K'^T V.  z, z_bias as in dl_gla_scan.
 template <typename T>
 __global__ void __launch_bounds__(CK_GLA_THREADS)
 gla_chunk_states_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, long ld, const float* __restrict__ z, long z_ld,
-                        const float* __restrict__ z_bias, const int32_t* __restrict__ cu_new, const int32_t* __restrict__ slots, int n_slots, CkGla out, int H,
-                        int dim, int vdim, float q_scale, float inv_tau, int n_chunks) {
+                        const float* __restrict__ z_bias, const int32_t* __restrict__ cu_new, const int32_t* __restrict__ slots, int n_slots, int n_seqs,
+                        CkGla out, int H, int dim, int vdim, float q_scale, float inv_tau, int lo) {
     __shared__ __align__(16) float sq[CK_DIM * CK_LDT], sk[CK_DIM * CK_LDT], sa[CK_DIM * CK_LDT];
     __shared__ __align__(16) float part[4 * CK_L * CK_L];  // the warps' shares of A; then 64 columns of V
     dl_launch_dependents();
     dl_grid_dependency_wait();
-    const int chunk = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     CkRange r;
-    if (!ck_range(r, cu_new, slots, n_slots, b, chunk)) return;
-    const long piece = ((long)b * n_chunks + chunk) * H + h;
+    if (!ck_find(r, cu_new, slots, n_slots, n_seqs, lo + blockIdx.x, lane)) return;
+    const long piece = (long)blockIdx.x * H + h;
     for (int e = tid; e < CK_L * CK_DIM; e += CK_GLA_THREADS) {
         const int t = e / CK_DIM, c = e % CK_DIM;
         float qv = 0.f, kv = 0.f, av = t < r.count ? 0.f : 1.f;    // a token that is not there decays nothing and adds nothing
@@ -485,31 +509,33 @@ gla_chunk_states_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
 }
 
 // The state before every chunk in place of the chunk's contribution: a thread per four neighbouring values of one (sequence, head).
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 gla_chunk_pass_kernel(CkGla io, const int32_t* __restrict__ cu_new, const int32_t* __restrict__ slots, float* __restrict__ state, int n_slots, int H,
-                      int dim, int vdim, int n_chunks) {
+                      int dim, int vdim, int lo, int n_pieces) {
     dl_launch_dependents();
     dl_grid_dependency_wait();
     const int b = blockIdx.z, h = blockIdx.y, at = (blockIdx.x * 256 + threadIdx.x) * 4, c = at / vdim;
     CkRange r;
-    if (at >= dim * vdim || !ck_range(r, cu_new, slots, n_slots, b, 0)) return;
-    const int chunks = (r.n + CK_L - 1) / CK_L;
+    if (at >= dim * vdim || !ck_sequence(r, cu_new, slots, n_slots, b)) return;
+    const int first = ck_piece0(r.t0, b) - lo;             // the sequence's first piece, from the window's
+    const int begin = max(0, -first), end = min((r.n + CK_L - 1) / CK_L, n_pieces - first);      // its chunks in the window
+    if (begin >= end) return;
     float4* S = reinterpret_cast<float4*>(state + ((long)r.slot * H + h) * dim * vdim + at);
     float4 s = *S;
-    const long piece0 = (long)b * n_chunks * H + h;
+    const long piece0 = (long)first * H + h;
     constexpr int AHEAD = 8;                               // chunks whose contributions are asked for together
-    for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
+    for (int c0 = begin; c0 < end; c0 += AHEAD) {
         float4 x[AHEAD];
         float keep[AHEAD];
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i) {
-            const long piece = piece0 + (long)min(c0 + i, chunks - 1) * H;
+            const long piece = piece0 + (long)min(c0 + i, end - 1) * H;
             x[i] = *reinterpret_cast<const float4*>(io.states + piece * CK_DIM * vdim + at);
             keep[i] = io.end[piece * CK_DIM + c];
         }
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i) {
-            if (c0 + i >= chunks) break;
+            if (c0 + i >= end) break;
             *reinterpret_cast<float4*>(io.states + (piece0 + (long)(c0 + i) * H) * CK_DIM * vdim + at) = s;
             s = make_float4(fmaf(keep[i], s.x, x[i].x), fmaf(keep[i], s.y, x[i].y), fmaf(keep[i], s.z, x[i].z), fmaf(keep[i], s.w, x[i].w));
         }
@@ -517,18 +543,18 @@ gla_chunk_pass_kernel(CkGla io, const int32_t* __restrict__ cu_new, const int32_
     *S = s;
 }
 
-// A block per (chunk, head, sequence): O = [Q+ | A] [S_0; V].
+// A block per (piece, head): O = [Q+ | A] [S_0; V].
 template <typename T>
 __global__ void __launch_bounds__(CK_GLA_THREADS)
 gla_chunk_out_kernel(const T* __restrict__ v, long v_ld, int v_silu, CkGla in, const int32_t* __restrict__ cu_new, const int32_t* __restrict__ slots,
-                     int n_slots, float* __restrict__ out, long out_ld, int H, int dim, int vdim, int n_chunks) {
+                     int n_slots, int n_seqs, float* __restrict__ out, long out_ld, int H, int dim, int vdim, int lo) {
     __shared__ __align__(16) float s_qa[CK_L * CK_LDX], s_x[CK_X * CK_GLA_COLS];
     dl_launch_dependents();
     dl_grid_dependency_wait();
-    const int chunk = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, rg = tid >> 4, cg = tid & 15;
+    const int h = blockIdx.y, tid = threadIdx.x, rg = tid >> 4, cg = tid & 15;
     CkRange r;
-    if (!ck_range(r, cu_new, slots, n_slots, b, chunk)) return;
-    const long piece = ((long)b * n_chunks + chunk) * H + h;
+    if (!ck_find(r, cu_new, slots, n_slots, n_seqs, lo + blockIdx.x, tid & 31)) return;
+    const long piece = (long)blockIdx.x * H + h;
     for (int e = tid; e < CK_L * (CK_X / 4); e += CK_GLA_THREADS)
         ck_copy16(s_qa + (e / (CK_X / 4)) * CK_LDX + 4 * (e % (CK_X / 4)), in.qa + piece * (CK_L * CK_X) + 4 * e, true);
     for (int col0 = 0; col0 < vdim; col0 += CK_GLA_COLS) {
@@ -554,7 +580,7 @@ gla_chunk_out_kernel(const T* __restrict__ v, long v_ld, int v_silu, CkGla in, c
                 float* dst = out + (long)(r.t0 + r.first + rg + 16 * i) * out_ld + (long)h * vdim + col;
                 ck_store<4>(dst, acc[i]);
                 if (!ck_all_finite(acc[i]))
-                    ck_row_again<4, CK_GLA_COLS>(dst, s_qa + (rg + 16 * i) * CK_LDX, s_x + 4 * cg, CK_DIM + rg + 16 * i + 1, make_float4(0.f, 0.f, 0.f, 0.f));
+                    ck_row_again<4, CK_GLA_COLS>(dst, s_qa + (rg + 16 * i) * CK_LDX, s_x + 4 * cg, CK_DIM + rg + 16 * i + 1, nullptr, 0);
             }
         __syncthreads();
     }
@@ -575,76 +601,86 @@ static cudaError_t ck_size(const void* kernel, std::atomic<unsigned long long>& 
 #define CK_CHECK(what)                                                                                                                \
     DL_REQUIRE(n_seqs >= 0 && H > 0 && H <= 65535 && n_seqs <= 65535 && dim > 0 && dim <= CK_DIM && vdim > 0 && vdim % 4 == 0 && n_slots > 0, \
                what ": sizes that the chunks do not take");                                                                           \
-    DL_REQUIRE(n_chunks >= 1 && scratch != nullptr && ((uintptr_t)scratch % 16) == 0, what ": no scratch");                           \
+    DL_REQUIRE(at_once >= 1 && scratch != nullptr && ((uintptr_t)scratch % 16) == 0, what ": no scratch");                            \
     DL_REQUIRE(out_ld % 4 == 0 && ((uintptr_t)out % 16) == 0, what ": unaligned rows");
 
-// Floats of scratch: for the delta rule, and for gated linear attention with values of vdim channels.
-extern "C" int dl_delta_chunk_scratch(int n_seqs, int n_chunks, int H, long long* floats) {
-    *floats = (long long)n_seqs * n_chunks * H * (CK_X * CK_X);
+// Pieces that the chunks of so many tokens and sequences lie in, and floats of scratch for one of them: for the delta rule, and for gated
+// linear attention with values of vdim channels.
+extern "C" int dl_chunk_pieces(int n_tokens, int n_seqs) { return (int)(((long long)n_tokens + (CK_L - 1) * (long long)n_seqs) / CK_L); }
+extern "C" int dl_delta_chunk_scratch(int H, long long* floats) {
+    *floats = (long long)H * (CK_X * CK_X);
     return DL_OK;
 }
-extern "C" int dl_gla_chunk_scratch(int n_seqs, int n_chunks, int H, int vdim, long long* floats) {
-    *floats = (long long)n_seqs * n_chunks * H * (CK_L * CK_X + CK_DIM + (long long)CK_DIM * vdim);
+extern "C" int dl_gla_chunk_scratch(int H, int vdim, long long* floats) {
+    *floats = (long long)H * (CK_L * CK_X + CK_DIM + (long long)CK_DIM * vdim);
     return DL_OK;
 }
 
-// As dl_gla_scan for bfloat16 rows; v's rows 8-byte aligned, the state's and out's rows 16-byte aligned.
+// As dl_gla_scan for bfloat16 rows; v's rows 8-byte aligned, the state's and out's rows 16-byte aligned.  scratch: for `at_once` pieces; where
+// there are more, a window of so many after the other (the states wait in `state` in between: the same bits).
 extern "C" int dl_gla_chunk(const void* q, const void* k, const void* v, int ld, const float* z, int z_stride, const float* z_bias,
                             const int32_t* cu_new, const int32_t* slots, float* state, int n_slots, float* out, int out_ld, float* scratch,
-                            int n_seqs, int n_tokens, int H, int dim, int vdim, float q_scale, float tau, int n_chunks, void* stream) {
+                            int n_seqs, int n_tokens, int H, int dim, int vdim, float q_scale, float tau, int at_once, void* stream) {
     CK_CHECK("gla_chunk");
     DL_REQUIRE(tau > 0.f && out_ld >= H * vdim && (z == nullptr || z_stride >= H * dim), "gla_chunk: bad arguments");
     DL_REQUIRE(ld % 4 == 0 && ((uintptr_t)v % 8) == 0 && ((uintptr_t)state % 16) == 0, "gla_chunk: unaligned values or states");
     if (n_seqs == 0 || n_tokens == 0) return DL_OK;
     cudaStream_t s = (cudaStream_t)stream;
     typedef __nv_bfloat16 T;
-    const long pieces = (long)n_seqs * n_chunks * H;
+    const long long pieces = dl_chunk_pieces(n_tokens, n_seqs), in_scratch = (long long)at_once * H;
     CkGla sc;
     sc.qa = scratch;
-    sc.end = sc.qa + pieces * CK_L * CK_X;
-    sc.states = sc.end + pieces * CK_DIM;
-    const dim3 grid(n_chunks, H, n_seqs);
-    cudaError_t e = dl_launch_dependent(gla_chunk_states_kernel<T>, grid, dim3(CK_GLA_THREADS), 0, s, (const T*)q, (const T*)k, (const T*)v, ld, z, z_stride,
-                                        z_bias, cu_new, slots, n_slots, sc, H, dim, vdim, q_scale, 1.0f / tau, n_chunks);
-    if (e == cudaSuccess)
-        e = dl_launch_dependent(gla_chunk_pass_kernel, dim3((dim * vdim / 4 + 255) / 256, H, n_seqs), dim3(256), 0, s, sc, cu_new, slots, state, n_slots, H,
-                                dim, vdim, n_chunks);
-    if (e == cudaSuccess)
-        e = dl_launch_dependent(gla_chunk_out_kernel<T>, grid, dim3(CK_GLA_THREADS), 0, s, (const T*)v, ld, z == nullptr ? 1 : 0, sc, cu_new, slots, n_slots, out,
-                                out_ld, H, dim, vdim, n_chunks);
+    sc.end = sc.qa + in_scratch * CK_L * CK_X;
+    sc.states = sc.end + in_scratch * CK_DIM;
+    cudaError_t e = cudaSuccess;
+    for (long long lo = 0; lo < pieces && e == cudaSuccess; lo += at_once) {
+        const int n = (int)(pieces - lo < at_once ? pieces - lo : at_once);
+        const dim3 grid(n, H);
+        e = dl_launch_dependent(gla_chunk_states_kernel<T>, grid, dim3(CK_GLA_THREADS), 0, s, (const T*)q, (const T*)k, (const T*)v, ld, z, z_stride,
+                                z_bias, cu_new, slots, n_slots, n_seqs, sc, H, dim, vdim, q_scale, 1.0f / tau, (int)lo);
+        if (e == cudaSuccess)
+            e = dl_launch_dependent(gla_chunk_pass_kernel, dim3((dim * vdim / 4 + 255) / 256, H, n_seqs), dim3(256), 0, s, sc, cu_new, slots, state,
+                                    n_slots, H, dim, vdim, (int)lo, n);
+        if (e == cudaSuccess)
+            e = dl_launch_dependent(gla_chunk_out_kernel<T>, grid, dim3(CK_GLA_THREADS), 0, s, (const T*)v, ld, z == nullptr ? 1 : 0, sc, cu_new, slots,
+                                    n_slots, n_seqs, out, out_ld, H, dim, vdim, (int)lo);
+    }
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "gla_chunk: %s", cudaGetErrorString(e));
     return DL_OK;
 }
 
 template <int CW>
 static cudaError_t ck_walk(const float* v, const float* G, const int32_t* cu_new, const int32_t* slots, float* state, long slot_stride, int n_slots,
-                           float* out, int n_seqs, int H, int dim, int vdim, int n_chunks, cudaStream_t s) {
+                           float* out, int n_seqs, int H, int dim, int vdim, int lo, int n_pieces, cudaStream_t s) {
     constexpr int smem = (CK_X * CK_LDX + 2 * CK_X * CW) * 4;
     static std::atomic<unsigned long long> sized{0};
     const cudaError_t e = ck_size((const void*)delta_chunk_walk_kernel<CW>, sized, smem);
     if (e != cudaSuccess) return e;
     // long-running blocks: they start when the kernel before has ended, spread over all multiprocessors
     return dl_launch_dependent_if(false, delta_chunk_walk_kernel<CW>, dim3((vdim + CW - 1) / CW, H, n_seqs), dim3(CK_THREADS), (size_t)smem, s, v, G, cu_new,
-                                  slots, state, slot_stride, n_slots, out, H, dim, vdim, n_chunks);
+                                  slots, state, slot_stride, n_slots, out, H, dim, vdim, lo, n_pieces);
 }
 
-// The recurrence of dl_delta_rule from its prepared rows: q, k [tokens, G*dim], v [tokens, H*vdim], g [tokens, H*dim], beta [tokens, H], all float32.
+// The recurrence of dl_delta_rule from its prepared rows: q, k [tokens, G*dim], v [tokens, H*vdim], g [tokens, H*dim], beta [tokens, H], all float32.  scratch
+// and at_once as in dl_gla_chunk.
 int dl_delta_chunk(const float* q, const float* k, const float* v, const float* g, const float* beta, const int32_t* cu_new, const int32_t* slots,
                    float* state, long slot_stride, int n_slots, float* out, float* scratch, int n_seqs, int n_tokens, int H, int G, int dim, int vdim,
-                   int n_chunks, cudaStream_t s) {
+                   int at_once, cudaStream_t s) {
     const int out_ld = H * vdim;
     CK_CHECK("delta_chunk");
     DL_REQUIRE(((uintptr_t)v % 16) == 0 && n_tokens >= 0, "delta_chunk: unaligned values");
     static std::atomic<unsigned long long> sized{0};
     cudaError_t e = ck_size((const void*)delta_chunk_prepare_kernel, sized, CK_DELTA_SMEM);
-    if (e == cudaSuccess)
-        e = dl_launch_dependent(delta_chunk_prepare_kernel, dim3(n_chunks, H, n_seqs), dim3(CK_THREADS), (size_t)CK_DELTA_SMEM, s, q, k, g, beta, cu_new, slots,
-                                n_slots, scratch, H, H / G, dim, n_chunks);
-    if (e == cudaSuccess) {
-        // 32 columns a block read G half as often as 16; 16 where 32 would leave multiprocessors without a block
-        const bool wide = (long)((vdim + 31) / 32) * H * n_seqs >= dl_sm_count();
-        e = wide ? ck_walk<32>(v, scratch, cu_new, slots, state, slot_stride, n_slots, out, n_seqs, H, dim, vdim, n_chunks, s)
-                 : ck_walk<16>(v, scratch, cu_new, slots, state, slot_stride, n_slots, out, n_seqs, H, dim, vdim, n_chunks, s);
+    // 32 columns a block read G half as often as 16; 16 where 32 would leave multiprocessors without a block
+    const bool wide = (long)((vdim + 31) / 32) * H * n_seqs >= dl_sm_count();
+    const long long pieces = dl_chunk_pieces(n_tokens, n_seqs);
+    for (long long lo = 0; lo < pieces && e == cudaSuccess; lo += at_once) {
+        const int m = (int)(pieces - lo < at_once ? pieces - lo : at_once);
+        e = dl_launch_dependent(delta_chunk_prepare_kernel, dim3(m, H), dim3(CK_THREADS), (size_t)CK_DELTA_SMEM, s, q, k, g, beta, cu_new, slots, n_slots,
+                                n_seqs, scratch, H, H / G, dim, (int)lo);
+        if (e == cudaSuccess)
+            e = wide ? ck_walk<32>(v, scratch, cu_new, slots, state, slot_stride, n_slots, out, n_seqs, H, dim, vdim, (int)lo, m, s)
+                     : ck_walk<16>(v, scratch, cu_new, slots, state, slot_stride, n_slots, out, n_seqs, H, dim, vdim, (int)lo, m, s);
     }
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "delta_chunk: %s", cudaGetErrorString(e));
     return DL_OK;

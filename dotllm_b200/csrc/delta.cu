@@ -275,7 +275,7 @@ delta_history_kernel(const T* __restrict__ x, int ld, int K, float* __restrict__
 // chunk_scan.cu
 int dl_delta_chunk(const float* q, const float* k, const float* v, const float* g, const float* beta, const int32_t* cu_new, const int32_t* slots,
                    float* state, long slot_stride, int n_slots, float* out, float* scratch, int n_seqs, int n_tokens, int H, int G, int dim, int vdim,
-                   int n_chunks, cudaStream_t s);
+                   int at_once, cudaStream_t s);
 
 #define DR_SPLIT 8                                        // lanes that share a column
 #define DR_WARPS 4
@@ -422,15 +422,15 @@ delta_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
 // `dtype`; b_logit [tokens, H] of `dtype` (rows b_stride apart); z float32 [tokens, H*dim] (rows z_stride apart);
 // dt_bias float32 [H*dim] (with `head_decay`: z [tokens, H] and dt_bias [H], one decay for all key channels of a head);
 // a_log float32 [H]; slot memory float32: S at `state`, the history at `hist`, both
-// slot_stride floats a slot.  chunk_scratch (dl_delta_chunk_scratch floats; NULL: token by token): the recurrence runs chunk by chunk
-// (chunk_scan.cu; n_chunks: of the longest sequence).  Outputs float32, contiguous: q, k [tokens, G*dim], v, o [tokens, H*vdim], g [tokens, H*dim],
+// slot_stride floats a slot.  chunk_scratch (NULL: token by token): the recurrence runs chunk by chunk (chunk_scan.cu),
+// the operands of chunk_pieces pieces at a time, dl_delta_chunk_scratch floats each.  Outputs float32, contiguous: q, k [tokens, G*dim], v, o [tokens, H*vdim], g [tokens, H*dim],
 // beta [tokens, H].
 extern "C" int dl_delta_rule(const void* x, int ld, const void* taps, int K, int dtype, const void* b_logit, int b_stride,
                              const float* z, int z_stride, const float* dt_bias, const float* a_log,
                              const int32_t* token_seq, const int32_t* cu_new, const int32_t* slots, float* state, float* hist,
                              long slot_stride, int n_slots, float* qo, float* ko, float* vo, float* go, float* bo, float* out,
                              int n_seqs, int n_tokens, int H, int G, int dim, int vdim, float q_scale, float unit_eps,
-                             int head_decay, float* chunk_scratch, int n_chunks, void* stream) {
+                             int head_decay, float* chunk_scratch, int chunk_pieces, void* stream) {
     DL_REQUIRE(n_seqs >= 0 && n_tokens >= 0 && H > 0 && G > 0 && dim > 0 && vdim > 0 && n_slots > 0 && K >= 1, "delta_rule: bad sizes");
     DL_REQUIRE(H % G == 0, "delta_rule: %d heads are not a multiple of %d key heads", H, G);
     DL_REQUIRE(K <= DP_MAX_TAPS, "delta_rule: a convolution of %d taps, the kernel takes up to %d", K, DP_MAX_TAPS);
@@ -480,7 +480,7 @@ extern "C" int dl_delta_rule(const void* x, int ld, const void* taps, int K, int
     }
     if (chunk_scratch != nullptr)
         return dl_delta_chunk(qo, ko, vo, go, bo, cu_new, slots, state, slot_stride, n_slots, out, chunk_scratch, n_seqs, n_tokens, H, G, dim, vdim,
-                              n_chunks, s);
+                              chunk_pieces, s);
     const dim3 grid((vdim + DR_COLS - 1) / DR_COLS, H, n_seqs), block(DR_THREADS);
     const int rows = (dim + DR_SPLIT - 1) / DR_SPLIT;
     // few blocks that walk a long run of tokens want a multiprocessor each: they start when the kernels before have ended

@@ -40,8 +40,9 @@ _library.register_signatures({
     "dl_delta_rule": [_P, _I, _P, _I, _I, _P, _I, _P, _I, _P, _P, _P, _P, _P, _P, _P, ctypes.c_long, _I,
                       _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _I, _P, _I, _P],
     "dl_gla_chunk": [_P, _P, _P, _I, _P, _I, _P, _P, _P, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _F, _F, _I, _P],
-    "dl_gla_chunk_scratch": [_I, _I, _I, _I, _P],
-    "dl_delta_chunk_scratch": [_I, _I, _I, _P],
+    "dl_gla_chunk_scratch": [_I, _I, _P],
+    "dl_delta_chunk_scratch": [_I, _P],
+    "dl_chunk_pieces": [_I, _I],
     "dl_expert_gate_up": [_P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P],
     "dl_expert_down": [_P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _I, _P, _I, _I, _P],
     "dl_expert_sort": [_P, _I, _I, _P, _P, _I, _P],
@@ -821,7 +822,7 @@ def gated_activation(gate_up, kind, limit=0.0, alpha=1.0, bias=None):
 # ------------------------------------------------------- gated linear attention
 CHUNK = 32                       # CK_L in csrc/chunk_scan.cu
 CHUNK_MAX_DIM = 64               # CK_DIM
-CHUNK_SCRATCH_BYTES = 4 << 30    # most scratch the chunks' operands may take (1.2 KB a token and head); more: token by token
+CHUNK_SCRATCH_BYTES = 512 << 20  # most scratch the chunks' operands take at a time (1.1 KB a token and head, 1.4 for linear attention with 128 value channels)
 # Steps whose longest sequence brings fewer tokens walk them one by one: a scan takes 0.11 (gated linear attention) to 0.19 us (delta rule)
 # a token, whatever else is in the batch, the chunks' launches 25 to 45 us (16 heads of 64 x 128, one sequence of 300 tokens: 33 and 58 us by
 # the scans, 20 and 59 by chunks; of 2,048: 227 and 320 against 95 and 199).
@@ -836,14 +837,15 @@ def chunk_hint(rows, plan):
     return {"max_new": plan.max_new}
 
 
-def _chunk_scratch(device, name, n_seqs, max_new, n_heads, *more):
-    """(scratch, chunks of the longest sequence) of a recurrence's chunked form, or (None, 0) where it would take too much."""
-    chunks = (int(max_new) + CHUNK - 1) // CHUNK
-    need = ctypes.c_longlong(0)
-    getattr(_library.library(), name)(n_seqs, chunks, n_heads, *more, ctypes.byref(need))
-    if 4 * need.value > CHUNK_SCRATCH_BYTES or n_seqs > 65535 or n_heads > 65535:
+def _chunk_scratch(device, name, n_tokens, n_seqs, n_heads, *more):
+    """(scratch, pieces it holds) of a recurrence's chunked form: a piece per chunk of 32 tokens; where all of them would take too much, as
+    many as fit, a window after the other; (None, 0) where not one fits."""
+    floats = ctypes.c_longlong(0)
+    getattr(_library.library(), name)(n_heads, *more, ctypes.byref(floats))
+    at_once = min(_library.library().dl_chunk_pieces(n_tokens, n_seqs), CHUNK_SCRATCH_BYTES // (4 * floats.value))
+    if at_once < 1 or n_seqs > 65535 or n_heads > 65535:
         return None, 0
-    return torch.empty(need.value, dtype=torch.float32, device=device), chunks
+    return torch.empty(at_once * floats.value, dtype=torch.float32, device=device), at_once
 
 
 def gla_scan(q, k, v, z, z_bias, cu_new, slots, state, n_heads, dim, vdim, q_scale, tau=1.0, max_new=1):
@@ -874,11 +876,11 @@ def gla_scan(q, k, v, z, z_bias, cu_new, slots, state, n_heads, dim, vdim, q_sca
     out = torch.empty((T, n_heads * vdim), dtype=torch.float32, device=q.device)
     if q.dtype == torch.bfloat16 and max_new >= CHUNK_MIN_TOKENS and dim <= CHUNK_MAX_DIM and vdim % 4 == 0 and ld % 4 == 0 and v.data_ptr() % 8 == 0 \
             and state.data_ptr() % 16 == 0:
-        scratch, chunks = _chunk_scratch(q.device, "dl_gla_chunk_scratch", slots.numel(), max_new, n_heads, vdim)
+        scratch, at_once = _chunk_scratch(q.device, "dl_gla_chunk_scratch", T, slots.numel(), n_heads, vdim)
         if scratch is not None:
             _library.call("dl_gla_chunk", _ptr(q), _ptr(k), _ptr(v), ld, _ptr(z), zs, _ptr(z_bias), _ptr(cu_new), _ptr(slots), _ptr(state),
                           state.shape[0], _ptr(out), out.stride(0), _ptr(scratch), slots.numel(), T, n_heads, dim, vdim, float(q_scale), float(tau),
-                          chunks, _stream())
+                          at_once, _stream())
             return out
     _library.call("dl_gla_scan", _ptr(q), _ptr(k), _ptr(v), ld, _ptr(z), zs, _ptr(z_bias), _code(q.dtype), _ptr(cu_new),
                   _ptr(slots), _ptr(state), state.shape[0], _ptr(out), out.stride(0), slots.numel(), T, n_heads, dim, vdim,
@@ -1124,14 +1126,14 @@ def delta_rule(x, taps, b_logit, z, dt_bias, a_log, token_seq, cu_new, slots, me
     qo, ko = torch.empty((T, G * dim), **f32), torch.empty((T, G * dim), **f32)
     vo, go = torch.empty((T, H * vdim), **f32), torch.empty((T, H * dim), **f32)
     bo, out = torch.empty((T, H), **f32), torch.empty((T, H * vdim), **f32)
-    scratch, chunks = None, 0
+    scratch, at_once = None, 0
     if x.dtype == torch.bfloat16 and max_new >= CHUNK_MIN_TOKENS and dim <= CHUNK_MAX_DIM and vdim % 4 == 0:
-        scratch, chunks = _chunk_scratch(x.device, "dl_delta_chunk_scratch", slots.numel(), max_new, H)
+        scratch, at_once = _chunk_scratch(x.device, "dl_delta_chunk_scratch", T, slots.numel(), H)
     _library.call("dl_delta_rule", _ptr(x), ld, _ptr(taps), K, _code(x.dtype), _ptr(b_logit), _rows_view(b_logit, "delta_rule b"),
                   _ptr(z), _rows_view(z, "delta_rule z"), _ptr(dt_bias), _ptr(a_log), _ptr(token_seq), _ptr(cu_new), _ptr(slots),
                   memory.data_ptr(), memory.data_ptr() + 4 * n_state, memory.stride(0), memory.shape[0],
                   _ptr(qo), _ptr(ko), _ptr(vo), _ptr(go), _ptr(bo), _ptr(out), slots.numel(), T, H, G, int(dim), int(vdim),
-                  float(q_scale), float(unit_eps), 1 if head_decay else 0, _ptr(scratch), chunks, _stream())
+                  float(q_scale), float(unit_eps), 1 if head_decay else 0, _ptr(scratch), at_once, _stream())
     return out
 
 

@@ -172,3 +172,72 @@ def test_delta_rule_of_a_token_that_is_no_number(what, token, H, G, monkeypatch)
     got, state = run(100)
     scan, scan_state = run(1)
     no_worse(got, state, clean, scan, scan_state, list(range(token)) + list(range(100, T)))
+
+
+def gla_call(lens, H, dim, vdim, seed=1):
+    from dotllm_b200.kernels import ops
+    T = sum(lens)
+    proj = g64(T, 2 * H * dim + H * vdim, seed=seed).to(torch.bfloat16).to(DEV)
+    z, bias = (g64(T, H * dim, seed=3) * 2).float().to(DEV), g64(H * dim, seed=5).float().to(DEV)
+    states = g64(len(lens), H, dim, vdim, seed=6).float().to(DEV)
+
+    def run(at, most):
+        """Sequences ``at`` of them, in this order."""
+        rows = torch.cat([torch.arange(sum(lens[:b]), sum(lens[:b + 1])) for b in at]).to(DEV)
+        p, s = proj[rows], states[at].clone()
+        q, k, v = p[:, :H * dim], p[:, H * dim:2 * H * dim], p[:, 2 * H * dim:]
+        cu, zz = i32([0] + list(np.cumsum([lens[b] for b in at]))), z[rows]
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        out = ops.gla_scan(q, k, v, zz, bias, cu, i32(range(len(at))), s, H, dim, vdim, 0.3, 5.0, max_new=most)
+        return out, s, torch.cuda.max_memory_allocated() - before
+    return run, H * (32 * 96 + 64 + 64 * vdim)
+
+
+def delta_call(lens, H, dim, vdim, K=4):
+    from dotllm_b200.kernels import ops
+    C, T, n_state = (2 * dim + vdim) * H, sum(lens), H * dim * vdim
+    taps, dt_bias, a_log = g64(C, K, seed=1, scale=0.5).to(torch.bfloat16).to(DEV), g64(H, seed=2).float().to(DEV), g64(H, seed=3, scale=0.5).float().to(DEV)
+    x, z = torch.randn(T, C + H, generator=torch.Generator().manual_seed(9)).to(torch.bfloat16).to(DEV), g64(T, H, seed=20).float().to(DEV)
+    memory = g64(len(lens), n_state + (K - 1) * C, seed=4).float().to(DEV)
+
+    def run(at, most):
+        rows = torch.cat([torch.arange(sum(lens[:b]), sum(lens[:b + 1])) for b in at]).to(DEV)
+        p, zz, m = x[rows], z[rows], memory[at].clone()
+        seq, cu = i32([i for i, b in enumerate(at) for _ in range(lens[b])]), i32([0] + list(np.cumsum([lens[b] for b in at])))
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        out = ops.delta_rule(p, taps, p[:, C:], zz, dt_bias, a_log, seq, cu, i32(range(len(at))), m, H, H, dim, vdim, dim ** -0.5, 1e-6,
+                             head_decay=True, max_new=most)
+        return out, m, torch.cuda.max_memory_allocated() - before
+    return run, H * 96 * 96
+
+
+@pytest.mark.parametrize("call", [gla_call, delta_call])
+@pytest.mark.parametrize("pieces", [1, 3, 7])
+def test_windows_of_chunks_give_the_same_bits(call, pieces, monkeypatch):
+    from dotllm_b200.kernels import ops
+    monkeypatch.setattr(ops, "CHUNK_MIN_TOKENS", 2)
+    lens = [1, 96, 31, 130, 2, 64, 33]
+    run, floats = call(lens, 3, 40, 72)
+    out, state, _ = run(list(range(7)), 130)
+    monkeypatch.setattr(ops, "CHUNK_SCRATCH_BYTES", 4 * floats * pieces + 3)
+    got, got_state, _ = run(list(range(7)), 130)
+    assert torch.equal(got, out) and torch.equal(got_state, state)
+    monkeypatch.setattr(ops, "CHUNK_SCRATCH_BYTES", 4 * floats - 1)      # not one piece: token by token
+    assert torch.equal(run(list(range(7)), 130)[0], run(list(range(7)), 1)[0])
+
+
+@pytest.mark.parametrize("call", [gla_call, delta_call])
+def test_scratch_follows_the_tokens(call):
+    """A prompt beside many single tokens takes the room of its own chunks and a piece for each of the others, and gets the bits it has alone."""
+    lens = [1] * 20 + [1500] + [1] * 27
+    run, floats = call(lens, 32, 64, 128)
+    out, state, peak = run(list(range(48)), 1500)
+    alone, alone_state, _ = run([20], 1500)
+    assert torch.equal(out[20:1520], alone) and torch.equal(state[20], alone_state[0])
+    _, _, scan_peak = run(list(range(48)), 1)
+    assert peak - scan_peak < 0.2 * 2 ** 30
+    assert peak - scan_peak <= 4 * floats * ((sum(lens) + 31 * 48) // 32) + (4 << 20)
