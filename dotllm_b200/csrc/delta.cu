@@ -146,7 +146,7 @@ delta_prepare_kernel(const T* __restrict__ x, int ld, const T* __restrict__ taps
     }
 }
 
-// The same for prompts that go chunk by chunk, bfloat16 rows, at most four taps and heads of 16, 32, 64 or 128 key channels: a thread
+// The same for prompts that go chunk by chunk, bfloat16 rows, at most four taps and heads of 16, 32 or 64 key channels: a thread
 // takes four neighbouring channels of four tokens in a row, so that its seven 8-byte rows are asked for at once (the kernel above
 // waits for one row after the other: 3,743 tokens of 8,192 channels in 205 us, this one in 105; the bytes alone are 37).  Tiles of
 // 256 channels along grid.y, then tiles of 256 decays (the step sizes with them).
@@ -216,7 +216,7 @@ delta_prepare_vec_kernel(const __nv_bfloat16* __restrict__ x, int ld, const __nv
         for (int d = 0; d < 4; ++d) e[d] = lag < K ? __bfloat162float(taps[(long)(cc + d) * K + (K - 1 - lag)]) : 0.f;
         tap[i] = make_float4(e[0], e[1], e[2], e[3]);
     }
-    const int lanes = dim / 4;                             // lanes of a head: 4, 8, 16 or 32, aligned (a tile starts at a whole head)
+    const int lanes = dim / 4;                             // lanes of a head: 4, 8 or 16, aligned (a tile starts at a whole head)
     const bool is_v = c >= qk;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -441,7 +441,7 @@ extern "C" int dl_delta_rule(const void* x, int ld, const void* taps, int K, int
     if (n_seqs == 0 || n_tokens == 0) return DL_OK;
     cudaStream_t s = (cudaStream_t)stream;
     const bool single = n_tokens == n_seqs;               // every sequence brings exactly one token
-    const bool vec = chunk_scratch != nullptr && dtype == DL_BF16 && K <= 4 && !single && (dim == 16 || dim == 32 || dim == 64 || dim == 128) && vdim % 4 == 0 &&
+    const bool vec = chunk_scratch != nullptr && dtype == DL_BF16 && K <= 4 && !single && (dim == 16 || dim == 32 || dim == 64) && vdim % 4 == 0 &&
                      ld % 4 == 0 && ((uintptr_t)x % 8) == 0 && slot_stride % 4 == 0 && ((uintptr_t)hist % 16) == 0 &&
                      (head_decay || (z_stride % 4 == 0 && ((uintptr_t)z % 16) == 0 && ((uintptr_t)dt_bias % 16) == 0));
     // enough blocks for a few rounds over the machine; beyond that a block walks a run of tokens

@@ -241,3 +241,49 @@ def test_scratch_follows_the_tokens(call):
     _, _, scan_peak = run(list(range(48)), 1)
     assert peak - scan_peak < 0.2 * 2 ** 30
     assert peak - scan_peak <= 4 * floats * ((sum(lens) + 31 * 48) // 32) + (4 << 20)
+
+
+@pytest.mark.parametrize("K", [1, 2, 3, 4])
+@pytest.mark.parametrize("dim", [16, 32, 64])
+@pytest.mark.parametrize("head_decay", [False, True])
+def test_preparation_of_prompts(K, dim, head_decay, monkeypatch):
+    """Fewer taps than the kernel's four places, heads of 4, 8 and 16 lanes, tokens that do not fill a block, sequences shorter than the taps."""
+    from dotllm_b200.kernels import ops
+    monkeypatch.setattr(ops, "CHUNK_MIN_TOKENS", 2)
+    H, G, vdim, lens = 4, 2, 36, [37, 1, 2, 50, 3]
+    C, T, n_state = 2 * G * dim + H * vdim, sum(lens), H * dim * vdim
+    decays = H if head_decay else H * dim
+    taps = g64(C, K, seed=1, scale=0.5).to(torch.bfloat16)
+    dt_bias, a_log = g64(decays, seed=2).float(), g64(H, seed=3, scale=0.5).float()
+    x, z = g64(T, C + H, seed=10).to(torch.bfloat16), g64(T, decays, seed=20).float()
+    memory = g64(6, n_state + (K - 1) * C, seed=4).float()
+    slots, seq, cu = [4, 1, 5, 0, 2], [i for i, n in enumerate(lens) for _ in range(n)], [0] + list(np.cumsum(lens))
+    gx, gm = x.to(DEV), memory.clone().to(DEV)
+    assert gx.stride(0) % 4 == 0 and gm.stride(0) % 4 == 0     # the kernel's four channels a thread
+    got = ops.delta_rule(gx, taps.to(DEV), gx[:, C:], z.to(DEV), dt_bias.to(DEV), a_log.to(DEV), i32(seq), i32(cu), i32(slots), gm, H, G, dim, vdim,
+                         dim ** -0.5, 1e-6, head_decay=head_decay, max_new=max(lens))
+    want_mem = memory.clone()
+    want = kernel_refs.delta_rule(x, taps, x[:, C:], z.repeat_interleave(dim, 1) if head_decay else z,
+                                  dt_bias.repeat_interleave(dim) if head_decay else dt_bias, a_log, torch.tensor(seq), torch.tensor(cu),
+                                  torch.tensor(slots), want_mem, H, G, dim, vdim, dim ** -0.5, 1e-6)
+    assert float((got.cpu() - want).abs().max()) < 3 * TOL * (1 + float(want.abs().max()))
+    assert float((gm.cpu() - want_mem).abs().max()) < 3 * TOL * (1 + float(want_mem.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("vdim,gate", [(128, "silu"), (64, "sigmoid"), (20, "silu")])
+def test_head_norm_of_many_rows(dtype, vdim, gate):
+    """So many (token, head) pairs that a warp takes four, not a multiple of a block's sixteen; the gate is a column view of wider rows."""
+    from dotllm_b200.kernels import ops
+    H, T = 7, 1361
+    assert H * T % 16 and H * T >= 4 * 4 * 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    o, wide = g64(T, H * vdim, seed=1).float().to(DEV), g64(T, H * vdim + 8, seed=2).to(dtype).to(DEV)
+    g, gain = wide[:, 8:], g64(vdim, seed=3).float().to(DEV)
+    got = ops.head_norm_gate(o, g, gain, H, vdim, 1e-5, dtype, gate=gate)
+    od, gd = o.double().view(T, H, vdim), g.double().reshape(T, H, vdim)
+    want = od / (od.square().mean(-1, keepdim=True) + 1e-5).sqrt() * gain.double() * (torch.sigmoid(gd) * (gd if gate == "silu" else 1))
+    # float32: a sum of 128 squares and a handful of roundings; bfloat16: the result's own rounding
+    rel = 2e-6 if dtype == torch.float32 else 2.0 ** -8
+    assert bool(((got.double().view(T, H, vdim) - want).abs() <= rel * want.abs() + 1e-6).all())
+    few = ops.head_norm_gate(o[:3], g[:3], gain, H, vdim, 1e-5, dtype, gate=gate)          # a pair a warp: the same bits
+    assert torch.equal(few, got[:3])

@@ -122,3 +122,38 @@ def test_results_that_are_not_finite_cost_an_ffma_product(M, N, K):
     finite, infinite, product = time(lambda: ops.linear(x, w)), time(lambda: ops.linear(bad, w)), time(lambda: ffma(x))
     print(f"observed {M} x {N} x {K}: finite {finite * 1e3:.0f} us, not finite {infinite * 1e3:.0f}, FFMA {product * 1e3:.0f}")
     assert infinite < finite + 10 * product                    # (8 rows: 7.8 times; a cut tile's chains are single lanes' and read rows of W side by side)
+
+
+@pytest.mark.parametrize("M,N,K", [(4, 300, 256), (9, 256, 2048), (24, 200, 516), (50, 256, 768), (200, 256, 2048), (300, 128, 4096), (20, 144, 14336)])
+def test_no_further_off_than_the_ffma_product(M, N, K):
+    """Norms: the bound above leaves room for a product without its smallest pieces (4e-6 off), this does not.  Every number of tokens a
+    tile may have, whole and cut tiles."""
+    from dotllm_b200.kernels import library, ops
+    x, w = make(M, N, K, seed=12)
+    want = x.double() @ w.double().T
+    chain = torch.empty(M, N, device=DEV)
+    library.call("dl_gemm_f32", x.data_ptr(), K, w.data_ptr(), chain.data_ptr(), N, M, N, K, library.current_stream())
+    far = lambda y: float((y.double() - want).norm() / want.norm())
+    assert far(ops.linear(x, w)) < min(5e-7, 1.1 * far(chain) + 2e-8), (far(ops.linear(x, w)), far(chain))
+
+
+@pytest.mark.parametrize("M", [4, 24, 50, 200])
+@pytest.mark.parametrize("K", [512, 8192])
+@pytest.mark.parametrize("whose", ["x", "w"])
+def test_the_last_eight_bits_alone(M, K, whose):
+    """Neighbours in k that cancel but for their last pieces: what is left is 2^-17 of the terms, the sums' own rounding 2^-24 of them."""
+    from dotllm_b200.kernels import ops
+    a, b = make(M, 144, K, seed=13)
+    a, b = (a, b) if whose == "x" else (b, a)
+
+    def last(t):                                               # pairs (v, -(v without its last piece)); the other side's pairs are equal
+        v = t[:, ::2].contiguous()
+        hi = v.to(torch.bfloat16).float()
+        mid = (v - hi).to(torch.bfloat16).float()
+        return torch.stack([v, -(hi + mid)], dim=2).reshape(t.shape).contiguous()
+
+    first, second = last(a), b[:, ::2].to(torch.bfloat16).float().repeat_interleave(2, 1).contiguous()
+    x, w = (first, second) if whose == "x" else (second, first)
+    want = x.double() @ w.double().T
+    assert 0 < float(want.norm()) < 1e-4 * float((x.abs().double() @ w.abs().double().T).norm())
+    assert float((ops.linear(x, w).double() - want).norm() / want.norm()) < 0.1
