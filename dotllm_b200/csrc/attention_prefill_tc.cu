@@ -58,6 +58,8 @@
 #define PT_BLOCKS(hd) ((hd) > 64 ? 1 : 2)    // blocks of a multiprocessor
 #define PT_BUFS(hd) ((hd) > 64 ? 2 : 1)      // buffers a tile has for its scores, and for its weights
 #define PT_TMEM_COLS(hd) (PT_TILES * (PT_BUFS(hd) * DL_PAGE + (hd)))    // 512 for heads of 128, 256 for heads of 64
+#define PT_ISSUE_REGS 40                     // registers a thread, heads of 64: of the four warps that issue copies and products,
+#define PT_SOFTMAX_REGS 96                   // and of the eight that hold a row's scores (the kernel is built with 80)
 #define PT_RESCALE_STEP 8.0f                 // log2 units a row's maximum may grow before O is rescaled
 
 __device__ __forceinline__ float pt_ex2(float x) {             // 2^x, 2 ulp; ex2(-inf) = 0
@@ -198,7 +200,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
     // Two blocks a multiprocessor leave 80 registers a thread, 30,720 a block: the four issuing warps give some up for the
     // threads that hold a row's scores (40 x 128 + 96 x 256 = 29,696)
     if (warp < 4) {
-        if (BUFS == 1) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (BUFS == 1) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PT_ISSUE_REGS));
         if (warp == 0) {
             // ------------------------------------------------------------ copies
             bool stop = false;
@@ -325,7 +327,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
             }
         }
     } else {
-        if (BUFS == 1) asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
+        if (BUFS == 1) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PT_SOFTMAX_REGS));
         // ------------------------------------------------------------ softmax: thread -> row of tile `t`
         const int t = (warp - 4) >> 2, quarter = warp & 3;
         const PtTile T = tiles[t];
@@ -544,6 +546,10 @@ static int pt_launch(dim3 grid, cudaStream_t s, const void* q, int q_stride, int
         cudaFuncAttributes attr;
         cudaError_t e = cudaFuncGetAttributes(&attr, attention_prefill_tc_kernel<HD, SHAPE>);
         if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "attention_prefill_tc: %s", cudaGetErrorString(e));
+        // a warp that asks for registers waits until the block's own have room: a build with fewer must not run
+        if (PT_BUFS(HD) == 1 && attr.numRegs * PT_THREADS < PT_ISSUE_REGS * 128 + PT_SOFTMAX_REGS * 256)
+            return dl_fail(DL_ERR_UNSUPPORTED, "attention_prefill_tc: built with %d registers a thread, the split between its warps needs %d", attr.numRegs,
+                           (PT_ISSUE_REGS * 128 + PT_SOFTMAX_REGS * 256 + PT_THREADS - 1) / PT_THREADS);
         const size_t ask = data + 1024 - (attr.sharedSizeBytes < 1024 ? attr.sharedSizeBytes : 0);
         e = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD, SHAPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ask);
         if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "attention_prefill_tc: shared memory %zu: %s", ask, cudaGetErrorString(e));
