@@ -20,7 +20,7 @@
 // packed multiply-adds issue half as often at the same rate and leave it there).  One prompt of 1,000 tokens, 32 heads of 128: 1,858 -> 295 us,
 // 28 TFLOP/s over the visible scores, issue slots 70 % and shared memory 65 % busy.  Decode: the bytes of K and V; the generic kernel
 // walked a sequence's keys one tile after the other, 64 blocks in all.  Here a page is a block's work, for all query heads of
-// the KV head, and a second kernel merges the pages' parts: 8 sequences of up to 1,500 tokens, 8 KV heads of 64: 144 -> 18 us
+// the KV head (several pages where the machine is full), and a second kernel merges the pages' parts: 8 sequences of up to 1,500 tokens, 8 KV heads of 64: 144 -> 18 us
 // (blocks that walked four pages each took 22).
 #include "common.cuh"
 #include <atomic>

@@ -206,11 +206,11 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
             bool stop = false;
             int issued = 0;
             if (lane == 0) {
-    #pragma unroll
+#pragma unroll
                 for (int t = 0; t < PT_TILES; ++t) {
                     if (tiles[t].rows <= 0) continue;
                     tc_mbar_expect(&q_full[t], Q_BYTES);
-    #pragma unroll
+#pragma unroll
                     for (int a = 0; a < ATOMS; ++a)
                         dl_tma_load_2d(q_smem + t * Q_BYTES + a * (PT_ROWS * 128), &tmap_q, head * HD + a * 64,
                                        cu_new[b] + row0 + t * PT_ROWS, &q_full[t]);
@@ -232,7 +232,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
                         } else {
                             unsigned char* k_dst = kv_smem + (size_t)s * STAGE_BYTES;
                             tc_mbar_expect(&kv_full[s], STAGE_BYTES);
-    #pragma unroll
+#pragma unroll
                             for (int a = 0; a < ATOMS; ++a)
                                 dl_tma_load_2d(k_dst + a * (DL_PAGE * 128), &tmap_k, a * 64, (page * nkv + kvh) * DL_PAGE, &kv_full[s]);
                             dl_tma_load_2d(k_dst + K_BYTES, &tmap_v, 0, (page * nkv + kvh) * HD, &kv_full[s]);
@@ -282,7 +282,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
                     }
                     tc_fence_after();
                     const uint32_t k_addr = tc_smem(kv_smem + (size_t)s * STAGE_BYTES);
-    #pragma unroll
+#pragma unroll
                     for (int k = 0; k < HD / 16; ++k) {
                         const int a = k / 4, kk = k % 4;            // 64-dim slice, 16-dim step inside it (32 bytes)
                         tc_mma(tmem_s + (uint32_t)((BUFS * t + sb) * DL_PAGE), tc_operand_desc(q_addr + a * (PT_ROWS * 128)) + (uint64_t)(kk * 2),
@@ -301,7 +301,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
                 for (int j = 0; j < n_kv && ok; ++j) {
                     const int s = j % STAGES;
                     const uint32_t v_addr = tc_smem(kv_smem + (size_t)s * STAGE_BYTES + K_BYTES);
-    #pragma unroll
+#pragma unroll
                     for (int t = 0; t < PT_TILES; ++t) {
                         if (j < tiles[t].j_lo || j > tiles[t].j_hi) continue;
                         const int c = j - tiles[t].j_lo, pb = c % BUFS;
@@ -314,7 +314,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
                         }
                         tc_fence_after();
                         const uint32_t p_addr = tc_smem(p_smem + (BUFS * t + pb) * P_BYTES);
-    #pragma unroll
+#pragma unroll
                         for (int k = 0; k < DL_PAGE / 16; ++k)
                             tc_mma(tmem_o + (uint32_t)(t * HD), tc_operand_desc(p_addr) + (uint64_t)(k * 2), tc_operand_desc(v_addr) + (uint64_t)(k * 2),
                                    idesc_pv, (c | k) != 0 ? 1u : 0u);
@@ -423,6 +423,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
 #pragma unroll
                     for (int i = 0; i < 8; ++i) o[i] *= corr;
                     tc_tmem_store8(my_o + (uint32_t)c0, o);
+                    tc_tmem_store_wait();
                 }
                 tc_fence_before();
             }

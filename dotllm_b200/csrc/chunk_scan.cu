@@ -1,11 +1,13 @@
-// The two recurrences with a decay per key channel over prompts, 32 tokens at a time, in float32 throughout:
+// The two recurrences with a decay per key channel over prompts, 32 tokens at a time, in float32 throughout (the chunked forms of Yang et
+// al., "Gated Linear Attention Transformers with Hardware-Efficient Training" and "Parallelizing Linear Transformers with the Delta
+// Rule over Sequence Length", here without divisions by running products of decays):
 //
 //   gated linear attention (gla.cu)    S_t = diag(a_t) S_(t-1) + k_t v_t^T                        o_t = S_t^T q_t
 //   gated delta rule (delta.cu)        S_t = diag(a_t) S_(t-1) + k_t u_t^T,                       o_t = S_t^T q_t
 //                                      u_t = b_t (v_t - (diag(a_t) S_(t-1))^T k_t)
 //
 // The scans of those files walk a sequence token by token: a chain of dependent steps, two warps a scheduler waiting for it (2,048
-// tokens of 16 heads 227 us for the first, 388 for the second; at no time is a pipe or the memory busy).  Over a chunk of L tokens that
+// tokens of 16 heads 227 us for the first, 320 for the second; at no time is a pipe or the memory busy).  Over a chunk of L tokens that
 // starts from S_0, with P_t = a_1 ... a_t (per channel), both are matrix products:
 //
 //   A[t][j] = sum_c q_t[c] k_j[c] (a_(j+1) ... a_t)[c]  (j <= t),      N[t][j] = b_t sum_c k_t[c] k_j[c] (a_(j+1) ... a_t)[c]  (j < t)
@@ -427,8 +429,7 @@ struct CkGla {                           // per (piece of the window, head), flo
 };
 
 // The chunk's rows of v, columns col0 .. + 63, through silu where asked, zeros beyond, into [L][64].
-template <typename T>
-__device__ __forceinline__ void ck_bring_v(float* s_v, const T* v, long v_ld, int v_silu, const CkRange& r, int h, int vdim, int col0, int tid) {
+__device__ __forceinline__ void ck_bring_v(float* s_v, const __nv_bfloat16* v, long v_ld, int v_silu, const CkRange& r, int h, int vdim, int col0, int tid) {
     for (int e = tid; e < CK_L * (CK_GLA_COLS / 4); e += CK_GLA_THREADS) {
         const int t = e / (CK_GLA_COLS / 4), c = (e % (CK_GLA_COLS / 4)) * 4;
         float x[4] = {0.f, 0.f, 0.f, 0.f};
@@ -444,9 +445,8 @@ __device__ __forceinline__ void ck_bring_v(float* s_v, const T* v, long v_ld, in
 }
 
 // A block per (piece, head): Q+, A, P_L and K'^T V.  z, z_bias as in dl_gla_scan.
-template <typename T>
 __global__ void __launch_bounds__(CK_GLA_THREADS)
-gla_chunk_states_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, long ld, const float* __restrict__ z, long z_ld,
+gla_chunk_states_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, long ld, const float* __restrict__ z, long z_ld,
                         const float* __restrict__ z_bias, const int32_t* __restrict__ cu_new, const int32_t* __restrict__ slots, int n_slots, int n_seqs,
                         CkGla out, int H, int dim, int vdim, float q_scale, float inv_tau, int lo) {
     __shared__ __align__(16) float sq[CK_DIM * CK_LDT], sk[CK_DIM * CK_LDT], sa[CK_DIM * CK_LDT];
@@ -462,7 +462,7 @@ gla_chunk_states_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
         float qv = 0.f, kv = 0.f, av = t < r.count ? 0.f : 1.f;    // a token that is not there decays nothing and adds nothing
         if (t < r.count && c < dim) {
             const long row = r.t0 + r.first + t;
-            qv = dl_to_f32<T>(q[row * ld + (long)h * dim + c]), kv = dl_to_f32<T>(k[row * ld + (long)h * dim + c]);
+            qv = dl_to_f32<__nv_bfloat16>(q[row * ld + (long)h * dim + c]), kv = dl_to_f32<__nv_bfloat16>(k[row * ld + (long)h * dim + c]);
             if (z != nullptr) {
                 const float zz = z[row * z_ld + (long)h * dim + c] + z_bias[h * dim + c];
                 av = expf((fminf(zz, 0.f) - log1pf(expf(-fabsf(zz)))) * inv_tau);
@@ -492,7 +492,7 @@ gla_chunk_states_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
     for (int e = tid; e < CK_L * CK_DIM; e += CK_GLA_THREADS) qa[(e / CK_DIM) * CK_X + e % CK_DIM] = sq[(e % CK_DIM) * CK_LDT + e / CK_DIM];
     const int rg = tid >> 4, cg = tid & 15;
     for (int col0 = 0; col0 < vdim; col0 += CK_GLA_COLS) {
-        ck_bring_v<T>(part, v, ld, z == nullptr ? 1 : 0, r, h, vdim, col0, tid);
+        ck_bring_v(part, v, ld, z == nullptr ? 1 : 0, r, h, vdim, col0, tid);
         __syncthreads();
         float acc[4][4];
 #pragma unroll
@@ -544,9 +544,8 @@ gla_chunk_pass_kernel(CkGla io, const int32_t* __restrict__ cu_new, const int32_
 }
 
 // A block per (piece, head): O = [Q+ | A] [S_0; V].
-template <typename T>
 __global__ void __launch_bounds__(CK_GLA_THREADS)
-gla_chunk_out_kernel(const T* __restrict__ v, long v_ld, int v_silu, CkGla in, const int32_t* __restrict__ cu_new, const int32_t* __restrict__ slots,
+gla_chunk_out_kernel(const __nv_bfloat16* __restrict__ v, long v_ld, int v_silu, CkGla in, const int32_t* __restrict__ cu_new, const int32_t* __restrict__ slots,
                      int n_slots, int n_seqs, float* __restrict__ out, long out_ld, int H, int dim, int vdim, int lo) {
     __shared__ __align__(16) float s_qa[CK_L * CK_LDX], s_x[CK_X * CK_GLA_COLS];
     dl_launch_dependents();
@@ -564,7 +563,7 @@ gla_chunk_out_kernel(const T* __restrict__ v, long v_ld, int v_silu, CkGla in, c
             ck_copy16(s_x + 4 * e, in.states + (live ? (piece * CK_DIM + c) * vdim + col : 0), live);
         }
         ck_commit();
-        ck_bring_v<T>(s_x + CK_DIM * CK_GLA_COLS, v, v_ld, v_silu, r, h, vdim, col0, tid);
+        ck_bring_v(s_x + CK_DIM * CK_GLA_COLS, v, v_ld, v_silu, r, h, vdim, col0, tid);
         ck_wait<0>();
         __syncthreads();
         float acc[2][4];
@@ -626,7 +625,6 @@ extern "C" int dl_gla_chunk(const void* q, const void* k, const void* v, int ld,
     DL_REQUIRE(ld % 4 == 0 && ((uintptr_t)v % 8) == 0 && ((uintptr_t)state % 16) == 0, "gla_chunk: unaligned values or states");
     if (n_seqs == 0 || n_tokens == 0) return DL_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    typedef __nv_bfloat16 T;
     const long long pieces = dl_chunk_pieces(n_tokens, n_seqs), in_scratch = (long long)at_once * H;
     CkGla sc;
     sc.qa = scratch;
@@ -636,13 +634,13 @@ extern "C" int dl_gla_chunk(const void* q, const void* k, const void* v, int ld,
     for (long long lo = 0; lo < pieces && e == cudaSuccess; lo += at_once) {
         const int n = (int)(pieces - lo < at_once ? pieces - lo : at_once);
         const dim3 grid(n, H);
-        e = dl_launch_dependent(gla_chunk_states_kernel<T>, grid, dim3(CK_GLA_THREADS), 0, s, (const T*)q, (const T*)k, (const T*)v, ld, z, z_stride,
+        e = dl_launch_dependent(gla_chunk_states_kernel, grid, dim3(CK_GLA_THREADS), 0, s, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, ld, z, z_stride,
                                 z_bias, cu_new, slots, n_slots, n_seqs, sc, H, dim, vdim, q_scale, 1.0f / tau, (int)lo);
         if (e == cudaSuccess)
             e = dl_launch_dependent(gla_chunk_pass_kernel, dim3((dim * vdim / 4 + 255) / 256, H, n_seqs), dim3(256), 0, s, sc, cu_new, slots, state,
                                     n_slots, H, dim, vdim, (int)lo, n);
         if (e == cudaSuccess)
-            e = dl_launch_dependent(gla_chunk_out_kernel<T>, grid, dim3(CK_GLA_THREADS), 0, s, (const T*)v, ld, z == nullptr ? 1 : 0, sc, cu_new, slots,
+            e = dl_launch_dependent(gla_chunk_out_kernel, grid, dim3(CK_GLA_THREADS), 0, s, (const __nv_bfloat16*)v, ld, z == nullptr ? 1 : 0, sc, cu_new, slots,
                                     n_slots, n_seqs, out, out_ld, H, dim, vdim, (int)lo);
     }
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "gla_chunk: %s", cudaGetErrorString(e));

@@ -1,4 +1,5 @@
-// y = x W^T for float32 matrices on the fifth-generation tensor cores, with float32 accuracy.
+// y = x W^T for float32 matrices on the fifth-generation tensor cores, with float32 accuracy.  (Splitting float32 values into three
+// bfloat16 ones: Henry, Tang and Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations".)
 //
 // What bounds the product: on the FFMA pipes 74 TFLOP/s (the kernels of gemm_f32.cu reach 24), for a few rows the four
 // bytes of every weight.  Here every operand value is split into three bfloat16 values, v = hi + mid + lo, each rounded to
@@ -537,13 +538,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 }
                 if (seg + 1 < s1) {
 #pragma unroll
-                    for (int c = 0; c < COLS; c += 8)
-                        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                                     ::"r"(lane_at + TOTAL_AT + c), "r"(__float_as_uint(sum[c])), "r"(__float_as_uint(sum[c + 1])),
-                                       "r"(__float_as_uint(sum[c + 2])), "r"(__float_as_uint(sum[c + 3])), "r"(__float_as_uint(sum[c + 4])),
-                                       "r"(__float_as_uint(sum[c + 5])), "r"(__float_as_uint(sum[c + 6])), "r"(__float_as_uint(sum[c + 7]))
-                                     : "memory");
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    for (int c = 0; c < COLS; c += 8) {
+                        const float v[8] = {sum[c], sum[c + 1], sum[c + 2], sum[c + 3], sum[c + 4], sum[c + 5], sum[c + 6], sum[c + 7]};
+                        tc_tmem_store8(lane_at + TOTAL_AT + c, v);
+                    }
+                    tc_tmem_store_wait();
                 } else {
                     float* dst = wk.y + (size_t)m0 * wk.y_stride + n;
                     bool fine = true;

@@ -233,7 +233,7 @@ F32_TILE_ROWS = 64                   # AF_ROWS
 # (32 heads of 64, one sequence, kernels alone; a tile's time does not depend on how full it is): 8 new tokens after 1,500 25 against
 # 208 us, 32 after 1,500 60 against 208, 32 after 200 20 against 40; a token's pages are read again for every token, so where tiles
 # fill the machine the line is lower.
-F32_SPLIT_TOKENS, F32_SPLIT_TOKENS_FEW, F32_FULL_BLOCKS = 8, 32, 148
+F32_SPLIT_TOKENS, F32_SPLIT_TOKENS_FEW = 8, 32
 F32_PARTS_BYTES = 256 << 20          # most room the pages' parts of a launch may take (head_dim + 2 floats a token, head and page); more tokens: more launches
 
 
@@ -250,7 +250,7 @@ def run_f32(q, q_stride, out, k_pool, v_pool, n_pages, token_seq, token_pos, blo
 
     pools = (k_pool.data_ptr(), v_pool.data_ptr(), n_pages)
     T = q.shape[0]
-    few = sum(-(-n // F32_TILE_ROWS) for n in plan.news) * n_heads <= F32_FULL_BLOCKS
+    few = sum(-(-n // F32_TILE_ROWS) for n in plan.news) * n_heads <= _library.library().dl_sm_count()
     if plan.max_new <= (F32_SPLIT_TOKENS_FEW if few else F32_SPLIT_TOKENS):
         a_token = n_heads * block_table.shape[1]           # parts
         at_once = max(1, min(T, 65535, F32_PARTS_BYTES // (4 * a_token * (head_dim + 2))))

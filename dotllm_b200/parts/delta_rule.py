@@ -14,7 +14,7 @@ head's state and the convolutions' last taps - 1 inputs - is the layer execution
 vector per slot, zero when a sequence opens; convolution sums, unit lengths, step sizes, decays, the recurrence and the
 per-head norm are float32 in either run dtype.  The kernels walk a sequence's new tokens in order from that entry; in a
 float32 run prompts, parts of prompts and decoded tokens are that one code path (the same bits however a sequence is
-cut), in a bfloat16 run the recurrence of prompts of 256 tokens and more goes a chunk of tokens at a time.
+cut), in a bfloat16 run the recurrence of a step whose longest sequence brings 256 tokens and more goes a chunk at a time.
 
 Two simpler forms, each a parameter: ``decay`` "head" - one decay per head, g = exp(-exp(A_h) softplus(a_h . x + dt_h)),
 from a projection of its own with one row per head (no low-rank pair), the same for all key channels of the head; and

@@ -9,8 +9,8 @@ stacked matrix, so one product feeds the scan.  The state is the layer execution
 (float32, zero when a sequence opens, carried from step to step); the decay logits leave their product in
 float32, and decays, recurrence and the per-head norm are float32 in either run dtype.  The scan walks a
 sequence's new tokens in order from the cached state; in a float32 run prompts, parts of prompts and decoded
-tokens are that one code path (the same bits however a sequence is cut), in a bfloat16 run prompts of 256 tokens
-and more go a chunk of tokens at a time, equal to float32 rounding.
+tokens are that one code path (the same bits however a sequence is cut), in a bfloat16 run the tokens of a step whose
+longest sequence brings 256 and more go a chunk at a time, equal to float32 rounding.
 """
 from __future__ import annotations
 

@@ -223,6 +223,7 @@ def test_windows_of_chunks_give_the_same_bits(call, pieces, monkeypatch):
     lens = [1, 96, 31, 130, 2, 64, 33]
     run, floats = call(lens, 3, 40, 72)
     out, state, _ = run(list(range(7)), 130)
+    assert torch.equal(run(list(range(7)), 2)[0], out)         # the most tokens of a sequence choose the form, nothing else
     monkeypatch.setattr(ops, "CHUNK_SCRATCH_BYTES", 4 * floats * pieces + 3)
     got, got_state, _ = run(list(range(7)), 130)
     assert torch.equal(got, out) and torch.equal(got_state, state)
