@@ -27,7 +27,7 @@
 // run as three launches.
 //
 // Measured (bfloat16 rows, kernels alone, state of 64 x 128 a head): gated linear attention, one sequence of 2,048 tokens, 16 heads: 227 ->
-// 95 us (46 the states, 14 the pass, 35 the outputs), eight such sequences 1,131 -> 668.  Delta rule, three sequences of 3,743 tokens in all, 32 heads:
+// 95 us (46 the states, 14 the pass, 35 the outputs), eight such sequences 1,131 -> 720.  Delta rule, three sequences of 3,743 tokens in all, 32 heads:
 // 734 -> 489 us (208 for G, 281 the walk); one of 2,048, 16 heads: 320 -> 199.  What bounds them now is the FFMA pipes' issue
 // (18 and 50 million multiply-adds a thousand tokens and head).
 //

@@ -826,7 +826,7 @@ CHUNK_SCRATCH_BYTES = 512 << 20  # most scratch the chunks' operands take at a t
 # Steps whose longest sequence brings fewer tokens walk them one by one.  The line lies where one sequence breaks even, which is where the
 # scans are at their best: their blocks then have multiprocessors to themselves and take 0.11 (gated linear attention) to 0.19 us (delta
 # rule) a token, the chunks' launches 25 to 45 us (16 heads of 64 x 128, 300 tokens: 33 and 58 us by the scans, 20 and 59 by chunks; of
-# 2,048: 227 and 320 against 95 and 199).  With more sequences a scan's token costs more (eight of 2,048: 1,131 us against 668).
+# 2,048: 227 and 320 against 95 and 199).  With more sequences a scan's token costs more (eight of 2,048: 1,131 us against 720).
 CHUNK_MIN_TOKENS = 256
 
 
