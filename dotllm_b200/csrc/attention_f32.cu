@@ -18,7 +18,7 @@
 // kernel ran a warp per (token, head) and brought every tile of keys into shared memory once per token.  Here 64 rows share a
 // page, a thread holds 4 rows x 4 scores and 4 rows x hd/16 outputs (128 threads with 8 rows each: 315 us where this takes 291; the
 // packed multiply-adds issue half as often at the same rate and leave it there).  One prompt of 1,000 tokens, 32 heads of 128: 1,858 -> 295 us,
-// 28 TFLOP/s over the visible scores, issue slots 70 % and shared memory 65 % busy.  Decode: the bytes of K and V; the generic kernel
+// 28 TFLOP/s over the visible scores, issue slots 50 % and shared memory 68 % busy.  Decode: the bytes of K and V; the generic kernel
 // walked a sequence's keys one tile after the other, 64 blocks in all.  Here a page is a block's work, for all query heads of
 // the KV head (several pages where the machine is full), and a second kernel merges the pages' parts: 8 sequences of up to 1,500 tokens, 8 KV heads of 64: 144 -> 18 us
 // (blocks that walked four pages each took 22).
