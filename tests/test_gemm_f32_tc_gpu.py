@@ -113,7 +113,7 @@ def test_results_that_are_not_finite_cost_an_ffma_product(M, N, K):
             b.record()
             torch.cuda.synchronize()
             times.append(a.elapsed_time(b))
-        return sorted(times[3:])[2]
+        return min(times[3:])                                  # (the host may be slow, the device is not slow by chance)
 
     y = ops.linear(bad, w)
     ffma(bad)
