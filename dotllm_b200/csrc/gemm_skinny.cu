@@ -20,6 +20,14 @@
 // 0-7 are gate rows and rows 8-15 the matching up rows, and the epilogue writes silu(gate) * up
 // (native/kernels/swiglu.cu:7-41).
 //
+// Eight consumer warps of three stages and shares from one chunk on, over the whole GPU, against six of
+// four stages and shares of four chunks or more (192 KB in flight either way), kernels alone in a graph, 8 rows: 3,072 x 2,048 (12.6 MB)
+// 6.8 -> 5.6 us, 2,048 x 2,048 6.7 -> 5.1, 2,048 x 8,192 10.6 -> 8.9, 4,096 x 14,336 23.0 -> 21.7, gated 14,336 x 4,096 40.4 -> 39.8, 128,256 x
+// 2,048 90.9 -> 89.7 (5.9 TB/s); a decode step of 16 layers of the smaller widths, 8 sequences at 2,000 tokens, 991 -> 898 us.  A small
+// matrix is a chain of latencies (start, rows of x, hand-over of cut tiles) with few bytes between: what helps is that all multiprocessors take part.
+// Two blocks a multiprocessor of half the ring, so that the next product's first weights arrive under this one, lost more in
+// the stream than it gained at the edges (the step 1,217 us); asking for chunks in the L2 ahead of the ring, shares that differ by a chunk (their
+// bounds cost divisions on the way to a cut tile's sum: 1,088 us) and shares of neighbours in different blocks (932) likewise.
 //
 // Two optional fusions take the add + RMSNorm between two products of a decode step into the products
 // themselves (the reference's fused_add_rmsnorm, native/kernels/fused_add_rmsnorm.cu:9-72, is a kernel
@@ -40,10 +48,10 @@
 #include <unordered_map>
 
 #ifndef GS_CONSUMERS
-#define GS_CONSUMERS 6
+#define GS_CONSUMERS 8
 #endif
 #ifndef GS_SLOTS
-#define GS_SLOTS 4                         // ring stages per consumer warp
+#define GS_SLOTS 3                         // ring stages per consumer warp
 #endif
 #define GS_BK 256                          // k per chunk
 #define GS_STAGE_ELEMS (16 * GS_BK)         // a stage is the dense box the copy engine writes: [16 rows][256 k]
@@ -211,7 +219,7 @@ struct GsWork {
     int x_stride;
     void* out;
     int out_stride;
-    int M, N, K, up_offset, cpt, total_chunks, share;
+    int M, N, K, up_offset, cpt, total_chunks, active, share;      // active: consumer warps of a block that have a share
     GsFuse fuse;
 };
 
@@ -231,26 +239,31 @@ struct GsRings {
 // chunk.  `cnt` counts the chunks of this ring.  False: gave up.
 template <bool FUSE_SWIGLU>
 __device__ __forceinline__ bool gs_produce(const CUtensorMap* tmap, const GsWork& w, const GsRings& r, int lane, int& cnt) {
-    const int gw = blockIdx.x * GS_CONSUMERS + lane;
+    const int gw = blockIdx.x * w.active + lane;
     int cur = min(w.total_chunks, gw * w.share);
     const int end = min(w.total_chunks, (gw + 1) * w.share);
     const uint64_t policy = dl_stream_policy();             // W is read once a step: first out of the L2
-    for (; cur < end; ++cur, ++cnt) {
+    // Every lane whose slot is free issues its next chunk; none waits inside for another lane's slot.
+    long long t0 = clock64();
+    while (cur < end) {
         const int slot = cnt % GS_SLOTS;
-        if (cnt >= GS_SLOTS && !gs_mbar_wait(&r.empty_bar[lane][slot], ((cnt / GS_SLOTS) - 1) & 1, r.gave_up)) {
+        if (cnt < GS_SLOTS || gs_mbar_try(&r.empty_bar[lane][slot], ((cnt / GS_SLOTS) - 1) & 1)) {
+            const int tile = cur / w.cpt, kc = cur - tile * w.cpt;
+            __nv_bfloat16* dst = r.stage_mem + (size_t)(lane * GS_SLOTS + slot) * GS_STAGE_ELEMS;
+            // a box is always written whole: parts outside the matrix arrive as zeros
+            gs_mbar_expect(&r.full_bar[lane][slot], GS_STAGE_ELEMS * 2);
+            if (FUSE_SWIGLU) {
+                dl_tma_load_2d_hint(dst, tmap, kc * GS_BK, tile * 8, &r.full_bar[lane][slot], policy);
+                dl_tma_load_2d_hint(dst + 8 * GS_BK, tmap, kc * GS_BK, w.up_offset + tile * 8, &r.full_bar[lane][slot], policy);
+            } else {
+                dl_tma_load_2d_hint(dst, tmap, kc * GS_BK, tile * 16, &r.full_bar[lane][slot], policy);
+            }
+            ++cur, ++cnt;
+            t0 = clock64();
+        } else if (*r.gave_up || clock64() - t0 > GS_WAIT_CYCLES) {
             if (!*r.gave_up) atomicExch(r.status, 1);
             *r.gave_up = 1;
             return false;
-        }
-        const int tile = cur / w.cpt, kc = cur - tile * w.cpt;
-        __nv_bfloat16* dst = r.stage_mem + (size_t)(lane * GS_SLOTS + slot) * GS_STAGE_ELEMS;
-        // a box is always written whole: parts outside the matrix arrive as zeros
-        gs_mbar_expect(&r.full_bar[lane][slot], GS_STAGE_ELEMS * 2);
-        if (FUSE_SWIGLU) {
-            dl_tma_load_2d_hint(dst, tmap, kc * GS_BK, tile * 8, &r.full_bar[lane][slot], policy);
-            dl_tma_load_2d_hint(dst + 8 * GS_BK, tmap, kc * GS_BK, w.up_offset + tile * 8, &r.full_bar[lane][slot], policy);
-        } else {
-            dl_tma_load_2d_hint(dst, tmap, kc * GS_BK, tile * 16, &r.full_bar[lane][slot], policy);
         }
     }
     return true;
@@ -270,7 +283,7 @@ template <int NT, typename TOut, bool FUSE_SWIGLU>
 __device__ __forceinline__ void gs_consume(const GsWork& w, const GsRings& r, float* __restrict__ partials,
                                            int* __restrict__ counters, int warp, int lane, int& cnt, bool& dead) {
     const int g = lane >> 2, t = lane & 3;
-    const int gw = blockIdx.x * GS_CONSUMERS + warp;
+    const int gw = blockIdx.x * w.active + warp;
     const int begin = min(w.total_chunks, gw * w.share), end = min(w.total_chunks, (gw + 1) * w.share);
     const int cpt = w.cpt, share = w.share, M = w.M, N = w.N, K = w.K;
     const __nv_bfloat16* x = w.x;
@@ -450,7 +463,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap, const GsWork work, 
         // producer does not wait for the kernel before this one: while that kernel finishes, the
         // rings fill.
         if (!early_weights) dl_grid_dependency_wait();
-        if (lane < GS_CONSUMERS) {
+        if (lane < work.active) {
             int cnt = 0;
             if (!gs_produce<FUSE_SWIGLU>(&tmap, work, rings, lane, cnt)) gs_drain(rings, lane, cnt);
         }
@@ -496,7 +509,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap, const GsWork work, 
             __syncwarp();
             if (lane == 0) gs_mbar_arrive(&scale_bar);
         }
-    } else {
+    } else if (warp < work.active) {
         // ------------------------------------------------------------ consumer warp
         dl_grid_dependency_wait();       // x comes from the kernel before this one; out, partials and counters may be in use by it
         int cnt = 0;
@@ -509,9 +522,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap, const GsWork work, 
 }
 
 // How the work of an (N, K) matrix is cut: tiles of 16 rows (8 gate + 8 up when gated), chunks per
-// tile, blocks, chunks per consumer warp.  Depends on the matrix and the device only, never on M.
+// tile, consumer warps of a block with a share, chunks of a share, blocks.  Depends on the matrix and the device only, never on M.
 struct GsPlan {
-    int tiles, cpt, total, blocks, share;
+    int tiles, cpt, total, active, share, blocks;
 };
 
 static GsPlan gs_plan(int N, int K, int fuse_swiglu, int sms) {
@@ -519,12 +532,16 @@ static GsPlan gs_plan(int N, int K, int fuse_swiglu, int sms) {
     p.tiles = fuse_swiglu ? (N + 7) / 8 : (N + 15) / 16;
     p.cpt = (K + GS_BK - 1) / GS_BK;
     p.total = p.tiles * p.cpt;
-    const int per_block = GS_CONSUMERS * 4;                  // at least about four chunks per warp
-    p.blocks = (p.total + per_block - 1) / per_block;
-    if (p.blocks > sms) p.blocks = sms;
+    // A share is a whole number of chunks, so the last multiprocessors get less, or nothing: of eight, seven and six warps those that leave the
+    // busiest multiprocessor with the fewest chunks (more warps where it is the same: they have more of the ring).  1,024 chunks of a
+    // 2,048 x 2,048 matrix: 8, 7 or 12; 14,336 of a 4,096 x 14,336 one: 104, 98 or 102 (22.1 against 21.5 us with eight and six).
+    p.active = GS_CONSUMERS;
+    for (int c = GS_CONSUMERS; c >= GS_CONSUMERS - 2; --c) {
+        const int share = (p.total + sms * c - 1) / (sms * c);
+        if (c == GS_CONSUMERS || share * c < p.share * p.active) p.share = share, p.active = c;
+    }
+    p.blocks = (p.total + p.active * p.share - 1) / (p.active * p.share);
     if (p.blocks < 1) p.blocks = 1;
-    const int warps = p.blocks * GS_CONSUMERS;
-    p.share = (p.total + warps - 1) / warps;
     return p;
 }
 
@@ -584,7 +601,7 @@ static int gs_launch(const GsPlan& p, cudaStream_t s, const __nv_bfloat16* x, in
     CUtensorMap tmap;
     const int rc = gs_weight_map(&tmap, w, N, K, FUSE);
     if (rc != DL_OK) return rc;
-    const GsWork work{x, x_stride, out, out_stride, M, N, K, up_offset, p.cpt, p.total, p.share, fuse};
+    const GsWork work{x, x_stride, out, out_stride, M, N, K, up_offset, p.cpt, p.total, p.active, p.share, fuse};
     cudaError_t le = dl_launch_dependent(gemm_skinny_kernel<NT, TOut, FUSE>, dim3(p.blocks), dim3(GS_THREADS), smem, s, tmap, work,
                                          early_weights, partials, counters, status);
     if (le != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "gemm_skinny: %s", cudaGetErrorString(le));

@@ -38,6 +38,7 @@ MAX_ROWS = 128           # rows the two kernels take between them; beyond this t
 TC_PLAIN = False
 SUM_STRIDE = 16          # floats between the sums of squares of two 16-column tiles (mma.sync kernel)
 _MAX_TILES = 1 << 16
+CONSUMER_WARPS = 8       # of a block (GS_CONSUMERS in csrc/gemm_skinny.cu): each may hand over two cut tiles of 16 rows x 16 tokens
 _state = {}
 
 
@@ -47,7 +48,7 @@ def _device_state(device):
         sms = _library.library().dl_sm_count()
         counters = torch.zeros(_MAX_TILES, dtype=torch.int32, device=device)
         _library.register_counters(counters)
-        partials = torch.empty(max(sms, 1) * 6 * 2 * 2 * 128, dtype=torch.float32, device=device)
+        partials = torch.empty(max(sms, 1) * CONSUMER_WARPS * 2 * 2 * 128, dtype=torch.float32, device=device)
         _state[key] = (counters, partials, sms)
     return _state[key]
 

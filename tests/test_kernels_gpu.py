@@ -494,6 +494,27 @@ def test_gemm_skinny_repeats_with_full_rings(monkeypatch):
         assert torch.equal(gemm_skinny.run(x, w, torch.float32), first)
 
 
+@pytest.mark.parametrize("N,K", [(16, 8), (1, 264), (17, 256), (40, 2048), (2048, 2048), (1184 * 16 + 5, 256), (9, 16384), (2368 * 2 + 16, 2048)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_gemm_skinny_shares(N, K, gated, monkeypatch):
+    """Shares of unequal length (some warps one chunk of 256 k more than others, fewer chunks than warps, tiles over many shares): against
+    float64, the same bits for one row as for eight and on every launch.  Bound: float32 sums of K products, K / 16 rounded additions deep."""
+    from dotllm_b200.kernels import gemm_skinny
+    g = torch.Generator().manual_seed(N * 7 + K)
+    x = torch.randn(8, K, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn((2 if gated else 1) * N, K, generator=g) * 0.05).to(torch.bfloat16).to(DEV)
+    y = gemm_skinny.run(x, w, torch.float32, fuse_swiglu=gated)
+    p = x.double() @ w.double().T
+    size = x.double().abs() @ w.double().abs().T
+    ref = torch.nn.functional.silu(p[:, :N]) * p[:, N:] if gated else p
+    # the gating multiplies an error of the gate by at most 1.1 |up| and one of the up product by at most |gate|
+    size = 1.1 * (size[:, :N] * (p[:, N:].abs() + 1e-3) + p[:, :N].abs() * size[:, N:]) if gated else size
+    assert ((y.double() - ref).abs() <= (K / 16 + 16) * 2 ** -24 * size + 1e-12).all()
+    assert torch.equal(gemm_skinny.run(x[:1].contiguous(), w, torch.float32, fuse_swiglu=gated), y[:1])
+    for _ in range(3):
+        assert torch.equal(gemm_skinny.run(x, w, torch.float32, fuse_swiglu=gated), y)
+
+
 @pytest.mark.parametrize("M,H,K,N2", [(8, 4096, 512, 1024), (1, 1000, 384, 272), (13, 1000, 384, 272), (16, 72, 64, 40),
                                       (17, 1000, 384, 272), (64, 4096, 512, 1024), (100, 1000, 4096, 272), (128, 72, 64, 40)])
 def test_products_that_add_and_normalise(M, H, K, N2, monkeypatch):
