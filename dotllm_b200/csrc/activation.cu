@@ -175,3 +175,9 @@ extern "C" int dl_head_gate(void* o, int o_stride, const void* gate, int gate_st
     DL_CHECK_LAUNCH("head_gate");
     return DL_OK;
 }
+
+DL_PACKED(dl_swiglu)
+DL_PACKED(dl_gated_activation)
+DL_PACKED(dl_unary_activation)
+DL_PACKED(dl_softcap)
+DL_PACKED(dl_head_gate)

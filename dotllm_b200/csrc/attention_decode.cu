@@ -1117,3 +1117,7 @@ extern "C" int dl_attention_decode_gated_bf16(const void* q, int q_stride, const
     return ad_dispatch(q, q_stride, out, out_stride, k_pool, v_pool, n_pages, seq_len, block_table, bt_stride, n_seqs, nh, nkv,
                        hd, scale, window, blocks, part_o, part_ml, part_slots, pair_counters, n_counters, fresh, status, stream);
 }
+
+DL_PACKED(dl_attention_decode_bf16)
+DL_PACKED(dl_attention_decode_fresh_bf16)
+DL_PACKED(dl_attention_decode_gated_bf16)

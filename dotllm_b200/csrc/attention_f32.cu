@@ -526,3 +526,6 @@ extern "C" int dl_attention_f32_split(const float* q, int q_stride, float* out, 
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "attention_f32_split: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_attention_f32_tile)
+DL_PACKED(dl_attention_f32_split)

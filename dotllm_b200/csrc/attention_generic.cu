@@ -288,3 +288,5 @@ extern "C" int dl_attention_generic(const void* q, int q_stride, void* out, int 
     DL_CHECK_LAUNCH("attention_generic");
     return DL_OK;
 }
+
+DL_PACKED(dl_attention_generic)

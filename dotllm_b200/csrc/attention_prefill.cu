@@ -431,3 +431,5 @@ extern "C" int dl_attention_prefill_bf16(const void* q, int q_stride, void* out,
 #undef AP_CASE
     return dl_fail(DL_ERR_UNSUPPORTED, "attention_prefill: head_dim %d (takes 32, 64, 96, 128)", hd);
 }
+
+DL_PACKED(dl_attention_prefill_bf16)

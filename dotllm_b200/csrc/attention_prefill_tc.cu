@@ -614,3 +614,5 @@ extern "C" int dl_attention_prefill_tc_bf16(const void* q, int q_stride, int n_t
 #undef PT_CASE
     return dl_fail(DL_ERR_UNSUPPORTED, "attention_prefill_tc: head_dim %d (takes 64 and 128)", hd);
 }
+
+DL_PACKED(dl_attention_prefill_tc_bf16)

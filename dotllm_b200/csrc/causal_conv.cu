@@ -160,3 +160,5 @@ extern "C" int dl_causal_conv(const void* x, int dtype, int ld, const float* tap
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "causal_conv: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_causal_conv)

@@ -683,3 +683,8 @@ int dl_delta_chunk(const float* q, const float* k, const float* v, const float* 
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "delta_chunk: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_chunk_pieces)
+DL_PACKED(dl_delta_chunk_scratch)
+DL_PACKED(dl_gla_chunk_scratch)
+DL_PACKED(dl_gla_chunk)

@@ -10,6 +10,9 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <math.h>
+#include <string.h>
+#include <type_traits>
+#include <utility>
 
 #define DL_PAGE 64            // tokens per cache page
 
@@ -31,6 +34,35 @@ int dl_fail(int status, const char* fmt, ...);
         if (e__ != cudaSuccess)                                                       \
             return dl_fail(DL_ERR_LAUNCH, "%s: %s", name, cudaGetErrorString(e__));   \
     } while (0)
+
+// The packed form of an entry point, for callers that know its signature only at run time (host/entry.cpp): the arguments as 64-bit
+// words, a float in the low half, and their kinds as letters.
+template <typename T> static inline T dl_unpack(unsigned long long word) {
+    T v;
+    static_assert(sizeof(T) <= 8, "arguments of at most 64 bits");
+    memcpy(&v, &word, sizeof(T));
+    return v;
+}
+template <typename T> static constexpr char dl_kind() {
+    return std::is_pointer<T>::value ? 'p' : std::is_same<T, float>::value ? 'f' : sizeof(T) == 8 ? 'l' : 'i';
+}
+template <typename... A, size_t... I>
+static inline int dl_call_packed(int (*fn)(A...), const unsigned long long* a, int n, std::index_sequence<I...>) {
+    if (n != (int)sizeof...(A)) return dl_fail(DL_ERR_ARGUMENT, "an entry point of %d arguments was called with %d", (int)sizeof...(A), n);
+    return fn(dl_unpack<A>(a[I])...);
+}
+template <typename... A> static inline int dl_call_packed(int (*fn)(A...), const unsigned long long* a, int n) {
+    return dl_call_packed(fn, a, n, std::index_sequence_for<A...>());
+}
+template <typename... A> static inline int dl_write_kinds(int (*)(A...), char* out, int room) {
+    const char kinds[] = {dl_kind<A>()..., 0};
+    if (room < (int)sizeof(kinds)) return -1;
+    memcpy(out, kinds, sizeof(kinds));
+    return (int)sizeof(kinds) - 1;
+}
+#define DL_PACKED(name)                                                                                              \
+    extern "C" int name##_packed(const unsigned long long* words, int n) { return dl_call_packed(name, words, n); }  \
+    extern "C" int name##_kinds(char* out, int room) { return dl_write_kinds(name, out, room); }
 
 // Programmatic dependent launch.  A kernel launched through dl_launch_dependent may begin while its
 // predecessor on the stream is still running: its blocks start as soon as every block of the

@@ -503,3 +503,5 @@ extern "C" int dl_delta_rule(const void* x, int ld, const void* taps, int K, int
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "delta_scan: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_delta_rule)

@@ -165,3 +165,7 @@ extern "C" int dl_embed_pairs(const void* table, const void* pairs, int dtype, c
     DL_CHECK_LAUNCH("embed_pairs");
     return DL_OK;
 }
+
+DL_PACKED(dl_gather_rows)
+DL_PACKED(dl_embed_positions)
+DL_PACKED(dl_embed_pairs)

@@ -482,3 +482,10 @@ extern "C" int dl_expert_combine(const float* y, int y_stride, const int32_t* pl
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "expert_combine: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_route_topk)
+DL_PACKED(dl_expert_gate_up)
+DL_PACKED(dl_expert_down)
+DL_PACKED(dl_expert_sort)
+DL_PACKED(dl_expert_gather)
+DL_PACKED(dl_expert_combine)

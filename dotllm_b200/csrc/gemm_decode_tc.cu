@@ -682,3 +682,6 @@ extern "C" int dl_gemm_decode_tc_bf16(const void* x, int x_stride, const void* w
 #undef GD_CASE
     return dl_fail(DL_ERR_UNSUPPORTED, "gemm_decode_tc: mode %d", p.mode);
 }
+
+DL_PACKED(dl_gemm_decode_tc_scratch)
+DL_PACKED(dl_gemm_decode_tc_bf16)

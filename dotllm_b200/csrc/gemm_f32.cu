@@ -203,3 +203,5 @@ extern "C" int dl_gemm_f32(const float* x, int x_stride, const float* w, float* 
     DL_CHECK_LAUNCH("gemm_f32");
     return DL_OK;
 }
+
+DL_PACKED(dl_gemm_f32)

@@ -665,3 +665,6 @@ extern "C" int dl_gemm_f32_tc(const float* x, int x_stride, const float* w, floa
     }
     return DL_OK;
 }
+
+DL_PACKED(dl_gemm_f32_tc_scratch)
+DL_PACKED(dl_gemm_f32_tc)

@@ -785,3 +785,8 @@ extern "C" int dl_gemm_skinny_static_status(int* code, void* stream) {
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "gemm_skinny_static_status: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_gemm_skinny_scratch)
+DL_PACKED(dl_gemm_skinny_bf16)
+DL_PACKED(dl_gemm_skinny_gated_bf16)
+DL_PACKED(dl_gemm_skinny_fused_bf16)

@@ -559,3 +559,8 @@ extern "C" int dl_gemm_tc_qkv_bf16(const void* x, int x_stride, const void* w, v
     return gt_launch<__nv_bfloat16, GT_QKV>((cudaStream_t)stream, x, x_stride, w, q_out, q_stride, M, q_cols + 2 * kv_cols, K, blocks,
                                             status, qkv);
 }
+
+DL_PACKED(dl_gemm_tc_bf16)
+DL_PACKED(dl_gemm_tc_gated_bf16)
+DL_PACKED(dl_gemm_tc_grouped_bf16)
+DL_PACKED(dl_gemm_tc_qkv_bf16)

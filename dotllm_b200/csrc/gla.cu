@@ -370,3 +370,6 @@ extern "C" int dl_head_norm_gate(const float* o, int o_stride, const void* g, in
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "head_norm_gate: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_gla_scan)
+DL_PACKED(dl_head_norm_gate)

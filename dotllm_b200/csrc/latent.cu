@@ -450,3 +450,8 @@ extern "C" int dl_per_head_rows(const void* x, int x_ld, int x_head, const void*
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "per_head_rows: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_latent_rows)
+DL_PACKED(dl_latent_query_tail)
+DL_PACKED(dl_channel_gate)
+DL_PACKED(dl_per_head_rows)

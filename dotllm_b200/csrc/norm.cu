@@ -419,3 +419,9 @@ extern "C" int dl_head_rmsnorm(const void* x, int x_stride, void* y, int y_strid
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "head_rmsnorm: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_add_rmsnorm)
+DL_PACKED(dl_branch_norm_add)
+DL_PACKED(dl_add_bias)
+DL_PACKED(dl_add_rows)
+DL_PACKED(dl_head_rmsnorm)

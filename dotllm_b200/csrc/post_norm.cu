@@ -262,3 +262,5 @@ extern "C" int dl_post_norm(float* x, const void* y, int y_dtype, int y_stride, 
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "post_norm: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_post_norm)

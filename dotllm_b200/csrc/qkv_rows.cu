@@ -175,3 +175,5 @@ extern "C" int dl_qkv_rows(const void* x, int dtype, int ld, const float* q_bias
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "qkv_rows: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_qkv_rows)

@@ -431,3 +431,5 @@ extern "C" int dl_rope_cache_write(void* q, int q_stride, const void* k, int k_s
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "rope_cache_write: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_rope_cache_write)

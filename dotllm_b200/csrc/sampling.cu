@@ -940,3 +940,6 @@ extern "C" int dl_repetition_penalty(float* logits, int row_stride, int rows, in
     DL_CHECK_LAUNCH("repetition_penalty");
     return DL_OK;
 }
+
+DL_PACKED(dl_sample)
+DL_PACKED(dl_repetition_penalty)

@@ -725,3 +725,7 @@ extern "C" int dl_gated_group_norm(const float* y, int y_ld, const void* g, int 
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "gated_group_norm: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_ssd_chunk)
+DL_PACKED(dl_ssd_scan)
+DL_PACKED(dl_gated_group_norm)

@@ -409,3 +409,10 @@ extern "C" int dl_scale_values(float* values, long long n, float factor, void* s
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "scale_values: %s", cudaGetErrorString(e));
     return DL_OK;
 }
+
+DL_PACKED(dl_stream_norm)
+DL_PACKED(dl_embed_copies)
+DL_PACKED(dl_stream_copies)
+DL_PACKED(dl_group_rmsnorm)
+DL_PACKED(dl_pair_norm_sum)
+DL_PACKED(dl_scale_values)

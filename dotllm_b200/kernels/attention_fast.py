@@ -68,12 +68,12 @@ def _decode(q, q_stride, out, k_pool, v_pool, n_pages, block_table, n_heads, n_k
     group = n_heads // tiles
     part_o, part_ml, slots = _decode_scratch(plan, group, head_dim, q.device)
     counters = _pair_counters(q.device)
-    _library.call("dl_attention_decode_bf16", q.data_ptr(), q_stride, out.data_ptr(), out.stride(0),
-                  k_pool.data_ptr(), v_pool.data_ptr(), n_pages, plan.seq_total.data_ptr(),
-                  block_table.data_ptr(), block_table.shape[1], B, n_heads, tiles, head_dim,
-                  scale, window, int(keep_first), None if sinks is None else sinks.data_ptr(), float(softcap),
-                  None if slopes is None else slopes.data_ptr(), *_gate_args(gate), n_kv_heads, DECODE_BLOCKS,
-                  part_o.data_ptr(), part_ml.data_ptr(), slots, counters.data_ptr(), counters.numel(),
+    _library.call("dl_attention_decode_bf16", q, q_stride, out, out.stride(0),
+                  k_pool, v_pool, n_pages, plan.seq_total,
+                  block_table, block_table.shape[1], B, n_heads, tiles, head_dim,
+                  scale, window, int(keep_first), sinks, float(softcap),
+                  slopes, *_gate_args(gate), n_kv_heads, DECODE_BLOCKS,
+                  part_o, part_ml, slots, counters, counters.numel(),
                   _library.status_word(q.device).data_ptr(), _library.current_stream())
     return True
 
@@ -92,7 +92,7 @@ def _pair_counters(device):
 
 
 def _decode_scratch(plan, group, head_dim, device):
-    slots = 2 * max(1, _library.library().dl_sm_count())
+    slots = 2 * max(1, _library.sm_count())
     key = ("decode", group, head_dim)
     if key not in plan.scratch:
         plan.scratch[key] = (torch.empty(slots * group * head_dim, dtype=torch.float32, device=device),
@@ -137,27 +137,27 @@ def decode_fresh(q, k, v, cos, sin, rotary_dim, block_table, k_pool, v_pool, n_h
                        or cos.data_ptr() % 16 or sin.data_ptr() % 16):
         return None
     B = plan.n_seqs
-    out = torch.empty((B, n_heads * head_dim), dtype=q.dtype, device=q.device)
+    out = _library.empty(B, n_heads * head_dim, q.dtype, q)
     part_o, part_ml, slots = _decode_scratch(plan, group, head_dim, q.device)
     counters = _pair_counters(q.device)
     if extras:
         qb, kb, vb = biases if biases is not None else (None, None, None)
         ptr = lambda t: None if t is None else t.data_ptr()
-        _library.call("dl_attention_decode_gated_bf16", q.data_ptr(), qs, ptr(k), ks, ptr(v), vs,
-                      cos.data_ptr() if rotary_dim else None, sin.data_ptr() if rotary_dim else None,
-                      cos.shape[0] if rotary_dim else 0, 1 if rotary_dim else 0, ptr(qb), ptr(kb) if k is not None else None,
-                      ptr(vb) if k is not None else None, ptr(gate), rows(gate) if gate is not None else 0, ptr(sinks), float(softcap), ptr(slopes), n_kv_heads,
-                      out.data_ptr(), out.stride(0), k_pool.data_ptr(), v_pool.data_ptr(), k_pool.shape[0],
-                      plan.seq_total.data_ptr(), block_table.data_ptr(), block_table.shape[1], B, n_heads, tiles, head_dim,
-                      scale, window, DECODE_BLOCKS, part_o.data_ptr(), part_ml.data_ptr(), slots, counters.data_ptr(),
+        _library.call("dl_attention_decode_gated_bf16", q, qs, k, ks, v, vs,
+                      cos if rotary_dim else None, sin if rotary_dim else None,
+                      cos.shape[0] if rotary_dim else 0, 1 if rotary_dim else 0, qb, kb if k is not None else None,
+                      vb if k is not None else None, gate, rows(gate) if gate is not None else 0, sinks, float(softcap), slopes, n_kv_heads,
+                      out, out.stride(0), k_pool, v_pool, k_pool.shape[0],
+                      plan.seq_total, block_table, block_table.shape[1], B, n_heads, tiles, head_dim,
+                      scale, window, DECODE_BLOCKS, part_o, part_ml, slots, counters,
                       counters.numel(), _library.status_word(q.device).data_ptr(), _library.current_stream())
         return out
-    _library.call("dl_attention_decode_fresh_bf16", q.data_ptr(), qs, k.data_ptr(), ks, v.data_ptr(), vs,
-                  cos.data_ptr() if rotary_dim else None, sin.data_ptr() if rotary_dim else None,
-                  cos.shape[0] if rotary_dim else 0, 1 if rotary_dim else 0, out.data_ptr(), out.stride(0),
-                  k_pool.data_ptr(), v_pool.data_ptr(), k_pool.shape[0], plan.seq_total.data_ptr(),
-                  block_table.data_ptr(), block_table.shape[1], B, n_heads, n_kv_heads, head_dim, scale, window,
-                  DECODE_BLOCKS, part_o.data_ptr(), part_ml.data_ptr(), slots, counters.data_ptr(), counters.numel(),
+    _library.call("dl_attention_decode_fresh_bf16", q, qs, k, ks, v, vs,
+                  cos if rotary_dim else None, sin if rotary_dim else None,
+                  cos.shape[0] if rotary_dim else 0, 1 if rotary_dim else 0, out, out.stride(0),
+                  k_pool, v_pool, k_pool.shape[0], plan.seq_total,
+                  block_table, block_table.shape[1], B, n_heads, n_kv_heads, head_dim, scale, window,
+                  DECODE_BLOCKS, part_o, part_ml, slots, counters, counters.numel(),
                   _library.status_word(q.device).data_ptr(), _library.current_stream())
     return out
 
@@ -183,19 +183,19 @@ def _prefill(q, q_stride, out, k_pool, v_pool, n_pages, block_table, n_heads, n_
         and (PREFILL_TC_SPECIAL or (not keep_first and sinks is None)) and (slopes is None or softcap <= 0)
     tile_seq, tile_row0, n_tiles = _prompt_tiles(plan, PREFILL_TC_ROWS if tc else PREFILL_ROWS, q.device)
     if tc:
-        _library.call("dl_attention_prefill_tc_bf16", q.data_ptr(), q_stride, q.shape[0], out.data_ptr(), out.stride(0),
-                      k_pool.data_ptr(), v_pool.data_ptr(), n_pages, tile_seq.data_ptr(), tile_row0.data_ptr(),
-                      n_tiles, plan.seq_start.data_ptr(), plan.seq_new.data_ptr(), plan.cu_new.data_ptr(),
-                      block_table.data_ptr(), block_table.shape[1], n_heads, n_kv_heads, head_dim, scale, window,
-                      int(keep_first), None if sinks is None else sinks.data_ptr(), float(softcap),
-                      None if slopes is None else slopes.data_ptr(), *_gate_args(gate), _library.status_word(q.device).data_ptr(), _library.current_stream())
+        _library.call("dl_attention_prefill_tc_bf16", q, q_stride, q.shape[0], out, out.stride(0),
+                      k_pool, v_pool, n_pages, tile_seq, tile_row0,
+                      n_tiles, plan.seq_start, plan.seq_new, plan.cu_new,
+                      block_table, block_table.shape[1], n_heads, n_kv_heads, head_dim, scale, window,
+                      int(keep_first), sinks, float(softcap),
+                      slopes, *_gate_args(gate), _library.status_word(q.device).data_ptr(), _library.current_stream())
         return True
-    _library.call("dl_attention_prefill_bf16", q.data_ptr(), q_stride, out.data_ptr(), out.stride(0),
-                  k_pool.data_ptr(), v_pool.data_ptr(), n_pages, tile_seq.data_ptr(), tile_row0.data_ptr(),
-                  n_tiles, plan.seq_start.data_ptr(), plan.seq_new.data_ptr(), plan.cu_new.data_ptr(),
-                  block_table.data_ptr(), block_table.shape[1], n_heads, n_kv_heads, head_dim, scale, window,
-                  int(keep_first), None if sinks is None else sinks.data_ptr(), float(softcap),
-                  None if slopes is None else slopes.data_ptr(), *_gate_args(gate), _library.status_word(q.device).data_ptr(), _library.current_stream())
+    _library.call("dl_attention_prefill_bf16", q, q_stride, out, out.stride(0),
+                  k_pool, v_pool, n_pages, tile_seq, tile_row0,
+                  n_tiles, plan.seq_start, plan.seq_new, plan.cu_new,
+                  block_table, block_table.shape[1], n_heads, n_kv_heads, head_dim, scale, window,
+                  int(keep_first), sinks, float(softcap),
+                  slopes, *_gate_args(gate), _library.status_word(q.device).data_ptr(), _library.current_stream())
     return True
 
 
@@ -250,7 +250,7 @@ def run_f32(q, q_stride, out, k_pool, v_pool, n_pages, token_seq, token_pos, blo
 
     pools = (k_pool.data_ptr(), v_pool.data_ptr(), n_pages)
     T = q.shape[0]
-    few = sum(-(-n // F32_TILE_ROWS) for n in plan.news) * n_heads <= _library.library().dl_sm_count()
+    few = sum(-(-n // F32_TILE_ROWS) for n in plan.news) * n_heads <= _library.sm_count()
     if plan.max_new <= (F32_SPLIT_TOKENS_FEW if few else F32_SPLIT_TOKENS):
         a_token = n_heads * block_table.shape[1]           # parts
         at_once = max(1, min(T, 65535, F32_PARTS_BYTES // (4 * a_token * (head_dim + 2))))
@@ -261,13 +261,13 @@ def run_f32(q, q_stride, out, k_pool, v_pool, n_pages, token_seq, token_pos, blo
         parts = (plan.scratch[key].data_ptr(), plan.scratch[key].data_ptr() + 4 * n * head_dim)
         for lo in range(0, T, at_once):
             _library.call("dl_attention_f32_split", q.data_ptr() + 4 * lo * q_stride, q_stride, out.data_ptr() + 4 * lo * out.stride(0), out.stride(0),
-                          *pools, token_seq.data_ptr() + 4 * lo, token_pos.data_ptr() + 4 * lo, block_table.data_ptr(), block_table.shape[1],
+                          *pools, token_seq.data_ptr() + 4 * lo, token_pos.data_ptr() + 4 * lo, block_table, block_table.shape[1],
                           min(at_once, T - lo), *tail(None if gate is None else gate[lo:]), *parts, _library.current_stream())
         return True
     tile_seq, tile_row0, n_tiles = _prompt_tiles(plan, F32_TILE_ROWS, q.device)
     if n_tiles > 65535:
         return False
-    _library.call("dl_attention_f32_tile", q.data_ptr(), q_stride, out.data_ptr(), out.stride(0), *pools, tile_seq.data_ptr(), tile_row0.data_ptr(), n_tiles, plan.seq_start.data_ptr(),
-                  plan.seq_new.data_ptr(), plan.cu_new.data_ptr(), block_table.data_ptr(), block_table.shape[1], *tail(gate),
+    _library.call("dl_attention_f32_tile", q, q_stride, out, out.stride(0), *pools, tile_seq, tile_row0, n_tiles, plan.seq_start,
+                  plan.seq_new, plan.cu_new, block_table, block_table.shape[1], *tail(gate),
                   _library.current_stream())
     return True

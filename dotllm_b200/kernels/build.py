@@ -172,5 +172,43 @@ def build(verbose=True, ptxas_info=False):
         return out_dir / LIB_NAME
 
 
+ENTRY = "dotllm_entry"                     # the CPython module of csrc/host/entry.cpp
+
+
+def build_entry(verbose=True):
+    """The module that calls the library's entry points from Python (csrc/host/entry.cpp), built beside the library with the host
+    compiler; its path.  It depends on the interpreter and on torch, so both are part of what decides whether it is current."""
+    import sysconfig
+    import torch
+    source = CSRC / "host" / "entry.cpp"
+    root = Path(torch.__file__).resolve().parent
+    cuda = str(Path(find_nvcc()).resolve().parent.parent / "include") if shutil.which("nvcc") or os.environ.get("NVCC") else "/usr/local/cuda/include"
+    flags = ["-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    digest = _digest([source], " ".join(flags) + torch.__version__ + sys.version)
+    for folder in (CSRC / "_build", None):
+        folder = folder or build_dir()
+        so, mark = folder / (ENTRY + ".so"), folder / (ENTRY + ".digest")
+        if so.is_file() and mark.is_file() and mark.read_text() == digest:
+            return so
+    import fcntl
+    with open(folder / ".lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        if so.is_file() and mark.is_file() and mark.read_text() == digest:
+            return so
+        t0 = time.time()
+        cmd = [os.environ.get("CXX") or shutil.which("g++") or "c++", *flags, "-I", str(root / "include"), "-I", str(root / "include/torch/csrc/api/include"),
+               "-I", sysconfig.get_paths()["include"], "-I", cuda, str(source), "-o", str(so) + ".tmp", "-L", str(root / "lib"),
+               "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise KernelError(f"the host compiler failed on {source.name}:\n{res.stdout}\n{res.stderr}")
+        os.replace(str(so) + ".tmp", so)
+        mark.write_text(digest)
+        if verbose:
+            _log(f"built {so.name} in {time.time() - t0:.0f} s")
+    return so
+
+
 if __name__ == "__main__":
     print(build(ptxas_info="-v" in sys.argv))
+    print(build_entry())

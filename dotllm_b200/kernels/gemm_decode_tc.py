@@ -36,7 +36,7 @@ def scratch_need(M, N, K, gated=False, sms=148):
 def _device_state(device):
     key = device.index
     if key not in _state:
-        sms = _library.library().dl_sm_count()
+        sms = _library.sm_count()
         counters = torch.zeros(_MAX_TILES, dtype=torch.int32, device=device)
         _library.register_counters(counters)
         # Two parts per block of at most 256 accumulator columns by 128 outputs: the largest product
@@ -65,19 +65,19 @@ def run(x, w, out_dtype, fuse_swiglu=False, resident=False, row_sums=None, into=
     sums_in, parts, width, eps = row_sums if row_sums is not None else (None, 0, 1, 0.0)
     if into is not None:
         stream, gain = into
-        scaled = torch.empty((M, n_out), dtype=torch.bfloat16, device=x.device)
+        scaled = _library.empty(M, n_out, torch.bfloat16, x)
         sums_out = torch.empty(((n_out + 127) // 128) * SUM_STRIDE, dtype=torch.float32, device=x.device)
         out, out_stride, result = stream, stream.stride(0), (scaled, sums_out)
     else:
         gain = scaled = sums_out = None
-        out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
+        out = _library.empty(M, n_out, out_dtype, x)
         out_stride, result = n_out, out
-    _library.call("dl_gemm_decode_tc_bf16", x.data_ptr(), x_stride, w.data_ptr(), out.data_ptr(),
+    _library.call("dl_gemm_decode_tc_bf16", x, x_stride, w, out,
                   0 if out.dtype == torch.float32 else 1, out_stride, M, n_out, K, flags,
-                  gain.data_ptr() if gain is not None else None, scaled.data_ptr() if scaled is not None else None, n_out,
-                  sums_out.data_ptr() if sums_out is not None else None,
-                  sums_in.data_ptr() if sums_in is not None else None, parts, 1.0 / width, float(eps),
-                  None if bias is None else bias.data_ptr(), partials.data_ptr(), partials.numel(), counters.data_ptr(),
+                  gain, scaled, n_out,
+                  sums_out,
+                  sums_in, parts, 1.0 / width, float(eps),
+                  bias, partials, partials.numel(), counters,
                   counters.numel(),
                   _library.status_word(x.device).data_ptr(), _library.current_stream())
     return result

@@ -41,14 +41,14 @@ def run(x, x_stride, w, resident=False):
     """y = x W^T, float32 [M, N]; x [M, K] with rows ``x_stride`` apart."""
     M, K = x.shape
     N = w.shape[0]
-    y = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    y = _library.empty(M, N, torch.float32, x)
     if M == 0:
         return y
     if M <= SELF_SPLIT and (x_stride % 4 or x.data_ptr() % 16):
-        x, x_stride = torch.empty((M, K), dtype=torch.float32, device=x.device).copy_(x), K
-    n_planes, n_sums = scratch_need(M, N, K, _library.library().dl_sm_count())
+        x, x_stride = _library.empty(M, K, torch.float32, x).copy_(x), K
+    n_planes, n_sums = scratch_need(M, N, K, _library.sm_count())
     scratch = torch.empty(n_sums + (n_planes + 1) // 2, dtype=torch.float32, device=x.device) if n_sums or n_planes else None
     at = 0 if scratch is None else scratch.data_ptr()      # the planes (a multiple of 8 values a row) in front, the sums behind
-    _library.call("dl_gemm_f32_tc", x.data_ptr(), x_stride, w.data_ptr(), y.data_ptr(), N, M, N, K, at, n_planes, at + 2 * n_planes, n_sums,
+    _library.call("dl_gemm_f32_tc", x, x_stride, w, y, N, M, N, K, at, n_planes, at + 2 * n_planes, n_sums,
                   1 if resident else 0, _library.status_word(x.device).data_ptr(), _library.current_stream())
     return y

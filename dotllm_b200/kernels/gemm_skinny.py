@@ -45,11 +45,11 @@ _state = {}
 def _device_state(device):
     key = device.index
     if key not in _state:
-        sms = _library.library().dl_sm_count()
+        sms = _library.sm_count()
         counters = torch.zeros(_MAX_TILES, dtype=torch.int32, device=device)
         _library.register_counters(counters)
         partials = torch.empty(max(sms, 1) * CONSUMER_WARPS * 2 * 2 * 128, dtype=torch.float32, device=device)
-        _state[key] = (counters, partials, sms)
+        _state[key] = (counters, partials, _library.status_word(device))
     return _state[key]
 
 
@@ -70,41 +70,42 @@ def takes(x, w, fuse_swiglu=False, max_rows=None):
             and w.data_ptr() % 16 == 0 and tiles <= _MAX_TILES)
 
 
-def run(x, w, out_dtype, fuse_swiglu=False, resident=False, row_sums=None, into=None):
+def run(x, w, out_dtype, fuse_swiglu=False, resident=False, row_sums=None, into=None, sizes=None):
     """``row_sums`` = (sums float32 [parts * 16], parts, width, eps): x is a stream times a norm's gain,
     and every output row is multiplied by rsqrt(sum of the row's parts / width + eps); the sums must come
     from a product of the same number of rows (``sum_stride``).
     ``into`` = (stream float32 [M, N], gain float32 [N]): the product is added into the stream in place;
-    returns (stream * gain as bfloat16 [M, N], sums of squares float32 [ceil(N / 16) * 16])."""
-    M, K = x.shape
+    returns (stream * gain as bfloat16 [M, N], sums of squares float32 [ceil(N / 16) * 16]).
+    ``sizes``: of x and w, where the caller has them (``product`` in csrc/host/entry.cpp)."""
+    M, K, N, x_stride = sizes[:4] if sizes is not None else (*x.shape, w.shape[0], None)
     if M > SKINNY_ROWS:
         return gemm_decode_tc.run(x, w, out_dtype, fuse_swiglu, resident, row_sums, into)
-    n_out = w.shape[0] // 2 if fuse_swiglu else w.shape[0]
-    counters, partials, sms = _device_state(x.device)
-    x_stride = x.stride(0) if M > 1 else max(K, x.stride(0))
+    n_out = N // 2 if fuse_swiglu else N
+    counters, partials, status = _device_state(x.device)
+    if x_stride is None:
+        x_stride = x.stride(0) if M > 1 else max(K, x.stride(0))
     flags = (1 if fuse_swiglu else 0) | (2 if resident else 0)
-    tail = (partials.data_ptr(), partials.numel(), counters.data_ptr(), counters.numel(),
-            _library.status_word(x.device).data_ptr(), _library.current_stream())
+    tail = (partials, partials.numel(), counters, _MAX_TILES, status, _library.current_stream())
     if row_sums is None and into is None:
-        out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
-        _library.call("dl_gemm_skinny_bf16", x.data_ptr(), x_stride, w.data_ptr(), out.data_ptr(),
-                      0 if out_dtype == torch.float32 else 1, n_out, M, n_out, K, flags, *tail)
+        half = out_dtype == torch.bfloat16
+        out = _library.empty(M, n_out, out_dtype, x)
+        _library.call("dl_gemm_skinny_bf16", x, x_stride, w, out, 1 if half else 0, n_out, M, n_out, K, flags, *tail)
         return out
     sums_in, parts, width, eps = row_sums if row_sums is not None else (None, 0, 1, 0.0)
     if into is not None:
         stream, gain = into
-        scaled = torch.empty((M, n_out), dtype=torch.bfloat16, device=x.device)
+        scaled = _library.empty(M, n_out, torch.bfloat16, x)
         sums_out = torch.empty(((n_out + 15) // 16) * 16, dtype=torch.float32, device=x.device)
         out, out_stride, result = stream, stream.stride(0), (scaled, sums_out)
     else:
         gain = scaled = sums_out = None
-        out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
+        out = _library.empty(M, n_out, out_dtype, x)
         out_stride, result = n_out, out
-    _library.call("dl_gemm_skinny_fused_bf16", x.data_ptr(), x_stride, w.data_ptr(), out.data_ptr(),
+    _library.call("dl_gemm_skinny_fused_bf16", x, x_stride, w, out,
                   0 if out.dtype == torch.float32 else 1, out_stride, M, n_out, K, flags,
-                  gain.data_ptr() if gain is not None else None, scaled.data_ptr() if scaled is not None else None, n_out,
-                  sums_out.data_ptr() if sums_out is not None else None,
-                  sums_in.data_ptr() if sums_in is not None else None, parts, 1.0 / width, float(eps), *tail)
+                  gain, scaled, n_out,
+                  sums_out,
+                  sums_in, parts, 1.0 / width, float(eps), *tail)
     return result
 
 
@@ -118,12 +119,12 @@ def run_gating(x, w, gate_kind, limit, alpha, resident=False, bias=None):
     [2N] or None)."""
     M, K = x.shape
     n_out = w.shape[0] // 2
-    counters, partials, sms = _device_state(x.device)
+    counters, partials, status = _device_state(x.device)
     x_stride = x.stride(0) if M > 1 else max(K, x.stride(0))
-    out = torch.empty((M, n_out), dtype=x.dtype, device=x.device)
-    _library.call("dl_gemm_skinny_gated_bf16", x.data_ptr(), x_stride, w.data_ptr(), out.data_ptr(), 1, n_out, M, n_out, K,
-                  1 | (2 if resident else 0), int(gate_kind), float(limit), float(alpha), None if bias is None else bias.data_ptr(), partials.data_ptr(), partials.numel(),
-                  counters.data_ptr(), counters.numel(), _library.status_word(x.device).data_ptr(), _library.current_stream())
+    out = _library.empty(M, n_out, x.dtype, x)
+    _library.call("dl_gemm_skinny_gated_bf16", x, x_stride, w, out, 1, n_out, M, n_out, K,
+                  1 | (2 if resident else 0), int(gate_kind), float(limit), float(alpha), bias, partials, partials.numel(),
+                  counters, counters.numel(), status, _library.current_stream())
     return out
 
 
@@ -131,12 +132,12 @@ def run_activated(x, w, kind, resident=False):
     """act(x W^T) in x's dtype for W [N, K] and an activation of one product (``ops.UNGATED``) in the product's epilogue."""
     M, K = x.shape
     n_out = w.shape[0]
-    counters, partials, sms = _device_state(x.device)
+    counters, partials, status = _device_state(x.device)
     x_stride = x.stride(0) if M > 1 else max(K, x.stride(0))
-    out = torch.empty((M, n_out), dtype=x.dtype, device=x.device)
-    _library.call("dl_gemm_skinny_gated_bf16", x.data_ptr(), x_stride, w.data_ptr(), out.data_ptr(), 1, n_out, M, n_out, K,
-                  2 if resident else 0, int(kind), 0.0, 0.0, None, partials.data_ptr(), partials.numel(),
-                  counters.data_ptr(), counters.numel(), _library.status_word(x.device).data_ptr(), _library.current_stream())
+    out = _library.empty(M, n_out, x.dtype, x)
+    _library.call("dl_gemm_skinny_gated_bf16", x, x_stride, w, out, 1, n_out, M, n_out, K,
+                  2 if resident else 0, int(kind), 0.0, 0.0, None, partials, partials.numel(),
+                  counters, counters.numel(), status, _library.current_stream())
     return out
 
 
@@ -147,9 +148,12 @@ def scratch_need(M, N, K, fuse_swiglu=False, sms=148):
     return a.value, b.value
 
 
-def maybe_run(x, w, out_dtype, fuse_swiglu=False, resident=False):
+def maybe_run(x, w, out_dtype, fuse_swiglu=False, resident=False, sizes=None):
     """y = x W^T (or the gated form) by the skinny kernel when it takes the sizes, else None.
-    ``resident``: no work still pending on the stream writes W."""
-    if not takes(x, w, fuse_swiglu):
+    ``resident``: no work still pending on the stream writes W.  ``sizes`` as in ``run``: they say all that ``takes`` would look up."""
+    if sizes is not None and sizes[0] <= SKINNY_ROWS:
+        if sizes[4] != 2 or sizes[2] > 16 * _MAX_TILES:
+            return None
+    elif not takes(x, w, fuse_swiglu):
         return None
-    return run(x, w, out_dtype, fuse_swiglu, resident)
+    return run(x, w, out_dtype, fuse_swiglu, resident, sizes=sizes)

@@ -36,8 +36,8 @@ def takes(x, w, fuse_swiglu=False):
 def run(x, w, out_dtype, fuse_swiglu=False):
     M, K = x.shape
     n_out = w.shape[0] // 2 if fuse_swiglu else w.shape[0]
-    out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
-    _library.call("dl_gemm_tc_bf16", x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(),
+    out = _library.empty(M, n_out, out_dtype, x)
+    _library.call("dl_gemm_tc_bf16", x, x.stride(0), w, out,
                   0 if out_dtype == torch.float32 else 1, n_out, M, n_out, K, 1 if fuse_swiglu else 0, BLOCKS,
                   _library.status_word(x.device).data_ptr(), _library.current_stream())
     return out
@@ -48,9 +48,9 @@ def run_gated(x, w, gate_kind, limit, alpha, bias=None):
     ``bias`` (float32 [2N] or None)."""
     M, K = x.shape
     n_out = w.shape[0] // 2
-    out = torch.empty((M, n_out), dtype=torch.bfloat16, device=x.device)
-    _library.call("dl_gemm_tc_gated_bf16", x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), n_out, M, n_out, K,
-                  int(gate_kind), float(limit), float(alpha), None if bias is None else bias.data_ptr(), BLOCKS, _library.status_word(x.device).data_ptr(),
+    out = _library.empty(M, n_out, torch.bfloat16, x)
+    _library.call("dl_gemm_tc_gated_bf16", x, x.stride(0), w, out, n_out, M, n_out, K,
+                  int(gate_kind), float(limit), float(alpha), bias, BLOCKS, _library.status_word(x.device).data_ptr(),
                   _library.current_stream())
     return out
 
@@ -59,8 +59,8 @@ def run_activated(x, w, kind):
     """act(x W^T) for W [N, K] and an activation of one product (``ops.UNGATED``) in the product's epilogue."""
     M, K = x.shape
     n_out = w.shape[0]
-    out = torch.empty((M, n_out), dtype=torch.bfloat16, device=x.device)
-    _library.call("dl_gemm_tc_gated_bf16", x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), n_out, M, n_out, K,
+    out = _library.empty(M, n_out, torch.bfloat16, x)
+    _library.call("dl_gemm_tc_gated_bf16", x, x.stride(0), w, out, n_out, M, n_out, K,
                   int(kind), 0.0, 0.0, None, BLOCKS, _library.status_word(x.device).data_ptr(), _library.current_stream())
     return out
 
@@ -78,9 +78,9 @@ def takes_qkv(x, w, q_cols, kv_cols, head_dim, rotary_dim, cos, sin, k_pool, v_p
 def run_qkv(x, w, q_cols, kv_cols, head_dim, n_kv_heads, cos, sin, token_pos, token_seq, block_table, k_pool, v_pool):
     """The rotated queries [M, q_cols]; the rotated keys and the values are in the cache when the kernel is done."""
     M, K = x.shape
-    q = torch.empty((M, q_cols), dtype=torch.bfloat16, device=x.device)
-    _library.call("dl_gemm_tc_qkv_bf16", x.data_ptr(), x.stride(0), w.data_ptr(), q.data_ptr(), q_cols, M, K, q_cols, kv_cols,
-                  head_dim, n_kv_heads, cos.data_ptr(), sin.data_ptr(), cos.shape[0], token_pos.data_ptr(), token_seq.data_ptr(),
-                  block_table.data_ptr(), block_table.shape[1], k_pool.data_ptr(), v_pool.data_ptr(), k_pool.shape[0], BLOCKS,
+    q = _library.empty(M, q_cols, torch.bfloat16, x)
+    _library.call("dl_gemm_tc_qkv_bf16", x, x.stride(0), w, q, q_cols, M, K, q_cols, kv_cols,
+                  head_dim, n_kv_heads, cos, sin, cos.shape[0], token_pos, token_seq,
+                  block_table, block_table.shape[1], k_pool, v_pool, k_pool.shape[0], BLOCKS,
                   _library.status_word(x.device).data_ptr(), _library.current_stream())
     return q

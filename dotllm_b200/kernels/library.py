@@ -1,4 +1,4 @@
-"""Loads the compiled kernel library through ctypes and declares its entry points.
+"""Loads the compiled kernel library, declares its entry points, and calls them (through csrc/host/entry.cpp).
 
 There is no fallback: if the library cannot be built or loaded, or the device is not
 sm_100, every call raises ``KernelError``.
@@ -30,6 +30,9 @@ _SIGNATURES = {
 _lock = threading.Lock()
 _lib = None
 _checked_device = False
+_entry = None                # the CPython module of csrc/host/entry.cpp
+_callables = {}              # entry point -> its callable
+_KINDS = {_P: "p", _I: "i", _F: "f", ctypes.c_long: "l", ctypes.c_longlong: "l"}
 
 
 def declare(lib, signatures):
@@ -78,6 +81,39 @@ def register_signatures(signatures):
         declare(_lib, signatures)
 
 
+def entry():
+    """The module that calls the library's entry points (built on first use, like the library): tensors are passed as they are."""
+    global _entry
+    if _entry is None:
+        import importlib.machinery
+        import importlib.util
+        from . import build
+        lib = library()
+        with _lock:
+            if _entry is None:
+                path = str(build.build_entry())
+                loader = importlib.machinery.ExtensionFileLoader(build.ENTRY, path)
+                try:
+                    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location(build.ENTRY, path, loader=loader))
+                    loader.exec_module(module)
+                except ImportError as exc:
+                    raise KernelError(f"cannot load {path}: {exc}") from exc
+                module.handle = lib._handle
+                _entry = module
+    return _entry
+
+
+def _bind(name):
+    """The callable of an entry point, whose own kinds of arguments must be the declared ones."""
+    module = entry()
+    declared = "".join(_KINDS[t] for t in _SIGNATURES[name])
+    found = module.kinds(module.handle, name)
+    if found != declared:
+        raise KernelError(f"{name}: the library's arguments ({found}) are not the declared ones ({declared})")
+    _callables[name] = fn = module.bind(module.handle, name)
+    return fn
+
+
 def require_device():
     """Raise unless the current CUDA device can run the sm_100a kernels."""
     global _checked_device
@@ -101,29 +137,51 @@ def set_dependent_launch(on):
     library().dl_set_dependent_launch(1 if on else 0)
 
 
-_raw_stream = None
-
-
 def current_stream():
     """The current CUDA stream's handle, for a kernel launch.  ``torch.cuda.current_stream()`` builds
     a Python stream object after several device-index and environment look-ups, 10 - 15 us a call with
-    a few hundred launches a step; the handle alone comes from the binding underneath it."""
-    global _raw_stream
-    if _raw_stream is None:
+    a few hundred launches a step."""
+    return (_entry or entry()).stream()
+
+
+_empty_kinds = None
+
+
+def empty(rows, width, dtype, like):
+    """A contiguous [rows, width] tensor on ``like``'s device: ``torch.empty`` without its parsing of arguments for the two types that
+    kernels write most."""
+    global _empty_kinds
+    if _empty_kinds is None:
         import torch
-        raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
-        if raw is not None and device is not None:
-            _raw_stream = lambda: raw(device())
-        else:
-            _raw_stream = lambda: torch.cuda.current_stream().cuda_stream
-    return _raw_stream()
+        _empty_kinds = {torch.float32: False, torch.bfloat16: True}
+    half = _empty_kinds.get(dtype)
+    if half is None or _entry is None:
+        import torch
+        return torch.empty((rows, width), dtype=dtype, device=like.device)
+    return _entry.empty(rows, width, half, like)
 
 
 def call(name, *args):
-    lib = library()
-    status = getattr(lib, name)(*args)
+    """Call an entry point; pointers may be given as tensors (their first element), as addresses or as None."""
+    fn = _callables.get(name)
+    status = (fn or _bind(name))(*args)
     if status != 0:
-        raise KernelError(f"{name}: {lib.dl_last_error().decode(errors='replace')} (status {status})")
+        raise KernelError(f"{name}: {library().dl_last_error().decode(errors='replace')} (status {status})")
+
+
+_sm_counts = {}
+
+
+def sm_count():
+    """Multiprocessors of the current device (0 without one)."""
+    import torch
+    device = torch._C._cuda_getDevice() if torch.cuda.is_initialized() else None
+    if device not in _sm_counts:
+        count = library().dl_sm_count()
+        if device is None:
+            return count
+        _sm_counts[device] = count
+    return _sm_counts[device]
 
 
 _status = {}

@@ -74,6 +74,8 @@ def _stream():
 
 
 def _need_cuda(*tensors):
+    if _library._checked_device and _library._entry is not None and _library._entry.all_cuda(*tensors):
+        return
     for t in tensors:
         if t is not None and not t.is_cuda:
             raise KernelError("kernels run on CUDA tensors only: there is no CPU fallback")
@@ -86,6 +88,10 @@ def _ptr(t):
 
 def _rows_view(t, what):
     """A 2-D tensor whose rows are contiguous (a column slice of a wider matrix is fine)."""
+    if _library._entry is not None:
+        stride = _library._entry.row_stride(t)
+        if stride >= 0:
+            return stride
     if t.dim() != 2 or (t.shape[1] > 1 and t.stride(1) != 1):
         raise KernelError(f"{what}: need a 2-D tensor with contiguous rows, got shape "
                           f"{tuple(t.shape)} strides {t.stride()}")
@@ -108,12 +114,12 @@ def gather_rows(table, ids, out=None, out_dtype=torch.float32):
     n, width = table.shape
     rows = ids.numel()
     if out is None:
-        out = torch.empty((rows, width), dtype=out_dtype, device=table.device)
+        out = _library.empty(rows, width, out_dtype, table)
     elif out.shape != (rows, width) or out.dtype != out_dtype or not out.is_contiguous():
         raise KernelError(f"gather_rows: out must be contiguous {out_dtype} [rows, width]")
     if out_dtype != torch.float32 and out_dtype != table.dtype:
         raise KernelError(f"gather_rows: rows of {table.dtype} are gathered as float32 or as they are, not as {out_dtype}")
-    _library.call("dl_gather_rows", _ptr(table), _code(table.dtype), stride, _ptr(ids), _ptr(out), _code(out_dtype),
+    _library.call("dl_gather_rows", table, _code(table.dtype), stride, ids, out, _code(out_dtype),
                   rows, width, n, _stream())
     return out
 
@@ -130,9 +136,9 @@ def embed_positions(table, pos_table, ids, positions):
     rows = ids.numel()
     if positions.numel() != rows:
         raise KernelError("embed_positions: one position per id")
-    out = torch.empty((rows, table.shape[1]), dtype=torch.float32, device=table.device)
-    _library.call("dl_embed_positions", _ptr(table), _ptr(pos_table), _code(table.dtype), _ptr(ids), _ptr(positions),
-                  _ptr(out), rows, table.shape[1], table.shape[0], pos_table.shape[0], _stream())
+    out = _library.empty(rows, table.shape[1], torch.float32, table)
+    _library.call("dl_embed_positions", table, pos_table, _code(table.dtype), ids, positions,
+                  out, rows, table.shape[1], table.shape[0], pos_table.shape[0], _stream())
     return out
 
 
@@ -151,9 +157,9 @@ def embed_pairs(table, pairs, step, last, mul_prev, mul_cur, scale=1.0):
                     (step.slots, "slots")):
         _int32(t, "embed_pairs " + what)
     rows = step.tokens.numel()
-    out = torch.empty((rows, table.shape[1]), dtype=torch.float32, device=table.device)
-    _library.call("dl_embed_pairs", _ptr(table), _ptr(pairs), _code(table.dtype), _ptr(step.tokens), _ptr(step.token_seq), _ptr(step.token_pos),
-                  _ptr(step.cu_new), _ptr(step.slots), _ptr(last), last.stride(0), last.shape[0], _ptr(out), rows, table.shape[1], table.shape[0],
+    out = _library.empty(rows, table.shape[1], torch.float32, table)
+    _library.call("dl_embed_pairs", table, pairs, _code(table.dtype), step.tokens, step.token_seq, step.token_pos,
+                  step.cu_new, step.slots, last, last.stride(0), last.shape[0], out, rows, table.shape[1], table.shape[0],
                   pairs.shape[0] - 1, int(mul_prev), int(mul_cur), float(scale), _stream())
     return out
 
@@ -209,7 +215,7 @@ def add_bias(x, bias):
     _need_cuda(x, bias)
     if x.dtype != torch.float32 or x.dim() != 2 or not x.is_contiguous() or bias.dtype != torch.float32 or bias.shape != (x.shape[1],):
         raise KernelError("add_bias: contiguous float32 rows and one float32 value per column")
-    _library.call("dl_add_bias", _ptr(x), _ptr(bias), x.shape[0], x.shape[1], _stream())
+    _library.call("dl_add_bias", x, bias, x.shape[0], x.shape[1], _stream())
     return x
 
 
@@ -303,9 +309,9 @@ def add_rmsnorm(residual, delta, gain, eps, out_dtype, lazy=False):
         raise KernelError(f"rmsnorm: gain must be float32 [{width}]")
     if delta is not None and (delta.shape != residual.shape or not delta.is_contiguous()):
         raise KernelError("rmsnorm: delta must be contiguous with the residual's shape")
-    out = torch.empty((rows, width), dtype=out_dtype, device=residual.device)
-    _library.call("dl_add_rmsnorm", _ptr(residual), _ptr(delta),
-                  _code(delta.dtype) if delta is not None else 0, _ptr(gain), _ptr(out),
+    out = _library.empty(rows, width, out_dtype, residual)
+    _library.call("dl_add_rmsnorm", residual, delta,
+                  _code(delta.dtype) if delta is not None else 0, gain, out,
                   _code(out_dtype), rows, width, float(eps), _stream())
     return out
 
@@ -328,9 +334,9 @@ def add_normed_branch(residual, branch, gain=None, eps=0.0, out_dtype=None):
     extra = branch.extra
     if extra is not None and (extra.dtype != torch.float32 or tuple(extra.shape) != (rows, width) or not extra.is_contiguous()):
         raise KernelError("normed branch: the extra addend must be contiguous float32 with the stream's shape")
-    out = torch.empty((rows, width), dtype=out_dtype, device=residual.device) if gain is not None else None
-    _library.call("dl_branch_norm_add", _ptr(residual), _ptr(data), _code(data.dtype), stride, _ptr(bias), _ptr(branch.gain),
-                  branch.eps, _ptr(extra), _ptr(gain), _ptr(out), _code(out_dtype) if out is not None else 0, rows, width,
+    out = _library.empty(rows, width, out_dtype, residual) if gain is not None else None
+    _library.call("dl_branch_norm_add", residual, data, _code(data.dtype), stride, bias, branch.gain,
+                  branch.eps, extra, gain, out, _code(out_dtype) if out is not None else 0, rows, width,
                   float(eps), _stream())
     return out
 
@@ -341,7 +347,7 @@ def add_rows(residual, other):
     if residual.dtype != torch.float32 or other.dtype != torch.float32 or residual.shape != other.shape \
             or residual.dim() != 2 or not residual.is_contiguous() or not other.is_contiguous():
         raise KernelError("add_rows: need two contiguous float32 tensors of one shape")
-    _library.call("dl_add_rows", _ptr(residual), _ptr(other), residual.shape[0], residual.shape[1], _stream())
+    _library.call("dl_add_rows", residual, other, residual.shape[0], residual.shape[1], _stream())
     return residual
 
 
@@ -386,10 +392,10 @@ def stream_norm(x, copies, write, read, gain, bias, eps, out_dtype, kind="layern
         ys = _rows_view(y, "stream_norm y")
         if tuple(y.shape) != (T, H):
             raise KernelError(f"stream_norm: a sublayer's output of shape {tuple(y.shape)} does not fit a stream of {(T, H)}")
-    normed = torch.empty((T, H), dtype=out_dtype, device=x.device) if gain is not None else None
-    u = torch.empty((T, H), dtype=torch.float32, device=x.device) if summed else None
-    _library.call("dl_stream_norm", _ptr(x), _ptr(y), _code(y.dtype) if y is not None else 0, ys, _ptr(scale), _ptr(mix), _ptr(outw),
-                  _ptr(read), _ptr(gain), _ptr(bias), _ptr(normed), _code(out_dtype) if normed is not None else 0, _ptr(u), T, S, H,
+    normed = _library.empty(T, H, out_dtype, x) if gain is not None else None
+    u = _library.empty(T, H, torch.float32, x) if summed else None
+    _library.call("dl_stream_norm", x, y, _code(y.dtype) if y is not None else 0, ys, scale, mix, outw,
+                  read, gain, bias, normed, _code(out_dtype) if normed is not None else 0, u, T, S, H,
                   float(eps), STREAM_NORMS[kind], _stream())
     return (normed, u) if summed else normed
 
@@ -399,8 +405,8 @@ def stream_copies(x, copies, factor=1.0):
     _need_cuda(x)
     if x.dtype != torch.float32 or x.dim() != 2 or not x.is_contiguous():
         raise KernelError("stream_copies: need contiguous float32 [T, H]")
-    out = torch.empty((x.shape[0], int(copies) * x.shape[1]), dtype=torch.float32, device=x.device)
-    _library.call("dl_stream_copies", _ptr(x), _ptr(out), x.shape[0], int(copies), x.shape[1], float(factor), _stream())
+    out = _library.empty(x.shape[0], int(copies) * x.shape[1], torch.float32, x)
+    _library.call("dl_stream_copies", x, out, x.shape[0], int(copies), x.shape[1], float(factor), _stream())
     return out
 
 
@@ -411,8 +417,8 @@ def embed_copies(table, ids, copies, factor=1.0):
     stride = _rows_view(table, "embed_copies table")
     _int32(ids, "embed_copies ids")
     n, width = table.shape
-    out = torch.empty((ids.numel(), int(copies) * width), dtype=torch.float32, device=table.device)
-    _library.call("dl_embed_copies", _ptr(table), _code(table.dtype), stride, _ptr(ids), _ptr(out), ids.numel(), int(copies), width, n,
+    out = _library.empty(ids.numel(), int(copies) * width, torch.float32, table)
+    _library.call("dl_embed_copies", table, _code(table.dtype), stride, ids, out, ids.numel(), int(copies), width, n,
                   float(factor), _stream())
     return out
 
@@ -426,8 +432,8 @@ def group_rmsnorm(x, gain, width_a, width_b, eps):
     width = int(width_a) + int(width_b)
     if x.dim() != 2 or x.shape[1] != width or gain.dtype != torch.float32 or gain.shape != (width,) or not gain.is_contiguous():
         raise KernelError(f"group_rmsnorm: x [T, {width}] and a float32 gain per column")
-    out = torch.empty((x.shape[0], width), dtype=x.dtype, device=x.device)
-    _library.call("dl_group_rmsnorm", _ptr(x), _rows_view(x, "group_rmsnorm x"), _ptr(out), out.stride(0), _code(x.dtype), _ptr(gain),
+    out = _library.empty(x.shape[0], width, x.dtype, x)
+    _library.call("dl_group_rmsnorm", x, _rows_view(x, "group_rmsnorm x"), out, out.stride(0), _code(x.dtype), gain,
                   x.shape[0], int(width_a), int(width_b), float(eps), _stream())
     return out
 
@@ -458,9 +464,9 @@ def qkv_rows(x, n_heads, n_kv_heads, dim, vdim, lay_k, lay_v, biases=None, gains
             raise KernelError("qkv_rows: the other values are [T, G*lay] of x's dtype, their weight one float32 number")
     width = (H + G) * lay_k + G * lay_v
     ld = -(-width // 8) * 8
-    out = torch.empty((T, ld), dtype=x.dtype, device=x.device)
-    _library.call("dl_qkv_rows", _ptr(x), _code(x.dtype), _rows_view(x, "qkv_rows x"), _ptr(qb), _ptr(kb), _ptr(vb), _ptr(qg), _ptr(kg), float(eps),
-                  H, G, d, vd, int(lay_k), int(lay_v), _ptr(first), first_ld, first_lay, _ptr(mix), _ptr(out), ld, T, _stream())
+    out = _library.empty(T, ld, x.dtype, x)
+    _library.call("dl_qkv_rows", x, _code(x.dtype), _rows_view(x, "qkv_rows x"), qb, kb, vb, qg, kg, float(eps),
+                  H, G, d, vd, int(lay_k), int(lay_v), first, first_ld, first_lay, mix, out, ld, T, _stream())
     return out[:, :H * lay_k], out[:, H * lay_k:(H + G) * lay_k], out[:, (H + G) * lay_k:width]
 
 
@@ -474,7 +480,7 @@ def pair_norm_sum(a, b, gain_a, gain_b, eps, weight_a=0.5, weight_b=0.5):
         if g.dtype != torch.float32 or g.shape != (a.shape[1],) or not g.is_contiguous():
             raise KernelError(f"pair_norm_sum: gains must be contiguous float32 [{a.shape[1]}]")
     out = torch.empty_like(a)
-    _library.call("dl_pair_norm_sum", _ptr(a), _ptr(b), _ptr(gain_a), _ptr(gain_b), _ptr(out), a.shape[0], a.shape[1], float(eps),
+    _library.call("dl_pair_norm_sum", a, b, gain_a, gain_b, out, a.shape[0], a.shape[1], float(eps),
                   float(weight_a), float(weight_b), _stream())
     return out
 
@@ -484,7 +490,7 @@ def scale_values(values, factor):
     _need_cuda(values)
     if values.dtype != torch.float32 or not values.is_contiguous():
         raise KernelError("scale_values: need a contiguous float32 tensor")
-    _library.call("dl_scale_values", _ptr(values), values.numel(), float(factor), _stream())
+    _library.call("dl_scale_values", values, values.numel(), float(factor), _stream())
     return values
 
 
@@ -534,12 +540,12 @@ def post_norm(x, write, out_dtype=None, last=None, conv=None):
             if write is None:
                 return x
         else:
-            out = torch.empty((T, H), dtype=out_dtype, device=x.device)
-    _library.call("dl_post_norm", _ptr(x), _ptr(y), _code(y.dtype) if y is not None else 0,
-                  _rows_view(y, "post_norm y") if y is not None else 0, alpha, _ptr(gain), gain.numel() if gain is not None else 1, eps,
-                  _ptr(gain2), gain2.numel() if gain2 is not None else 1, float(eps2), _ptr(out), _code(out_dtype) if out is not None else 0,
-                  T, H, _ptr(memory), memory.stride(0) if memory is not None else 0, memory.shape[0] if memory is not None else 0, _ptr(slots),
-                  _ptr(taps), K, _stream())
+            out = _library.empty(T, H, out_dtype, x)
+    _library.call("dl_post_norm", x, y, _code(y.dtype) if y is not None else 0,
+                  _rows_view(y, "post_norm y") if y is not None else 0, alpha, gain, gain.numel() if gain is not None else 1, eps,
+                  gain2, gain2.numel() if gain2 is not None else 1, float(eps2), out, _code(out_dtype) if out is not None else 0,
+                  T, H, memory, memory.stride(0) if memory is not None else 0, memory.shape[0] if memory is not None else 0, slots,
+                  taps, K, _stream())
     return x if out is None and out_dtype is not None else out
 
 
@@ -561,10 +567,10 @@ def causal_conv(x, taps, memory, cu_new, slots, max_new, bias=None, activation=N
         raise KernelError("causal_conv: a slot's memory must hold the last K - 1 inputs in float32")
     _int32(cu_new, "causal_conv cu_new")
     _int32(slots, "causal_conv slots")
-    out = torch.empty((T, C), dtype=out_dtype or torch.float32, device=x.device)
-    _library.call("dl_causal_conv", _ptr(x), _code(x.dtype), _rows_view(x, "causal_conv x"), _ptr(taps), K, _ptr(bias),
-                  1 if activation == "silu" else 0, 1 if add_input else 0, _ptr(memory), memory.stride(0), memory.shape[0], _ptr(cu_new),
-                  _ptr(slots), _ptr(out), _code(out.dtype), out.stride(0), slots.numel(), int(max_new), C, _stream())
+    out = _library.empty(T, C, out_dtype or torch.float32, x)
+    _library.call("dl_causal_conv", x, _code(x.dtype), _rows_view(x, "causal_conv x"), taps, K, bias,
+                  1 if activation == "silu" else 0, 1 if add_input else 0, memory, memory.stride(0), memory.shape[0], cu_new,
+                  slots, out, _code(out.dtype), out.stride(0), slots.numel(), int(max_new), C, _stream())
     return out
 
 
@@ -624,14 +630,14 @@ def rope_cache_write(q, k, v, cos, sin, rotary_dim, token_seq, token_pos, block_
                 or not sin.is_contiguous():
             raise KernelError("rope: cos/sin must be contiguous float32 [positions, rotary_dim/2]")
         table_rows = cos.shape[0]
-    _library.call("dl_rope_cache_write", _ptr(q), qs, _ptr(k) if write_cache else None, ks,
-                  _ptr(v) if write_cache else None, vs, _code(q.dtype),
-                  _ptr(cos) if rotary_dim else None, _ptr(sin) if rotary_dim else None,
-                  int(rotary_dim), table_rows, _ptr(token_seq) if write_cache else None, _ptr(token_pos),
-                  _ptr(block_table) if write_cache else None, bt_stride,
-                  _ptr(k_pool) if write_cache else None, _ptr(v_pool) if write_cache else None, n_pages,
-                  T, n_heads, n_kv_heads, head_dim, vd, _ptr(qb), _ptr(kb) if write_cache else None,
-                  _ptr(vb) if write_cache else None, 1 if write_cache else 0, _stream())
+    _library.call("dl_rope_cache_write", q, qs, k if write_cache else None, ks,
+                  v if write_cache else None, vs, _code(q.dtype),
+                  cos if rotary_dim else None, sin if rotary_dim else None,
+                  int(rotary_dim), table_rows, token_seq if write_cache else None, token_pos,
+                  block_table if write_cache else None, bt_stride,
+                  k_pool if write_cache else None, v_pool if write_cache else None, n_pages,
+                  T, n_heads, n_kv_heads, head_dim, vd, qb, kb if write_cache else None,
+                  vb if write_cache else None, 1 if write_cache else 0, _stream())
 
 
 def _check_pools(k_pool, v_pool, n_kv_heads, head_dim, value_dim=None):
@@ -651,7 +657,7 @@ def head_gate(o, gate, n_heads, width):
     _need_cuda(o, gate)
     if o.dim() != 2 or o.shape[1] != n_heads * width or gate.shape != (o.shape[0], n_heads) or gate.dtype != o.dtype:
         raise KernelError("head_gate: o [T, heads*width] and one gate logit per (row, head) of o's dtype")
-    _library.call("dl_head_gate", _ptr(o), _rows_view(o, "head_gate o"), _ptr(gate), _rows_view(gate, "head_gate gate"),
+    _library.call("dl_head_gate", o, _rows_view(o, "head_gate o"), gate, _rows_view(gate, "head_gate gate"),
                   _code(o.dtype), o.shape[0], n_heads, width, _stream())
     return o
 
@@ -708,7 +714,7 @@ def attention(q, k_pool, v_pool, token_seq, token_pos, block_table, n_heads, n_k
     _int32(token_seq, "token_seq")
     _int32(token_pos, "token_pos")
     _int32(block_table, "block_table")
-    out = torch.empty((T, n_heads * vd), dtype=q.dtype, device=q.device)
+    out = _library.empty(T, n_heads * vd, q.dtype, q)
     softcap, slopes = 0.0, None
     if score_hook:
         softcap, slopes = score_hook.softcap, score_hook.slopes
@@ -724,10 +730,10 @@ def attention(q, k_pool, v_pool, token_seq, token_pos, block_table, n_heads, n_k
         if attention_fast.run_f32(q, qs, out, k_pool, v_pool, n_pages, token_seq, token_pos, block_table, n_heads, n_kv_heads, head_dim,
                                   float(scale), int(window), plan, int(keep_first), sinks, softcap, slopes, gate):
             return out
-    _library.call("dl_attention_generic", _ptr(q), qs, _ptr(out), out.stride(0), _code(q.dtype),
-                  _ptr(k_pool), _ptr(v_pool), n_pages, _ptr(token_seq), _ptr(token_pos),
-                  _ptr(block_table), block_table.shape[1], T, n_heads, n_kv_heads, head_dim, vd,
-                  float(scale), int(window), float(softcap), _ptr(slopes), _ptr(gate), gs, int(keep_first), _ptr(sinks), _stream())
+    _library.call("dl_attention_generic", q, qs, out, out.stride(0), _code(q.dtype),
+                  k_pool, v_pool, n_pages, token_seq, token_pos,
+                  block_table, block_table.shape[1], T, n_heads, n_kv_heads, head_dim, vd,
+                  float(scale), int(window), float(softcap), slopes, gate, gs, int(keep_first), sinks, _stream())
     return out
 
 
@@ -783,10 +789,10 @@ def swiglu(gate_up):
         raise KernelError("swiglu: need a contiguous [T, 2I] tensor")
     rows, two_i = gate_up.shape
     width = two_i // 2
-    out = torch.empty((rows, width), dtype=gate_up.dtype, device=gate_up.device)
+    out = _library.empty(rows, width, gate_up.dtype, gate_up)
     esize = gate_up.element_size()
-    _library.call("dl_swiglu", gate_up.data_ptr(), gate_up.data_ptr() + width * esize, two_i,
-                  _ptr(out), _code(gate_up.dtype), rows, width, _stream())
+    _library.call("dl_swiglu", gate_up, gate_up.data_ptr() + width * esize, two_i,
+                  out, _code(gate_up.dtype), rows, width, _stream())
     return out
 
 
@@ -812,9 +818,9 @@ def gated_activation(gate_up, kind, limit=0.0, alpha=1.0, bias=None):
         raise KernelError("gated_activation: need a contiguous [T, 2I] tensor")
     rows, two_i = gate_up.shape
     width = two_i // 2
-    out = torch.empty((rows, width), dtype=gate_up.dtype, device=gate_up.device)
-    _library.call("dl_gated_activation", gate_up.data_ptr(), gate_up.data_ptr() + width * gate_up.element_size(), two_i,
-                  _ptr(out), _code(gate_up.dtype), rows, width, GATINGS[kind], float(limit), float(alpha),
+    out = _library.empty(rows, width, gate_up.dtype, gate_up)
+    _library.call("dl_gated_activation", gate_up, gate_up.data_ptr() + width * gate_up.element_size(), two_i,
+                  out, _code(gate_up.dtype), rows, width, GATINGS[kind], float(limit), float(alpha),
                   _ptr(_gate_bias(bias, two_i, "gated_activation")), _stream())
     return out
 
@@ -874,17 +880,17 @@ def gla_scan(q, k, v, z, z_bias, cu_new, slots, state, n_heads, dim, vdim, q_sca
         raise KernelError("gla_scan: the state must be contiguous float32 [slots, H, dim, vdim]")
     _int32(cu_new, "gla cu_new")
     _int32(slots, "gla slots")
-    out = torch.empty((T, n_heads * vdim), dtype=torch.float32, device=q.device)
+    out = _library.empty(T, n_heads * vdim, torch.float32, q)
     if q.dtype == torch.bfloat16 and max_new >= CHUNK_MIN_TOKENS and dim <= CHUNK_MAX_DIM and vdim % 4 == 0 and ld % 4 == 0 and v.data_ptr() % 8 == 0 \
             and state.data_ptr() % 16 == 0:
         scratch, at_once = _chunk_scratch(q.device, "dl_gla_chunk_scratch", T, slots.numel(), n_heads, vdim)
         if scratch is not None:
-            _library.call("dl_gla_chunk", _ptr(q), _ptr(k), _ptr(v), ld, _ptr(z), zs, _ptr(z_bias), _ptr(cu_new), _ptr(slots), _ptr(state),
-                          state.shape[0], _ptr(out), out.stride(0), _ptr(scratch), slots.numel(), T, n_heads, dim, vdim, float(q_scale), float(tau),
+            _library.call("dl_gla_chunk", q, k, v, ld, z, zs, z_bias, cu_new, slots, state,
+                          state.shape[0], out, out.stride(0), scratch, slots.numel(), T, n_heads, dim, vdim, float(q_scale), float(tau),
                           at_once, _stream())
             return out
-    _library.call("dl_gla_scan", _ptr(q), _ptr(k), _ptr(v), ld, _ptr(z), zs, _ptr(z_bias), _code(q.dtype), _ptr(cu_new),
-                  _ptr(slots), _ptr(state), state.shape[0], _ptr(out), out.stride(0), slots.numel(), T, n_heads, dim, vdim,
+    _library.call("dl_gla_scan", q, k, v, ld, z, zs, z_bias, _code(q.dtype), cu_new,
+                  slots, state, state.shape[0], out, out.stride(0), slots.numel(), T, n_heads, dim, vdim,
                   float(q_scale), float(tau), _stream())
     return out
 
@@ -904,8 +910,8 @@ def head_norm_gate(o, g, gain, n_heads, vdim, eps, out_dtype, gate="silu"):
     if o.dtype != torch.float32 or not o.is_contiguous() or o.shape != (T, n_heads * vdim) or g.shape != o.shape \
             or g.dtype != out_dtype or gain.dtype != torch.float32 or gain.shape != (vdim,) or not gain.is_contiguous():
         raise KernelError("head_norm_gate: o float32 [T, H*vdim], g of the output's dtype and shape, gain float32 [vdim]")
-    out = torch.empty((T, n_heads * vdim), dtype=out_dtype, device=o.device)
-    _library.call("dl_head_norm_gate", _ptr(o), o.stride(0), _ptr(g), gs, _ptr(gain), _ptr(out), out.stride(0),
+    out = _library.empty(T, n_heads * vdim, out_dtype, o)
+    _library.call("dl_head_norm_gate", o, o.stride(0), g, gs, gain, out, out.stride(0),
                   _code(out_dtype), T, n_heads, vdim, float(eps), HEAD_GATES[gate], _stream())
     return out
 
@@ -923,9 +929,9 @@ def head_rmsnorm(x, gain_a, heads_a, dim, eps, gain_b=None, heads_b=0, lay=None)
     for g, n in ((gain_a, heads_a), (gain_b, heads_b)):
         if n and (g is None or g.dtype != torch.float32 or g.shape != (dim,) or not g.is_contiguous()):
             raise KernelError(f"head_rmsnorm: a gain must be contiguous float32 [{dim}]")
-    out = torch.empty((T, (heads_a + heads_b) * lay), dtype=x.dtype, device=x.device)
-    _library.call("dl_head_rmsnorm", _ptr(x), _rows_view(x, "head_rmsnorm x"), _ptr(out), out.stride(0), _code(x.dtype),
-                  _ptr(gain_a), _ptr(gain_b), T, int(heads_a), int(heads_b), int(dim), lay, float(eps), _stream())
+    out = _library.empty(T, (heads_a + heads_b) * lay, x.dtype, x)
+    _library.call("dl_head_rmsnorm", x, _rows_view(x, "head_rmsnorm x"), out, out.stride(0), _code(x.dtype),
+                  gain_a, gain_b, T, int(heads_a), int(heads_b), int(dim), lay, float(eps), _stream())
     return out
 
 
@@ -955,7 +961,7 @@ def ssd_scan(xbc, z, dt_bias, a_log, skip, cu_new, slots, memory, n_heads, group
         raise KernelError(f"ssd_scan: a slot's memory must hold {H * N * P} float32 values")
     _int32(cu_new, "ssd_scan cu_new")
     _int32(slots, "ssd_scan slots")
-    out = torch.empty((T, H * P), dtype=torch.float32, device=xbc.device)
+    out = _library.empty(T, H * P, torch.float32, xbc)
     ld, zld = _rows_view(xbc, "ssd_scan xbc"), _rows_view(z, "ssd_scan z")
     if SSD_CHUNKED and xbc.dtype == torch.bfloat16 and max_new >= SSD_CHUNK_MIN_TOKENS and N % 8 == 0 and P % 8 == 0 and N <= SSD_CHUNK_MAX_STATE \
             and ld % 8 == 0 and xbc.data_ptr() % 16 == 0:
@@ -964,13 +970,13 @@ def ssd_scan(xbc, z, dt_bias, a_log, skip, cu_new, slots, memory, n_heads, group
         if chunks > 2 and B * H * ((P + SSD_CHUNK_COLS - 1) // SSD_CHUNK_COLS) < SSD_SIDE_BLOCKS and B * chunks <= 65535 \
                 and B * chunks * H * N * P * 4 <= SSD_SIDE_BYTES and memory.stride(0) % 4 == 0 and memory.data_ptr() % 16 == 0:
             part = torch.empty((B * chunks, H, N, P), dtype=torch.float32, device=xbc.device)
-            decay = torch.empty((B * chunks, H), dtype=torch.float32, device=xbc.device)
-        _library.call("dl_ssd_chunk", _ptr(xbc), ld, _ptr(z), zld, _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(cu_new), _ptr(slots), _ptr(memory),
-                      memory.stride(0), memory.shape[0], _ptr(out), out.stride(0), B, H, G, N, P, chunks, _ptr(part), _ptr(decay), _stream())
+            decay = _library.empty(B * chunks, H, torch.float32, xbc)
+        _library.call("dl_ssd_chunk", xbc, ld, z, zld, dt_bias, a_log, skip, cu_new, slots, memory,
+                      memory.stride(0), memory.shape[0], out, out.stride(0), B, H, G, N, P, chunks, part, decay, _stream())
         return out
-    _library.call("dl_ssd_scan", _ptr(xbc), _code(xbc.dtype), ld, _ptr(z), zld,
-                  _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(cu_new), _ptr(slots), _ptr(memory), memory.stride(0), memory.shape[0],
-                  _ptr(out), out.stride(0), slots.numel(), T, H, G, N, P, _stream())
+    _library.call("dl_ssd_scan", xbc, _code(xbc.dtype), ld, z, zld,
+                  dt_bias, a_log, skip, cu_new, slots, memory, memory.stride(0), memory.shape[0],
+                  out, out.stride(0), slots.numel(), T, H, G, N, P, _stream())
     return out
 
 
@@ -992,8 +998,8 @@ def gated_group_norm(y, gate, gain, parts, eps, scale=1.0, out=None):
     if y.dtype != torch.float32 or gate.shape != (T, W) or gain.dtype != torch.float32 or gain.shape != (W,) or W % parts:
         raise KernelError(f"gated_group_norm: y float32 [T, W], a gate of its shape, gains [W], W a multiple of {parts} parts")
     out = _out_view(out, T, W, gate.dtype, y.device, "gated_group_norm")
-    _library.call("dl_gated_group_norm", _ptr(y), _rows_view(y, "gated_group_norm y"), _ptr(gate), _rows_view(gate, "gated_group_norm gate"),
-                  _ptr(gain), _ptr(out), _rows_view(out, "gated_group_norm out"), _code(gate.dtype), T, W, int(parts), float(eps),
+    _library.call("dl_gated_group_norm", y, _rows_view(y, "gated_group_norm y"), gate, _rows_view(gate, "gated_group_norm gate"),
+                  gain, out, _rows_view(out, "gated_group_norm out"), _code(gate.dtype), T, W, int(parts), float(eps),
                   float(scale), _stream())
     return out
 
@@ -1022,10 +1028,10 @@ def latent_rows(x, q_gain, kv_gain, eps, rot, tables, token_pos, lay):
     if x.shape[1] != rq + r + rot or dims > rot or lay < r + rot:
         raise KernelError(f"latent_rows: rows of {rq} + {r} + {rot} channels into {lay}, {dims} of them rotated")
     _int32(token_pos, "latent_rows positions")
-    cq = torch.empty((T, rq), dtype=x.dtype, device=x.device) if rq else None
-    kv = torch.empty((T, lay), dtype=x.dtype, device=x.device)
-    _library.call("dl_latent_rows", _ptr(x), _code(x.dtype), _rows_view(x, "latent_rows x"), rq, r, int(rot), dims, _ptr(q_gain), _ptr(kv_gain),
-                  float(eps), _ptr(cos), _ptr(sin), rows, _ptr(token_pos), _ptr(cq), _ptr(kv), int(lay), T, _stream())
+    cq = _library.empty(T, rq, x.dtype, x) if rq else None
+    kv = _library.empty(T, lay, x.dtype, x)
+    _library.call("dl_latent_rows", x, _code(x.dtype), _rows_view(x, "latent_rows x"), rq, r, int(rot), dims, q_gain, kv_gain,
+                  float(eps), cos, sin, rows, token_pos, cq, kv, int(lay), T, _stream())
     return cq, kv
 
 
@@ -1047,9 +1053,9 @@ def latent_values(a, w_value, lay, gate=None):
     if a.shape[1] != H * lay or lay < r or (gate is not None and (gate.shape != (T, H * vd) or gate.dtype != a.dtype)):
         raise KernelError(f"latent_values: {H} heads of {r} in {lay} channels and a gate [T, {H * vd}]")
     if _per_head_rows_takes(a, w_value, lay):
-        out = torch.empty((T, H * vd), dtype=a.dtype, device=a.device)
-        _library.call("dl_per_head_rows", _ptr(a), _rows_view(a, "latent_values a"), int(lay), _ptr(w_value), H, vd, r, _ptr(out), out.stride(0), vd,
-                      _ptr(gate), _rows_view(gate, "latent_values gate") if gate is not None else 0, -1, 0, None, None, 0, None, T, _stream())
+        out = _library.empty(T, H * vd, a.dtype, a)
+        _library.call("dl_per_head_rows", a, _rows_view(a, "latent_values a"), int(lay), w_value, H, vd, r, out, out.stride(0), vd,
+                      gate, _rows_view(gate, "latent_values gate") if gate is not None else 0, -1, 0, None, None, 0, None, T, _stream())
         return out
     o = linear_per_head(a, w_value, x_head=lay)
     return o if gate is None else channel_gate(o, gate, H, vd, out=o)
@@ -1065,14 +1071,14 @@ def latent_queries(q, w_key, rot, tables, token_pos, lay):
     if q.shape[1] != H * (d + rot) or dims > rot or lay < r + rot:
         raise KernelError(f"latent_queries: {H} heads of {d} + {rot} channels into {lay}")
     _int32(token_pos, "latent_queries positions")
-    out = torch.empty((T, H * lay), dtype=q.dtype, device=q.device)
+    out = _library.empty(T, H * lay, q.dtype, q)
     if _per_head_rows_takes(q, w_key, d + rot):
-        _library.call("dl_per_head_rows", _ptr(q), _rows_view(q, "latent_queries q"), d + rot, _ptr(w_key), H, r, d, _ptr(out), out.stride(0),
-                      int(lay), None, 0, int(rot), dims, _ptr(cos), _ptr(sin), rows, _ptr(token_pos), T, _stream())
+        _library.call("dl_per_head_rows", q, _rows_view(q, "latent_queries q"), d + rot, w_key, H, r, d, out, out.stride(0),
+                      int(lay), None, 0, int(rot), dims, cos, sin, rows, token_pos, T, _stream())
         return out
     linear_per_head(q, w_key, x_head=d + rot, out=out, out_head=lay)
-    _library.call("dl_latent_query_tail", _ptr(q), _code(q.dtype), _rows_view(q, "latent_queries q"), d, int(rot), dims, _ptr(cos), _ptr(sin),
-                  rows, _ptr(token_pos), _ptr(out), out.stride(0), r, int(lay), H, T, _stream())
+    _library.call("dl_latent_query_tail", q, _code(q.dtype), _rows_view(q, "latent_queries q"), d, int(rot), dims, cos, sin,
+                  rows, token_pos, out, out.stride(0), r, int(lay), H, T, _stream())
     return out
 
 
@@ -1084,8 +1090,8 @@ def channel_gate(o, gate, heads, width, lay=None, scale=1.0, out=None):
     if o.shape[1] < (heads - 1) * lay + width or (gate is not None and (gate.shape != (T, heads * width) or gate.dtype != o.dtype)):
         raise KernelError(f"channel_gate: o with {heads} heads {lay} apart and one gate logit per channel of o's dtype")
     out = _out_view(out, T, heads * width, o.dtype, o.device, "channel_gate")
-    _library.call("dl_channel_gate", _ptr(o), _rows_view(o, "channel_gate o"), lay, _ptr(gate),
-                  _rows_view(gate, "channel_gate gate") if gate is not None else heads * width, _ptr(out),
+    _library.call("dl_channel_gate", o, _rows_view(o, "channel_gate o"), lay, gate,
+                  _rows_view(gate, "channel_gate gate") if gate is not None else heads * width, out,
                   _rows_view(out, "channel_gate out"), _code(o.dtype), T, int(heads), int(width), float(scale), _stream())
     return out
 
@@ -1123,18 +1129,15 @@ def delta_rule(x, taps, b_logit, z, dt_bias, a_log, token_seq, cu_new, slots, me
     _int32(token_seq, "delta_rule token_seq")
     _int32(cu_new, "delta_rule cu_new")
     _int32(slots, "delta_rule slots")
-    f32 = dict(dtype=torch.float32, device=x.device)
-    qo, ko = torch.empty((T, G * dim), **f32), torch.empty((T, G * dim), **f32)
-    vo, go = torch.empty((T, H * vdim), **f32), torch.empty((T, H * dim), **f32)
-    bo, out = torch.empty((T, H), **f32), torch.empty((T, H * vdim), **f32)
+    qo, ko, vo, go, bo, out = (_library.empty(T, n, torch.float32, x) for n in (G * dim, G * dim, H * vdim, H * dim, H, H * vdim))
     scratch, at_once = None, 0
     if x.dtype == torch.bfloat16 and max_new >= CHUNK_MIN_TOKENS and dim <= CHUNK_MAX_DIM and vdim % 4 == 0:
         scratch, at_once = _chunk_scratch(x.device, "dl_delta_chunk_scratch", T, slots.numel(), H)
-    _library.call("dl_delta_rule", _ptr(x), ld, _ptr(taps), K, _code(x.dtype), _ptr(b_logit), _rows_view(b_logit, "delta_rule b"),
-                  _ptr(z), _rows_view(z, "delta_rule z"), _ptr(dt_bias), _ptr(a_log), _ptr(token_seq), _ptr(cu_new), _ptr(slots),
-                  memory.data_ptr(), memory.data_ptr() + 4 * n_state, memory.stride(0), memory.shape[0],
-                  _ptr(qo), _ptr(ko), _ptr(vo), _ptr(go), _ptr(bo), _ptr(out), slots.numel(), T, H, G, int(dim), int(vdim),
-                  float(q_scale), float(unit_eps), 1 if head_decay else 0, _ptr(scratch), at_once, _stream())
+    _library.call("dl_delta_rule", x, ld, taps, K, _code(x.dtype), b_logit, _rows_view(b_logit, "delta_rule b"),
+                  z, _rows_view(z, "delta_rule z"), dt_bias, a_log, token_seq, cu_new, slots,
+                  memory, memory.data_ptr() + 4 * n_state, memory.stride(0), memory.shape[0],
+                  qo, ko, vo, go, bo, out, slots.numel(), T, H, G, int(dim), int(vdim),
+                  float(q_scale), float(unit_eps), 1 if head_decay else 0, scratch, at_once, _stream())
     return out
 
 
@@ -1177,10 +1180,10 @@ def route_topk(x, w_router, bias, top, scoring="softmax_chosen", experts=None, w
         raise KernelError("route_topk: a correction, normalised weights and a scale go with 'softmax_all' without groups")
     T = x.shape[0]
     z = linear(x, w_router, out_dtype=torch.float32, resident=True)         # float32 accumulation, float32 logits
-    ids = torch.empty((T, top), dtype=torch.int32, device=x.device)
-    weights = torch.empty((T, top), dtype=torch.float32, device=x.device)
-    _library.call("dl_route_topk", _ptr(z), z.stride(0) if T > 1 else rows_w, _ptr(bias), _ptr(ids), _ptr(weights), T, E, top,
-                  ROUTER_SCORINGS[scoring], n_groups, keep_groups, _ptr(correction), 1 if normalise else 0, float(weight_scale),
+    ids = _library.empty(T, top, torch.int32, x)
+    weights = _library.empty(T, top, torch.float32, x)
+    _library.call("dl_route_topk", z, z.stride(0) if T > 1 else rows_w, bias, ids, weights, T, E, top,
+                  ROUTER_SCORINGS[scoring], n_groups, keep_groups, correction, 1 if normalise else 0, float(weight_scale),
                   _stream())
     return (ids, weights, z) if with_logits else (ids, weights)
 
@@ -1221,8 +1224,8 @@ def expert_gate_up(x, ids, w_gate_up, kind, limit=0.0, alpha=1.0, row_scale=None
     E, rows_w, K = w_gate_up.shape
     ff = rows_w // halves
     T, top = ids.shape
-    out = torch.empty((T * top, ff), dtype=x.dtype, device=x.device)
-    _library.call("dl_expert_gate_up", _ptr(x), xs, _ptr(ids), _ptr(w_gate_up), _ptr(out), _code(x.dtype), T, top, K,
+    out = _library.empty(T * top, ff, x.dtype, x)
+    _library.call("dl_expert_gate_up", x, xs, ids, w_gate_up, out, _code(x.dtype), T, top, K,
                   ff, E, GATINGS[kind], float(limit), float(alpha), _ptr(_row_scale(row_scale, ids, "expert_gate_up")), _stream())
     return out
 
@@ -1253,9 +1256,9 @@ def expert_down(h, ids, weights, w_down, addend=None, addend_gate=None, identity
     E, N, ff = w_down.shape
     astride, gstride = _addend(addend, addend_gate, T, N, "expert_down")
     irows, istride, icount = _identity(identity, T, N, h.dtype, "expert_down")
-    out = torch.empty((T, N), dtype=torch.float32, device=h.device)
-    _library.call("dl_expert_down", _ptr(h), _ptr(ids), _ptr(weights), _ptr(w_down), _ptr(addend), astride, _ptr(out),
-                  _code(h.dtype), T, top, ff, N, E, _ptr(addend_gate), gstride, _ptr(irows), istride, icount, _stream())
+    out = _library.empty(T, N, torch.float32, h)
+    _library.call("dl_expert_down", h, ids, weights, w_down, addend, astride, out,
+                  _code(h.dtype), T, top, ff, N, E, addend_gate, gstride, irows, istride, icount, _stream())
     return out
 
 
@@ -1316,22 +1319,22 @@ def experts_grouped(x, ids, weights, w_gate_up, w_down, kind, limit=0.0, alpha=1
     dev = x.device
     place = torch.empty(rows, dtype=torch.int32, device=dev)
     tile_expert = torch.empty(tiles, dtype=torch.int32, device=dev)
-    _library.call("dl_expert_sort", _ptr(ids), rows, E, _ptr(place), _ptr(tile_expert), tiles, _stream())
+    _library.call("dl_expert_sort", ids, rows, E, place, tile_expert, tiles, _stream())
     sorted_x = torch.empty((tiles * EXPERT_TILE, K), dtype=torch.bfloat16, device=dev)
-    _library.call("dl_expert_gather", _ptr(x), x.stride(0) if T > 1 else K, _ptr(place), _ptr(sorted_x), rows, top, K,
+    _library.call("dl_expert_gather", x, x.stride(0) if T > 1 else K, place, sorted_x, rows, top, K,
                   _ptr(_row_scale(row_scale, ids, "experts_grouped")), _stream())
     status = _library.status_word(dev).data_ptr()
     h = torch.empty((tiles * EXPERT_TILE, ff), dtype=torch.bfloat16, device=dev)
-    _library.call("dl_gemm_tc_grouped_bf16", _ptr(sorted_x), K, _ptr(w_gate_up), _ptr(h), 1, ff, tiles * EXPERT_TILE, ff, K, E,
-                  _ptr(tile_expert), 1 if gated else 0, GATINGS[kind], float(limit), float(alpha), 0, status, _stream())
+    _library.call("dl_gemm_tc_grouped_bf16", sorted_x, K, w_gate_up, h, 1, ff, tiles * EXPERT_TILE, ff, K, E,
+                  tile_expert, 1 if gated else 0, GATINGS[kind], float(limit), float(alpha), 0, status, _stream())
     y = torch.empty((tiles * EXPERT_TILE, N), dtype=torch.float32, device=dev)
-    _library.call("dl_gemm_tc_grouped_bf16", _ptr(h), ff, _ptr(w_down), _ptr(y), 0, N, tiles * EXPERT_TILE, N, ff, E,
-                  _ptr(tile_expert), 0, 0, 0.0, 0.0, 0, status, _stream())
+    _library.call("dl_gemm_tc_grouped_bf16", h, ff, w_down, y, 0, N, tiles * EXPERT_TILE, N, ff, E,
+                  tile_expert, 0, 0, 0.0, 0.0, 0, status, _stream())
     astride, gstride = _addend(addend, addend_gate, T, N, "experts_grouped")
     irows, istride, icount = _identity(identity, T, N, torch.bfloat16, "experts_grouped")
     out = torch.empty((T, N), dtype=torch.float32, device=dev)
-    _library.call("dl_expert_combine", _ptr(y), N, _ptr(place), _ptr(weights), _ptr(addend), astride, _ptr(out), T, top, N,
-                  _ptr(addend_gate), gstride, _ptr(ids), _ptr(irows), istride, E, icount, _stream())
+    _library.call("dl_expert_combine", y, N, place, weights, addend, astride, out, T, top, N,
+                  addend_gate, gstride, ids, irows, istride, E, icount, _stream())
     return out
 
 
@@ -1349,7 +1352,7 @@ def linear_per_head(x, w, x_head=None, out=None, out_head=None):
     T = x.shape[0]
     xs = _rows_view(x, "linear_per_head x")
     if out is None:
-        y = torch.empty((T, H * oh), dtype=x.dtype, device=x.device)
+        y = _library.empty(T, H * oh, x.dtype, x)
     else:
         y = out
         if y.shape != (T, H * oh) or y.dtype != x.dtype or not y.is_contiguous():
@@ -1358,12 +1361,18 @@ def linear_per_head(x, w, x_head=None, out=None, out_head=None):
         return y
     if x.dtype == torch.float32:
         for h in range(H):
-            _library.call("dl_gemm_f32", x.data_ptr() + 4 * h * xh, xs, w[h].data_ptr(), y.data_ptr() + 4 * h * oh, H * oh,
+            _library.call("dl_gemm_f32", x.data_ptr() + 4 * h * xh, xs, w[h], y.data_ptr() + 4 * h * oh, H * oh,
                           T, b, a, _stream())
         return y
     xv = x.as_strided((H, T, a), (xh, xs, 1), x.storage_offset())
     torch.bmm(xv, w.transpose(1, 2), out=y.as_strided((H, T, b), (oh, H * oh, 1), y.storage_offset()))
     return y
+
+
+def _product_sizes(x, w):
+    """(rows, k, n, row stride of x, kind) of x W^T, read in one call; None where the caller's own checks have to say what is wrong
+    or take an unusual layout (``product`` in csrc/host/entry.cpp)."""
+    return _library._entry.product(x, w) if _library._checked_device and _library._entry is not None else None
 
 
 def linear(x, w, out_dtype=None, resident=False, lazy=False):
@@ -1383,14 +1392,18 @@ def linear(x, w, out_dtype=None, resident=False, lazy=False):
             rows, x = x.row_sums(), x.data
         else:
             given = x = x.tensor()
-    _need_cuda(x, w)
-    if w.dim() != 2 or not w.is_contiguous() or x.dim() != 2 or x.shape[1] != w.shape[1]:
-        raise KernelError(f"linear: x {tuple(x.shape)} does not match W {tuple(w.shape)}")
-    if x.dtype != w.dtype:
-        raise KernelError(f"linear: x is {x.dtype} but W is {w.dtype}")
+    sizes = _product_sizes(x, w)
+    if sizes is None:
+        _need_cuda(x, w)
+        if w.dim() != 2 or not w.is_contiguous() or x.dim() != 2 or x.shape[1] != w.shape[1]:
+            raise KernelError(f"linear: x {tuple(x.shape)} does not match W {tuple(w.shape)}")
+        if x.dtype != w.dtype:
+            raise KernelError(f"linear: x is {x.dtype} but W is {w.dtype}")
+        M, K = x.shape
+        N = w.shape[0]
+    else:
+        M, K, N = sizes[:3]
     out_dtype = out_dtype or x.dtype
-    M, K = x.shape
-    N = w.shape[0]
     if lazy and out_dtype == torch.float32 and x.dtype == torch.bfloat16 and M > 0:
         return PendingProduct(given, w, resident)
     if rows is not None:
@@ -1401,13 +1414,13 @@ def linear(x, w, out_dtype=None, resident=False, lazy=False):
         xs = _rows_view(x, "linear x")
         if gemm_f32_tc.takes(w):
             return gemm_f32_tc.run(x, xs, w, resident)
-        y = torch.empty((M, N), dtype=torch.float32, device=x.device)
-        _library.call("dl_gemm_f32", _ptr(x), xs, _ptr(w), _ptr(y), N, M, N, K, _stream())
+        y = _library.empty(M, N, torch.float32, x)
+        _library.call("dl_gemm_f32", x, xs, w, y, N, M, N, K, _stream())
         return y
     if x.dtype != torch.bfloat16:
         raise KernelError(f"linear: unsupported dtype {x.dtype}")
     if M > 0:
-        y = gemm_skinny.maybe_run(x, w, out_dtype, resident=resident)
+        y = gemm_skinny.maybe_run(x, w, out_dtype, resident=resident, sizes=sizes)
         if y is not None:
             return y
     if out_dtype == torch.bfloat16:
@@ -1421,7 +1434,7 @@ def unary_activation(x, kind):
     if kind not in UNGATED:
         raise KernelError(f"unary_activation: {kind!r} is no activation of one product; known: {sorted(UNGATED)}")
     out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
-    _library.call("dl_unary_activation", _ptr(x), _rows_view(x, "unary_activation x"), _ptr(out), _code(x.dtype), x.shape[0],
+    _library.call("dl_unary_activation", x, _rows_view(x, "unary_activation x"), out, _code(x.dtype), x.shape[0],
                   x.shape[1], GATINGS[kind], _stream())
     return out
 
@@ -1451,7 +1464,7 @@ def softcap(values, cap):
     _need_cuda(values)
     if values.dtype != torch.float32 or not values.is_contiguous() or not cap > 0:
         raise KernelError("softcap: contiguous float32 values and a positive cap")
-    _library.call("dl_softcap", _ptr(values), values.numel(), float(cap), _stream())
+    _library.call("dl_softcap", values, values.numel(), float(cap), _stream())
     return values
 
 
@@ -1485,12 +1498,14 @@ def gated_linear(x, w_gate_up, resident=False, kind="silu", limit=0.0, alpha=1.0
             _need_cuda(x.data, w_gate_up)
             return gemm_skinny.run(x.data, w_gate_up, x.dtype, fuse_swiglu=True, resident=resident, row_sums=x.row_sums())
         x = x.tensor()
-    _need_cuda(x, w_gate_up)
-    if w_gate_up.dim() != 2 or w_gate_up.shape[0] % 2 or not w_gate_up.is_contiguous() or x.dim() != 2 \
-            or x.shape[1] != w_gate_up.shape[1]:
-        raise KernelError(f"gated_linear: x {tuple(x.shape)} does not match W {tuple(w_gate_up.shape)}")
+    sizes = _product_sizes(x, w_gate_up)
+    if sizes is None or sizes[2] % 2:
+        _need_cuda(x, w_gate_up)
+        if w_gate_up.dim() != 2 or w_gate_up.shape[0] % 2 or not w_gate_up.is_contiguous() or x.dim() != 2 \
+                or x.shape[1] != w_gate_up.shape[1]:
+            raise KernelError(f"gated_linear: x {tuple(x.shape)} does not match W {tuple(w_gate_up.shape)}")
     if x.dtype == torch.bfloat16 and x.shape[0] > 0:
-        y = gemm_skinny.maybe_run(x, w_gate_up, x.dtype, fuse_swiglu=True, resident=resident)
+        y = gemm_skinny.maybe_run(x, w_gate_up, x.dtype, fuse_swiglu=True, resident=resident, sizes=sizes)
         if y is not None:
             return y
         if gemm_tc.takes(x, w_gate_up, fuse_swiglu=True):
@@ -1519,8 +1534,8 @@ def sample(logits, temperature=None, top_k=None, top_p=None, min_p=None, uniform
         out = torch.empty((rows,), dtype=torch.int32, device=logits.device)
     elif out.dtype != torch.int32 or out.shape != (rows,) or not out.is_contiguous() or not out.is_cuda:
         raise KernelError("sample: out must be a contiguous int32 CUDA tensor of one id per row")
-    _library.call("dl_sample", _ptr(logits), logits.stride(0) if rows > 1 else vocab, rows, vocab,
-                  _ptr(temperature), _ptr(top_k), _ptr(top_p), _ptr(min_p), _ptr(uniform), _ptr(out),
+    _library.call("dl_sample", logits, logits.stride(0) if rows > 1 else vocab, rows, vocab,
+                  temperature, top_k, top_p, min_p, uniform, out,
                   0 if split is None else (2 if split else 1), _stream())
     return out
 
@@ -1553,7 +1568,7 @@ def repetition_penalty(logits, prev, prev_len, penalty, window, row_map=None, ap
                     ("append ids", tok)):
         if t is not None and t.numel() != rows:
             raise KernelError(f"repetition_penalty: {name} must hold one value per row ({rows}), got {t.numel()}")
-    _library.call("dl_repetition_penalty", _ptr(logits), logits.stride(0) if rows > 1 else vocab, rows,
-                  vocab, _ptr(prev), prev.shape[1], prev.shape[0], _ptr(row_map), _ptr(pos), _ptr(tok), _ptr(prev_len),
-                  _ptr(penalty), _ptr(window), _stream())
+    _library.call("dl_repetition_penalty", logits, logits.stride(0) if rows > 1 else vocab, rows,
+                  vocab, prev, prev.shape[1], prev.shape[0], row_map, pos, tok, prev_len,
+                  penalty, window, _stream())
     return logits
