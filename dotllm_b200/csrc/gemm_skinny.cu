@@ -7,33 +7,32 @@
 // 32-wide slice of k, lane (g, t) holds k = 8t..8t+7 of rows g and g+8 and the same slice of token
 // g's activations, which is a consistent permutation of k for both operands of two MMAs.
 //
-// Shape: persistent, warp-specialised, stream-K.  The work is the list of (16-row tile, 256-wide
-// chunk of k) pairs in tile-major order, cut into equal contiguous shares, one per consumer warp of
-// the whole grid, so every warp streams the same number of bytes whatever N and K are.  One producer
-// warp per block (lane c serving consumer warp c) copies chunks as tiled boxes of a tensor map over W
-// (cp.async.bulk.tensor.2d, 16 rows by 256 k) into a private ring of shared-memory stages for each
-// consumer warp, signalling an mbarrier per stage; copies run ahead of the arithmetic by the depth
-// of the ring.  A consumer never synchronises with another warp of
-// its block.  A tile that lies wholly inside one share is finished by that warp; a tile cut between
-// shares is summed, in share order, by whichever of its warps arrives last, so the result is
-// deterministic and does not depend on the number of rows of x.  With FUSE_SWIGLU a tile's rows
-// 0-7 are gate rows and rows 8-15 the matching up rows, and the epilogue writes silu(gate) * up
-// (native/kernels/swiglu.cu:7-41).
+// Shape: persistent, warp-specialised, in two forms.  One producer warp per block (lane c serving consumer warp c) copies chunks of W as tiled
+// boxes of a tensor map (cp.async.bulk.tensor.2d) into a private ring of shared-memory stages for each of eight consumer warps, signalling an
+// mbarrier per stage; copies run ahead of the arithmetic by the depth of the ring.  Either way a result does not depend on the number of rows of x and
+// is the same on every launch.  With FUSE_SWIGLU a tile's rows 0-7 are gate rows and rows 8-15 the matching up rows, and the epilogue
+// writes silu(gate) * up (native/kernels/swiglu.cu:7-41).
 //
-// Eight consumer warps of three stages and shares from one chunk on, over the whole GPU, against six of
-// four stages and shares of four chunks or more (192 KB in flight either way), kernels alone in a graph, 8 rows: 3,072 x 2,048 (12.6 MB)
-// 6.8 -> 5.6 us, 2,048 x 2,048 6.7 -> 5.1, 2,048 x 8,192 10.6 -> 8.9, 4,096 x 14,336 23.0 -> 21.7, gated 14,336 x 4,096 40.4 -> 39.8, 128,256 x
-// 2,048 90.9 -> 89.7 (5.9 TB/s); a decode step of 16 layers of the smaller widths, 8 sequences at 2,000 tokens, 991 -> 898 us.  A small
-// matrix is a chain of latencies (start, rows of x, hand-over of cut tiles) with few bytes between: what helps is that all multiprocessors take part.
-// Two blocks a multiprocessor of half the ring, so that the next product's first weights arrive under this one, lost more in
-// the stream than it gained at the edges (the step 1,217 us); asking for chunks in the L2 ahead of the ring, shares that differ by a chunk (their
-// bounds cost divisions on the way to a cut tile's sum: 1,088 us) and shares of neighbours in different blocks (932) likewise.
+// * By rows (gemm_skinny_rows_kernel; nearly all sizes): every multiprocessor owns the same number of rows of W over all of k.  The consumer warps split k,
+//   their sums meet in shared memory, and warps of their own add them in a fixed order and run the epilogue.  Nothing passes between blocks: no
+//   partial sums through global memory, no counters.  A pass holds up to 48 rows, so a chunk's slice of x is read once for all of them (x is 8 / 48 of what
+//   W is; with 16-row tiles it was half, and its loads' latency set the pace).
+// * By shares (gemm_skinny_kernel; where a block's rows are one tile and 4,096 < K < 12,288): the list of (16-row tile, 256-wide chunk of k) pairs in
+//   tile-major order is cut into equal contiguous shares, one per consumer warp of the whole grid.  A tile cut between shares is summed, in share
+//   order, by whichever of its warps arrives last.
+//
+// By rows against by shares, each product in a graph of many, 8 rows: 3,072 x 2,048 5.5 -> 5.0 us, 2,048 x 2,048 5.1 -> 4.2, 64 x 2,048 3.8 -> 2.7, gated
+// 8,192 x 2,048 15.4 -> 13.3, 6,144 x 4,096 12.7 -> 11.1, 4,096 x 14,336 22.1 -> 20.9, gated 14,336 x 4,096 40.3 -> 38.5, 128,256 x 2,048
+// 87.0 -> 80.6 (6.5 TB/s); the small ones are a chain of latencies (start, rows of x, sums).  One tile a block leaves x at half the bytes of W again:
+// 2,048 x 4,096 by rows 6.3, by shares 6.4; x 6,144 8.2 and 7.7; x 8,192 9.9 and 9.2; x 16,384 15.3 and 16.1.  A decode step of 16 layers of the smaller
+// widths, 8 sequences at 2,000 tokens: 905 -> 849 us.  Tried: rings of half the size, so that the next product's first weights arrive under this one
+// (941 us), x asked for three chunks ahead (2,048 x 2,048 4.3 -> 4.7), passes of 32 rows (5,120 x 13,824, 35 rows a block: 25.5 -> 30.1).
 //
 // Two optional fusions take the add + RMSNorm between two products of a decode step into the products
 // themselves (the reference's fused_add_rmsnorm, native/kernels/fused_add_rmsnorm.cu:9-72, is a kernel
 // of its own).  A float32 product with `gain` set adds its result into the float32 residual stream it
 // is given as `out`, writes the sum times the norm's gain as bfloat16 (`scaled`) and the sum of squares
-// of every 16-column tile and row (`sumsq_out`).  The product that follows takes `scaled` as its x
+// of every tile and row (`sumsq_out`, a part of 16 floats a tile).  The product that follows takes `scaled` as its x
 // and `sumsq_in`: a warp of its own adds the tiles' sums in tile order, and every output row is
 // multiplied by rsqrt(sum / n + eps) in the epilogue - x W^T of the normalised row, since the
 // normalisation is one factor per row.  All of it in float32 and in a fixed order.
@@ -43,6 +42,7 @@
 #include "common.cuh"
 #include "gating.cuh"
 #include "tma.cuh"
+#include <atomic>
 #include <mutex>
 #include <type_traits>
 #include <unordered_map>
@@ -54,10 +54,22 @@
 #define GS_SLOTS 3                         // ring stages per consumer warp
 #endif
 #define GS_BK 256                          // k per chunk
+// ... and where rows are shared out evenly (gemm_skinny_rows_kernel)
+#define GR_MOST 48                         // rows of a pass, at most (gated: 16 pairs)
+#define GR_MAX_SLOTS 8                     // ring stages per consumer warp, at most
+#define GR_THREADS(TILES) (32 * (GS_CONSUMERS + 1 + (TILES)))   // consumers, the producer warp, a warp a tile that adds
+#define GR_SMEM 231168                     // bytes of shared memory for the rings and the sums, at most: what a block can have less the barriers
 #define GS_STAGE_ELEMS (16 * GS_BK)         // a stage is the dense box the copy engine writes: [16 rows][256 k]
 #define GS_THREADS (32 * (GS_CONSUMERS + 2))   // consumers, the producer warp, the row-statistics warp
 #define GS_WAIT_CYCLES (1ll << 31)
 #define GS_MAX_ROWS 16
+// Rows of a stage (gated: the up rows lie behind room for all tiles' gate rows), and bytes of a block's rings with what a read of the missing
+// rows of the last tile reaches beyond them.
+__host__ __device__ static inline int GR_stage_rows(int rows, bool gated, int tiles) { return gated ? 8 * tiles + rows : rows; }
+__host__ __device__ static inline int GR_ring_bytes(int rows, int slots, bool gated, int tiles, int bk) {
+    const int stage = GR_stage_rows(rows, gated, tiles);
+    return (GS_CONSUMERS * slots * stage + 16 * tiles - stage) * bk * 2;
+}
 
 __device__ __forceinline__ void gs_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                        uint32_t b0, uint32_t b1) {
@@ -122,8 +134,9 @@ struct GsFuse {
 // acc[j] = {(row g, tok 2t), (row g, tok 2t+1), (row g+8, tok 2t), (row g+8, tok 2t+1)} of 8-token group j
 // `row_scale`: null, or the factor of every output row (token).  `fuse.gain` (float32 plain products
 // only): add into `out` and leave the scaled copy and the tile's sums of squares for the next product.
+// The tile's rows of W are `base` .. `end` - 1 (at most 16, gated: pairs, at most 8); its sums of squares are part `part`.
 template <int NT, typename TOut, bool FUSE_SWIGLU>
-__device__ __forceinline__ void gs_epilogue(const float (&acc_in)[NT][4], TOut* out, int out_stride, int tile, int M,
+__device__ __forceinline__ void gs_epilogue(const float (&acc_in)[NT][4], TOut* out, int out_stride, int part, int base, int end, int M,
                                             int N, int g, int t, const float* row_scale, const GsFuse& fuse,
                                             const float (&stream_in)[NT][4], const float (&gain_in)[2]) {
 #pragma unroll
@@ -135,8 +148,8 @@ __device__ __forceinline__ void gs_epilogue(const float (&acc_in)[NT][4], TOut* 
             acc[0] *= s0, acc[1] *= s1, acc[2] *= s0, acc[3] *= s1;
         }
         if (FUSE_SWIGLU) {
-            const int col = tile * 8 + g;
-            if (col < N) {
+            const int col = base + g;
+            if (col < end) {
                 if (fuse.gate_bias != nullptr) {
                     const float bg = __ldg(fuse.gate_bias + col), bu = __ldg(fuse.gate_bias + N + col);
                     acc[0] += bg, acc[1] += bg, acc[2] += bu, acc[3] += bu;
@@ -157,33 +170,33 @@ __device__ __forceinline__ void gs_epilogue(const float (&acc_in)[NT][4], TOut* 
             float ss[2] = {0.f, 0.f};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int row = tile * 16 + g + (e >> 1) * 8, tok = tok0 + (e & 1);
-                if (row < N && tok < M) {
+                const int row = base + g + (e >> 1) * 8, tok = tok0 + (e & 1);
+                if (row < end && tok < M) {
                     const float h = stream_in[j][e] + acc[e];
                     stream[(size_t)tok * out_stride + row] = h;
                     fuse.scaled[(size_t)tok * fuse.scaled_stride + row] = __float2bfloat16_rn(h * gain_in[e >> 1]);
                     ss[e & 1] = fmaf(h, h, ss[e & 1]);
                 }
             }
-            // the tile's 16 columns of a token lie in the 8 lanes that share t: add them in a fixed order
+            // the tile's columns of a token lie in the 8 lanes that share t: add them in a fixed order
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 ss[e] += __shfl_xor_sync(0xffffffffu, ss[e], 4);
                 ss[e] += __shfl_xor_sync(0xffffffffu, ss[e], 8);
                 ss[e] += __shfl_xor_sync(0xffffffffu, ss[e], 16);
-                if (g == 0 && tok0 + e < M) fuse.sumsq_out[(size_t)tile * 16 + tok0 + e] = ss[e];
+                if (g == 0 && tok0 + e < M) fuse.sumsq_out[(size_t)part * 16 + tok0 + e] = ss[e];
             }
         } else {
             if (!dl_gate_is_gated(fuse.gate_kind)) {         // an activation of the one product
 #pragma unroll
                 for (int e = 0; e < 4; ++e) acc[e] = dl_unary_value(fuse.gate_kind, acc[e]);
             }
-            const int row_lo = tile * 16 + g, row_hi = row_lo + 8;
-            if (row_lo < N) {
+            const int row_lo = base + g, row_hi = row_lo + 8;
+            if (row_lo < end) {
                 if (tok0 < M) gs_store<TOut>(out + (size_t)tok0 * out_stride + row_lo, acc[0]);
                 if (tok0 + 1 < M) gs_store<TOut>(out + (size_t)(tok0 + 1) * out_stride + row_lo, acc[1]);
             }
-            if (row_hi < N) {
+            if (row_hi < end) {
                 if (tok0 < M) gs_store<TOut>(out + (size_t)tok0 * out_stride + row_hi, acc[2]);
                 if (tok0 + 1 < M) gs_store<TOut>(out + (size_t)(tok0 + 1) * out_stride + row_hi, acc[3]);
             }
@@ -191,7 +204,7 @@ __device__ __forceinline__ void gs_epilogue(const float (&acc_in)[NT][4], TOut* 
     }
 }
 
-// Built with -DGS_TIMELINE (DOTLLM_NVCC_EXTRA), every warp stamps the global nanosecond timer at six
+// Built with -DGS_TIMELINE (DOTLLM_NVCC_EXTRA), every warp of a product by shares stamps the global nanosecond timer at six
 // points of a launch into gs_timeline, which dl_gemm_skinny_timeline copies out
 // (`python -m dotllm_b200.kernels.microbench gemm_skinny --timeline` prints the spread over the grid).
 #ifdef GS_TIMELINE
@@ -381,7 +394,7 @@ __device__ __forceinline__ void gs_consume(const GsWork& w, const GsRings& r, fl
                 }
             }
             if (whole) {
-                gs_epilogue<NT, TOut, FUSE_SWIGLU>(acc, out, w.out_stride, tile, M, N, g, t, row_scale, w.fuse, stream_in, gain_in);
+                gs_epilogue<NT, TOut, FUSE_SWIGLU>(acc, out, w.out_stride, tile, tile * (FUSE_SWIGLU ? 8 : 16), N, M, N, g, t, row_scale, w.fuse, stream_in, gain_in);
             } else {
                 // a warp's first tile may be shared with the share before, its last with the share after
                 const int which = (tile == begin / cpt) ? 0 : 1;
@@ -416,7 +429,7 @@ __device__ __forceinline__ void gs_consume(const GsWork& w, const GsRings& r, fl
 #pragma unroll
                             for (int e = 0; e < 4; ++e) acc[j][e] += __ldcg(theirs + (j * 4 + e) * 32 + lane);
                     }
-                    gs_epilogue<NT, TOut, FUSE_SWIGLU>(acc, out, w.out_stride, tile, M, N, g, t, row_scale, w.fuse, stream_in, gain_in);
+                    gs_epilogue<NT, TOut, FUSE_SWIGLU>(acc, out, w.out_stride, tile, tile * (FUSE_SWIGLU ? 8 : 16), N, M, N, g, t, row_scale, w.fuse, stream_in, gain_in);
                 }
             }
 #pragma unroll
@@ -450,6 +463,49 @@ __device__ __forceinline__ void gs_consume(const GsWork& w, const GsRings& r, fl
     const GsRings rings{reinterpret_cast<__nv_bfloat16*>(gs_smem_raw), full_bar, empty_bar, &gave_up, status, &scale_bar,  \
                         row_scale_smem}
 
+// The row-statistics warp: the factors of the output rows from the sums that the product before left (`scale_bar` completes when they are written).
+__device__ __forceinline__ void gs_row_factors(const GsFuse& fuse, float* factors, uint64_t* scale_bar, int lane) {
+    if (fuse.sumsq_in == nullptr) return;
+    dl_grid_dependency_wait();   // the sums come from the kernel before this one
+    // A warp-wide float4 load covers 8 parts x 16 rows: lane -> (rows 4q .. 4q+3, part l/4 of
+    // every 8).  All loads of a batch are in flight together; a lane adds its parts in part
+    // order, then the 8 lanes of a row group are added in a fixed order: the same bits on
+    // every launch.
+    const int q = lane & 3, sub = lane >> 2;
+    const float4* in = reinterpret_cast<const float4*>(fuse.sumsq_in) + q;
+    float4 acc4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int p0 = 0; p0 < fuse.n_parts; p0 += 8 * 16) {
+        float4 v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int p = p0 + 8 * i + sub;
+            v[i] = p < fuse.n_parts ? __ldcg(in + (size_t)p * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc4.x += v[i].x, acc4.y += v[i].y, acc4.z += v[i].z, acc4.w += v[i].w;
+    }
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+        // both partners add (lower lane's value) + (higher lane's value)
+        const float4 other = make_float4(__shfl_xor_sync(0xffffffffu, acc4.x, o), __shfl_xor_sync(0xffffffffu, acc4.y, o),
+                                         __shfl_xor_sync(0xffffffffu, acc4.z, o), __shfl_xor_sync(0xffffffffu, acc4.w, o));
+        const bool low = (lane & o) == 0;
+        acc4.x = low ? acc4.x + other.x : other.x + acc4.x;
+        acc4.y = low ? acc4.y + other.y : other.y + acc4.y;
+        acc4.z = low ? acc4.z + other.z : other.z + acc4.z;
+        acc4.w = low ? acc4.w + other.w : other.w + acc4.w;
+    }
+    if (lane < 4) {
+        factors[4 * lane + 0] = rsqrtf(acc4.x * fuse.inv_n + fuse.eps);
+        factors[4 * lane + 1] = rsqrtf(acc4.y * fuse.inv_n + fuse.eps);
+        factors[4 * lane + 2] = rsqrtf(acc4.z * fuse.inv_n + fuse.eps);
+        factors[4 * lane + 3] = rsqrtf(acc4.w * fuse.inv_n + fuse.eps);
+    }
+    __threadfence_block();
+    __syncwarp();
+    if (lane == 0) gs_mbar_arrive(scale_bar);
+}
+
 template <int NT, typename TOut, bool FUSE_SWIGLU>
 __global__ void __launch_bounds__(GS_THREADS, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap, const GsWork work, int early_weights,
@@ -469,46 +525,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap, const GsWork work, 
         }
     } else if (warp == GS_CONSUMERS + 1) {
         // ------------------------------------------------------------ row-statistics warp
-        if (work.fuse.sumsq_in != nullptr) {
-            dl_grid_dependency_wait();   // the sums come from the kernel before this one
-            // A warp-wide float4 load covers 8 parts x 16 rows: lane -> (rows 4q .. 4q+3, part l/4 of
-            // every 8).  All loads of a batch are in flight together; a lane adds its parts in part
-            // order, then the 8 lanes of a row group are added in a fixed order: the same bits on
-            // every launch.
-            const int q = lane & 3, sub = lane >> 2;
-            const float4* in = reinterpret_cast<const float4*>(work.fuse.sumsq_in) + q;
-            float4 acc4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int p0 = 0; p0 < work.fuse.n_parts; p0 += 8 * 16) {
-                float4 v[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int p = p0 + 8 * i + sub;
-                    v[i] = p < work.fuse.n_parts ? __ldcg(in + (size_t)p * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-#pragma unroll
-                for (int i = 0; i < 16; ++i) acc4.x += v[i].x, acc4.y += v[i].y, acc4.z += v[i].z, acc4.w += v[i].w;
-            }
-#pragma unroll
-            for (int o = 4; o < 32; o <<= 1) {
-                // both partners add (lower lane's value) + (higher lane's value)
-                const float4 other = make_float4(__shfl_xor_sync(0xffffffffu, acc4.x, o), __shfl_xor_sync(0xffffffffu, acc4.y, o),
-                                                 __shfl_xor_sync(0xffffffffu, acc4.z, o), __shfl_xor_sync(0xffffffffu, acc4.w, o));
-                const bool low = (lane & o) == 0;
-                acc4.x = low ? acc4.x + other.x : other.x + acc4.x;
-                acc4.y = low ? acc4.y + other.y : other.y + acc4.y;
-                acc4.z = low ? acc4.z + other.z : other.z + acc4.z;
-                acc4.w = low ? acc4.w + other.w : other.w + acc4.w;
-            }
-            if (lane < 4) {
-                row_scale_smem[4 * lane + 0] = rsqrtf(acc4.x * work.fuse.inv_n + work.fuse.eps);
-                row_scale_smem[4 * lane + 1] = rsqrtf(acc4.y * work.fuse.inv_n + work.fuse.eps);
-                row_scale_smem[4 * lane + 2] = rsqrtf(acc4.z * work.fuse.inv_n + work.fuse.eps);
-                row_scale_smem[4 * lane + 3] = rsqrtf(acc4.w * work.fuse.inv_n + work.fuse.eps);
-            }
-            __threadfence_block();
-            __syncwarp();
-            if (lane == 0) gs_mbar_arrive(&scale_bar);
-        }
+        gs_row_factors(work.fuse, row_scale_smem, &scale_bar, lane);
     } else if (warp < work.active) {
         // ------------------------------------------------------------ consumer warp
         dl_grid_dependency_wait();       // x comes from the kernel before this one; out, partials and counters may be in use by it
@@ -519,6 +536,258 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap, const GsWork work, 
     }
     __syncthreads();                                         // nobody leaves while copies may still land
     GS_STAMP(5);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Rows shared out evenly: block b owns rows R b .. R (b + 1) - 1 of W (R = ceil(N / multiprocessors)) over all of k, in `passes` passes of `rows` <= 48
+// of them (gated: pairs, <= 16), TILES tiles of 16 (8 pairs) at most.  A pass's chunks of BK k go round the block's eight consumer warps; at its end the warps' sums meet in
+// shared memory, where a warp a tile adds them in warp order while the others go on with the next pass.  Nothing passes between blocks.
+struct GsRowsWork {
+    const __nv_bfloat16* x;
+    int x_stride;
+    void* out;
+    int out_stride;
+    int M, N, K, up_offset, cpt, block_rows, rows, passes, slots;     // slots: ring stages of a consumer warp
+    GsFuse fuse;
+};
+
+// Tiles of 16 rows that n rows make in passes of `rows`.
+__host__ __device__ static inline int gs_rows_tiles(int n, int rows) {
+    const int full = n / rows, rest = n - full * rows;
+    return full * ((rows + 15) / 16) + (rest + 15) / 16;
+}
+
+template <int NT, int BK>
+__device__ __forceinline__ void gs_rows_x(uint4 (&xf)[BK / 32][NT], const GsRowsWork& w, int k0, int g, int t) {
+#pragma unroll
+    for (int s = 0; s < BK / 32; ++s)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            const int tok = j * 8 + g, k = k0 + 32 * s + 8 * t;
+            xf[s][j] = make_uint4(0u, 0u, 0u, 0u);
+            if (tok < w.M && k < w.K) xf[s][j] = __ldg(reinterpret_cast<const uint4*>(w.x + (size_t)tok * w.x_stride + k));
+        }
+}
+
+template <int NT, typename TOut, bool FUSE_SWIGLU, int TILES, int BK>
+__global__ void __launch_bounds__(GR_THREADS(TILES), 1)
+gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWork w, int early_weights, int* __restrict__ status) {
+    constexpr int TILE = FUSE_SWIGLU ? 8 : 16;               // rows (gated: pairs) of a tile
+    extern __shared__ __align__(128) unsigned char gs_smem_raw[];
+    __shared__ uint64_t full_bar[GS_CONSUMERS][GR_MAX_SLOTS], empty_bar[GS_CONSUMERS][GR_MAX_SLOTS], scale_bar, sums_full[2], sums_empty[2];
+    __shared__ volatile int gave_up;
+    __shared__ float row_scale_smem[GS_MAX_ROWS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    if (threadIdx.x == 0) {
+        gave_up = 0;
+        gs_mbar_init(&scale_bar, 1);
+        for (int h = 0; h < 2; ++h) gs_mbar_init(&sums_full[h], GS_CONSUMERS), gs_mbar_init(&sums_empty[h], TILES);
+        for (int c = 0; c < GS_CONSUMERS; ++c)
+            for (int s = 0; s < w.slots; ++s) {
+                gs_mbar_init(&full_bar[c][s], 1);
+                gs_mbar_init(&empty_bar[c][s], 1);
+            }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    dl_launch_dependents();
+    const int first = blockIdx.x * w.block_rows, end_row = min(w.N, first + w.block_rows);      // this block's rows
+    const int passes = (end_row - first + w.rows - 1) / w.rows, total = passes * w.cpt;
+    const uint32_t box_bytes = w.rows * (BK * 2), stage_bytes = GR_stage_rows(w.rows, FUSE_SWIGLU, TILES) * (BK * 2);
+    // the sums of a pass, of two passes in turn: [2][warp][tile][NT][lane]
+    float4* sums = reinterpret_cast<float4*>(gs_smem_raw + GR_ring_bytes(w.rows, w.slots, FUSE_SWIGLU, TILES, BK));
+    if (warp < GS_CONSUMERS) {
+        // ------------------------------------------------------------ consumer warp
+        dl_grid_dependency_wait();       // x comes from the kernel before this one
+        uint4 xf[BK / 32][NT];
+        int cur = warp, slot = 0, phase = 0;
+        bool dead = false;
+        auto gave = [&](int code) {
+            if (!gave_up) atomicExch(status, code);
+            gave_up = 1;
+            dead = true;
+        };
+        if (cur < total) gs_rows_x<NT, BK>(xf, w, (cur % w.cpt) * BK, g, t);
+        for (int p = 0; p < passes; ++p) {
+            float acc[TILES][NT][4];
+#pragma unroll
+            for (int i = 0; i < TILES; ++i)
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+            for (const int pass_end = (p + 1) * w.cpt; cur < pass_end; cur += GS_CONSUMERS) {
+                if (!dead && !gs_mbar_wait(&full_bar[warp][slot], phase, &gave_up)) gave(3);
+                uint4 xn[BK / 32][NT];                    // the next chunk's rows of x, asked for before this one's arithmetic
+                const int next = cur + GS_CONSUMERS;
+                gs_rows_x<NT, BK>(xn, w, next < total ? (next % w.cpt) * BK : w.K, g, t);
+                if (!dead) {
+                    // rows beyond the box are whatever lies behind it: they reach output rows that are not stored
+                    const uint32_t st = gs_smem(gs_smem_raw + (size_t)(warp * w.slots + slot) * stage_bytes) + (uint32_t)(g * BK + 8 * t) * 2u;
+                    const int tiles = (w.rows + TILE - 1) / TILE;
+#pragma unroll
+                    for (int s = 0; s < BK / 32; ++s) {
+#pragma unroll
+                        for (int i = 0; i < TILES; ++i) {
+                            if (i >= tiles) break;
+                            // a plain tile's upper eight rows lie behind its lower eight, a gated one's behind all gate rows
+                            const uint4 a_lo = gs_lds128(st + (uint32_t)((TILE * i * BK + 32 * s) * 2));
+                            const uint4 a_hi = gs_lds128(st + (uint32_t)(((FUSE_SWIGLU ? TILE * TILES + TILE * i : TILE * i + 8) * BK + 32 * s) * 2));
+#pragma unroll
+                            for (int j = 0; j < NT; ++j) {
+                                gs_mma(acc[i][j], a_lo.x, a_hi.x, a_lo.y, a_hi.y, xf[s][j].x, xf[s][j].y);
+                                gs_mma(acc[i][j], a_lo.z, a_hi.z, a_lo.w, a_hi.w, xf[s][j].z, xf[s][j].w);
+                            }
+                        }
+                    }
+                    // as in gs_consume: the slot is released when every read of it is done
+#pragma unroll
+                    for (int i = 0; i < TILES; ++i)
+#pragma unroll
+                        for (int j = 0; j < NT; ++j) asm volatile("" : "+f"(acc[i][j][0]), "+f"(acc[i][j][1]), "+f"(acc[i][j][2]), "+f"(acc[i][j][3]));
+                    __threadfence_block();
+                    __syncwarp();
+                    if (lane == 0) gs_mbar_arrive(&empty_bar[warp][slot]);
+                }
+                if (++slot == w.slots) slot = 0, phase ^= 1;
+#pragma unroll
+                for (int s = 0; s < BK / 32; ++s)
+#pragma unroll
+                    for (int j = 0; j < NT; ++j) xf[s][j] = xn[s][j];
+            }
+            const int h = p & 1;
+            if (p >= 2 && !dead && !gs_mbar_wait(&sums_empty[h], ((p >> 1) - 1) & 1, &gave_up)) gave(6);
+            float4* mine = sums + (size_t)(h * GS_CONSUMERS + warp) * TILES * NT * 32 + lane;
+            if (!dead) {
+#pragma unroll
+                for (int i = 0; i < TILES; ++i)
+#pragma unroll
+                    for (int j = 0; j < NT; ++j) mine[(i * NT + j) * 32] = make_float4(acc[i][j][0], acc[i][j][1], acc[i][j][2], acc[i][j][3]);
+            }
+            __threadfence_block();
+            __syncwarp();
+            if (lane == 0) gs_mbar_arrive(&sums_full[h]);
+        }
+    } else if (warp == GS_CONSUMERS) {
+        // ------------------------------------------------------------ producer warp: lane c serves consumer warp c
+        // When the caller vouches that no pending work writes the weights (early_weights), the rings fill while the kernel before this one finishes.
+        if (!early_weights) dl_grid_dependency_wait();
+        if (lane < GS_CONSUMERS) {
+            const uint64_t policy = dl_stream_policy();      // W is read once a step: first out of the L2
+            int cnt = 0, cur = lane, slot = 0, phase = 1;
+            bool ok = true;
+            long long t0 = clock64();
+            while (cur < total) {
+                if (cnt < w.slots || gs_mbar_try(&empty_bar[lane][slot], phase)) {
+                    const int pass = cur / w.cpt, kc = cur - pass * w.cpt, row = first + pass * w.rows;
+                    unsigned char* dst = gs_smem_raw + (size_t)(lane * w.slots + slot) * stage_bytes;
+                    // a box is always written whole: parts outside the matrix arrive as zeros
+                    gs_mbar_expect(&full_bar[lane][slot], FUSE_SWIGLU ? 2 * box_bytes : box_bytes);
+                    dl_tma_load_2d_hint(dst, &tmap, kc * BK, row, &full_bar[lane][slot], policy);
+                    if (FUSE_SWIGLU) dl_tma_load_2d_hint(dst + TILES * TILE * BK * 2, &tmap, kc * BK, w.up_offset + row, &full_bar[lane][slot], policy);
+                    cur += GS_CONSUMERS, ++cnt;
+                    if (++slot == w.slots) slot = 0, phase ^= 1;
+                    t0 = clock64();
+                } else if (gave_up || clock64() - t0 > GS_WAIT_CYCLES) {
+                    if (!gave_up) atomicExch(status, 1);
+                    gave_up = 1;
+                    ok = false;
+                    break;
+                }
+            }
+            if (!ok)                                         // copies already issued must land before the block's shared memory is released
+                for (int i = max(0, cnt - w.slots); i < cnt; ++i) {
+                    const long long t1 = clock64();
+                    while (!gs_mbar_try(&full_bar[lane][i % w.slots], (i / w.slots) & 1) && clock64() - t1 < GS_WAIT_CYCLES) {}
+                }
+        }
+    } else {
+        // ------------------------------------------------------------ adding warps: one a tile of a pass; the first makes the row factors before that
+        const int tile = warp - GS_CONSUMERS - 1, N = w.N, M = w.M;
+        if (tile == 0) gs_row_factors(w.fuse, row_scale_smem, &scale_bar, lane);
+        dl_grid_dependency_wait();                           // out may be in use by the kernel before this one
+        TOut* out = reinterpret_cast<TOut*>(w.out);
+        const bool into = std::is_same<TOut, float>::value && !FUSE_SWIGLU && w.fuse.gain != nullptr;
+        const float* row_scale = nullptr;
+        bool dead = false;
+        for (int p = 0; p < passes && !dead; ++p) {
+            const int h = p & 1, pass_end = min(end_row, first + (p + 1) * w.rows);
+            const int base = first + p * w.rows + tile * TILE;
+            // the stream's values and the gains, asked for early so that the epilogue does not wait for them (only this warp ever writes them)
+            float stream_in[NT][4], gain_in[2] = {0.f, 0.f};
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) stream_in[j][e] = 0.f;
+            if (into) {
+                const float* stream = reinterpret_cast<const float*>(w.out);
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const int row = base + g + 8 * r;
+                    gain_in[r] = row < pass_end ? __ldg(w.fuse.gain + row) : 0.f;
+#pragma unroll
+                    for (int j = 0; j < NT; ++j)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const int tok = j * 8 + 2 * t + e;
+                            stream_in[j][2 * r + e] = (row < pass_end && tok < M) ? __ldcg(stream + (size_t)tok * w.out_stride + row) : 0.f;
+                        }
+                }
+            }
+            if (!gs_mbar_wait(&sums_full[h], (p >> 1) & 1, &gave_up) ||
+                (w.fuse.sumsq_in != nullptr && row_scale == nullptr && !gs_mbar_wait(&scale_bar, 0, &gave_up))) {
+                if (!gave_up) atomicExch(status, 5);
+                gave_up = 1;
+                dead = true;
+                continue;
+            }
+            if (w.fuse.sumsq_in != nullptr) row_scale = row_scale_smem;
+            float acc[NT][4];
+            const float4* theirs = sums + (size_t)(h * GS_CONSUMERS * TILES + tile) * NT * 32 + lane;
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                float4 v[GS_CONSUMERS];
+#pragma unroll
+                for (int c = 0; c < GS_CONSUMERS; ++c) v[c] = theirs[(c * TILES * NT + j) * 32];
+                acc[j][0] = v[0].x, acc[j][1] = v[0].y, acc[j][2] = v[0].z, acc[j][3] = v[0].w;
+#pragma unroll
+                for (int c = 1; c < GS_CONSUMERS; ++c) acc[j][0] += v[c].x, acc[j][1] += v[c].y, acc[j][2] += v[c].z, acc[j][3] += v[c].w;
+            }
+            __syncwarp();
+            if (lane == 0) gs_mbar_arrive(&sums_empty[h]);
+            if (base < pass_end)
+                gs_epilogue<NT, TOut, FUSE_SWIGLU>(acc, out, w.out_stride, blockIdx.x * gs_rows_tiles(w.block_rows, w.rows) + p * ((w.rows + 15) / 16) + tile, base, pass_end, M, N, g, t, row_scale, w.fuse, stream_in, gain_in);
+        }
+    }
+    __syncthreads();                                         // nobody leaves while copies may still land
+}
+
+// How rows are shared out: rows of a block, passes of a block, rows of a pass, blocks.  By N and the device alone, so that the parts of a row's
+// sum of squares lie the same for every product of that width.
+struct GsRowsPlan {
+    int block_rows, passes, rows, blocks;
+};
+static GsRowsPlan gs_rows_plan(int N, bool gated, int sms) {
+    const int most = gated ? 16 : GR_MOST;
+    GsRowsPlan p;
+    p.block_rows = (N + sms - 1) / sms;
+    p.passes = (p.block_rows + most - 1) / most;
+    p.rows = (p.block_rows + p.passes - 1) / p.passes;
+    p.blocks = (N + p.block_rows - 1) / p.block_rows;
+    return p;
+}
+// Which products go that way; the others by shares.  With one tile of rows a block, x is half as many bytes as W, and by shares it is asked for
+// further ahead; below 4,096 what passes between blocks costs more than that, at 16,384 the rows' distance of a power of two slows the shares down
+// (both sides measured at the top of this file).
+static bool gs_by_rows(int N, int K, bool gated, int sms) { return gated || (N + sms - 1) / sms > 16 || K <= 4096 || K >= 12288; }
+
+// Parts of the sums of squares (16 floats each) that a product of N output columns over K leaves.
+extern "C" int dl_gemm_skinny_parts(int N, int K) {
+    const int sms = dl_sm_count();
+    if (!gs_by_rows(N, K, false, sms)) return (N + 15) / 16;
+    const GsRowsPlan p = gs_rows_plan(N, false, sms);
+    const int last = N - (p.blocks - 1) * p.block_rows;      // the last block may have fewer rows
+    return (p.blocks - 1) * gs_rows_tiles(p.block_rows, p.rows) + gs_rows_tiles(last, p.rows);
 }
 
 // How the work of an (N, K) matrix is cut: tiles of 16 rows (8 gate + 8 up when gated), chunks per
@@ -556,29 +825,28 @@ extern "C" int dl_gemm_skinny_scratch(int M, int N, int K, int fuse_swiglu, int 
     return DL_OK;
 }
 
-// Tensor map of W: rows of K bfloat16, boxes of 16 rows (8 for gate + up) by 256 columns.  Encoding
+// Tensor map of W: `rows` rows of K bfloat16, boxes of `box` rows by `bk` columns.  Encoding
 // costs a driver call, so maps are kept per (matrix, shape).
 struct GsMapKey {
     const void* w;
-    int rows, k, box;
-    bool operator==(const GsMapKey& o) const { return w == o.w && rows == o.rows && k == o.k && box == o.box; }
+    int rows, k, box, bk;
+    bool operator==(const GsMapKey& o) const { return w == o.w && rows == o.rows && k == o.k && box == o.box && bk == o.bk; }
 };
 struct GsMapKeyHash {
     size_t operator()(const GsMapKey& k) const {
-        return std::hash<const void*>()(k.w) ^ ((size_t)k.rows * 1000003u) ^ ((size_t)k.k * 10007u) ^ (size_t)k.box;
+        return std::hash<const void*>()(k.w) ^ ((size_t)k.rows * 1000003u) ^ ((size_t)k.k * 10007u) ^ (size_t)(k.box + 32 * k.bk);
     }
 };
 
-static int gs_weight_map(CUtensorMap* out, const void* w, int N, int K, bool gated) {
+static int gs_weight_map(CUtensorMap* out, const void* w, int rows, int K, int box, int bk) {
     static std::unordered_map<GsMapKey, CUtensorMap, GsMapKeyHash> maps;
     static std::mutex maps_mutex;
-    const int rows = gated ? 2 * N : N, box = gated ? 8 : 16;
     std::lock_guard<std::mutex> lock(maps_mutex);
-    const GsMapKey key{w, rows, K, box};
+    const GsMapKey key{w, rows, K, box, bk};
     auto it = maps.find(key);
     if (it == maps.end()) {
         CUtensorMap fresh;
-        if (dl_tmap_encode_2d_bf16(&fresh, w, (uint64_t)rows, (uint64_t)K, (uint64_t)K * 2, box, GS_BK, DL_TMAP_SWIZZLE_NONE) != 0)
+        if (dl_tmap_encode_2d_bf16(&fresh, w, (uint64_t)rows, (uint64_t)K, (uint64_t)K * 2, box, bk, DL_TMAP_SWIZZLE_NONE) != 0)
             return DL_ERR_LAUNCH;
         if (maps.size() > 4096) maps.clear();
         it = maps.emplace(key, fresh).first;
@@ -599,13 +867,51 @@ static int gs_launch(const GsPlan& p, cudaStream_t s, const __nv_bfloat16* x, in
         configured = true;
     }
     CUtensorMap tmap;
-    const int rc = gs_weight_map(&tmap, w, N, K, FUSE);
+    const int rc = gs_weight_map(&tmap, w, FUSE ? 2 * N : N, K, FUSE ? 8 : 16, GS_BK);
     if (rc != DL_OK) return rc;
     const GsWork work{x, x_stride, out, out_stride, M, N, K, up_offset, p.cpt, p.total, p.active, p.share, fuse};
     cudaError_t le = dl_launch_dependent(gemm_skinny_kernel<NT, TOut, FUSE>, dim3(p.blocks), dim3(GS_THREADS), smem, s, tmap, work,
                                          early_weights, partials, counters, status);
     if (le != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "gemm_skinny: %s", cudaGetErrorString(le));
     return DL_OK;
+}
+
+template <int NT, typename TOut, bool FUSE, int TILES, int BK>
+static int gs_launch_rows_of(const GsRowsPlan& p, cudaStream_t s, const __nv_bfloat16* x, int x_stride, const __nv_bfloat16* w, void* out, int out_stride, int M,
+                          int N, int K, int early_weights, int* status, const GsFuse& fuse) {
+    const int cpt = (K + BK - 1) / BK;
+    const int a_warp = (p.passes * cpt + GS_CONSUMERS - 1) / GS_CONSUMERS;     // the busiest warp's chunks: no stages beyond them
+    const int sums = (p.passes > 1 ? 2 : 1) * GS_CONSUMERS * TILES * NT * 512;
+    int slots = a_warp < GR_MAX_SLOTS ? a_warp : GR_MAX_SLOTS;
+    while (slots > 1 && GR_ring_bytes(p.rows, slots, FUSE, TILES, BK) + sums > GR_SMEM) --slots;
+    const int smem = GR_ring_bytes(p.rows, slots, FUSE, TILES, BK) + sums;
+    static std::atomic<unsigned long long> sized{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess && (dev >= 64 || !(sized.load() >> dev & 1))) {
+        e = cudaFuncSetAttribute(gemm_skinny_rows_kernel<NT, TOut, FUSE, TILES, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM);
+        if (e == cudaSuccess && dev < 64) sized.fetch_or(1ull << dev);
+    }
+    if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "gemm_skinny: shared memory %d: %s", smem, cudaGetErrorString(e));
+    CUtensorMap tmap;
+    const int rc = gs_weight_map(&tmap, w, FUSE ? 2 * N : N, K, p.rows, BK);
+    if (rc != DL_OK) return rc;
+    const GsRowsWork work{x, x_stride, out, out_stride, M, N, K, N, cpt, p.block_rows, p.rows, p.passes, slots, fuse};
+    e = dl_launch_dependent(gemm_skinny_rows_kernel<NT, TOut, FUSE, TILES, BK>, dim3(p.blocks), dim3(GR_THREADS(TILES)), (size_t)smem, s, tmap, work, early_weights, status);
+    if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "gemm_skinny: %s", cudaGetErrorString(e));
+    return DL_OK;
+}
+
+template <int NT, typename TOut, bool FUSE>
+static int gs_launch_rows(int sms, cudaStream_t s, const __nv_bfloat16* x, int x_stride, const __nv_bfloat16* w, void* out, int out_stride, int M,
+                          int N, int K, int early_weights, int* status, const GsFuse& fuse) {
+    const GsRowsPlan p = gs_rows_plan(N, FUSE, sms);
+#define GR_OF(TILES, BK) gs_launch_rows_of<NT, TOut, FUSE, TILES, BK>(p, s, x, x_stride, w, out, out_stride, M, N, K, early_weights, status, fuse)
+    const int tiles = (p.rows + (FUSE ? 7 : 15)) / (FUSE ? 8 : 16);
+    if (tiles == 1) return GR_OF(1, 256);
+    if (FUSE || tiles == 2) return GR_OF(2, 128);
+    if constexpr (!FUSE) return GR_OF(3, 128);
+#undef GR_OF
 }
 
 // x: bf16 [M, K] rows x_stride apart, M <= 16.  w: bf16, contiguous rows of K.
@@ -630,8 +936,21 @@ static int gs_run(const void* x, int x_stride, const void* w, void* out, int out
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return dl_fail(DL_ERR_LAUNCH, "gemm_skinny: cannot query the device");
-    const GsPlan p = gs_plan(N, K, fuse_swiglu, sms);
     const int nt = M <= 8 ? 1 : 2;
+    if (gs_by_rows(N, K, fuse_swiglu != 0, sms)) {
+        cudaStream_t s = (cudaStream_t)stream;
+        const __nv_bfloat16 *xb = (const __nv_bfloat16*)x, *wb = (const __nv_bfloat16*)w;
+#define GR_CASE(NTV)                                                                                                                               \
+    if (nt == NTV) {                                                                                                                               \
+        if (fuse_swiglu && out_dtype == DL_F32) return gs_launch_rows<NTV, float, true>(sms, s, xb, x_stride, wb, out, out_stride, M, N, K, early, status, fuse);        \
+        if (fuse_swiglu) return gs_launch_rows<NTV, __nv_bfloat16, true>(sms, s, xb, x_stride, wb, out, out_stride, M, N, K, early, status, fuse); \
+        if (out_dtype == DL_F32) return gs_launch_rows<NTV, float, false>(sms, s, xb, x_stride, wb, out, out_stride, M, N, K, early, status, fuse); \
+        return gs_launch_rows<NTV, __nv_bfloat16, false>(sms, s, xb, x_stride, wb, out, out_stride, M, N, K, early, status, fuse);                 \
+    }
+        GR_CASE(1) GR_CASE(2)
+#undef GR_CASE
+    }
+    const GsPlan p = gs_plan(N, K, fuse_swiglu, sms);
     DL_REQUIRE(partial_floats >= p.blocks * GS_CONSUMERS * 2 * nt * 4 * 32 && n_counters >= p.tiles,
                "gemm_skinny: scratch too small (%d floats, %d counters)", partial_floats, n_counters);
     cudaStream_t s = (cudaStream_t)stream;
@@ -677,7 +996,7 @@ extern "C" int dl_gemm_skinny_gated_bf16(const void* x, int x_stride, const void
 // The same with the fusions of an add + RMSNorm between two products (either, both or neither):
 // gain set (float32 [N]; out must be float32 and the product plain): out is the float32 residual
 //   stream and is added to in place; scaled bf16 [M, N] (rows scaled_stride apart) receives
-//   out * gain, sumsq_out float32 [ceil(N / 16) * 16] the sum of squares per 16-column tile and row.
+//   out * gain, sumsq_out float32 [dl_gemm_skinny_parts(N, K) * 16] the sum of squares per tile and row.
 // sumsq_in set (float32 [n_parts * 16], as a product before this one left it): every output row m
 //   is multiplied by rsqrt(sum_p sumsq_in[p * 16 + m] / n + eps), n = 1 / inv_n the width of x's norm.
 extern "C" int dl_gemm_skinny_fused_bf16(const void* x, int x_stride, const void* w, void* out, int out_dtype,
@@ -787,6 +1106,7 @@ extern "C" int dl_gemm_skinny_static_status(int* code, void* stream) {
 }
 
 DL_PACKED(dl_gemm_skinny_scratch)
+DL_PACKED(dl_gemm_skinny_parts)
 DL_PACKED(dl_gemm_skinny_bf16)
 DL_PACKED(dl_gemm_skinny_gated_bf16)
 DL_PACKED(dl_gemm_skinny_fused_bf16)

@@ -1,14 +1,15 @@
 """Dispatch to the weight-streaming products for steps of a few rows (decode).
 
 Up to ``SKINNY_ROWS`` rows go to the mma.sync kernel of csrc/gemm_skinny.cu (it can take 16), more, up
-to 128, to the tcgen05 kernel of csrc/gemm_decode_tc.cu (``gemm_decode_tc.run``, same contract).  The first cuts its work into
-equal shares per warp; tiles that straddle two shares are summed through a scratch buffer with
-arrival counters.  Both are kept here per device (they are small and every launch leaves the
+to 128, to the tcgen05 kernel of csrc/gemm_decode_tc.cu (``gemm_decode_tc.run``, same contract).  The first gives every multiprocessor
+the same rows of W, or (few sizes) cuts its work into equal shares per warp, where tiles that straddle two shares are summed through a
+scratch buffer with arrival counters.  Both are kept here per device (they are small and every launch leaves the
 counters zero).  Launches that share them must be on one stream.
 """
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 
@@ -21,6 +22,7 @@ _library.register_signatures({
     "dl_gemm_skinny_fused_bf16": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P, _P, _I, _F, _F,
                                   _P, _I, _P, _I, _P, _P],
     "dl_gemm_skinny_gated_bf16": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P, _I, _P, _I, _P, _P],
+    "dl_gemm_skinny_parts": [_I, _I],
     "dl_gemm_skinny_scratch": [_I, _I, _I, _I, _I, _P, _P],
 })
 
@@ -36,7 +38,7 @@ MAX_ROWS = 128           # rows the two kernels take between them; beyond this t
 # gating at the 8B shape and 64 rows).  The plain products do too when TC_PLAIN is set; measured inside a decode
 # step the library's are about 7 us a product faster at those sizes, so they stay with the library.
 TC_PLAIN = False
-SUM_STRIDE = 16          # floats between the sums of squares of two 16-column tiles (mma.sync kernel)
+SUM_STRIDE = 16          # floats between the sums of squares of two tiles (mma.sync kernel)
 _MAX_TILES = 1 << 16
 CONSUMER_WARPS = 8       # of a block (GS_CONSUMERS in csrc/gemm_skinny.cu): each may hand over two cut tiles of 16 rows x 16 tokens
 _state = {}
@@ -51,6 +53,12 @@ def _device_state(device):
         partials = torch.empty(max(sms, 1) * CONSUMER_WARPS * 2 * 2 * 128, dtype=torch.float32, device=device)
         _state[key] = (counters, partials, _library.status_word(device))
     return _state[key]
+
+
+@functools.lru_cache(maxsize=None)
+def _parts(n_out, k):
+    """Parts of the sums of squares that a product of these sizes leaves (its plan: of the sizes and the multiprocessors)."""
+    return _library.library().dl_gemm_skinny_parts(n_out, k)
 
 
 def sum_stride(rows):
@@ -75,7 +83,7 @@ def run(x, w, out_dtype, fuse_swiglu=False, resident=False, row_sums=None, into=
     and every output row is multiplied by rsqrt(sum of the row's parts / width + eps); the sums must come
     from a product of the same number of rows (``sum_stride``).
     ``into`` = (stream float32 [M, N], gain float32 [N]): the product is added into the stream in place;
-    returns (stream * gain as bfloat16 [M, N], sums of squares float32 [ceil(N / 16) * 16]).
+    returns (stream * gain as bfloat16 [M, N], sums of squares float32 [_parts(N, K) * 16]).
     ``sizes``: of x and w, where the caller has them (``product`` in csrc/host/entry.cpp)."""
     M, K, N, x_stride = sizes[:4] if sizes is not None else (*x.shape, w.shape[0], None)
     if M > SKINNY_ROWS:
@@ -95,7 +103,7 @@ def run(x, w, out_dtype, fuse_swiglu=False, resident=False, row_sums=None, into=
     if into is not None:
         stream, gain = into
         scaled = _library.empty(M, n_out, torch.bfloat16, x)
-        sums_out = torch.empty(((n_out + 15) // 16) * 16, dtype=torch.float32, device=x.device)
+        sums_out = torch.empty(_parts(n_out, K) * SUM_STRIDE, dtype=torch.float32, device=x.device)
         out, out_stride, result = stream, stream.stride(0), (scaled, sums_out)
     else:
         gain = scaled = sums_out = None

@@ -515,6 +515,38 @@ def test_gemm_skinny_shares(N, K, gated, monkeypatch):
         assert torch.equal(gemm_skinny.run(x, w, torch.float32, fuse_swiglu=gated), y)
 
 
+@pytest.mark.parametrize("N,K,gated", [(1, 8, False), (148, 136, False), (149, 4096, False), (148 * 16, 384, False), (148 * 16 + 1, 384, False),
+                                       (148 * 32, 520, False), (148 * 33 - 1, 1160, False), (148 * 48, 128, False), (148 * 49, 264, False), (20000, 72, False),
+                                       (8, 1288, True), (148 * 8 + 1, 2048, True), (148 * 17, 136, True), (148 * 48 - 5, 264, True),
+                                       (148 * 16, 4104, False), (2000, 8192, False), (2368, 12280, False), (2368, 12288, False), (2369, 8192, False)])
+@pytest.mark.parametrize("M", [1, 8, 11])
+def test_gemm_skinny_rows(N, K, gated, M, monkeypatch):
+    """A block's rows at the edges of tiles, passes and rings, the last block with fewer, and both sides of the rule that chooses between rows and
+    shares: against float64, with the bits of one row alone, launch after launch, and the sums of squares that an adding product leaves.
+    Bound as in test_gemm_skinny_shares."""
+    from dotllm_b200.kernels import gemm_skinny, library
+    monkeypatch.setattr(gemm_skinny, "SKINNY_ROWS", gemm_skinny.KERNEL_ROWS)
+    g = torch.Generator().manual_seed(N * 5 + K)
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn((2 if gated else 1) * N, K, generator=g) * 0.05).to(torch.bfloat16).to(DEV)
+    y = gemm_skinny.run(x, w, torch.float32, fuse_swiglu=gated)
+    p, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    ref = torch.nn.functional.silu(p[:, :N]) * p[:, N:] if gated else p
+    size = 1.1 * (size[:, :N] * (p[:, N:].abs() + 1e-3) + p[:, :N].abs() * size[:, N:]) if gated else size
+    assert ((y.double() - ref).abs() <= (K / 16 + 16) * 2 ** -24 * size + 1e-12).all()
+    assert torch.equal(gemm_skinny.run(x[:1].contiguous(), w, torch.float32, fuse_swiglu=gated), y[:1])
+    for _ in range(3):
+        assert torch.equal(gemm_skinny.run(x, w, torch.float32, fuse_swiglu=gated), y)
+    if not gated:
+        stream, gain = torch.randn(M, N, generator=g).to(DEV), torch.rand(N, generator=g).to(DEV)
+        want = stream + y
+        scaled, sums = gemm_skinny.run(x, w, torch.float32, into=(stream, gain))
+        assert torch.equal(stream, want) and torch.equal(scaled, (want * gain).to(torch.bfloat16))
+        total = sums.view(-1, gemm_skinny.SUM_STRIDE)[:, :M].double().sum(0)
+        assert ((total - want.double().square().sum(1)).abs() <= 2 ** -20 * total).all()
+    library.check_status()
+
+
 @pytest.mark.parametrize("M,H,K,N2", [(8, 4096, 512, 1024), (1, 1000, 384, 272), (13, 1000, 384, 272), (16, 72, 64, 40),
                                       (17, 1000, 384, 272), (64, 4096, 512, 1024), (100, 1000, 4096, 272), (128, 72, 64, 40)])
 def test_products_that_add_and_normalise(M, H, K, N2, monkeypatch):
