@@ -41,76 +41,20 @@
 // a code in `status` and returns after waiting (bounded) for copies in flight.
 #include "common.cuh"
 #include "gating.cuh"
+#include "stream_rows.cuh"
 #include "tma.cuh"
 #include <atomic>
 #include <mutex>
 #include <type_traits>
 #include <unordered_map>
 
-#ifndef GS_CONSUMERS
-#define GS_CONSUMERS 8
-#endif
 #ifndef GS_SLOTS
 #define GS_SLOTS 3                         // ring stages per consumer warp
 #endif
 #define GS_BK 256                          // k per chunk
-// ... and where rows are shared out evenly (gemm_skinny_rows_kernel)
-#define GR_MOST 48                         // rows of a pass, at most (gated: 16 pairs)
-#define GR_MAX_SLOTS 8                     // ring stages per consumer warp, at most
-#define GR_THREADS(TILES) (32 * (GS_CONSUMERS + 1 + (TILES)))   // consumers, the producer warp, a warp a tile that adds
-#define GR_SMEM 231168                     // bytes of shared memory for the rings and the sums, at most: what a block can have less the barriers
 #define GS_STAGE_ELEMS (16 * GS_BK)         // a stage is the dense box the copy engine writes: [16 rows][256 k]
 #define GS_THREADS (32 * (GS_CONSUMERS + 2))   // consumers, the producer warp, the row-statistics warp
-#define GS_WAIT_CYCLES (1ll << 31)
 #define GS_MAX_ROWS 16
-// Rows of a stage (gated: the up rows lie behind room for all tiles' gate rows), and bytes of a block's rings with what a read of the missing
-// rows of the last tile reaches beyond them.
-__host__ __device__ static inline int GR_stage_rows(int rows, bool gated, int tiles) { return gated ? 8 * tiles + rows : rows; }
-__host__ __device__ static inline int GR_ring_bytes(int rows, int slots, bool gated, int tiles, int bk) {
-    const int stage = GR_stage_rows(rows, gated, tiles);
-    return (GS_CONSUMERS * slots * stage + 16 * tiles - stage) * bk * 2;
-}
-
-__device__ __forceinline__ void gs_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                       uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-__device__ __forceinline__ uint32_t gs_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void gs_mbar_init(uint64_t* bar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gs_smem(bar)), "r"(count));
-}
-__device__ __forceinline__ void gs_mbar_expect(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(gs_smem(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void gs_mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gs_smem(bar)) : "memory");
-}
-__device__ __forceinline__ bool gs_mbar_try(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(gs_smem(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool gs_mbar_wait(uint64_t* bar, uint32_t parity, volatile int* gave_up) {
-    if (gs_mbar_try(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!gs_mbar_try(bar, parity)) {
-        if (*gave_up || clock64() - t0 > GS_WAIT_CYCLES) return false;
-    }
-    return true;
-}
-__device__ __forceinline__ uint4 gs_lds128(uint32_t addr) {     // 16 bytes from a shared-space byte address
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-
 template <typename TOut> __device__ __forceinline__ void gs_store(TOut* p, float v);
 template <> __device__ __forceinline__ void gs_store<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void gs_store<__nv_bfloat16>(__nv_bfloat16* p, float v) {
@@ -573,6 +517,7 @@ template <int NT, typename TOut, bool FUSE_SWIGLU, int TILES, int BK>
 __global__ void __launch_bounds__(GR_THREADS(TILES), 1)
 gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWork w, int early_weights, int* __restrict__ status) {
     constexpr int TILE = FUSE_SWIGLU ? 8 : 16;               // rows (gated: pairs) of a tile
+    constexpr int CHAINS = GR_CHAINS(TILES);                 // accumulators that a chunk's instructions go round: they wait for one another otherwise
     extern __shared__ __align__(128) unsigned char gs_smem_raw[];
     __shared__ uint64_t full_bar[GS_CONSUMERS][GR_MAX_SLOTS], empty_bar[GS_CONSUMERS][GR_MAX_SLOTS], scale_bar, sums_full[2], sums_empty[2];
     __shared__ volatile int gave_up;
@@ -609,13 +554,13 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
         };
         if (cur < total) gs_rows_x<NT, BK>(xf, w, (cur % w.cpt) * BK, g, t);
         for (int p = 0; p < passes; ++p) {
-            float acc[TILES][NT][4];
+            float acc[TILES][NT][CHAINS][4];
 #pragma unroll
             for (int i = 0; i < TILES; ++i)
 #pragma unroll
                 for (int j = 0; j < NT; ++j)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+                    for (int e = 0; e < 4 * CHAINS; ++e) acc[i][j][e / 4][e % 4] = 0.f;
             for (const int pass_end = (p + 1) * w.cpt; cur < pass_end; cur += GS_CONSUMERS) {
                 if (!dead && !gs_mbar_wait(&full_bar[warp][slot], phase, &gave_up)) gave(3);
                 uint4 xn[BK / 32][NT];                    // the next chunk's rows of x, asked for before this one's arithmetic
@@ -635,8 +580,8 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
                             const uint4 a_hi = gs_lds128(st + (uint32_t)(((FUSE_SWIGLU ? TILE * TILES + TILE * i : TILE * i + 8) * BK + 32 * s) * 2));
 #pragma unroll
                             for (int j = 0; j < NT; ++j) {
-                                gs_mma(acc[i][j], a_lo.x, a_hi.x, a_lo.y, a_hi.y, xf[s][j].x, xf[s][j].y);
-                                gs_mma(acc[i][j], a_lo.z, a_hi.z, a_lo.w, a_hi.w, xf[s][j].z, xf[s][j].w);
+                                gs_mma(acc[i][j][2 * s % CHAINS], a_lo.x, a_hi.x, a_lo.y, a_hi.y, xf[s][j].x, xf[s][j].y);
+                                gs_mma(acc[i][j][(2 * s + 1) % CHAINS], a_lo.z, a_hi.z, a_lo.w, a_hi.w, xf[s][j].z, xf[s][j].w);
                             }
                         }
                     }
@@ -644,7 +589,10 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
 #pragma unroll
                     for (int i = 0; i < TILES; ++i)
 #pragma unroll
-                        for (int j = 0; j < NT; ++j) asm volatile("" : "+f"(acc[i][j][0]), "+f"(acc[i][j][1]), "+f"(acc[i][j][2]), "+f"(acc[i][j][3]));
+                        for (int j = 0; j < NT; ++j)
+#pragma unroll
+                            for (int c = 0; c < CHAINS; ++c)
+                                asm volatile("" : "+f"(acc[i][j][c][0]), "+f"(acc[i][j][c][1]), "+f"(acc[i][j][c][2]), "+f"(acc[i][j][c][3]));
                     __threadfence_block();
                     __syncwarp();
                     if (lane == 0) gs_mbar_arrive(&empty_bar[warp][slot]);
@@ -662,7 +610,14 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
 #pragma unroll
                 for (int i = 0; i < TILES; ++i)
 #pragma unroll
-                    for (int j = 0; j < NT; ++j) mine[(i * NT + j) * 32] = make_float4(acc[i][j][0], acc[i][j][1], acc[i][j][2], acc[i][j][3]);
+                    for (int j = 0; j < NT; ++j) {
+                        float (&a)[4] = acc[i][j][0];
+#pragma unroll
+                        for (int c = 1; c < CHAINS; ++c)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) a[e] += acc[i][j][c][e];
+                        mine[(i * NT + j) * 32] = make_float4(a[0], a[1], a[2], a[3]);
+                    }
             }
             __threadfence_block();
             __syncwarp();
@@ -762,20 +717,6 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
     __syncthreads();                                         // nobody leaves while copies may still land
 }
 
-// How rows are shared out: rows of a block, passes of a block, rows of a pass, blocks.  By N and the device alone, so that the parts of a row's
-// sum of squares lie the same for every product of that width.
-struct GsRowsPlan {
-    int block_rows, passes, rows, blocks;
-};
-static GsRowsPlan gs_rows_plan(int N, bool gated, int sms) {
-    const int most = gated ? 16 : GR_MOST;
-    GsRowsPlan p;
-    p.block_rows = (N + sms - 1) / sms;
-    p.passes = (p.block_rows + most - 1) / most;
-    p.rows = (p.block_rows + p.passes - 1) / p.passes;
-    p.blocks = (N + p.block_rows - 1) / p.block_rows;
-    return p;
-}
 // Which products go that way; the others by shares.  With one tile of rows a block, x is half as many bytes as W, and by shares it is asked for
 // further ahead; below 4,096 what passes between blocks costs more than that, at 16,384 the rows' distance of a power of two slows the shares down
 // (both sides measured at the top of this file).

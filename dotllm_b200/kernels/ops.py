@@ -7,6 +7,7 @@ CPU path.  Parts call these functions through the module (``ops.add_rmsnorm(...)
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 
@@ -45,6 +46,9 @@ _library.register_signatures({
     "dl_chunk_pieces": [_I, _I],
     "dl_expert_gate_up": [_P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P],
     "dl_expert_down": [_P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _I, _P, _I, _I, _P],
+    "dl_expert_gate_up_rows": [_P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P],
+    "dl_expert_down_rows_takes": [_I, _I],
+    "dl_expert_down_rows": [_P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _P, _I, _P, _I, _I, _P, _P],
     "dl_expert_sort": [_P, _I, _I, _P, _P, _I, _P],
     "dl_expert_gather": [_P, _I, _P, _P, _I, _I, _I, _P, _P],
     "dl_expert_combine": [_P, _I, _P, _P, _P, _I, _P, _I, _I, _I, _P, _I, _P, _P, _I, _I, _I, _P],
@@ -1209,6 +1213,34 @@ def _addend(addend, addend_gate, T, N, what):
     return astride, gstride
 
 
+# Tokens up to which the chosen experts' matrices are read once each (csrc/experts_rows.cu), and the megabytes of an expert's matrices from which
+# that pays with up to eight tokens and with more: an expert costs it about 2.5 (3.6) us however small it is.  Measured, once each / row by row /
+# as tiles, us: 16 experts of 25 MB, two a token, 8 tokens 53 / 84 / -, 16 tokens 70 / 149 / 130; 32 of 50 MB, four, 8 tokens 180 / 335 / 309,
+# 16 tokens 212 / 561 / 333; 64 of 17 MB, six, 8 tokens 120 / 203 / 201, 16 tokens 230 / 350 / 275; 128 of 9 MB, eight, 1 token 31 / 57 / -, 8 tokens
+# 140 / 150 / 184, 16 tokens 320 / 257 / 268; 32 of 9 MB, four, 8 tokens 65 / 79 / 110, 16 tokens 115 / 136 / 115; 16 of 3 MB, two, 8 tokens 33 / 18 / -.
+EXPERT_ROWS_TOKENS = 16
+EXPERT_ROWS_MB = (8.0, 16.0)
+
+
+def _expert_rows_take(x, x_stride, ids, w, k, mb):
+    T, top = ids.shape
+    return (T <= EXPERT_ROWS_TOKENS and mb >= EXPERT_ROWS_MB[T > 8] and T * top <= 128 and w.shape[0] <= 512 and x.dtype == torch.bfloat16 and x.is_cuda and k % 8 == 0
+            and x_stride % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+@functools.lru_cache(maxsize=None)
+def _down_rows_take(rows, n):
+    return bool(_library.library().dl_expert_down_rows_takes(rows, n))
+
+
+def experts_by_rows(x, ids, w_gate_up, w_down, kind, row_scale=None):
+    """Do ``expert_gate_up`` and ``expert_down`` read every chosen expert's matrices once for this step?  Then nothing else is faster."""
+    return (row_scale is None and kind not in UNGATED and x.stride(1) == 1 and x.shape[1] <= 12288
+            and _expert_rows_take(x, x.stride(0) if x.shape[0] > 1 else x.shape[1], ids, w_gate_up, x.shape[1], 6e-6 * w_down.shape[2] * x.shape[1])
+            and w_down.data_ptr() % 16 == 0 and w_down.shape[2] % 8 == 0 and ids.shape[1] * (-(-w_down.shape[2] // 256) * 256) <= 24576
+            and _down_rows_take(ids.numel(), w_down.shape[1]))
+
+
 def expert_gate_up(x, ids, w_gate_up, kind, limit=0.0, alpha=1.0, row_scale=None):
     """Row (t, j) = act(G_e x_t, U_e x_t) for e = ids[t, j].  x [T, K]; w_gate_up [E, 2*ff, K] (an expert's gate
     rows, then its up rows); returns [T*top, ff] in x's dtype.  For an activation of one product (``UNGATED``) the
@@ -1225,6 +1257,10 @@ def expert_gate_up(x, ids, w_gate_up, kind, limit=0.0, alpha=1.0, row_scale=None
     ff = rows_w // halves
     T, top = ids.shape
     out = _library.empty(T * top, ff, x.dtype, x)
+    if row_scale is None and halves == 2 and _expert_rows_take(x, xs, ids, w_gate_up, K, 6e-6 * ff * K) and K <= 12288:
+        _library.call("dl_expert_gate_up_rows", x, xs, ids, w_gate_up, out, T, top, K, ff, E, GATINGS[kind], float(limit), float(alpha),
+                      _library.status_word(x.device), _stream())
+        return out
     _library.call("dl_expert_gate_up", x, xs, ids, w_gate_up, out, _code(x.dtype), T, top, K,
                   ff, E, GATINGS[kind], float(limit), float(alpha), _ptr(_row_scale(row_scale, ids, "expert_gate_up")), _stream())
     return out
@@ -1257,6 +1293,10 @@ def expert_down(h, ids, weights, w_down, addend=None, addend_gate=None, identity
     astride, gstride = _addend(addend, addend_gate, T, N, "expert_down")
     irows, istride, icount = _identity(identity, T, N, h.dtype, "expert_down")
     out = _library.empty(T, N, torch.float32, h)
+    if _expert_rows_take(h, ff, ids, w_down, ff, 6e-6 * ff * N) and top * (-(-ff // 256) * 256) <= 24576 and _down_rows_take(T * top, N):
+        _library.call("dl_expert_down_rows", h, ids, weights, w_down, addend, astride, out, T, top, ff, N, E, addend_gate, gstride, irows,
+                      istride, icount, _library.status_word(h.device), _stream())
+        return out
     _library.call("dl_expert_down", h, ids, weights, w_down, addend, astride, out,
                   _code(h.dtype), T, top, ff, N, E, addend_gate, gstride, irows, istride, icount, _stream())
     return out

@@ -83,3 +83,68 @@ def test_scaled_rows_keep_their_digits(tokens):
     x, w_in, w_out, ids, weights = step(tokens, 2, 4, 2048, 1536)
     assert ops.experts_as_tiles(x, ids, w_in, w_out)
     assert ops.experts_as_tiles(x, ids, w_in, w_out, row_scale=weights) == (2 * tokens >= 128)
+
+
+@pytest.mark.parametrize("tokens,top,E,K,ff,N", [(1, 1, 1, 8, 8, 8), (1, 4, 40, 264, 24, 136), (5, 3, 7, 520, 148 * 8 + 8, 160), (8, 2, 16, 2048, 512, 2048),
+                                                 (8, 16, 20, 136, 40, 296), (9, 4, 33, 1024, 2376, 264), (16, 8, 300, 256, 72, 2376), (16, 1, 3, 392, 4744, 7120),
+                                                 (12, 2, 5, 128, 264, 4744)])
+def test_chosen_experts_read_once(tokens, top, E, K, ff, N, monkeypatch):
+    """The kernels that read each chosen expert once, against float64: edges of a block's rows, tiles and passes, more rows of one expert than an instruction
+    has columns (a token may name an expert twice), ids without matrices, identity experts, no weights; and a token's bits do not depend on
+    the others.  Bounds: float32 sums of K products of bfloat16 (K / 16 additions deep), h rounded to bfloat16 once."""
+    from dotllm_b200.kernels import library, ops
+    monkeypatch.setattr(ops, "EXPERT_ROWS_MB", (0.0, 0.0))
+    g = torch.Generator().manual_seed(tokens * 31 + K)
+    make = lambda *s, scale=1.0: (torch.randn(*s, generator=g) * scale).to(torch.bfloat16).to(DEV)
+    x, w_in, w_out, other = make(tokens, K), make(E, 2 * ff, K, scale=0.06), make(E, N, ff, scale=0.09), make(tokens, N)
+    ids = torch.randint(0, E + 2, (tokens, top), generator=g).to(torch.int32)
+    if tokens > 4:
+        ids[:, 0] = 0                                        # one expert for every token
+        ids[2, -1] = -1
+    ids = ids.to(DEV)
+    weights, addend, gate = torch.rand(tokens, top, generator=g).to(DEV), torch.randn(tokens, N, generator=g).to(DEV), torch.randn(tokens, 3, generator=g).to(DEV)
+    assert ops.experts_by_rows(x, ids, w_in, w_out, "silu")
+    h = ops.expert_gate_up(x, ids, w_in, "clamped_sigmoid", 1.5, 1.702)
+    flat = ids.flatten().tolist()
+    for r, e in enumerate(flat):
+        if not 0 <= e < E:
+            assert (h[r] == 0).all()
+            continue
+        z = w_in[e].double() @ x[r // top].double()
+        size = (K / 16 + 16) * 2.0 ** -24 * (w_in[e].double().abs() @ x[r // top].double().abs())
+        a, b = z[:ff].clamp(max=1.5), z[ff:].clamp(-1.5, 1.5)
+        want = a * torch.sigmoid(1.702 * a) * (b + 1)
+        # |d/da a sigmoid(1.702 a)| <= 1.1, |b + 1| <= 2.5, |a sigmoid| <= 1.5
+        assert ((h[r].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.75 * size[:ff] + 1.5 * size[ff:] + 1e-6).all()
+    for kw in (dict(weights=weights, addend=addend, addend_gate=gate, identity=(other, 1)), dict(weights=None), dict(weights=weights, addend=addend)):
+        got = ops.expert_down(h, ids, kw.get("weights"), w_out, addend=kw.get("addend"), addend_gate=kw.get("addend_gate"), identity=kw.get("identity"))
+        want, bound = torch.zeros(tokens, N, dtype=torch.float64, device=DEV), torch.zeros(tokens, N, dtype=torch.float64, device=DEV)
+        if "addend" in kw:
+            want += addend.double() * (torch.sigmoid(gate[:, :1].double()) if "addend_gate" in kw else 1.0)
+        for r, e in enumerate(flat):
+            f = weights.flatten()[r].double() if kw["weights"] is not None else 1.0
+            if 0 <= e < E:
+                want[r // top] += f * (w_out[e].double() @ h[r].double())
+                bound[r // top] += f * (w_out[e].double().abs() @ h[r].double().abs())
+            elif e == E and "identity" in kw:
+                want[r // top] += f * other[r // top].double()
+        assert ((got.double() - want).abs() <= (ff / 16 + 16 + top) * 2.0 ** -24 * (bound + want.abs()) + 1e-5 * want.abs() + 1e-6).all()
+        alone = ops.expert_down(h[-top:].contiguous(), ids[-1:].contiguous(), kw["weights"][-1:].contiguous() if kw["weights"] is not None else None, w_out,
+                                addend=addend[-1:].contiguous() if "addend" in kw else None, addend_gate=gate[-1:] if "addend_gate" in kw else None,
+                                identity=(other[-1:], 1) if "identity" in kw else None)
+        assert torch.equal(alone, got[-1:])
+    assert torch.equal(ops.expert_gate_up(x[-1:].contiguous(), ids[-1:].contiguous(), w_in, "clamped_sigmoid", 1.5, 1.702), h[-top:])
+    library.check_status()
+
+
+@pytest.mark.parametrize("tokens,top,E,K,ff,once", [(8, 2, 16, 2048, 2048, True), (16, 2, 16, 2048, 2048, True), (17, 2, 16, 2048, 2048, False), (8, 4, 32, 2048, 768, True),
+                                                    (9, 4, 32, 2048, 768, False), (8, 2, 16, 1024, 512, False), (16, 9, 16, 2048, 2048, False)])
+def test_experts_read_once_where_it_pays(tokens, top, E, K, ff, once):
+    """Experts of some size and steps of few tokens; never an activation of one product, a row scale or unaligned rows."""
+    from dotllm_b200.kernels import ops
+    x, ids = torch.empty(tokens, K, dtype=torch.bfloat16, device=DEV), torch.zeros(tokens, top, dtype=torch.int32, device=DEV)
+    w_in, w_out = (torch.empty(s, dtype=torch.bfloat16, device=DEV) for s in ((E, 2 * ff, K), (E, K, ff)))
+    assert ops.experts_by_rows(x, ids, w_in, w_out, "silu") == once
+    assert not ops.experts_by_rows(x, ids, w_in, w_out, "relu2") and not ops.experts_by_rows(x, ids, w_in, w_out, "silu", row_scale=x)
+    odd = torch.empty(tokens, K + 1, dtype=torch.bfloat16, device=DEV)[:, 1:]
+    assert not ops.experts_by_rows(odd, ids, w_in, w_out, "silu")
