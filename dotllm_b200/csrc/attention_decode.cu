@@ -9,7 +9,8 @@
 //
 // Shape: persistent, warp-specialised, stream-K.  The step's work is the list of all visible cache
 // pages ordered by (sequence, KV head, page); it is cut into equal contiguous shares, one per block
-// (one block per multiprocessor), whatever the lengths of the sequences are - the kernel computes
+// (one block per multiprocessor), whatever the lengths of the sequences are, or, where that is hardly less even, into
+// segments that do not cross a pair (AdCut below) - the kernel computes
 // the cut itself from the lengths on the device, so a captured launch serves any lengths.  A share
 // is a few segments, each a run of pages of one (sequence, KV head).  A cache page of one KV head
 // is two contiguous pieces (K [64][hd], V [hd][64]); one producer thread copies them with
@@ -141,28 +142,70 @@ __device__ __forceinline__ int ad_pages_of(int len, AdWin win) {
 
 // The work of a step is the list of all visible pages, ordered by (sequence, KV head, page), cut into
 // equal contiguous shares, one per block.  AdCut is that cut, computed by every warp for itself.
+//
+// A share may hold the end of one pair's pages and the beginning of the next one's: two segments, each with its queries, its merge
+// of the block's warps and its part of the output (about 3.4 us more than one segment of as many pages; a block's 11 pages of
+// 8 sequences of 1,100 to 2,000 tokens and heads of 64 take 4).  Where the pairs are no more than the blocks, a pair's pages are cut into
+// segments of at most `len` instead, a block each, as long as the longest is at most `slack` pages longer than a share would be; and not cut at
+// all if the longest pair is at most `slack` pages longer than that (parts that pass between blocks cost 3 us as well).  128 KB of
+// pages stream to a multiprocessor in that time.  An attention layer (three launches, in a graph): 8 sequences of 1,100 to 2,000 tokens, 32 heads of 64,
+// 24.4 -> 23.2 us; 8 of 280 to 500, heads of 128, 31.8 -> 29.2; 18 of 360 to 700 47.0 -> 39.6; a decode step of 16 such layers (the first) 855 -> 840.
 struct AdCut {
     int total, share;        // pages in the step, pages per block
+    int len;                 // 0: shares; else pages of a pair's segment, at most
 };
+#define AD_SLACK_BYTES (128 * 1024)
 
-__device__ __forceinline__ AdCut ad_cut(const int32_t* seq_len, int n_seqs, int nkv, AdWin window, int n_blocks, int min_share, int lane) {
-    int sum = 0;
-    for (int b0 = 0; b0 < n_seqs; b0 += 32)
-        if (b0 + lane < n_seqs) sum += ad_pages_of(seq_len[b0 + lane], window);
+__device__ __forceinline__ AdCut ad_cut(const int32_t* seq_len, int n_seqs, int nkv, AdWin window, int n_blocks, int min_share, int slack, int lane) {
+    int sum = 0, longest = 0, mine = 0;
+    bool beyond = false;                                     // sequences with pages beyond the first 32
+    for (int b0 = 0; b0 < n_seqs; b0 += 32) {
+        const int pages = b0 + lane < n_seqs ? ad_pages_of(seq_len[b0 + lane], window) : 0;
+        if (b0 == 0) mine = pages;
+        else beyond = beyond || pages > 0;
+        sum += pages, longest = max(longest, pages);
+    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    for (int o = 16; o > 0; o >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+    }
     AdCut c;
     c.total = sum * nkv;
     c.share = max(min_share, (c.total + n_blocks - 1) / n_blocks);
+    c.len = 0;
+    // Only what the lengths say decides, so that rows without pages (a captured step wider than its batch) change nothing.  Long shares are left
+    // alone: the search takes 0.3 us, and what it saves is little of theirs.
+    const int live = 32 - __clz(__ballot_sync(0xffffffffu, mine > 0));
+    if (c.share <= 3 * slack && live * nkv <= n_blocks && !__any_sync(0xffffffffu, beyond)) {
+        // lane j tries segments of share + j pages; slack < 32
+        const int try_len = c.share + lane;
+        const float per_page = 1.0f / (float)try_len;
+        int segments = 0;
+#pragma unroll 1
+        for (int b = 0; b < live; ++b) {                     // ceil(pages / try_len); the quotient in float32 is at most one off
+            const int pages = __shfl_sync(0xffffffffu, mine, b);
+            int n = (int)((float)pages * per_page);
+            n += n * try_len < pages ? 1 : 0;
+            n += n * try_len < pages ? 1 : 0;
+            n -= (n - 1) * try_len >= pages ? 1 : 0;
+            segments += n;
+        }
+        const unsigned fits = __ballot_sync(0xffffffffu, segments * nkv <= n_blocks && lane <= slack);
+        const int shortest = fits != 0 ? c.share + __ffs(fits) - 1 : c.share;
+        c.len = longest <= shortest + slack ? longest : fits != 0 ? shortest : 0;      // (longest 0: no pages at all)
+    }
     return c;
 }
+// Blocks' units that a pair's pages make: pages of a share, or segments.
+__device__ __forceinline__ int ad_units(int pages, int len) { return len > 0 ? (pages + len - 1) / len : pages; }
 
-// The sequence that holds page r of the list (r < total), and the pages of the list before it.
-__device__ __forceinline__ void ad_locate(const int32_t* seq_len, int n_seqs, int nkv, AdWin window, int r, int lane,
+// The sequence that holds unit r of the list (r < total), and the units of the list before it.
+__device__ __forceinline__ void ad_locate(const int32_t* seq_len, int n_seqs, int nkv, AdWin window, int len, int r, int lane,
                                           int* b_out, int* before_out) {
     int before = 0, b = n_seqs, b_before = 0;
     for (int b0 = 0; b0 < n_seqs; b0 += 32) {
-        const int np = (b0 + lane < n_seqs) ? ad_pages_of(seq_len[b0 + lane], window) * nkv : 0;
+        const int np = (b0 + lane < n_seqs) ? ad_units(ad_pages_of(seq_len[b0 + lane], window), len) * nkv : 0;
         int incl = np;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -188,6 +231,7 @@ struct AdWalk {
     int b, kvh, pg;          // where r lies: sequence, KV head, page among the sequence's visible pages
     int len, np;             // of sequence b: keys, visible pages
     bool first;              // the next segment is the block's first
+    int i0, n_seg;           // segments of a pair (AdCut::len): the block of its first, how many
 };
 struct AdSeg {
     int b, kvh, len, first_key, n_pages, slot;
@@ -199,23 +243,29 @@ struct AdSeg {
 __device__ __forceinline__ AdWalk ad_walk_begin(const AdCut& c, const int32_t* seq_len, int n_seqs, int nkv, AdWin window,
                                                 int block, int lane) {
     AdWalk w;
-    w.r = min(c.total, block * c.share);
-    w.r_end = min(c.total, w.r + c.share);
+    w.r = c.len > 0 ? block : min(c.total, block * c.share);
+    w.r_end = c.len > 0 ? block + 1 : min(c.total, w.r + c.share);
     w.first = true;
     w.b = n_seqs;
-    w.kvh = w.pg = w.len = w.np = 0;
+    w.kvh = w.pg = w.len = w.np = w.i0 = w.n_seg = 0;
     if (w.r < w.r_end) {
         int before;
-        ad_locate(seq_len, n_seqs, nkv, window, w.r, lane, &w.b, &before);
-        if (w.b >= n_seqs) {                                 // cannot happen while r < total
+        ad_locate(seq_len, n_seqs, nkv, window, c.len, w.r, lane, &w.b, &before);
+        if (w.b >= n_seqs) {                                 // (there are fewer segments than blocks)
             w.r = w.r_end;
             return w;
         }
         w.len = seq_len[w.b];
         w.np = ad_pages_of(w.len, window);
-        const int off = w.r - before;
-        w.kvh = off / w.np;
-        w.pg = off - w.kvh * w.np;
+        const int off = w.r - before, units = ad_units(w.np, c.len);
+        w.kvh = off / units;
+        w.pg = off - w.kvh * units;
+        if (c.len > 0) {                                     // w.pg is the segment's number so far
+            w.n_seg = units, w.i0 = block - w.pg;
+            w.r_end = (w.pg + 1) * w.np / units;
+            w.pg = w.pg * w.np / units;
+            w.r = w.pg;
+        }
     }
     return w;
 }
@@ -418,7 +468,8 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_
     __shared__ uint64_t full_bar[AD_MAX_RING], empty_bar[AD_MAX_RING];
     __shared__ float sm_m[AD_MAX_STAGES][16], sm_l[AD_MAX_STAGES][16];
     __shared__ volatile int gave_up;
-    __shared__ int last_of_pair;
+    __shared__ int last_of_pair[2];
+    __shared__ int cut_pair[2][5];       // per slot: the pair (sequence, -1: none; KV head), the block of its first segment, how many, the first one's slot
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -448,6 +499,9 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_
     }
     __syncthreads();
     dl_launch_dependents();
+    // Every warp for itself, from one copy of the code: it is cold at the start of a launch.
+    const AdCut cut = ad_cut(seq_len, n_seqs, nkv, window, gridDim.x, min_share, AD_SLACK_BYTES / (2 * (int)PAGE_BYTES), lane);
+    AdWalk walk = ad_walk_begin(cut, seq_len, n_seqs, nkv, window, blockIdx.x, lane);
 
     if (warp == AD_MAX_STAGES) {
         // ------------------------------------------------------------ producer
@@ -461,8 +515,6 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_
         int n = 0;                                           // pages issued so far, over all runs
         bool stop = false, waited = false;
         const uint64_t policy = ad_stream_policy();
-        const AdCut cut = ad_cut(seq_len, n_seqs, nkv, window, gridDim.x, min_share, lane);
-        AdWalk walk = ad_walk_begin(cut, seq_len, n_seqs, nkv, window, blockIdx.x, lane);
         AdSeg w;
         while (!stop && ad_walk_next(walk, w, seq_len, n_seqs, nkv, window)) {
             const int32_t* pages = block_table + (size_t)w.b * bt_stride;
@@ -515,22 +567,26 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_
         const float to_log2 = capped ? 1.f : scale * 1.4426950408889634f;   // scores in units of log2 (capped ones come in them)
         const float scale2 = sloped ? 1.f : to_log2;                        // ... and so do those that took a distance penalty
         int n0 = 0;                                          // pages of the runs before this one
-        const AdCut cut = ad_cut(seq_len, n_seqs, nkv, window, gridDim.x, min_share, lane);
-        AdWalk walk = ad_walk_begin(cut, seq_len, n_seqs, nkv, window, blockIdx.x, lane);
         AdSeg w;
-        dl_grid_dependency_wait();       // q comes from the kernel before this one; out and the scratch may be in use by it
-        while (ad_walk_next(walk, w, seq_len, n_seqs, nkv, window)) {      // the same segments in every warp
-            // Q rows g and g+8 of the group (zero beyond the group)
-            uint4 qf_lo[DC], qf_hi[DC];
-            {
-                const __nv_bfloat16* qb = q + (size_t)w.b * q_stride + (size_t)w.kvh * group * HD;
+        bool more = ad_walk_next(walk, w, seq_len, n_seqs, nkv, window);          // the same segments in every warp
+        uint4 qf_lo[DC], qf_hi[DC];                          // Q rows g and g+8 of the group (zero beyond the group)
+        auto load_q = [&](const AdSeg& seg) {
+            const __nv_bfloat16* qb = q + (size_t)seg.b * q_stride + (size_t)seg.kvh * group * HD;
 #pragma unroll
-                for (int c = 0; c < DC; ++c) {
-                    qf_lo[c] = make_uint4(0u, 0u, 0u, 0u);
-                    qf_hi[c] = make_uint4(0u, 0u, 0u, 0u);
-                    if (g < group) qf_lo[c] = *reinterpret_cast<const uint4*>(qb + (size_t)g * HD + c * 32 + t * 8);
-                    if (WIDE && g + 8 < group) qf_hi[c] = *reinterpret_cast<const uint4*>(qb + (size_t)(g + 8) * HD + c * 32 + t * 8);
-                }
+            for (int c = 0; c < DC; ++c) {
+                qf_lo[c] = make_uint4(0u, 0u, 0u, 0u);
+                qf_hi[c] = make_uint4(0u, 0u, 0u, 0u);
+                if (g < group) qf_lo[c] = *reinterpret_cast<const uint4*>(qb + (size_t)g * HD + c * 32 + t * 8);
+                if (WIDE && g + 8 < group) qf_hi[c] = *reinterpret_cast<const uint4*>(qb + (size_t)(g + 8) * HD + c * 32 + t * 8);
+            }
+        };
+        // A block cuts at most two pairs, the first's segment in slot 0 and the last's in slot 1 (pairs between them are whole).  Both are
+        // counted in behind the last segment: an atomic between segments would have every warp wait for it.
+        if (threadIdx.x == 0) cut_pair[0][0] = cut_pair[1][0] = -1, cut_pair[0][2] = walk.i0, cut_pair[0][3] = walk.n_seg;
+        dl_grid_dependency_wait();       // q comes from the kernel before this one; out and the scratch may be in use by it
+        if (more) load_q(w);
+        while (more) {
+            {
                 // the biases of rows g and g+8 (read only where the row exists)
                 const float* qbias_lo = (fresh.q_bias != nullptr && g < group) ? fresh.q_bias + (size_t)(w.kvh * group + g) * HD : nullptr;
                 const float* qbias_hi = (WIDE && fresh.q_bias != nullptr && g + 8 < group) ? fresh.q_bias + (size_t)(w.kvh * group + g + 8) * HD : nullptr;
@@ -839,6 +895,9 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_
                 if (lane == 0) ad_mbar_arrive(&empty_bar[s]);
             }
             n0 += w.n_pages;
+            AdSeg next;                                      // its queries are on their way while this segment is merged
+            more = ad_walk_next(walk, next, seq_len, n_seqs, nkv, window);
+            if (more) load_q(next);
 
             // ---- merge the block's warps (fixed order) and hand the run's result on
             l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
@@ -904,29 +963,41 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_
                     }
                 }
             }
-            ad_consumer_sync(n_stages);                              // the merge buffers are free for the next run
-            if (!w.whole) {
-                // The pair's pages are spread over the blocks i0 .. i1 of the cut.  Each of them counts itself
-                // in once its segment is written (one acquire-release atomic: the consumer warps' stores
-                // are ordered before it by the barrier above); whichever arrives last merges the
-                // segments in block order - the same bits whatever the order of arrival.
-                const int i0 = w.pair_begin / cut.share, i1 = (w.pair_begin + w.pair_pages - 1) / cut.share;
-                if (tid == 0) {
-                    int seen;
-                    int* counter = pair_counters + w.b * nkv + w.kvh;
-                    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(seen) : "l"(counter) : "memory");
-                    last_of_pair = (seen == i1 - i0) ? 1 : 0;
-                    if (seen == i1 - i0) *counter = 0;               // ready for the next launch
+            if (tid == 0 && !w.whole) {                      // the pair's pages are spread over the blocks i0 .. i0 + n - 1
+                int* c = cut_pair[w.slot];
+                c[0] = w.b, c[1] = w.kvh, c[4] = 0;
+                if (cut.len == 0) {                      // (else the walk's beginning has left them)
+                    const int i0 = w.pair_begin / cut.share;
+                    c[2] = i0, c[3] = (w.pair_begin + w.pair_pages - 1) / cut.share - i0 + 1, c[4] = w.pair_begin == i0 * cut.share ? 0 : 1;
                 }
-                ad_consumer_sync(n_stages);
-                const bool last = last_of_pair != 0;
-                ad_consumer_sync(n_stages);                          // everyone has read the flag before it is written again
-                if (last)
-                    ad_merge_pair<HD, WIDE ? 4 : 8>(out + (size_t)w.b * out_stride + (size_t)w.kvh * group * HD, group, i0, i1 - i0 + 1,
-                                      (w.pair_begin == i0 * cut.share) ? 0 : 1, part_o, part_ml, tid, 32 * n_stages,
-                                      fresh.gate != nullptr ? fresh.gate + (size_t)w.b * fresh.gate_stride + w.kvh * group : nullptr,
-                                      fresh.sinks != nullptr ? fresh.sinks + w.kvh * group : nullptr);
             }
+            ad_consumer_sync(n_stages);                              // the merge buffers are free for the next run
+            w = next;
+        }
+        // Each of a cut pair's blocks counts itself in once its segment is written (one
+        // acquire-release atomic: the consumer warps' stores are ordered before it by the barrier behind the merge above); whichever
+        // arrives last merges the segments in block order - the same bits whatever the order of arrival.
+        ad_consumer_sync(n_stages);                          // (a block without segments has none to wait for)
+        if (cut_pair[0][0] >= 0 || cut_pair[1][0] >= 0) {
+            const int tid = threadIdx.x;
+            if ((tid == 0 || tid == 32) && cut_pair[tid >> 5][0] >= 0) {
+                const int* c = cut_pair[tid >> 5];
+                int seen;
+                int* counter = pair_counters + c[0] * nkv + c[1];
+                asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(seen) : "l"(counter) : "memory");
+                last_of_pair[tid >> 5] = (seen == c[3] - 1) ? 1 : 0;
+                if (seen == c[3] - 1) *counter = 0;          // ready for the next launch
+            }
+            ad_consumer_sync(n_stages);
+#pragma unroll 1
+            for (int slot = 0; slot < 2; ++slot)
+                if (cut_pair[slot][0] >= 0 && last_of_pair[slot] != 0) {
+                    const int b = cut_pair[slot][0], kvh = cut_pair[slot][1];
+                    ad_merge_pair<HD, WIDE ? 4 : 8>(out + (size_t)b * out_stride + (size_t)kvh * group * HD, group, cut_pair[slot][2], cut_pair[slot][3],
+                                      cut_pair[slot][4], part_o, part_ml, tid, 32 * n_stages,
+                                      fresh.gate != nullptr ? fresh.gate + (size_t)b * fresh.gate_stride + kvh * group : nullptr,
+                                      fresh.sinks != nullptr ? fresh.sinks + kvh * group : nullptr);
+                }
         }
     }
     __syncthreads();                                         // nobody leaves while copies may still land

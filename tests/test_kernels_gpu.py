@@ -865,6 +865,43 @@ def test_attention_decode_with_the_new_token_inside(nh, nkv, hd, rotate, window,
     assert torch.equal(k_one, k_two) and torch.equal(v_one, v_two)
 
 
+@pytest.mark.parametrize("nh,nkv,hd,lengths", [
+    (8, 8, 64, [500, 460, 1, 64, 65, 300]),                                # pairs are not cut
+    (8, 8, 64, [2000, 1880, 1760, 1640, 1500, 1380, 1260, 1140]),          # segments of a pair, a block each
+    (4, 4, 128, [1500, 70, 1300, 1024, 1, 900]),
+    (8, 8, 64, [4500, 4000, 60, 3300, 3000]),                              # shares
+    (2, 2, 32, [2900, 2900, 40]), (24, 2, 64, [1900, 700, 1200]),
+    (3, 3, 64, [64 * (1 + i % 7) for i in range(32)]), (3, 3, 64, [64 * (1 + i % 7) for i in range(33)])])
+@pytest.mark.parametrize("window,blocks", [(0, 0), (700, 0), (0, 40)])
+def test_attention_decode_cuts(nh, nkv, hd, lengths, window, blocks, monkeypatch):
+    """The three ways in which a step's pages are cut, against float32 attention; the same bits on every launch and with rows that hold nothing behind
+    the sequences (a captured step wider than its batch)."""
+    from dotllm_b200.kernels import attention_fast, library
+    monkeypatch.setattr(attention_fast, "DECODE_BLOCKS", blocks)
+    B = len(lengths)
+    k_pool, v_pool, table, dense = make_paged(B, lengths, nkv, hd, torch.bfloat16, seed=25)
+    g = torch.Generator().manual_seed(26)
+    q = torch.randn(B + 9, nh * hd, generator=g).to(torch.bfloat16).to(DEV)
+    scale = 1.0 / math.sqrt(hd)
+    tables = torch.full((B + 9, table.shape[1] + 5), -1, dtype=torch.int32)
+    tables[:B, :table.shape[1]] = table
+    kp, vp = k_pool.to(DEV), v_pool.to(DEV)
+
+    def run(n, width):
+        lens = (lengths + [0] * 9)[:n]
+        plan = _decode_plan(lens)
+        pos = torch.tensor([max(0, v - 1) for v in lens], dtype=torch.int32, device=DEV)
+        plan.seq_start = pos
+        return ops().attention(q[:n], kp, vp, torch.arange(n, dtype=torch.int32, device=DEV), pos, tables[:n, :width].contiguous().to(DEV), nh, nkv, hd, scale,
+                               window, plan=plan)[:B]
+
+    got = run(B, table.shape[1])
+    ref = torch.stack([dense_attention(q[b].cpu(), *dense[b], nh, nkv, scale, lengths[b] - 1, window) for b in range(B)])
+    close(got, ref, 2e-3, 2 ** -7)
+    assert torch.equal(run(B, table.shape[1]), got) and torch.equal(run(B + 9, table.shape[1] + 5), got)
+    library.check_status()
+
+
 @pytest.mark.parametrize("fused", [False, True])
 def test_attention_decode_rows_that_hold_nothing(fused):
     """Rows whose length after the step is 0 (the idle rows of a captured step wider than its batch)
