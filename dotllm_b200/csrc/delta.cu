@@ -148,12 +148,14 @@ delta_prepare_kernel(const T* __restrict__ x, int ld, const T* __restrict__ taps
 
 // The same for prompts that go chunk by chunk, bfloat16 rows, at most four taps and heads of 16, 32 or 64 key channels: a thread
 // takes four neighbouring channels of four tokens in a row, so that its seven 8-byte rows are asked for at once (the kernel above
-// waits for one row after the other: 3,743 tokens of 8,192 channels in 205 us, this one in 105; the bytes alone are 37).  Tiles of
+// waits for one row after the other: 3,743 tokens of 8,192 channels in 205 us, this one in 73; the bytes alone are 37).  What bounds it is the
+// issue of instructions (silu's exponential and division above all): a run inside a sequence looks its place up once (a token at a time and with the
+// history's conditions it took 105 us), the taps come 16 bytes at a time, and values need no norm.  Runs of eight tokens took 85: 77 registers.  Tiles of
 // 256 channels along grid.y, then tiles of 256 decays (the step sizes with them).
 #define DP_VEC_TILE 256
-#define DP_VEC_TOKENS 8                                   // tokens a block: two runs of four
-__device__ __forceinline__ float4 dp_load4(const __nv_bfloat16* p) {
-    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+#define DP_VEC_RUN 4                                      // tokens of a thread
+#define DP_VEC_TOKENS (2 * DP_VEC_RUN)                    // tokens a block: two runs
+__device__ __forceinline__ float4 dp_widen4(const uint2& raw) {
     const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), b = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
     return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
 }
@@ -169,22 +171,22 @@ delta_prepare_vec_kernel(const __nv_bfloat16* __restrict__ x, int ld, const __nv
     dl_launch_dependents();
     dl_grid_dependency_wait();
     const int qk = 2 * G * dim, C = qk + H * vdim;
-    const int t0 = blockIdx.x * DP_VEC_TOKENS + (threadIdx.x >> 6) * 4, sub = (threadIdx.x & 63) * 4;
+    const int t_first = blockIdx.x * DP_VEC_TOKENS + (threadIdx.x >> 6) * DP_VEC_RUN, sub = (threadIdx.x & 63) * 4;
     if ((int)blockIdx.y >= channel_tiles) {                // decays and step sizes
         const int c = ((int)blockIdx.y - channel_tiles) * DP_VEC_TILE + sub, h = c / dim;     // dim is a multiple of 4: one head
         if (c >= H * dim) return;
         const float rate = expf(a_log[h]);
-        float4 zs[4];
         const float4 bias = head_decay ? make_float4(dt_bias[h], dt_bias[h], dt_bias[h], dt_bias[h]) : *reinterpret_cast<const float4*>(dt_bias + c);
+        float4 zs[DP_VEC_RUN];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const long row = min(t0 + i, n_tokens - 1);
+        for (int i = 0; i < DP_VEC_RUN; ++i) {
+            const long row = min(t_first + i, n_tokens - 1);
             if (head_decay) zs[i].x = z[row * z_stride + h];
             else zs[i] = *reinterpret_cast<const float4*>(z + row * z_stride + c);
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int t = t0 + i;
+        for (int i = 0; i < DP_VEC_RUN; ++i) {
+            const int t = t_first + i;
             if (t >= n_tokens) break;
             float4 g;
             g.x = expf(-rate * dr_softplus(zs[i].x + bias.x));
@@ -202,48 +204,82 @@ delta_prepare_vec_kernel(const __nv_bfloat16* __restrict__ x, int ld, const __nv
     const int c = blockIdx.y * DP_VEC_TILE + sub;
     const bool live = c < C;
     const int cc = live ? c : 0;
-    float4 in[7], tap[4];                                  // rows t0 - 3 .. t0 + 3; taps, place 3 - lag meets the input `lag` tokens back
+    float4 tap[4];                                         // place 3 - lag meets the input `lag` tokens back
+    const bool tap_vec = K == 4 && ((uintptr_t)taps % 16) == 0;      // the thread's sixteen taps are 32 aligned bytes
+    uint2 raw[DP_VEC_RUN + 3];                             // rows t_first - 3 ..
 #pragma unroll
-    for (int i = 0; i < 7; ++i) {
-        const int t = t0 - 3 + i;
-        in[i] = dp_load4(x + (long)min(max(t, 0), n_tokens - 1) * ld + cc);
-    }
+    for (int i = 0; i < DP_VEC_RUN + 3; ++i)
+        raw[i] = *reinterpret_cast<const uint2*>(x + (long)min(max(t_first - 3 + i, 0), n_tokens - 1) * ld + cc);
+    if (tap_vec) {
+        const uint4 lo = *reinterpret_cast<const uint4*>(taps + 4l * cc), hi = *reinterpret_cast<const uint4*>(taps + 4l * cc + 8);
+        const float4 c0 = dp_widen4(make_uint2(lo.x, lo.y)), c1 = dp_widen4(make_uint2(lo.z, lo.w)), c2 = dp_widen4(make_uint2(hi.x, hi.y)),
+                     c3 = dp_widen4(make_uint2(hi.z, hi.w));
+        tap[0] = make_float4(c0.x, c1.x, c2.x, c3.x), tap[1] = make_float4(c0.y, c1.y, c2.y, c3.y);
+        tap[2] = make_float4(c0.z, c1.z, c2.z, c3.z), tap[3] = make_float4(c0.w, c1.w, c2.w, c3.w);
+    } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int lag = 3 - i;
-        float e[4];
+        for (int i = 0; i < 4; ++i) {
+            const int lag = 3 - i;
+            float e[4];
 #pragma unroll
-        for (int d = 0; d < 4; ++d) e[d] = lag < K ? __bfloat162float(taps[(long)(cc + d) * K + (K - 1 - lag)]) : 0.f;
-        tap[i] = make_float4(e[0], e[1], e[2], e[3]);
+            for (int d = 0; d < 4; ++d) e[d] = lag < K ? __bfloat162float(taps[(long)(cc + d) * K + (K - 1 - lag)]) : 0.f;
+            tap[i] = make_float4(e[0], e[1], e[2], e[3]);
+        }
     }
     const int lanes = dim / 4;                             // lanes of a head: 4, 8 or 16, aligned (a tile starts at a whole head)
-    const bool is_v = c >= qk;
+    const bool is_v = c >= qk, query = c < G * dim, units = !__all_sync(0xffffffffu, is_v || !live);
+    // The run lies inside a sequence, behind its first K - 1 new tokens (all but a sequence's ends): nothing but the step's own rows is read, and every
+    // token has its place.  One look for the run instead of three dependent loads a token.
+    const int t_last = t_first + DP_VEC_RUN - 1, b_first = token_seq[min(t_first, n_tokens - 1)];
+    const int slot_first = slots[b_first];
+    const bool inner = t_last < n_tokens && token_seq[min(t_last, n_tokens - 1)] == b_first && t_first - cu_new[b_first] >= K - 1 && slot_first >= 0 &&
+                       slot_first < n_slots;
+    float4 in[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int t = t0 + i, row = min(t, n_tokens - 1), b = token_seq[row], slot = slots[b], j = row - cu_new[b];
+    for (int i = 0; i < 3; ++i) in[i + 1] = dp_widen4(raw[i]);
+#pragma unroll
+    for (int i = 0; i < DP_VEC_RUN; ++i) {
+        const int t = t_first + i;
+        in[0] = in[1], in[1] = in[2], in[2] = in[3], in[3] = dp_widen4(raw[i + 3]);
+        bool there = inner;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (inner) {
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {                      // oldest first; a place in front of the taps adds 0 * 0
-            const int lag = 3 - p;
-            float4 v = in[i + p];
-            if (lag >= K) v = make_float4(0.f, 0.f, 0.f, 0.f);
-            else if (lag > j)                              // before the sequence's new tokens: its history, whose row K - 2 is the newest
-                v = slot >= 0 && slot < n_slots ? *reinterpret_cast<const float4*>(hist + (long)slot * slot_stride + (long)(K - 1 - (lag - j)) * C + cc)
-                                                : make_float4(0.f, 0.f, 0.f, 0.f);
-            acc.x = fmaf(tap[p].x, v.x, acc.x);
-            acc.y = fmaf(tap[p].y, v.y, acc.y);
-            acc.z = fmaf(tap[p].z, v.z, acc.z);
-            acc.w = fmaf(tap[p].w, v.w, acc.w);
+            for (int p = 0; p < 4; ++p) {                  // oldest first; a place in front of the taps adds 0 * 0
+                const float4 v = 3 - p >= K ? make_float4(0.f, 0.f, 0.f, 0.f) : in[p];
+                acc.x = fmaf(tap[p].x, v.x, acc.x);
+                acc.y = fmaf(tap[p].y, v.y, acc.y);
+                acc.z = fmaf(tap[p].z, v.z, acc.z);
+                acc.w = fmaf(tap[p].w, v.w, acc.w);
+            }
+        } else {
+            const int row = min(t, n_tokens - 1), b = token_seq[row], slot = slots[b], j = row - cu_new[b];
+            there = t < n_tokens && slot >= 0 && slot < n_slots;
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const int lag = 3 - p;
+                float4 v = in[p];
+                if (lag >= K) v = make_float4(0.f, 0.f, 0.f, 0.f);
+                else if (lag > j)                          // before the sequence's new tokens: its history, whose row K - 2 is the newest
+                    v = slot >= 0 && slot < n_slots ? *reinterpret_cast<const float4*>(hist + (long)slot * slot_stride + (long)(K - 1 - (lag - j)) * C + cc)
+                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+                acc.x = fmaf(tap[p].x, v.x, acc.x);
+                acc.y = fmaf(tap[p].y, v.y, acc.y);
+                acc.z = fmaf(tap[p].z, v.z, acc.z);
+                acc.w = fmaf(tap[p].w, v.w, acc.w);
+            }
         }
-        float4 y = make_float4(dp_silu(acc.x), dp_silu(acc.y), dp_silu(acc.z), dp_silu(acc.w));
-        float ss = (y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w);
-        for (int o = lanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (!live || t >= n_tokens || slot < 0 || slot >= n_slots) continue;
+        const float4 y = make_float4(dp_silu(acc.x), dp_silu(acc.y), dp_silu(acc.z), dp_silu(acc.w));
+        float ss = 0.f;
+        if (units) {                                       // some channel of the warp's is a query's or a key's
+            ss = (y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w);
+            for (int o = lanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        }
+        if (!live || !there) continue;
         if (is_v) {
             *reinterpret_cast<float4*>(vo + (long)t * H * vdim + (c - qk)) = y;
             continue;
         }
-        const bool query = c < G * dim;
         const float r = (1.0f / sqrtf(ss + unit_eps)) * (query ? q_scale : 1.0f);
         float* dst = query ? qo + (long)t * G * dim + c : ko + (long)t * G * dim + (c - G * dim);
         *reinterpret_cast<float4*>(dst) = make_float4(y.x * r, y.y * r, y.z * r, y.w * r);

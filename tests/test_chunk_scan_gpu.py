@@ -271,6 +271,39 @@ def test_preparation_of_prompts(K, dim, head_decay, monkeypatch):
     assert float((gm.cpu() - want_mem).abs().max()) < 3 * TOL * (1 + float(want_mem.abs().max()))
 
 
+def test_preparation_places_and_taps(monkeypatch):
+    """Runs of four tokens that begin at every place of a sequence, one sequence without a slot among them, and taps that are not 16-byte aligned: the
+    same bits as each sequence alone (whose runs begin elsewhere) with aligned taps."""
+    from dotllm_b200.kernels import ops
+    monkeypatch.setattr(ops, "CHUNK_MIN_TOKENS", 2)
+    H, G, dim, vdim, K = 4, 4, 64, 128, 4
+    lens = [5, 6, 7, 9, 70, 3, 12, 33]
+    C, T, n_state = 2 * G * dim + H * vdim, sum(lens), H * dim * vdim
+    taps = g64(C, K, seed=1, scale=0.5).to(torch.bfloat16).to(DEV)
+    odd = torch.empty(C * K + 1, dtype=torch.bfloat16, device=DEV)[1:].view(C, K).copy_(taps)
+    assert taps.data_ptr() % 16 == 0 and odd.data_ptr() % 16 != 0
+    dt_bias, a_log = g64(H * dim, seed=2).float().to(DEV), g64(H, seed=3, scale=0.5).float().to(DEV)
+    x, z = g64(T, C + H, seed=10).to(torch.bfloat16).to(DEV), g64(T, H * dim, seed=20).float().to(DEV)
+    memory = g64(9, n_state + (K - 1) * C, seed=4).float().to(DEV)
+    slots = [4, 1, -1, 5, 0, 2, 8, 7]
+
+    def run(rows, w, lengths, where):
+        m = memory.clone()
+        seq, cu = [i for i, n in enumerate(lengths) for _ in range(n)], [0] + list(np.cumsum(lengths))
+        o = ops.delta_rule(x[rows], w, x[rows][:, C:], z[rows], dt_bias, a_log, i32(seq), i32(cu), i32(where), m, H, G, dim, vdim, dim ** -0.5, 1e-6,
+                           max_new=max(lengths))
+        return o, m
+
+    whole, mem = run(slice(0, T), odd, lens, slots)
+    at = 0
+    for n, slot in zip(lens, slots):
+        if slot >= 0:
+            alone, m = run(slice(at, at + n), taps, [n], [slot])
+            assert torch.equal(whole[at:at + n], alone) and torch.equal(mem[slot], m[slot])
+        at += n
+    assert torch.equal(mem[[3, 6]], memory[[3, 6]])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("vdim,gate", [(128, "silu"), (64, "sigmoid"), (20, "silu")])
 def test_head_norm_of_many_rows(dtype, vdim, gate):
