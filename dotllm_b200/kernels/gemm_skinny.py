@@ -55,9 +55,9 @@ def _device_state(device):
     return _state[key]
 
 
-@functools.lru_cache(maxsize=None)
-def _parts(n_out, k):
-    """Parts of the sums of squares that a product of these sizes leaves (its plan: of the sizes and the multiprocessors)."""
+@functools.lru_cache(maxsize=4096)
+def _parts(n_out, k, sms):
+    """Parts of the sums of squares that a product of these sizes leaves (its plan: of the sizes and ``sms``, the current device's multiprocessors)."""
     return _library.library().dl_gemm_skinny_parts(n_out, k)
 
 
@@ -83,7 +83,7 @@ def run(x, w, out_dtype, fuse_swiglu=False, resident=False, row_sums=None, into=
     and every output row is multiplied by rsqrt(sum of the row's parts / width + eps); the sums must come
     from a product of the same number of rows (``sum_stride``).
     ``into`` = (stream float32 [M, N], gain float32 [N]): the product is added into the stream in place;
-    returns (stream * gain as bfloat16 [M, N], sums of squares float32 [_parts(N, K) * 16]).
+    returns (stream * gain as bfloat16 [M, N], sums of squares float32 [parts * 16]).
     ``sizes``: of x and w, where the caller has them (``product`` in csrc/host/entry.cpp)."""
     M, K, N, x_stride = sizes[:4] if sizes is not None else (*x.shape, w.shape[0], None)
     if M > SKINNY_ROWS:
@@ -103,7 +103,7 @@ def run(x, w, out_dtype, fuse_swiglu=False, resident=False, row_sums=None, into=
     if into is not None:
         stream, gain = into
         scaled = _library.empty(M, n_out, torch.bfloat16, x)
-        sums_out = torch.empty(_parts(n_out, K) * SUM_STRIDE, dtype=torch.float32, device=x.device)
+        sums_out = torch.empty(_parts(n_out, K, _library.sm_count()) * SUM_STRIDE, dtype=torch.float32, device=x.device)
         out, out_stride, result = stream, stream.stride(0), (scaled, sums_out)
     else:
         gain = scaled = sums_out = None

@@ -1228,8 +1228,8 @@ def _expert_rows_take(x, x_stride, ids, w, k, mb):
             and x_stride % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
-@functools.lru_cache(maxsize=None)
-def _down_rows_take(rows, n):
+@functools.lru_cache(maxsize=4096)
+def _down_rows_take(rows, n, sms):
     return bool(_library.library().dl_expert_down_rows_takes(rows, n))
 
 
@@ -1238,7 +1238,7 @@ def experts_by_rows(x, ids, w_gate_up, w_down, kind, row_scale=None):
     return (row_scale is None and kind not in UNGATED and x.stride(1) == 1 and x.shape[1] <= 12288
             and _expert_rows_take(x, x.stride(0) if x.shape[0] > 1 else x.shape[1], ids, w_gate_up, x.shape[1], 6e-6 * w_down.shape[2] * x.shape[1])
             and w_down.data_ptr() % 16 == 0 and w_down.shape[2] % 8 == 0 and ids.shape[1] * (-(-w_down.shape[2] // 256) * 256) <= 24576
-            and _down_rows_take(ids.numel(), w_down.shape[1]))
+            and _down_rows_take(ids.numel(), w_down.shape[1], _library.sm_count()))
 
 
 def expert_gate_up(x, ids, w_gate_up, kind, limit=0.0, alpha=1.0, row_scale=None):
@@ -1293,7 +1293,7 @@ def expert_down(h, ids, weights, w_down, addend=None, addend_gate=None, identity
     astride, gstride = _addend(addend, addend_gate, T, N, "expert_down")
     irows, istride, icount = _identity(identity, T, N, h.dtype, "expert_down")
     out = _library.empty(T, N, torch.float32, h)
-    if _expert_rows_take(h, ff, ids, w_down, ff, 6e-6 * ff * N) and top * (-(-ff // 256) * 256) <= 24576 and _down_rows_take(T * top, N):
+    if _expert_rows_take(h, ff, ids, w_down, ff, 6e-6 * ff * N) and top * (-(-ff // 256) * 256) <= 24576 and _down_rows_take(T * top, N, _library.sm_count()):
         _library.call("dl_expert_down_rows", h, ids, weights, w_down, addend, astride, out, T, top, ff, N, E, addend_gate, gstride, irows,
                       istride, icount, _library.status_word(h.device), _stream())
         return out
