@@ -7,6 +7,10 @@
 // entry (an expert of more has several entries).  Nothing passes between blocks, and k is cut the same way for every
 // entry, so a row's result does not depend on what else is in the step.
 //
+// Sums keep the accuracy of float32 additions (GsTree in stream_rows.cuh): accumulators that live on in the tensor core left the down product's float32 results
+// 1.3e-7 (rows of 1,408 values) to 1.8e-6 (14,336) off, relative to float64, where chains of multiply-adds row by row are 0.8e-7 to 1.3e-7 off; these
+// are 0.8e-7 to 1.0e-7 off (rows of 704 to 1,408 values 1.02 to 1.05 of row by row's, longer ones 0.75 to 1), in the same time.
+//
 // The down product's block keeps its columns of every (token, choice) row in shared memory and at the end sums each token's choices in their order,
 // with weights, identity experts and addend, as the kernel of experts.cu does.
 //
@@ -95,16 +99,15 @@ __device__ __forceinline__ void xr_make_lists(XrLists& l, const XrWork& w) {
     __syncthreads();
 }
 
-template <int NT, int BK>
-__device__ __forceinline__ void xr_load_x(uint4 (&xf)[BK / 32][NT], const __nv_bfloat16* const (&rows)[NT], int K, int k0, int t) {
+// A lane's values of an instruction's columns, 32 k from k0 on.
+template <int NT>
+__device__ __forceinline__ void xr_load_x(uint4 (&xf)[NT], const __nv_bfloat16* const (&rows)[NT], int K, int k0, int t) {
 #pragma unroll
-    for (int s = 0; s < BK / 32; ++s)
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-            const int k = k0 + 32 * s + 8 * t;
-            xf[s][j] = make_uint4(0u, 0u, 0u, 0u);
-            if (rows[j] != nullptr && k < K) xf[s][j] = __ldg(reinterpret_cast<const uint4*>(rows[j] + k));
-        }
+    for (int j = 0; j < NT; ++j) {
+        const int k = k0 + 8 * t;
+        xf[j] = make_uint4(0u, 0u, 0u, 0u);
+        if (rows[j] != nullptr && k < K) xf[j] = __ldg(reinterpret_cast<const uint4*>(rows[j] + k));
+    }
 }
 
 // tmap: the experts' stacked matrices [E * expert_rows, K], boxes of pass_rows x BK.
@@ -112,7 +115,9 @@ template <int NT, bool DOWN, int TILES, int BK>
 __global__ void __launch_bounds__(GR_THREADS(TILES), 1)
 expert_rows_kernel(const __grid_constant__ CUtensorMap tmap, const XrWork w, int* __restrict__ status) {
     constexpr int TILE = DOWN ? 16 : 8;                      // rows (pairs) of a tile
-    constexpr int CHAINS = GR_CHAINS(TILES);                 // accumulators that a chunk's instructions go round: they wait for one another otherwise
+    // The next chunk's values of x are asked for before this one's arithmetic, into registers of their own; where that would spill (two groups of
+    // columns and chunks of 256), behind every step into the registers that it has left, which asks a little later (5 to 10 % slower where both fit).
+    constexpr bool IN_PLACE = NT == 2 && BK == 256;
     extern __shared__ __align__(128) unsigned char xr_smem[];
     __shared__ uint64_t full_bar[GS_CONSUMERS][GR_MAX_SLOTS], empty_bar[GS_CONSUMERS][GR_MAX_SLOTS], sums_full[2], sums_empty[2];
     __shared__ volatile int gave_up;
@@ -160,39 +165,42 @@ expert_rows_kernel(const __grid_constant__ CUtensorMap tmap, const XrWork w, int
             dead = true;
         };
         rows_of(0);
-        if (warp < chunks) xr_load_x<NT, BK>(xf, xr, w.K, (warp % w.cpt) * BK, t);
+#pragma unroll
+        for (int s = 0; s < BK / 32; ++s) xr_load_x<NT>(xf[s], xr, warp < chunks ? w.K : 0, (warp % w.cpt) * BK + 32 * s, t);
         const int tiles = (w.pass_rows + TILE - 1) / TILE;
         for (int d = 0, q = 0; d < entries; ++d) {
             int cur = warp;
             for (int p = 0; p < passes; ++p, ++q) {
-                float acc[TILES][NT][CHAINS][4];
+                float acc[TILES][NT][4];
 #pragma unroll
                 for (int i = 0; i < TILES; ++i)
 #pragma unroll
                     for (int j = 0; j < NT; ++j)
 #pragma unroll
-                        for (int e = 0; e < 4 * CHAINS; ++e) acc[i][j][e / 4][e % 4] = 0.f;
+                        for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
                 for (const int pass_end = (p + 1) * w.cpt; cur < pass_end; cur += GS_CONSUMERS) {
                     if (!dead && !gs_mbar_wait(&full_bar[warp][slot], phase, &gave_up)) gave(3);
-                    uint4 xn[BK / 32][NT];                   // the next chunk's rows of x, asked for before this one's arithmetic
                     int next = cur + GS_CONSUMERS;
                     if (next >= chunks) rows_of(d + 1), next = warp;
-                    xr_load_x<NT, BK>(xn, xr, w.K, (next % w.cpt) * BK, t);
+                    next = (next % w.cpt) * BK;
+                    uint4 xn[IN_PLACE ? 1 : BK / 32][NT];
+                    if (!IN_PLACE)
+#pragma unroll
+                        for (int s = 0; s < BK / 32; ++s) xr_load_x<NT>(xn[IN_PLACE ? 0 : s], xr, w.K, next + 32 * s, t);
                     if (!dead) {
                         // rows beyond the box are whatever lies behind it: they reach results that are not stored
                         const uint32_t st = gs_smem(xr_smem + (size_t)(warp * w.slots + slot) * stage_bytes) + (uint32_t)(g * BK + 8 * t) * 2u;
 #pragma unroll
-                        for (int s = 0; s < BK / 32; ++s) {
+                        for (int i = 0; i < TILES; ++i) {
+                            if (i >= tiles) break;
+                            GsTree<BK / 32> tree[NT];
 #pragma unroll
-                            for (int i = 0; i < TILES; ++i) {
-                                if (i >= tiles) break;
+                            for (int s = 0; s < BK / 32; ++s) {
                                 const uint4 a_lo = gs_lds128(st + (uint32_t)((TILE * i * BK + 32 * s) * 2));
                                 const uint4 a_hi = gs_lds128(st + (uint32_t)(((DOWN ? TILE * i + 8 : TILE * TILES + TILE * i) * BK + 32 * s) * 2));
 #pragma unroll
-                                for (int j = 0; j < NT; ++j) {
-                                    gs_mma(acc[i][j][2 * s % CHAINS], a_lo.x, a_hi.x, a_lo.y, a_hi.y, xf[s][j].x, xf[s][j].y);
-                                    gs_mma(acc[i][j][(2 * s + 1) % CHAINS], a_lo.z, a_hi.z, a_lo.w, a_hi.w, xf[s][j].z, xf[s][j].w);
-                                }
+                                for (int j = 0; j < NT; ++j) tree[j].add(s, acc[i][j], a_lo, a_hi, xf[s][j]);
+                                if (IN_PLACE && i == tiles - 1) xr_load_x<NT>(xf[s], xr, w.K, next + 32 * s, t);
                             }
                         }
                         // the slot is released when every read of it is done (gs_consume in gemm_skinny.cu)
@@ -200,18 +208,17 @@ expert_rows_kernel(const __grid_constant__ CUtensorMap tmap, const XrWork w, int
                         for (int i = 0; i < TILES; ++i)
 #pragma unroll
                             for (int j = 0; j < NT; ++j)
-#pragma unroll
-                                for (int c = 0; c < CHAINS; ++c)
-                                    asm volatile("" : "+f"(acc[i][j][c][0]), "+f"(acc[i][j][c][1]), "+f"(acc[i][j][c][2]), "+f"(acc[i][j][c][3]));
+                                asm volatile("" : "+f"(acc[i][j][0]), "+f"(acc[i][j][1]), "+f"(acc[i][j][2]), "+f"(acc[i][j][3]));
                         __threadfence_block();
                         __syncwarp();
                         if (lane == 0) gs_mbar_arrive(&empty_bar[warp][slot]);
                     }
                     if (++slot == w.slots) slot = 0, phase ^= 1;
+                    if (!IN_PLACE)
 #pragma unroll
-                    for (int s = 0; s < BK / 32; ++s)
+                        for (int s = 0; s < BK / 32; ++s)
 #pragma unroll
-                        for (int j = 0; j < NT; ++j) xf[s][j] = xn[s][j];
+                            for (int j = 0; j < NT; ++j) xf[s][j] = xn[IN_PLACE ? 0 : s][j];
                 }
                 const int h = q & 1;
                 if (q >= 2 && !dead && !gs_mbar_wait(&sums_empty[h], ((q >> 1) - 1) & 1, &gave_up)) gave(6);
@@ -220,14 +227,7 @@ expert_rows_kernel(const __grid_constant__ CUtensorMap tmap, const XrWork w, int
 #pragma unroll
                     for (int i = 0; i < TILES; ++i)
 #pragma unroll
-                        for (int j = 0; j < NT; ++j) {
-                            float (&a)[4] = acc[i][j][0];
-#pragma unroll
-                            for (int c = 1; c < CHAINS; ++c)
-#pragma unroll
-                                for (int e = 0; e < 4; ++e) a[e] += acc[i][j][c][e];
-                            mine[(i * NT + j) * 32] = make_float4(a[0], a[1], a[2], a[3]);
-                        }
+                        for (int j = 0; j < NT; ++j) mine[(i * NT + j) * 32] = make_float4(acc[i][j][0], acc[i][j][1], acc[i][j][2], acc[i][j][3]);
                 }
                 __threadfence_block();
                 __syncwarp();
@@ -289,9 +289,11 @@ expert_rows_kernel(const __grid_constant__ CUtensorMap tmap, const XrWork w, int
                     float4 v[GS_CONSUMERS];
 #pragma unroll
                     for (int c = 0; c < GS_CONSUMERS; ++c) v[c] = theirs[(c * TILES * NT + j) * 32];
-                    acc[j][0] = v[0].x, acc[j][1] = v[0].y, acc[j][2] = v[0].z, acc[j][3] = v[0].w;
 #pragma unroll
-                    for (int c = 1; c < GS_CONSUMERS; ++c) acc[j][0] += v[c].x, acc[j][1] += v[c].y, acc[j][2] += v[c].z, acc[j][3] += v[c].w;
+                    for (int half = GS_CONSUMERS / 2; half > 0; half /= 2)
+#pragma unroll
+                        for (int c = 0; c < half; ++c) v[c].x += v[c + half].x, v[c].y += v[c + half].y, v[c].z += v[c + half].z, v[c].w += v[c + half].w;
+                    acc[j][0] = v[0].x, acc[j][1] = v[0].y, acc[j][2] = v[0].z, acc[j][3] = v[0].w;
                 }
                 __syncwarp();
                 if (lane == 0) gs_mbar_arrive(&sums_empty[h]);

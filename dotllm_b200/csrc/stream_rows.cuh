@@ -21,6 +21,30 @@ __device__ __forceinline__ void gs_mma(float (&c)[4], uint32_t a0, uint32_t a1, 
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// A chunk's products where the sums keep float32's accuracy: every instruction starts from zero, and what they leave is added up as a binary tree of
+// rounded additions.  (The tensor core cuts an accumulator's low bits off with every instruction that adds to it, so a chain of them drifts.)
+// S steps of 32 k, a power of two; the last one adds the chunk's sum to acc.
+template <int S> struct GsTree {
+    float level[4][4];
+    __device__ __forceinline__ void add(int s, float (&acc)[4], const uint4& lo, const uint4& hi, const uint4& x) {
+        static_assert(S >= 1 && S <= 16 && (S & (S - 1)) == 0, "a power of two");
+        float u[4] = {0.f, 0.f, 0.f, 0.f}, v[4] = {0.f, 0.f, 0.f, 0.f};
+        gs_mma(u, lo.x, hi.x, lo.y, hi.y, x.x, x.y);
+        gs_mma(v, lo.z, hi.z, lo.w, hi.w, x.z, x.w);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            float sum = u[e] + v[e];
+#pragma unroll
+            for (int l = 0; l < 4; ++l) {
+                if (!(s >> l & 1)) break;                    // (constants once the caller's loop over s is unrolled)
+                sum += level[l][e];
+            }
+            if (s == S - 1) acc[e] += sum;
+            else level[s & 1 ? (s & 2 ? (s & 4 ? 3 : 2) : 1) : 0][e] = sum;
+        }
+    }
+};
+
 __device__ __forceinline__ uint32_t gs_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void gs_mbar_init(uint64_t* bar, int count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gs_smem(bar)), "r"(count));

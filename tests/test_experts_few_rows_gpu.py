@@ -148,3 +148,25 @@ def test_experts_read_once_where_it_pays(tokens, top, E, K, ff, once):
     assert not ops.experts_by_rows(x, ids, w_in, w_out, "relu2") and not ops.experts_by_rows(x, ids, w_in, w_out, "silu", row_scale=x)
     odd = torch.empty(tokens, K + 1, dtype=torch.bfloat16, device=DEV)[:, 1:]
     assert not ops.experts_by_rows(odd, ids, w_in, w_out, "silu")
+
+
+@pytest.mark.parametrize("tokens,top,E,ff,N", [(1, 2, 4, 2048, 2048), (8, 2, 8, 768, 2048), (8, 1, 4, 8192, 2048), (16, 4, 8, 2048, 4096), (5, 1, 2, 14336, 4096),
+                                               (16, 1, 3, 1408, 7104)])
+def test_sums_of_chosen_experts_keep_float32(tokens, top, E, ff, N, monkeypatch):
+    """The float32 results of experts read once are as near the exact sums as those of the kernel that goes row by row (chains of float32 multiply-adds).
+    A chain of m rounded additions is sqrt(m / 2) 2^-24 / sqrt(3) off (the partial sums grow as a random walk), a tree of m sqrt(log2 m) of it: at
+    most 4 for the widest here, so 2^-22 would be a chain that drifts; the kernels differ by a quarter at most."""
+    from dotllm_b200.kernels import library, ops
+    g = torch.Generator().manual_seed(ff + N)
+    h = torch.randn(tokens * top, ff, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(E, N, ff, generator=g) * 0.02).to(torch.bfloat16).to(DEV)
+    ids = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(tokens)]).to(torch.int32).to(DEV)
+    weights = torch.rand(tokens, top, generator=g).to(DEV)
+    want = torch.stack([sum(weights[t, j].double() * (w[int(ids[t, j])].double() @ h[t * top + j].double()) for j in range(top)) for t in range(tokens)])
+    error = {}
+    for name, limit in (("once", 0.0), ("by rows", float("inf"))):
+        monkeypatch.setattr(ops, "EXPERT_ROWS_MB", (limit, limit))
+        got = ops.expert_down(h, ids, weights, w)
+        error[name] = float((got.double() - want).norm() / want.norm())
+    library.check_status()
+    assert error["once"] < 1.25 * error["by rows"] and error["once"] < 2.0 ** -22, error
