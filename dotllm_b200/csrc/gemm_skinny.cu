@@ -491,7 +491,7 @@ struct GsRowsWork {
     int x_stride;
     void* out;
     int out_stride;
-    int M, N, K, up_offset, cpt, block_rows, rows, passes, slots;     // slots: ring stages of a consumer warp
+    int M, N, K, up_offset, cpt, block_rows, rows, passes, slots, sums;     // ring stages of a consumer warp; passes whose sums have room
     GsFuse fuse;
 };
 
@@ -501,16 +501,20 @@ __host__ __device__ static inline int gs_rows_tiles(int n, int rows) {
     return full * ((rows + 15) / 16) + (rest + 15) / 16;
 }
 
-template <int NT, int BK>
-__device__ __forceinline__ void gs_rows_x(uint4 (&xf)[BK / 32][NT], const GsRowsWork& w, int k0, int g, int t) {
+// A lane's values of the tokens: a step of 32 k, a chunk.
+template <int NT>
+__device__ __forceinline__ void gs_rows_x(uint4 (&xf)[NT], const GsRowsWork& w, int k0, int g, int t) {
 #pragma unroll
-    for (int s = 0; s < BK / 32; ++s)
+    for (int j = 0; j < NT; ++j) {
+        const int tok = j * 8 + g, k = k0 + 8 * t;
+        xf[j] = make_uint4(0u, 0u, 0u, 0u);
+        if (tok < w.M && k < w.K) xf[j] = __ldg(reinterpret_cast<const uint4*>(w.x + (size_t)tok * w.x_stride + k));
+    }
+}
+template <int NT, int S>
+__device__ __forceinline__ void gs_rows_x(uint4 (&xf)[S][NT], const GsRowsWork& w, int k0, int g, int t) {
 #pragma unroll
-        for (int j = 0; j < NT; ++j) {
-            const int tok = j * 8 + g, k = k0 + 32 * s + 8 * t;
-            xf[s][j] = make_uint4(0u, 0u, 0u, 0u);
-            if (tok < w.M && k < w.K) xf[s][j] = __ldg(reinterpret_cast<const uint4*>(w.x + (size_t)tok * w.x_stride + k));
-        }
+    for (int s = 0; s < S; ++s) gs_rows_x<NT>(xf[s], w, k0 + 32 * s, g, t);
 }
 
 template <int NT, typename TOut, bool FUSE_SWIGLU, int TILES, int BK>
@@ -518,6 +522,10 @@ __global__ void __launch_bounds__(GR_THREADS(TILES), 1)
 gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWork w, int early_weights, int* __restrict__ status) {
     constexpr int TILE = FUSE_SWIGLU ? 8 : 16;               // rows (gated: pairs) of a tile
     constexpr int CHAINS = GR_CHAINS(TILES);                 // accumulators that a chunk's instructions go round: they wait for one another otherwise
+    // The next chunk's values of x are asked for before this one's arithmetic, into registers of their own.  Chunks of 256 k ask behind every step, into the
+    // registers that it has left: two sets of 16 tokens spilled, and a spilled load is waited for (2,048 x 14,336, 10 rows: 25.8 us, this way 15.8; 8 rows
+    // 13.9 both ways; 2,048 x 4,096, 8 rows 6.0 and 5.9).  Chunks of 128 lose by it (4,096 x 8,192, 8 rows: 14.3 and 14.7).
+    constexpr bool IN_PLACE = BK == 256;
     extern __shared__ __align__(128) unsigned char gs_smem_raw[];
     __shared__ uint64_t full_bar[GS_CONSUMERS][GR_MAX_SLOTS], empty_bar[GS_CONSUMERS][GR_MAX_SLOTS], scale_bar, sums_full[2], sums_empty[2];
     __shared__ volatile int gave_up;
@@ -539,7 +547,7 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
     const int first = blockIdx.x * w.block_rows, end_row = min(w.N, first + w.block_rows);      // this block's rows
     const int passes = (end_row - first + w.rows - 1) / w.rows, total = passes * w.cpt;
     const uint32_t box_bytes = w.rows * (BK * 2), stage_bytes = GR_stage_rows(w.rows, FUSE_SWIGLU, TILES) * (BK * 2);
-    // the sums of a pass, of two passes in turn: [2][warp][tile][NT][lane]
+    // the sums of a pass, or of two passes in turn: [sums][warp][tile][NT][lane]
     float4* sums = reinterpret_cast<float4*>(gs_smem_raw + GR_ring_bytes(w.rows, w.slots, FUSE_SWIGLU, TILES, BK));
     if (warp < GS_CONSUMERS) {
         // ------------------------------------------------------------ consumer warp
@@ -552,7 +560,7 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
             gave_up = 1;
             dead = true;
         };
-        if (cur < total) gs_rows_x<NT, BK>(xf, w, (cur % w.cpt) * BK, g, t);
+        if (cur < total) gs_rows_x<NT>(xf, w, (cur % w.cpt) * BK, g, t);
         for (int p = 0; p < passes; ++p) {
             float acc[TILES][NT][CHAINS][4];
 #pragma unroll
@@ -563,9 +571,9 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
                     for (int e = 0; e < 4 * CHAINS; ++e) acc[i][j][e / 4][e % 4] = 0.f;
             for (const int pass_end = (p + 1) * w.cpt; cur < pass_end; cur += GS_CONSUMERS) {
                 if (!dead && !gs_mbar_wait(&full_bar[warp][slot], phase, &gave_up)) gave(3);
-                uint4 xn[BK / 32][NT];                    // the next chunk's rows of x, asked for before this one's arithmetic
-                const int next = cur + GS_CONSUMERS;
-                gs_rows_x<NT, BK>(xn, w, next < total ? (next % w.cpt) * BK : w.K, g, t);
+                const int next = cur + GS_CONSUMERS, k_next = next < total ? (next % w.cpt) * BK : w.K;
+                uint4 xn[BK / 32][NT];
+                if (!IN_PLACE) gs_rows_x<NT>(xn, w, k_next, g, t);
                 if (!dead) {
                     // rows beyond the box are whatever lies behind it: they reach output rows that are not stored
                     const uint32_t st = gs_smem(gs_smem_raw + (size_t)(warp * w.slots + slot) * stage_bytes) + (uint32_t)(g * BK + 8 * t) * 2u;
@@ -584,6 +592,7 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
                                 gs_mma(acc[i][j][(2 * s + 1) % CHAINS], a_lo.z, a_hi.z, a_lo.w, a_hi.w, xf[s][j].z, xf[s][j].w);
                             }
                         }
+                        if (IN_PLACE) gs_rows_x<NT>(xf[s], w, k_next + 32 * s, g, t);
                     }
                     // as in gs_consume: the slot is released when every read of it is done
 #pragma unroll
@@ -598,13 +607,15 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
                     if (lane == 0) gs_mbar_arrive(&empty_bar[warp][slot]);
                 }
                 if (++slot == w.slots) slot = 0, phase ^= 1;
+                if (!IN_PLACE) {
 #pragma unroll
-                for (int s = 0; s < BK / 32; ++s)
+                    for (int s = 0; s < BK / 32; ++s)
 #pragma unroll
-                    for (int j = 0; j < NT; ++j) xf[s][j] = xn[s][j];
+                        for (int j = 0; j < NT; ++j) xf[s][j] = xn[s][j];
+                }
             }
-            const int h = p & 1;
-            if (p >= 2 && !dead && !gs_mbar_wait(&sums_empty[h], ((p >> 1) - 1) & 1, &gave_up)) gave(6);
+            const int h = w.sums == 2 ? p & 1 : 0, turn = w.sums == 2 ? p >> 1 : p;      // whose turn it is with sums h
+            if (turn >= 1 && !dead && !gs_mbar_wait(&sums_empty[h], (turn - 1) & 1, &gave_up)) gave(6);
             float4* mine = sums + (size_t)(h * GS_CONSUMERS + warp) * TILES * NT * 32 + lane;
             if (!dead) {
 #pragma unroll
@@ -666,7 +677,7 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
         const float* row_scale = nullptr;
         bool dead = false;
         for (int p = 0; p < passes && !dead; ++p) {
-            const int h = p & 1, pass_end = min(end_row, first + (p + 1) * w.rows);
+            const int h = w.sums == 2 ? p & 1 : 0, turn = w.sums == 2 ? p >> 1 : p, pass_end = min(end_row, first + (p + 1) * w.rows);
             const int base = first + p * w.rows + tile * TILE;
             // the stream's values and the gains, asked for early so that the epilogue does not wait for them (only this warp ever writes them)
             float stream_in[NT][4], gain_in[2] = {0.f, 0.f};
@@ -689,7 +700,7 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
                         }
                 }
             }
-            if (!gs_mbar_wait(&sums_full[h], (p >> 1) & 1, &gave_up) ||
+            if (!gs_mbar_wait(&sums_full[h], turn & 1, &gave_up) ||
                 (w.fuse.sumsq_in != nullptr && row_scale == nullptr && !gs_mbar_wait(&scale_bar, 0, &gave_up))) {
                 if (!gave_up) atomicExch(status, 5);
                 gave_up = 1;
@@ -822,10 +833,16 @@ static int gs_launch_rows_of(const GsRowsPlan& p, cudaStream_t s, const __nv_bfl
                           int N, int K, int early_weights, int* status, const GsFuse& fuse) {
     const int cpt = (K + BK - 1) / BK;
     const int a_warp = (p.passes * cpt + GS_CONSUMERS - 1) / GS_CONSUMERS;     // the busiest warp's chunks: no stages beyond them
-    const int sums = (p.passes > 1 ? 2 : 1) * GS_CONSUMERS * TILES * NT * 512;
-    int slots = a_warp < GR_MAX_SLOTS ? a_warp : GR_MAX_SLOTS;
-    while (slots > 1 && GR_ring_bytes(p.rows, slots, FUSE, TILES, BK) + sums > GR_SMEM) --slots;
-    const int smem = GR_ring_bytes(p.rows, slots, FUSE, TILES, BK) + sums;
+    const int a_pass = GS_CONSUMERS * TILES * NT * 512;      // bytes of a pass's sums
+    auto stages = [&](int sums) {
+        int slots = a_warp < GR_MAX_SLOTS ? a_warp : GR_MAX_SLOTS;
+        while (slots > 1 && GR_ring_bytes(p.rows, slots, FUSE, TILES, BK) + sums * a_pass > GR_SMEM) --slots;
+        return slots;
+    };
+    // Sums of two passes, unless that leaves the rings a single stage where one pass's leave two (48 rows and 16 tokens: 128,256 x 2,048 of 10 rows
+    // 95.7 us with one stage, 80 with two).
+    const int sums = p.passes > 1 && (stages(2) > 1 || stages(1) == 1) ? 2 : 1, slots = stages(sums);
+    const int smem = GR_ring_bytes(p.rows, slots, FUSE, TILES, BK) + sums * a_pass;
     static std::atomic<unsigned long long> sized{0};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -837,7 +854,7 @@ static int gs_launch_rows_of(const GsRowsPlan& p, cudaStream_t s, const __nv_bfl
     CUtensorMap tmap;
     const int rc = gs_weight_map(&tmap, w, FUSE ? 2 * N : N, K, p.rows, BK);
     if (rc != DL_OK) return rc;
-    const GsRowsWork work{x, x_stride, out, out_stride, M, N, K, N, cpt, p.block_rows, p.rows, p.passes, slots, fuse};
+    const GsRowsWork work{x, x_stride, out, out_stride, M, N, K, N, cpt, p.block_rows, p.rows, p.passes, slots, sums, fuse};
     e = dl_launch_dependent(gemm_skinny_rows_kernel<NT, TOut, FUSE, TILES, BK>, dim3(p.blocks), dim3(GR_THREADS(TILES)), (size_t)smem, s, tmap, work, early_weights, status);
     if (e != cudaSuccess) return dl_fail(DL_ERR_LAUNCH, "gemm_skinny: %s", cudaGetErrorString(e));
     return DL_OK;

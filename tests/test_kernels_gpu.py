@@ -547,6 +547,41 @@ def test_gemm_skinny_rows(N, K, gated, M, monkeypatch):
     library.check_status()
 
 
+def _chained_us(make, n, runs=9):
+    """Microseconds of one of ``n`` launches back to back in a captured graph, the shortest of several runs."""
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        make()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            make()
+        times = []
+        for _ in range(runs):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(stream)
+            graph.replay()
+            b.record(stream)
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+    return min(times[1:]) * 1e3 / n
+
+
+@pytest.mark.parametrize("N,K,gated,most", [(2048, 14336, False, 1.6), (2048, 16384, False, 1.6), (1024, 14336, True, 1.6), (128256, 2048, False, 1.12)])
+def test_gemm_skinny_16_rows_cost_little_more_than_8(N, K, gated, most, monkeypatch):
+    """W is read once either way; x of 16 rows is twice that of 8: at most as many bytes more as W has with one tile of rows a block, next to
+    none for many rows.  (Registers that spill and a ring of a single stage made it 2.4 and 1.2 times.)"""
+    from dotllm_b200.kernels import gemm_skinny, library
+    monkeypatch.setattr(gemm_skinny, "SKINNY_ROWS", gemm_skinny.KERNEL_ROWS)
+    rows = (2 if gated else 1) * N
+    copies = (300 << 20) // (2 * rows * K) + 2               # more than the L2 holds
+    ws = [torch.full((rows, K), 0.01, dtype=torch.bfloat16, device=DEV) for _ in range(copies)]
+    x = torch.ones(16, K, dtype=torch.bfloat16, device=DEV)
+    t = {m: _chained_us(lambda: [gemm_skinny.run(x[:m], w, torch.bfloat16, fuse_swiglu=gated, resident=True) for w in ws], copies) for m in (8, 16)}
+    library.check_status()
+    assert t[16] < most * t[8], t
+
+
 @pytest.mark.parametrize("M,H,K,N2", [(8, 4096, 512, 1024), (1, 1000, 384, 272), (13, 1000, 384, 272), (16, 72, 64, 40),
                                       (17, 1000, 384, 272), (64, 4096, 512, 1024), (100, 1000, 4096, 272), (128, 72, 64, 40)])
 def test_products_that_add_and_normalise(M, H, K, N2, monkeypatch):
