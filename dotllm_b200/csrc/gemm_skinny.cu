@@ -13,18 +13,18 @@
 // is the same on every launch.  With FUSE_SWIGLU a tile's rows 0-7 are gate rows and rows 8-15 the matching up rows, and the epilogue
 // writes silu(gate) * up (native/kernels/swiglu.cu:7-41).
 //
-// * By rows (gemm_skinny_rows_kernel; nearly all sizes): every multiprocessor owns the same number of rows of W over all of k.  The consumer warps split k,
+// * By rows (gemm_skinny_rows_kernel; most sizes): every multiprocessor owns the same number of rows of W over all of k.  The consumer warps split k,
 //   their sums meet in shared memory, and warps of their own add them in a fixed order and run the epilogue.  Nothing passes between blocks: no
 //   partial sums through global memory, no counters.  A pass holds up to 48 rows, so a chunk's slice of x is read once for all of them (x is 8 / 48 of what
 //   W is; with 16-row tiles it was half, and its loads' latency set the pace).
-// * By shares (gemm_skinny_kernel; where a block's rows are one tile and 4,096 < K < 12,288): the list of (16-row tile, 256-wide chunk of k) pairs in
+// * By shares (gemm_skinny_kernel; few rows a block and K > 4,096, see gs_by_rows): the list of (16-row tile, 256-wide chunk of k) pairs in
 //   tile-major order is cut into equal contiguous shares, one per consumer warp of the whole grid.  A tile cut between shares is summed, in share
 //   order, by whichever of its warps arrives last.
 //
 // By rows against by shares, each product in a graph of many, 8 rows: 3,072 x 2,048 5.5 -> 5.0 us, 2,048 x 2,048 5.1 -> 4.2, 64 x 2,048 3.8 -> 2.7, gated
 // 8,192 x 2,048 15.4 -> 13.3, 6,144 x 4,096 12.7 -> 11.1, 4,096 x 14,336 22.1 -> 20.9, gated 14,336 x 4,096 40.3 -> 38.5, 128,256 x 2,048
-// 87.0 -> 80.6 (6.5 TB/s); the small ones are a chain of latencies (start, rows of x, sums).  One tile a block leaves x at half the bytes of W again:
-// 2,048 x 4,096 by rows 6.3, by shares 6.4; x 6,144 8.2 and 7.7; x 8,192 9.9 and 9.2; x 16,384 15.3 and 16.1.  A decode step of 16 layers of the smaller
+// 87.0 -> 80.6 (6.5 TB/s); the small ones are a chain of latencies (start, rows of x, sums).  One tile a block leaves x at half the bytes of W again.
+// A decode step of 16 layers of the smaller
 // widths, 8 sequences at 2,000 tokens: 905 -> 849 us.  Tried: rings of half the size, so that the next product's first weights arrive under this one
 // (941 us), x asked for three chunks ahead (2,048 x 2,048 4.3 -> 4.7), passes of 32 rows (5,120 x 13,824, 35 rows a block: 25.5 -> 30.1).
 //
@@ -728,10 +728,20 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
     __syncthreads();                                         // nobody leaves while copies may still land
 }
 
-// Which products go that way; the others by shares.  With one tile of rows a block, x is half as many bytes as W, and by shares it is asked for
-// further ahead; below 4,096 what passes between blocks costs more than that, at 16,384 the rows' distance of a power of two slows the shares down
-// (both sides measured at the top of this file).
-static bool gs_by_rows(int N, int K, bool gated, int sms) { return gated || (N + sms - 1) / sms > 16 || K <= 4096 || K >= 12288; }
+// Which products go that way; the others by shares.  By rows every block reads all of x, by shares what passes between blocks takes its time: rows
+// for short k and where a block has many rows, shares for a few rows of long k.  By the sizes alone, so that a row's bits do not depend on the
+// number of rows of x.  Measured at 8 and at 10 rows of x, by rows / by shares, us (2,048 columns: 14 rows of W a block of 148; 1,536: 11; 2,400: 17):
+//   2,048 x 4,096   6.0 6.7 / 6.3 6.7      2,048 x 8,192   9.7 11.1 / 9.3 10.0      2,048 x 14,336  13.9 15.8 / 13.4 14.3
+//   2,048 x 5,120   7.3 8.2 / 8.0 8.6      2,048 x 12,288 12.6 14.2 / 11.8 12.8     2,048 x 16,384  15.1 17.6 / 15.9 16.6
+//   1,536 x 14,336 12.6 14.5 / 11.1 12.2   512 x 4,096      4.5  5.3 / 5.1  5.8      512 x 14,336   10.2 12.6 / 8.0 9.1
+//   2,400 x 4,096 and less as 2,048        2,400 x 8,192  12.6 14.3 / 11.4 12.2     3,072 x 8,192   13.4 14.2 / 13.2 13.9
+// Gated: 1,024 x 14,336 (14 rows: 7 pairs) 13.9 15.8 / 13.1 13.9, 512 x 8,192 7.6 9.0 / 6.9 8.0, 512 x 14,336 10.8 13.5 / 9.4 10.6, 64 x 14,336 9.5 12.2 / 7.7 8.8.
+static bool gs_by_rows(int N, int K, bool gated, int sms) {
+    const int rows = (gated ? 2 : 1) * ((N + sms - 1) / sms);     // of W a block
+    if (K <= 4096 || rows > 20) return true;
+    if (gated) return rows >= 14;
+    return rows >= 14 && rows <= 16 && (K <= 5120 || K >= 12288);
+}
 
 // Parts of the sums of squares (16 floats each) that a product of N output columns over K leaves.
 extern "C" int dl_gemm_skinny_parts(int N, int K) {
@@ -753,17 +763,32 @@ static GsPlan gs_plan(int N, int K, int fuse_swiglu, int sms) {
     p.tiles = fuse_swiglu ? (N + 7) / 8 : (N + 15) / 16;
     p.cpt = (K + GS_BK - 1) / GS_BK;
     p.total = p.tiles * p.cpt;
-    // A share is a whole number of chunks, so the last multiprocessors get less, or nothing: of eight, seven and six warps those that leave the
-    // busiest multiprocessor with the fewest chunks (more warps where it is the same: they have more of the ring).  1,024 chunks of a
-    // 2,048 x 2,048 matrix: 8, 7 or 12; 14,336 of a 4,096 x 14,336 one: 104, 98 or 102 (22.1 against 21.5 us with eight and six).
-    p.active = GS_CONSUMERS;
-    for (int c = GS_CONSUMERS; c >= GS_CONSUMERS - 2; --c) {
-        const int share = (p.total + sms * c - 1) / (sms * c);
-        if (c == GS_CONSUMERS || share * c < p.share * p.active) p.share = share, p.active = c;
+    // A share is a whole number of chunks, so the last multiprocessors get less, or nothing: the number of warps, and the share, that leave the busiest
+    // multiprocessor the fewest chunks.  Shares that do not divide a tile's chunks count six more: their warps end one tile and begin another, about 1 us
+    // (1,536 x 8,192, 8 rows: seven warps of 3 of 32 chunks 8.75 us, six of 4 7.9; 1,024 x 10,240: six of 3 of 40 8.9, six of 4 8.1).  And a tile is cut
+    // into 28 parts at most, or fewer where k is long, since one warp adds them all (512 x 8,192: 32 parts 7.3 us, 16 6.3; 512 x 12,288: 24
+    // parts 7.3, 12 7.2; 16 x 16,384: 64 parts 9.0, 32 7.1, 16 6.7).  Of equals the one with more warps: they have more of the ring.
+    const int least = p.cpt >= 48 ? 4 : p.cpt >= 32 ? 2 : 1;
+    int best = 0;
+    for (int c = GS_CONSUMERS; c >= GS_CONSUMERS / 2; --c) {
+        const int even = (p.total + sms * c - 1) / (sms * c), first = even > least ? even : least;
+        for (int share = first; share <= first + 1; ++share) {
+            const int cost = 2 * (c * share + (p.cpt % share != 0 ? 6 : 0)) + (p.cpt % share != 0 ? 1 : 0);
+            if (best == 0 || cost < best) best = cost, p.active = c, p.share = share;
+        }
     }
     p.blocks = (p.total + p.active * p.share - 1) / (p.active * p.share);
     if (p.blocks < 1) p.blocks = 1;
     return p;
+}
+
+// The form and the cut of a product on a device of `sms` multiprocessors: by rows (1) or by shares (0), and by shares the warps of a block that have one,
+// its chunks, blocks.
+extern "C" int dl_gemm_skinny_plan(int N, int K, int gated, int sms, int* by_rows, int* active, int* share, int* blocks) {
+    DL_REQUIRE(N > 0 && K > 0 && sms > 0, "gemm_skinny_plan: bad sizes");
+    const GsPlan p = gs_plan(N, K, gated, sms);
+    *by_rows = gs_by_rows(N, K, gated != 0, sms) ? 1 : 0, *active = p.active, *share = p.share, *blocks = p.blocks;
+    return DL_OK;
 }
 
 // Scratch the product needs: float32 partial sums and int32 arrival counters (zero before the first
@@ -1065,6 +1090,7 @@ extern "C" int dl_gemm_skinny_static_status(int* code, void* stream) {
 
 DL_PACKED(dl_gemm_skinny_scratch)
 DL_PACKED(dl_gemm_skinny_parts)
+DL_PACKED(dl_gemm_skinny_plan)
 DL_PACKED(dl_gemm_skinny_bf16)
 DL_PACKED(dl_gemm_skinny_gated_bf16)
 DL_PACKED(dl_gemm_skinny_fused_bf16)

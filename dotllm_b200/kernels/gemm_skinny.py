@@ -23,6 +23,7 @@ _library.register_signatures({
                                   _P, _I, _P, _I, _P, _P],
     "dl_gemm_skinny_gated_bf16": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P, _I, _P, _I, _P, _P],
     "dl_gemm_skinny_parts": [_I, _I],
+    "dl_gemm_skinny_plan": [_I, _I, _I, _I, _P, _P, _P, _P],
     "dl_gemm_skinny_scratch": [_I, _I, _I, _I, _I, _P, _P],
 })
 
@@ -147,6 +148,14 @@ def run_activated(x, w, kind, resident=False):
                   2 if resident else 0, int(kind), 0.0, 0.0, None, partials, partials.numel(),
                   counters, counters.numel(), status, _library.current_stream())
     return out
+
+
+def plan(N, K, gated=False, sms=148):
+    """How a product is cut on a device of ``sms`` multiprocessors: ("rows", 0, 0, 0), or ("shares", warps of a block with a share, its chunks, blocks)."""
+    v = [ctypes.c_int() for _ in range(4)]
+    if _library.library().dl_gemm_skinny_plan(N, K, 1 if gated else 0, sms, *(ctypes.byref(i) for i in v)) != 0:
+        raise _library.KernelError(f"gemm_skinny: no plan for {N} x {K}")
+    return ("rows", 0, 0, 0) if v[0].value else ("shares", v[1].value, v[2].value, v[3].value)
 
 
 def scratch_need(M, N, K, fuse_swiglu=False, sms=148):

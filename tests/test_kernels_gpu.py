@@ -497,7 +497,7 @@ def test_gemm_skinny_repeats_with_full_rings(monkeypatch):
 @pytest.mark.parametrize("N,K", [(16, 8), (1, 264), (17, 256), (40, 2048), (2048, 2048), (1184 * 16 + 5, 256), (9, 16384), (2368 * 2 + 16, 2048)])
 @pytest.mark.parametrize("gated", [False, True])
 def test_gemm_skinny_shares(N, K, gated, monkeypatch):
-    """Shares of unequal length (some warps one chunk of 256 k more than others, fewer chunks than warps, tiles over many shares): against
+    """Few rows and many, short k and long (all but the smallest of them go by rows; the products by shares are test_gemm_skinny_by_shares'): against
     float64, the same bits for one row as for eight and on every launch.  Bound: float32 sums of K products, K / 16 rounded additions deep."""
     from dotllm_b200.kernels import gemm_skinny
     g = torch.Generator().manual_seed(N * 7 + K)
@@ -537,6 +537,58 @@ def test_gemm_skinny_rows(N, K, gated, M, monkeypatch):
     assert torch.equal(gemm_skinny.run(x[:1].contiguous(), w, torch.float32, fuse_swiglu=gated), y[:1])
     for _ in range(3):
         assert torch.equal(gemm_skinny.run(x, w, torch.float32, fuse_swiglu=gated), y)
+    if not gated:
+        stream, gain = torch.randn(M, N, generator=g).to(DEV), torch.rand(N, generator=g).to(DEV)
+        want = stream + y
+        scaled, sums = gemm_skinny.run(x, w, torch.float32, into=(stream, gain))
+        assert torch.equal(stream, want) and torch.equal(scaled, (want * gain).to(torch.bfloat16))
+        total = sums.view(-1, gemm_skinny.SUM_STRIDE)[:, :M].double().sum(0)
+        assert ((total - want.double().square().sum(1)).abs() <= 2 ** -20 * total).all()
+    library.check_status()
+
+
+SHARES = [(1, 8192, False), (16, 4104, False), (17, 6144, False), (40, 12280, False), (300, 8200, False), (512, 16384, False), (768, 6144, False), (1000, 10240, False),
+          (1536, 8192, False), (2000, 8192, False), (2368, 6144, False), (2400, 7168, False), (2560, 6912, False), (1, 12296, True), (17, 4104, True), (64, 14336, True), (888, 8192, True)]
+
+
+def test_gemm_skinny_shares_sizes_are_cut_into_shares():
+    """The sizes below go by shares, with every number of warps that has one, shares that divide a tile and shares that do not, one chunk and many."""
+    from dotllm_b200.kernels import gemm_skinny, library
+    plans = {size: gemm_skinny.plan(*size, sms=library.sm_count()) for size in SHARES}
+    assert all(form == "shares" for form, *_ in plans.values()), plans
+    if library.sm_count() == 148:
+        assert {p[1] for p in plans.values()} == {4, 5, 6, 7, 8} and {1, 2, 3, 4} <= {p[2] for p in plans.values()}, plans
+        assert any(-(-k // 256) % plans[n, k, gated][2] for n, k, gated in SHARES)
+
+
+@pytest.mark.parametrize("N,K,gated", SHARES)
+@pytest.mark.parametrize("M", [1, 9, 16])
+def test_gemm_skinny_by_shares(N, K, gated, M, monkeypatch):
+    """Products cut into shares: tiles that many warps of many blocks hand over, fewer chunks than warps, the last share shorter, row factors from the
+    product before and sums of squares for the next.  Against float64 (bound as in test_gemm_skinny_shares), with the bits of one row alone, and the
+    same bits on every launch: partial sums, counters and ring slots are used again at once."""
+    from dotllm_b200.kernels import gemm_skinny, library
+    monkeypatch.setattr(gemm_skinny, "SKINNY_ROWS", gemm_skinny.KERNEL_ROWS)
+    g = torch.Generator().manual_seed(N * 3 + K)
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn((2 if gated else 1) * N, K, generator=g) * 0.05).to(torch.bfloat16).to(DEV)
+    p, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+
+    def close_to(y, factor=1.0):
+        q, e = p * factor, size * factor
+        ref = torch.nn.functional.silu(q[:, :N]) * q[:, N:] if gated else q
+        e = 1.1 * (e[:, :N] * (q[:, N:].abs() + 1e-3) + q[:, :N].abs() * e[:, N:]) if gated else e
+        assert ((y.double() - ref).abs() <= ((K / 16 + 16) * 2 ** -24 + 2 ** -21 * isinstance(factor, torch.Tensor)) * e + 1e-12).all()
+
+    y = gemm_skinny.run(x, w, torch.float32, fuse_swiglu=gated)
+    close_to(y)
+    assert torch.equal(gemm_skinny.run(x[:1].contiguous(), w, torch.float32, fuse_swiglu=gated), y[:1])
+    for _ in range(30 if M == 16 else 3):
+        assert torch.equal(gemm_skinny.run(x, w, torch.float32, fuse_swiglu=gated), y)
+    # an output row's factor is rsqrt(the sum of its parts / width + eps): a float32 division, sum and root, 2^-21 of it
+    parts = torch.rand(5, gemm_skinny.SUM_STRIDE, generator=g).to(DEV)
+    factor = (parts.double().sum(0)[:M, None] / 70 + 1e-5).rsqrt()
+    close_to(gemm_skinny.run(x, w, torch.float32, fuse_swiglu=gated, row_sums=(parts.flatten(), 5, 70, 1e-5)), factor)
     if not gated:
         stream, gain = torch.randn(M, N, generator=g).to(DEV), torch.rand(N, generator=g).to(DEV)
         want = stream + y
