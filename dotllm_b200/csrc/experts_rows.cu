@@ -165,8 +165,10 @@ expert_rows_kernel(const __grid_constant__ CUtensorMap tmap, const XrWork w, int
             dead = true;
         };
         rows_of(0);
+        if (warp < chunks) {
 #pragma unroll
-        for (int s = 0; s < BK / 32; ++s) xr_load_x<NT>(xf[s], xr, warp < chunks ? w.K : 0, (warp % w.cpt) * BK + 32 * s, t);
+            for (int s = 0; s < BK / 32; ++s) xr_load_x<NT>(xf[s], xr, w.K, (warp % w.cpt) * BK + 32 * s, t);
+        }
         const int tiles = (w.pass_rows + TILE - 1) / TILE;
         for (int d = 0, q = 0; d < entries; ++d) {
             int cur = warp;

@@ -1213,32 +1213,53 @@ def _addend(addend, addend_gate, T, N, what):
     return astride, gstride
 
 
-# Tokens up to which the chosen experts' matrices are read once each (csrc/experts_rows.cu), and the megabytes of an expert's matrices from which
-# that pays with up to eight tokens and with more: an expert costs it about 2.5 (3.6) us however small it is.  Measured, once each / row by row /
-# as tiles, us: 16 experts of 25 MB, two a token, 8 tokens 53 / 84 / -, 16 tokens 70 / 149 / 130; 32 of 50 MB, four, 8 tokens 180 / 335 / 309,
-# 16 tokens 212 / 561 / 333; 64 of 17 MB, six, 8 tokens 120 / 203 / 201, 16 tokens 230 / 350 / 275; 128 of 9 MB, eight, 1 token 31 / 57 / -, 8 tokens
-# 140 / 150 / 184, 16 tokens 320 / 257 / 268; 32 of 9 MB, four, 8 tokens 65 / 79 / 110, 16 tokens 115 / 136 / 115; 16 of 3 MB, two, 8 tokens 33 / 18 / -.
+# Tokens up to which the chosen experts' matrices are read once each (csrc/experts_rows.cu), and the megabytes from which that pays, with up to eight
+# tokens and with more: of a gated expert's three matrices, so 1.5 times those of the gate/up product and 3 times those of the down product, each of
+# which is asked for itself.  An entry (an expert and its rows) costs each product about 1.25 us (1.8 with more than eight tokens) however small it is.
+# Measured, once each / row by row / as tiles, us: 16 experts of 25 MB, two a token, 8 tokens 49 / 84 / -, 16 tokens 72 / 149 / 130; 32 of 50 MB, four, 8 tokens
+# 151 / 335 / 309, 16 tokens 225 / 561 / 333; 64 of 17 MB, six, 8 tokens 120 / 203 / 201, 16 tokens 215 / 350 / 275; 128 of 9 MB, eight, 1 token 30 / 57 / -, 8 tokens
+# 133 / 150 / 184, 16 tokens 320 / 257 / 268; 32 of 9 MB, four, 8 tokens 60 / 79 / 110, 16 tokens 115 / 136 / 115; 16 of 3 MB, two, 8 tokens 33 / 18 / -.
+# The second number also holds for gate/up products of at most four pairs a block with more than four tokens (128 experts, two of 512 x 4,096 pairs,
+# 4 tokens 1.1 times as fast as row by row, 8 tokens 38 / 33).  An expert whose width is no multiple of 8 goes row by row altogether (256, eight of 700 x 2,048
+# pairs: the gate/up product of 6 tokens 62 / 52).
+# A down product behind a gate/up product that went row by row (no gate, or weights on the way in) cannot begin under it, since a block takes a whole
+# multiprocessor: with short sums, which row by row are short chains, that is more than reading once saves.  Such steps, top x ff < 1,536: 8 experts, one
+# of 768, N 2,048: 3 tokens 19.8 / 15.3, 16, one of 1,024, N 4,096: 1 token 26 / 21, 3 tokens 30 / 23.5, 8 tokens as fast; up to 2,304: 16 experts, two of
+# 1,024, N 2,048: 1 token 24 / 23, 8 tokens 1.1 times as fast.
 EXPERT_ROWS_TOKENS = 16
 EXPERT_ROWS_MB = (8.0, 16.0)
 
 
-def _expert_rows_take(x, x_stride, ids, w, k, mb):
+def _expert_rows_take(x, x_stride, ids, w, k, mb, more):
     T, top = ids.shape
-    return (T <= EXPERT_ROWS_TOKENS and mb >= EXPERT_ROWS_MB[T > 8] and T * top <= 128 and w.shape[0] <= 512 and x.dtype == torch.bfloat16 and x.is_cuda and k % 8 == 0
-            and x_stride % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+    return (T <= EXPERT_ROWS_TOKENS and mb >= EXPERT_ROWS_MB[more or T > 8] and T * top <= 128 and w.shape[0] <= 512 and x.dtype == torch.bfloat16 and x.is_cuda
+            and k % 8 == 0 and x_stride % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 @functools.lru_cache(maxsize=4096)
-def _down_rows_take(rows, n, sms):
+def _down_rows_fit(rows, n, sms):
     return bool(_library.library().dl_expert_down_rows_takes(rows, n))
+
+
+def _gate_up_by_rows(x, x_stride, ids, w, ff, row_scale, gated):
+    K = x.shape[1]
+    return (row_scale is None and gated and K <= 12288 and ff % 8 == 0
+            and _expert_rows_take(x, x_stride, ids, w, K, 6e-6 * ff * K, ids.shape[0] > 4 and ff <= 4 * _library.sm_count()))
+
+
+def _down_by_rows(h, ids, w, ff, N, read_once):
+    """``h``: any tensor of its type at its alignment; its rows are ff apart.  ``read_once`` as in ``expert_down``."""
+    top, rows = ids.shape[1], ids.numel()
+    short = 0 if read_once else top * ff
+    return (top * (-(-ff // 256) * 256) <= 24576 and _expert_rows_take(h, ff, ids, w, ff, 6e-6 * ff * N, 0 < short < 1536)
+            and not (0 < short < 2304 and rows <= 3) and _down_rows_fit(rows, N, _library.sm_count()))
 
 
 def experts_by_rows(x, ids, w_gate_up, w_down, kind, row_scale=None):
     """Do ``expert_gate_up`` and ``expert_down`` read every chosen expert's matrices once for this step?  Then nothing else is faster."""
-    return (row_scale is None and kind not in UNGATED and x.stride(1) == 1 and x.shape[1] <= 12288
-            and _expert_rows_take(x, x.stride(0) if x.shape[0] > 1 else x.shape[1], ids, w_gate_up, x.shape[1], 6e-6 * w_down.shape[2] * x.shape[1])
-            and w_down.data_ptr() % 16 == 0 and w_down.shape[2] % 8 == 0 and ids.shape[1] * (-(-w_down.shape[2] // 256) * 256) <= 24576
-            and _down_rows_take(ids.numel(), w_down.shape[1], _library.sm_count()))
+    N, ff = w_down.shape[1:]
+    return (x.stride(1) == 1 and _gate_up_by_rows(x, x.stride(0) if x.shape[0] > 1 else x.shape[1], ids, w_gate_up, ff, row_scale, kind not in UNGATED)
+            and _down_by_rows(x, ids, w_down, ff, N, True))
 
 
 def expert_gate_up(x, ids, w_gate_up, kind, limit=0.0, alpha=1.0, row_scale=None):
@@ -1257,7 +1278,7 @@ def expert_gate_up(x, ids, w_gate_up, kind, limit=0.0, alpha=1.0, row_scale=None
     ff = rows_w // halves
     T, top = ids.shape
     out = _library.empty(T * top, ff, x.dtype, x)
-    if row_scale is None and halves == 2 and _expert_rows_take(x, xs, ids, w_gate_up, K, 6e-6 * ff * K) and K <= 12288:
+    if _gate_up_by_rows(x, xs, ids, w_gate_up, ff, row_scale, halves == 2):
         _library.call("dl_expert_gate_up_rows", x, xs, ids, w_gate_up, out, T, top, K, ff, E, GATINGS[kind], float(limit), float(alpha),
                       _library.status_word(x.device), _stream())
         return out
@@ -1276,12 +1297,12 @@ def _identity(identity, T, N, dtype, what):
     return rows, _rows_view(rows, what + " identity"), int(count)
 
 
-def expert_down(h, ids, weights, w_down, addend=None, addend_gate=None, identity=None):
+def expert_down(h, ids, weights, w_down, addend=None, addend_gate=None, identity=None, read_once=False):
     """out[t] = sum_j weights[t, j] * D_e(t,j) h[t*top + j]  (+ addend[t]), float32 [T, N].  h [T*top, ff];
     w_down [E, N, ff] of h's dtype; weights float32 [T, top] or None (all 1); addend float32 [T, N] (rows contiguous)
     or None; ``addend_gate`` float32, one logit per token (column 0 of a [T, n] view): the addend times its sigmoid.
     ``identity`` (x [T, N] of h's dtype, n): ids E .. E + n - 1 name experts without matrices that give back their input,
-    weight * x[t]."""
+    weight * x[t].  ``read_once``: ``expert_gate_up`` read the chosen experts' matrices once for this step (``experts_by_rows``)."""
     _need_cuda(h, ids, weights, w_down, addend, addend_gate)
     _int32(ids, "expert ids")
     T, top = ids.shape
@@ -1293,7 +1314,7 @@ def expert_down(h, ids, weights, w_down, addend=None, addend_gate=None, identity
     astride, gstride = _addend(addend, addend_gate, T, N, "expert_down")
     irows, istride, icount = _identity(identity, T, N, h.dtype, "expert_down")
     out = _library.empty(T, N, torch.float32, h)
-    if _expert_rows_take(h, ff, ids, w_down, ff, 6e-6 * ff * N) and top * (-(-ff // 256) * 256) <= 24576 and _down_rows_take(T * top, N, _library.sm_count()):
+    if _down_by_rows(h, ids, w_down, ff, N, read_once):
         _library.call("dl_expert_down_rows", h, ids, weights, w_down, addend, astride, out, T, top, ff, N, E, addend_gate, gstride, irows,
                       istride, icount, _library.status_word(h.device), _stream())
         return out

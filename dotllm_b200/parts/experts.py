@@ -165,13 +165,13 @@ class RoutedExperts(FeedForward):
                 shared_gate = z[:, self.n_experts + self.identity:self.n_experts + self.identity + 1]   # the row behind the experts' rows
         # the weight on the expert's input scales the rows that go in; nothing is left to weigh on the way out
         scale, weights = (weights, None) if self.weight_on == "input" else (None, weights)
-        if not ops.experts_by_rows(x, ids, self.w_gate_up, self.w_down, self.activation, row_scale=scale) \
-                and ops.experts_as_tiles(x, ids, self.w_gate_up, self.w_down, row_scale=scale):
+        read_once = ops.experts_by_rows(x, ids, self.w_gate_up, self.w_down, self.activation, row_scale=scale)
+        if not read_once and ops.experts_as_tiles(x, ids, self.w_gate_up, self.w_down, row_scale=scale):
             # many rows: sorted by expert, both products as tensor-core tiles
             return ops.experts_grouped(x, ids, weights, self.w_gate_up, self.w_down, self.activation, self.limit, self.alpha,
                                        addend=shared, row_scale=scale, addend_gate=shared_gate, identity=identity)
         h = ops.expert_gate_up(x, ids, self.w_gate_up, self.activation, self.limit, self.alpha, row_scale=scale)
-        return ops.expert_down(h, ids, weights, self.w_down, addend=shared, addend_gate=shared_gate, identity=identity)
+        return ops.expert_down(h, ids, weights, self.w_down, addend=shared, addend_gate=shared_gate, identity=identity, read_once=read_once)
 
 
 register_feed_forward("routed_experts", RoutedExperts)

@@ -117,7 +117,7 @@ def test_chosen_experts_read_once(tokens, top, E, K, ff, N, monkeypatch):
         # |d/da a sigmoid(1.702 a)| <= 1.1, |b + 1| <= 2.5, |a sigmoid| <= 1.5
         assert ((h[r].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.75 * size[:ff] + 1.5 * size[ff:] + 1e-6).all()
     for kw in (dict(weights=weights, addend=addend, addend_gate=gate, identity=(other, 1)), dict(weights=None), dict(weights=weights, addend=addend)):
-        got = ops.expert_down(h, ids, kw.get("weights"), w_out, addend=kw.get("addend"), addend_gate=kw.get("addend_gate"), identity=kw.get("identity"))
+        got = ops.expert_down(h, ids, kw.get("weights"), w_out, addend=kw.get("addend"), addend_gate=kw.get("addend_gate"), identity=kw.get("identity"), read_once=True)
         want, bound = torch.zeros(tokens, N, dtype=torch.float64, device=DEV), torch.zeros(tokens, N, dtype=torch.float64, device=DEV)
         if "addend" in kw:
             want += addend.double() * (torch.sigmoid(gate[:, :1].double()) if "addend_gate" in kw else 1.0)
@@ -131,7 +131,7 @@ def test_chosen_experts_read_once(tokens, top, E, K, ff, N, monkeypatch):
         assert ((got.double() - want).abs() <= (ff / 16 + 16 + top) * 2.0 ** -24 * (bound + want.abs()) + 1e-5 * want.abs() + 1e-6).all()
         alone = ops.expert_down(h[-top:].contiguous(), ids[-1:].contiguous(), kw["weights"][-1:].contiguous() if kw["weights"] is not None else None, w_out,
                                 addend=addend[-1:].contiguous() if "addend" in kw else None, addend_gate=gate[-1:] if "addend_gate" in kw else None,
-                                identity=(other[-1:], 1) if "identity" in kw else None)
+                                identity=(other[-1:], 1) if "identity" in kw else None, read_once=True)
         assert torch.equal(alone, got[-1:])
     assert torch.equal(ops.expert_gate_up(x[-1:].contiguous(), ids[-1:].contiguous(), w_in, "clamped_sigmoid", 1.5, 1.702), h[-top:])
     library.check_status()
@@ -166,7 +166,36 @@ def test_sums_of_chosen_experts_keep_float32(tokens, top, E, ff, N, monkeypatch)
     error = {}
     for name, limit in (("once", 0.0), ("by rows", float("inf"))):
         monkeypatch.setattr(ops, "EXPERT_ROWS_MB", (limit, limit))
-        got = ops.expert_down(h, ids, weights, w)
+        got = ops.expert_down(h, ids, weights, w, read_once=True)
         error[name] = float((got.double() - want).norm() / want.norm())
     library.check_status()
     assert error["once"] < 1.25 * error["by rows"] and error["once"] < 2.0 ** -22, error
+
+
+@pytest.mark.parametrize("tokens,top,ff,N,E,once", [(1, 1, 768, 2048, 8, False), (8, 1, 768, 2048, 8, False), (8, 1, 1024, 2048, 64, False), (8, 1, 1408, 2048, 16, True),
+                                                    (8, 2, 704, 2048, 64, False), (2, 2, 512, 4096, 128, False), (1, 4, 768, 2048, 32, True), (8, 2, 768, 2048, 32, True),
+                                                    (8, 2, 664, 2048, 32, False), (1, 2, 1024, 2048, 16, False), (2, 2, 1024, 2048, 16, True),
+                                                    (9, 2, 1024, 2048, 16, False), (9, 2, 1408, 2048, 16, True), (9, 1, 1408, 2048, 16, True)])
+def test_down_products_read_once_where_that_pays(tokens, top, ff, N, E, once, monkeypatch):
+    """Whatever came before them (a gate or none, weights on the way in): by the down matrices' own size, and short sums row by row."""
+    from dotllm_b200.kernels import library, ops
+    called = []
+    real = library.call
+    monkeypatch.setattr(library, "call", lambda name, *a: (called.append(name), real(name, *a))[1])
+    h, w = torch.zeros(tokens * top, ff, dtype=torch.bfloat16, device=DEV), torch.zeros(E, N, ff, dtype=torch.bfloat16, device=DEV)
+    ids = torch.zeros(tokens, top, dtype=torch.int32, device=DEV)
+    assert (ops.expert_down(h, ids, None, w) == 0).all()
+    assert called == ["dl_expert_down_rows" if once else "dl_expert_down"]
+
+
+@pytest.mark.parametrize("tokens,top,ff,K,E,once", [(6, 8, 700, 2048, 16, False), (6, 8, 704, 2048, 16, True), (8, 2, 512, 4096, 32, False), (4, 2, 512, 4096, 32, True),
+                                                    (8, 2, 600, 4096, 32, True), (8, 2, 512, 6144, 16, True)])
+def test_gate_up_products_read_once_where_that_pays(tokens, top, ff, K, E, once, monkeypatch):
+    from dotllm_b200.kernels import library, ops
+    called = []
+    real = library.call
+    monkeypatch.setattr(library, "call", lambda name, *a: (called.append(name), real(name, *a))[1])
+    x, w = torch.zeros(tokens, K, dtype=torch.bfloat16, device=DEV), torch.zeros(E, 2 * ff, K, dtype=torch.bfloat16, device=DEV)
+    ids = torch.zeros(tokens, top, dtype=torch.int32, device=DEV)
+    assert (ops.expert_gate_up(x, ids, w, "silu") == 0).all()
+    assert called == ["dl_expert_gate_up_rows" if once else "dl_expert_gate_up"]
