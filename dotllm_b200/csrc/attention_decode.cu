@@ -150,6 +150,7 @@ __device__ __forceinline__ int ad_pages_of(int len, AdWin win) {
 // all if the longest pair is at most `slack` pages longer than that (parts that pass between blocks cost 3 us as well).  128 KB of
 // pages stream to a multiprocessor in that time.  An attention layer (three launches, in a graph): 8 sequences of 1,100 to 2,000 tokens, 32 heads of 64,
 // 24.4 -> 23.2 us; 8 of 280 to 500, heads of 128, 31.8 -> 29.2; 18 of 360 to 700 47.0 -> 39.6; a decode step of 16 such layers (the first) 855 -> 840.
+// Against shares alone, the attention in a chain of its own, heads of 64 (128): 18 of 360 to 700 16.0 -> 9.4 (22.1 -> 12.1), 16 of a page 6.2 -> 6.5 (7.9 -> 8.1).
 struct AdCut {
     int total, share;        // pages in the step, pages per block
     int len;                 // 0: shares; else pages of a pair's segment, at most
@@ -175,30 +176,38 @@ __device__ __forceinline__ AdCut ad_cut(const int32_t* seq_len, int n_seqs, int 
     c.share = max(min_share, (c.total + n_blocks - 1) / n_blocks);
     c.len = 0;
     // Only what the lengths say decides, so that rows without pages (a captured step wider than its batch) change nothing.  Long shares are left
-    // alone: the search takes 0.3 us, and what it saves is little of theirs.
+    // alone: the search takes 0.2 us, and what it saves is little of theirs.
     const int live = 32 - __clz(__ballot_sync(0xffffffffu, mine > 0));
     if (c.share <= 3 * slack && live * nkv <= n_blocks && !__any_sync(0xffffffffu, beyond)) {
+        if (longest <= c.share + slack) {                    // not cut, whatever the segments would be (16 sequences of a page or two: 1.3 us of search)
+            c.len = longest;                                 // (0: no pages at all)
+            return c;
+        }
         // lane j tries segments of share + j pages; slack < 32
         const int try_len = c.share + lane;
         const float per_page = 1.0f / (float)try_len;
         int segments = 0;
 #pragma unroll 1
-        for (int b = 0; b < live; ++b) {                     // ceil(pages / try_len); the quotient in float32 is at most one off
-            const int pages = __shfl_sync(0xffffffffu, mine, b);
-            int n = (int)((float)pages * per_page);
-            n += n * try_len < pages ? 1 : 0;
-            n += n * try_len < pages ? 1 : 0;
-            n -= (n - 1) * try_len >= pages ? 1 : 0;
-            segments += n;
+        for (int b0 = 0; b0 < live; b0 += 4) {               // ceil(pages / try_len); the quotient in float32 is at most one off
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {                    // (four of them on their way at once; rows behind the live ones have no pages)
+                const int pages = __shfl_sync(0xffffffffu, mine, b0 + i);
+                int n = (int)((float)pages * per_page);
+                n += n * try_len < pages ? 1 : 0;
+                n += n * try_len < pages ? 1 : 0;
+                n -= (n - 1) * try_len >= pages ? 1 : 0;
+                segments += n;
+            }
         }
         const unsigned fits = __ballot_sync(0xffffffffu, segments * nkv <= n_blocks && lane <= slack);
         const int shortest = fits != 0 ? c.share + __ffs(fits) - 1 : c.share;
-        c.len = longest <= shortest + slack ? longest : fits != 0 ? shortest : 0;      // (longest 0: no pages at all)
+        // (not longer than 1.25 slack beyond a share: a lone layer waits for its longest block, 12 sequences of 750 to 1,500, heads of 64, 27.6 against 25.1 us)
+        c.len = longest <= min(shortest, c.share + slack / 4) + slack ? longest : fits != 0 ? shortest : 0;
     }
     return c;
 }
 // Blocks' units that a pair's pages make: pages of a share, or segments.
-__device__ __forceinline__ int ad_units(int pages, int len) { return len > 0 ? (pages + len - 1) / len : pages; }
+__device__ __forceinline__ int ad_units(int pages, int len) { return len == 0 || pages == 0 ? pages : pages <= len ? 1 : (pages + len - 1) / len; }
 
 // The sequence that holds unit r of the list (r < total), and the units of the list before it.
 __device__ __forceinline__ void ad_locate(const int32_t* seq_len, int n_seqs, int nkv, AdWin window, int len, int r, int lane,
@@ -258,13 +267,18 @@ __device__ __forceinline__ AdWalk ad_walk_begin(const AdCut& c, const int32_t* s
         w.len = seq_len[w.b];
         w.np = ad_pages_of(w.len, window);
         const int off = w.r - before, units = ad_units(w.np, c.len);
-        w.kvh = off / units;
-        w.pg = off - w.kvh * units;
-        if (c.len > 0) {                                     // w.pg is the segment's number so far
-            w.n_seg = units, w.i0 = block - w.pg;
-            w.r_end = (w.pg + 1) * w.np / units;
-            w.pg = w.pg * w.np / units;
-            w.r = w.pg;
+        if (units == 1) {                                    // a page, or a whole pair: no divisions
+            w.kvh = off;
+            if (c.len > 0) w.n_seg = 1, w.i0 = block, w.r = 0, w.r_end = w.np;
+        } else {
+            w.kvh = off / units;
+            w.pg = off - w.kvh * units;
+            if (c.len > 0) {                                 // w.pg is the segment's number so far
+                w.n_seg = units, w.i0 = block - w.pg;
+                w.r_end = (w.pg + 1) * w.np / units;
+                w.pg = w.pg * w.np / units;
+                w.r = w.pg;
+            }
         }
     }
     return w;
@@ -580,11 +594,13 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_
                 if (WIDE && g + 8 < group) qf_hi[c] = *reinterpret_cast<const uint4*>(qb + (size_t)(g + 8) * HD + c * 32 + t * 8);
             }
         };
-        // A block cuts at most two pairs, the first's segment in slot 0 and the last's in slot 1 (pairs between them are whole).  Both are
-        // counted in behind the last segment: an atomic between segments would have every warp wait for it.
+        // A block cuts at most two pairs, the first's segment in slot 0 and the last's in slot 1 (pairs between them are whole).  A first segment with
+        // others behind it is counted in at once, by one thread that looks at the answer behind the last one (where both are counted in there, a block
+        // may have both to merge at its end: 24 sequences of 75 to 150, heads of 128, 15.4 against 14.1 us); the others behind the last segment.
         if (threadIdx.x == 0) cut_pair[0][0] = cut_pair[1][0] = -1, cut_pair[0][2] = walk.i0, cut_pair[0][3] = walk.n_seg;
         dl_grid_dependency_wait();       // q comes from the kernel before this one; out and the scratch may be in use by it
         if (more) load_q(w);
+        int seen_first = -1;                                 // thread 32: blocks counted in before this one
         while (more) {
             {
                 // the biases of rows g and g+8 (read only where the row exists)
@@ -972,6 +988,10 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_
                 }
             }
             ad_consumer_sync(n_stages);                              // the merge buffers are free for the next run
+            if (threadIdx.x == 32 && more && w.slot == 0 && !w.whole) {
+                int* counter = pair_counters + w.b * nkv + w.kvh;
+                asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(seen_first) : "l"(counter) : "memory");
+            }
             w = next;
         }
         // Each of a cut pair's blocks counts itself in once its segment is written (one
@@ -980,24 +1000,26 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_
         ad_consumer_sync(n_stages);                          // (a block without segments has none to wait for)
         if (cut_pair[0][0] >= 0 || cut_pair[1][0] >= 0) {
             const int tid = threadIdx.x;
-            if ((tid == 0 || tid == 32) && cut_pair[tid >> 5][0] >= 0) {
-                const int* c = cut_pair[tid >> 5];
-                int seen;
+            const int mine = tid == 32 ? 0 : 1;              // thread 32 counts slot 0, thread 0 slot 1
+            if ((tid == 0 || tid == 32) && cut_pair[mine][0] >= 0) {
+                const int* c = cut_pair[mine];
+                int seen = mine == 0 ? seen_first : -1;
                 int* counter = pair_counters + c[0] * nkv + c[1];
-                asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(seen) : "l"(counter) : "memory");
-                last_of_pair[tid >> 5] = (seen == c[3] - 1) ? 1 : 0;
+                if (seen < 0) asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(seen) : "l"(counter) : "memory");
+                last_of_pair[mine] = (seen == c[3] - 1) ? 1 : 0;
                 if (seen == c[3] - 1) *counter = 0;          // ready for the next launch
             }
             ad_consumer_sync(n_stages);
-#pragma unroll 1
-            for (int slot = 0; slot < 2; ++slot)
-                if (cut_pair[slot][0] >= 0 && last_of_pair[slot] != 0) {
-                    const int b = cut_pair[slot][0], kvh = cut_pair[slot][1];
-                    ad_merge_pair<HD, WIDE ? 4 : 8>(out + (size_t)b * out_stride + (size_t)kvh * group * HD, group, cut_pair[slot][2], cut_pair[slot][3],
-                                      cut_pair[slot][4], part_o, part_ml, tid, 32 * n_stages,
-                                      fresh.gate != nullptr ? fresh.gate + (size_t)b * fresh.gate_stride + kvh * group : nullptr,
-                                      fresh.sinks != nullptr ? fresh.sinks + kvh * group : nullptr);
-                }
+            // Where both are complete, half of the warps merge each: a merge is a chain of loads, seldom work for all threads.
+            const bool first = cut_pair[0][0] >= 0 && last_of_pair[0] != 0, second = cut_pair[1][0] >= 0 && last_of_pair[1] != 0;
+            const int half = n_stages / 2 * 32, slot = first ? (second && tid >= half ? 1 : 0) : 1;
+            if (first || second) {
+                const int b = cut_pair[slot][0], kvh = cut_pair[slot][1], n_threads = !(first && second) ? 32 * n_stages : slot == 0 ? half : 32 * n_stages - half;
+                ad_merge_pair<HD, WIDE ? 4 : 8>(out + (size_t)b * out_stride + (size_t)kvh * group * HD, group, cut_pair[slot][2], cut_pair[slot][3],
+                                  cut_pair[slot][4], part_o, part_ml, first && second && slot == 1 ? tid - half : tid, n_threads,
+                                  fresh.gate != nullptr ? fresh.gate + (size_t)b * fresh.gate_stride + kvh * group : nullptr,
+                                  fresh.sinks != nullptr ? fresh.sinks + kvh * group : nullptr);
+            }
         }
     }
     __syncthreads();                                         // nobody leaves while copies may still land

@@ -958,7 +958,9 @@ def test_attention_decode_with_the_new_token_inside(nh, nkv, hd, rotate, window,
     (4, 4, 128, [1500, 70, 1300, 1024, 1, 900]),
     (8, 8, 64, [4500, 4000, 60, 3300, 3000]),                              # shares
     (2, 2, 32, [2900, 2900, 40]), (24, 2, 64, [1900, 700, 1200]),
-    (3, 3, 64, [64 * (1 + i % 7) for i in range(32)]), (3, 3, 64, [64 * (1 + i % 7) for i in range(33)])])
+    (3, 3, 64, [64 * (1 + i % 7) for i in range(32)]), (3, 3, 64, [64 * (1 + i % 7) for i in range(33)]),
+    (8, 8, 64, [150 - 3 * i for i in range(24)]), (32, 8, 128, [150 - 3 * i for i in range(24)]),      # a block ends one pair, holds some, begins another
+    (8, 8, 64, [1500 - 62 * i for i in range(12)]), (8, 8, 64, [60] * 16), (8, 8, 64, [1, 64, 65, 129, 2])])
 @pytest.mark.parametrize("window,blocks", [(0, 0), (700, 0), (0, 40)])
 def test_attention_decode_cuts(nh, nkv, hd, lengths, window, blocks, monkeypatch):
     """The three ways in which a step's pages are cut, against float32 attention; the same bits on every launch and with rows that hold nothing behind
@@ -987,6 +989,22 @@ def test_attention_decode_cuts(nh, nkv, hd, lengths, window, blocks, monkeypatch
     close(got, ref, 2e-3, 2 ** -7)
     assert torch.equal(run(B, table.shape[1]), got) and torch.equal(run(B + 9, table.shape[1] + 5), got)
     library.check_status()
+
+
+def test_attention_decode_does_not_search_for_a_cut_of_short_sequences():
+    """128 pairs of a page each, of 4 sequences or of 32: the same blocks and bytes.  (A search through the sequences for a cut that their lengths do not
+    need took the 32 a third longer.)"""
+    from dotllm_b200.kernels import library
+    hd, t = 64, {}
+    for B, nkv in ((4, 32), (32, 4)):
+        k_pool, v_pool, table, _ = make_paged(B, [60] * B, nkv, hd, torch.bfloat16, seed=5)
+        plan = _decode_plan([60] * B)
+        plan.seq_start = pos = torch.full((B,), 59, dtype=torch.int32, device=DEV)
+        q, seq = torch.randn(B, 4 * nkv * hd, device=DEV).to(torch.bfloat16), torch.arange(B, dtype=torch.int32, device=DEV)
+        args = (q, k_pool.to(DEV), v_pool.to(DEV), seq, pos, table.to(DEV), 4 * nkv, nkv, hd, 0.125, 0)
+        t[B] = _chained_us(lambda: [ops().attention(*args, plan=plan) for _ in range(40)], 40)
+    library.check_status()
+    assert t[32] < 1.15 * t[4], t
 
 
 @pytest.mark.parametrize("fused", [False, True])
