@@ -45,8 +45,8 @@ int dl_gemm_skinny_bf16_static(const void* x, int x_stride, const void* w, void*
                                int out_stride, int M, int N, int K, int fuse_swiglu, void* stream);
 
 // Waits for `stream`, writes the give-up word of the static calls on the current device to *code
-// (0: all waits were served; 1, 3, 5: a producer's, a consumer's, the row factors' wait expired)
-// and clears it.  Allocates nothing.
+// (0: all waits were served; 1: a producer's wait expired, 3: a consumer's, 5: the sums' or
+// the row factors', 6: one for room for the sums) and clears it.  Allocates nothing.
 int dl_gemm_skinny_static_status(int* code, void* stream);
 
 #ifdef __cplusplus

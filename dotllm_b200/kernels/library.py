@@ -188,7 +188,9 @@ _status = {}
 _counters = []
 _STATUS_TEXT = {1: "a producer's wait for a free shared-memory stage expired",
                 2: "a block table named a page outside the pool",
-                3: "a consumer's wait for a bulk copy expired"}
+                3: "a consumer's wait for a bulk copy expired",
+                5: "an epilogue's wait for a product's sums or for its rows' factors expired",
+                6: "a consumer's wait for room for a product's sums expired"}
 
 
 def register_counters(tensor):

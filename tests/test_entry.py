@@ -68,6 +68,21 @@ def test_tensors_without_a_gpu(entry):
     assert library.empty(2, 3, torch.int32, x).dtype == torch.int32
 
 
+def test_every_code_that_kernels_share_has_a_text(monkeypatch):
+    """A wait that ran out says in words whose it was; codes from 10 on belong to one kernel each, whose source lists them."""
+    import re
+    from dotllm_b200.kernels import build
+    written = set()
+    for source in build.sources():
+        written |= {int(n) for n in re.findall(r"(?:atomicExch\(\w*\.?status, |\bgave\()(\d)\)", source.read_text())}
+    assert written == set(library._STATUS_TEXT)
+    for code in written:
+        monkeypatch.setattr(library, "_status", {None: torch.full((1,), code, dtype=torch.int32)})
+        with pytest.raises(KernelError, match="gave up: a.* (expired|pool)$"):
+            library.check_status()
+        library.check_status()                               # the word is clear again
+
+
 @pytest.mark.gpu
 def test_sizes_of_a_product_say_what_the_general_rule_says(entry):
     """``product`` against the rules it stands for, over types, strides, offsets and odd sizes."""
