@@ -148,11 +148,12 @@ __device__ __forceinline__ void gs_epilogue(const float (&acc_in)[NT][4], TOut* 
     }
 }
 
-// Built with -DGS_TIMELINE (DOTLLM_NVCC_EXTRA), every warp of a product by shares stamps the global nanosecond timer at six
+// Built with -DGS_TIMELINE (DOTLLM_NVCC_EXTRA), every warp of a product stamps the global nanosecond timer at six
 // points of a launch into gs_timeline, which dl_gemm_skinny_timeline copies out
 // (`python -m dotllm_b200.kernels.microbench gemm_skinny --timeline` prints the spread over the grid).
+#define GS_TIMELINE_WARPS 12                     // of a block, at most (GR_THREADS(3) / 32)
 #ifdef GS_TIMELINE
-__device__ long long gs_timeline[6][2048];       // [event][block * (GS_CONSUMERS + 2) + warp]
+__device__ long long gs_timeline[6][2048];       // [event][block * GS_TIMELINE_WARPS + warp]
 __device__ __forceinline__ long long gs_now() {
     long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -160,7 +161,7 @@ __device__ __forceinline__ long long gs_now() {
 }
 #define GS_STAMP(ev)                                                                                                     \
     do {                                                                                                                 \
-        const int slot__ = blockIdx.x * (GS_CONSUMERS + 2) + (threadIdx.x >> 5);                                          \
+        const int slot__ = blockIdx.x * GS_TIMELINE_WARPS + (threadIdx.x >> 5);                                             \
         if ((threadIdx.x & 31) == 0 && slot__ < 2048) gs_timeline[ev][slot__] = gs_now();                                 \
     } while (0)
 extern "C" int dl_gemm_skinny_timeline(long long* out) {
@@ -531,6 +532,7 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
     __shared__ volatile int gave_up;
     __shared__ float row_scale_smem[GS_MAX_ROWS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    GS_STAMP(0);                                             // block started
     if (threadIdx.x == 0) {
         gave_up = 0;
         gs_mbar_init(&scale_bar, 1);
@@ -544,6 +546,7 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
     }
     __syncthreads();
     dl_launch_dependents();
+    GS_STAMP(1);                                             // barriers ready
     const int first = blockIdx.x * w.block_rows, end_row = min(w.N, first + w.block_rows);      // this block's rows
     const int passes = (end_row - first + w.rows - 1) / w.rows, total = passes * w.cpt;
     const uint32_t box_bytes = w.rows * (BK * 2), stage_bytes = GR_stage_rows(w.rows, FUSE_SWIGLU, TILES) * (BK * 2);
@@ -571,6 +574,7 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
                     for (int e = 0; e < 4 * CHAINS; ++e) acc[i][j][e / 4][e % 4] = 0.f;
             for (const int pass_end = (p + 1) * w.cpt; cur < pass_end; cur += GS_CONSUMERS) {
                 if (!dead && !gs_mbar_wait(&full_bar[warp][slot], phase, &gave_up)) gave(3);
+                if (cur == warp) GS_STAMP(2);                // the warp's first chunk has landed
                 const int next = cur + GS_CONSUMERS, k_next = next < total ? (next % w.cpt) * BK : w.K;
                 uint4 xn[BK / 32][NT];
                 if (!IN_PLACE) gs_rows_x<NT>(xn, w, k_next, g, t);
@@ -607,6 +611,7 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
                     if (lane == 0) gs_mbar_arrive(&empty_bar[warp][slot]);
                 }
                 if (++slot == w.slots) slot = 0, phase ^= 1;
+                if (next >= total) GS_STAMP(3);              // the warp's last chunk is consumed
                 if (!IN_PLACE) {
 #pragma unroll
                     for (int s = 0; s < BK / 32; ++s)
@@ -634,6 +639,7 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
             __syncwarp();
             if (lane == 0) gs_mbar_arrive(&sums_full[h]);
         }
+        GS_STAMP(4);                                         // its sums are handed over
     } else if (warp == GS_CONSUMERS) {
         // ------------------------------------------------------------ producer warp: lane c serves consumer warp c
         // When the caller vouches that no pending work writes the weights (early_weights), the rings fill while the kernel before this one finishes.
@@ -726,6 +732,7 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
         }
     }
     __syncthreads();                                         // nobody leaves while copies may still land
+    GS_STAMP(5);
 }
 
 // Which products go that way; the others by shares.  By rows every block reads all of x, by shares what passes between blocks takes its time: rows

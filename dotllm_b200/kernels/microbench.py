@@ -87,6 +87,25 @@ def _paged(batch, context, nkv, hd, dev):
     return k_pool, v_pool, table
 
 
+TIMELINE_EVENTS = ("block_start", "barriers_ready", "first_chunk_landed", "last_chunk_consumed", "sums_handed_over", "block_end")
+TIMELINE_WARPS, TIMELINE_SLOTS = 12, 2048               # of a block (GS_TIMELINE_WARPS in csrc/gemm_skinny.cu), of an event
+
+
+def timeline_spread(stamps):
+    """{event: (first, mean, last)} in nanoseconds after the first block's start, from the stamps of one launch (0: no such warp)."""
+    blocks = TIMELINE_SLOTS // TIMELINE_WARPS
+    starts = [stamps[b * TIMELINE_WARPS] for b in range(blocks) if stamps[b * TIMELINE_WARPS]]
+    if not starts:
+        raise SystemExit("the launch left no time stamps")
+    spread = {}
+    for e, name in enumerate(TIMELINE_EVENTS):
+        warps = [0] if e in (0, 1, 5) else range(TIMELINE_WARPS)
+        v = [stamps[e * TIMELINE_SLOTS + b * TIMELINE_WARPS + w] - min(starts) for b in range(blocks) for w in warps
+             if stamps[e * TIMELINE_SLOTS + b * TIMELINE_WARPS + w]]
+        spread[name] = (min(v), sum(v) // len(v), max(v)) if v else None
+    return spread
+
+
 def main(argv=None):
     ap = argparse.ArgumentParser()
     ap.add_argument("kernel", choices=["attention_decode", "attention_prefill", "gemm_skinny", "gemm_tc", "norm", "rope", "sample"])
@@ -218,16 +237,7 @@ def main(argv=None):
             lib.dl_gemm_skinny_timeline.argtypes = [ctypes.c_void_p]
             if lib.dl_gemm_skinny_timeline(buf) != 0:
                 raise SystemExit("could not read the timeline")
-            stride = gemm_skinny.CONSUMER_WARPS + 2         # warps of a block: the consumers, the producer, the statistics warp
-            blocks = min(148, 2048 // stride)
-            first = min(buf[b * stride] for b in range(blocks) if buf[b * stride])
-            names = ["block_start", "barriers_ready", "first_chunk_landed", "last_chunk_consumed", "share_done", "block_end"]
-            spread = {}
-            for e, name in enumerate(names):
-                warps = [0] if e in (0, 1, 5) else range(gemm_skinny.CONSUMER_WARPS)
-                v = [buf[e * 2048 + b * stride + w] - first for b in range(blocks) for w in warps
-                     if buf[e * 2048 + b * stride + w]]
-                spread[name] = [min(v), sum(v) // len(v), max(v)]
+            spread = timeline_spread(buf)
             result["timeline_ns_min_mean_max"] = spread
         # The same product as a decode step issues it: launches back to back from a captured graph,
         # each on a different copy of W (together larger than the L2), with and without the
