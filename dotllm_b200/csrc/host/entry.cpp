@@ -187,6 +187,12 @@ PyObject* product(PyObject*, PyObject* const* args, Py_ssize_t n) {
     });
 }
 
+// The lock is given up while the allocator works, as torch.empty does: it may wait for the device, or for another thread's allocation.
+struct WithoutLock {
+    PyThreadState* state = PyEval_SaveThread();
+    ~WithoutLock() { PyEval_RestoreThread(state); }
+};
+
 // empty(rows, width, bfloat16, like): a contiguous tensor on like's device, float32 or bfloat16.
 PyObject* empty(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
@@ -198,7 +204,12 @@ PyObject* empty(PyObject*, PyObject* const* args, Py_ssize_t n) {
         const int64_t rows = PyLong_AsLongLong(args[0]), width = PyLong_AsLongLong(args[1]);
         const int half = PyObject_IsTrue(args[2]);
         if (half < 0 || ((rows == -1 || width == -1) && PyErr_Occurred())) return nullptr;
-        return THPVariable_Wrap(at::empty({rows, width}, at::TensorOptions().dtype(half ? at::kBFloat16 : at::kFloat).device(like->device())));
+        at::Tensor t;
+        {
+            WithoutLock unlocked;
+            t = at::empty({rows, width}, at::TensorOptions().dtype(half ? at::kBFloat16 : at::kFloat).device(like->device()));
+        }
+        return THPVariable_Wrap(std::move(t));
     });
 }
 

@@ -68,6 +68,24 @@ def test_tensors_without_a_gpu(entry):
     assert library.empty(2, 3, torch.int32, x).dtype == torch.int32
 
 
+def test_allocation_leaves_other_threads_running(entry):
+    """``empty`` gives up the interpreter's lock: another thread runs although the interpreter itself would not switch for a minute."""
+    import _thread
+    import sys
+    like, ran, kept = torch.zeros(1), [], []
+    before = sys.getswitchinterval()
+    sys.setswitchinterval(60.0)
+    try:
+        _thread.start_new_thread(lambda: ran.append(1), ())  # (threading's start() waits for the thread, and gives up the lock itself)
+        for _ in range(3000):                                # (kept: a tensor's end may give up the lock as well)
+            kept.append(entry.empty(512, 512, False, like))
+            if ran:
+                break
+        assert ran
+    finally:
+        sys.setswitchinterval(before)
+
+
 def test_every_code_that_kernels_share_has_a_text(monkeypatch):
     """A wait that ran out says in words whose it was; codes from 10 on belong to one kernel each, whose source lists them."""
     import re
