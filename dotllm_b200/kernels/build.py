@@ -2,7 +2,9 @@
 
 The library is built in-tree (``csrc/_build/``) the first time it is needed and again
 whenever a source, a header or the flags change.  Only ``nvcc`` is needed: the sources
-include no PyTorch headers and the library is loaded through ``ctypes``.  If the tree is
+include no PyTorch headers.  The module that calls the library from Python (``build_entry``)
+also needs a C++ compiler and the headers of Python and PyTorch; without them the calls go
+through ``ctypes`` (``library.entry``).  If the tree is
 not writable the build goes to a per-user folder under the system's temporary directory.
 Progress goes to standard error, one line per file, so that a first call that compiles
 for a minute is seen to be alive.
@@ -182,7 +184,9 @@ def build_entry(verbose=True):
     import torch
     source = CSRC / "host" / "entry.cpp"
     root = Path(torch.__file__).resolve().parent
+    python = sysconfig.get_paths()["include"]
     cuda = str(Path(find_nvcc()).resolve().parent.parent / "include") if shutil.which("nvcc") or os.environ.get("NVCC") else "/usr/local/cuda/include"
+    compiler = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
     flags = ["-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     digest = _digest([source], " ".join(flags) + torch.__version__ + sys.version)
     for folder in (CSRC / "_build", None):
@@ -195,9 +199,14 @@ def build_entry(verbose=True):
         fcntl.flock(lock, fcntl.LOCK_EX)
         if so.is_file() and mark.is_file() and mark.read_text() == digest:
             return so
+        if compiler is None:
+            raise KernelError(f"{source.name} needs a C++ compiler (g++ or c++ on PATH, or CXX)")
+        for folder_of, header in ((python, "Python.h"), (root / "include", "torch/csrc/autograd/python_variable.h"), (cuda, "cuda_runtime_api.h")):
+            if not (Path(folder_of) / header).is_file():
+                raise KernelError(f"{source.name} needs {header}, which is not in {folder_of}")
         t0 = time.time()
-        cmd = [os.environ.get("CXX") or shutil.which("g++") or "c++", *flags, "-I", str(root / "include"), "-I", str(root / "include/torch/csrc/api/include"),
-               "-I", sysconfig.get_paths()["include"], "-I", cuda, str(source), "-o", str(so) + ".tmp", "-L", str(root / "lib"),
+        cmd = [compiler, *flags, "-I", str(root / "include"), "-I", str(root / "include/torch/csrc/api/include"),
+               "-I", python, "-I", cuda, str(source), "-o", str(so) + ".tmp", "-L", str(root / "lib"),
                "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:

@@ -68,6 +68,62 @@ def test_tensors_without_a_gpu(entry):
     assert library.empty(2, 3, torch.int32, x).dtype == torch.int32
 
 
+@pytest.mark.parametrize("lacking", ["compiler", "Python.h", "broken"])
+def test_machines_without_the_modules_headers_call_by_ctypes(entry, lacking, monkeypatch, tmp_path, capsys):
+    """The kernel library alone is enough to run: where the module cannot be built, the missing piece is named and the calls go through ctypes."""
+    import sysconfig
+    from dotllm_b200.kernels import build
+    monkeypatch.setattr(library, "_entry", None)
+    monkeypatch.setattr(library, "_callables", {})
+    monkeypatch.setattr(build, "ENTRY", "dotllm_entry_of_a_test")
+    monkeypatch.setattr(build, "build_dir", lambda: tmp_path)
+    if lacking == "compiler":
+        monkeypatch.delenv("CXX", raising=False)
+        monkeypatch.setattr(build.shutil, "which", lambda name: None)
+    elif lacking == "Python.h":
+        paths = sysconfig.get_paths()
+        monkeypatch.setattr(sysconfig, "get_paths", lambda *a: {**paths, "include": str(tmp_path)})
+    else:
+        monkeypatch.setenv("CXX", "/bin/false")
+    pieces = library._bind("dl_chunk_pieces")
+    assert isinstance(library.entry(), library._CtypesEntry) and {"compiler": "C++ compiler", "Python.h": "Python.h", "broken": "failed"}[lacking] in capsys.readouterr().err
+    assert pieces(100, 3) == entry.bind(entry.handle, "dl_chunk_pieces")(100, 3)
+    for bad in ((1,), (1, 2, 3), (1, 1.5), (1, "1"), (1, None), (1, torch.zeros(1))):
+        with pytest.raises(TypeError):
+            pieces(*bad)
+    for name in library._SIGNATURES:
+        assert callable(library._bind(name))
+    with pytest.raises(KernelError, match="dl_scale_values"):
+        library.call("dl_scale_values", None, -1, 1.0, None)
+    assert library.empty(2, 3, torch.bfloat16, torch.zeros(1)).dtype == torch.bfloat16
+
+
+@pytest.mark.gpu
+def test_kernels_called_by_ctypes_give_the_same(entry, monkeypatch):
+    from dotllm_b200.kernels import ops
+    g = torch.Generator().manual_seed(3)
+    x, w = (torch.randn(*s, generator=g).to(torch.bfloat16).cuda() for s in ((5, 520), (96, 520)))
+    x32, gain = x.float(), torch.rand(520, generator=g).cuda()
+
+    def run():
+        return [ops.linear(x, w), ops.gated_linear(x, w), ops.linear(x32, w.float()), ops.add_rmsnorm(x32.clone(), None, gain, 1e-5, torch.bfloat16),
+                ops.linear(x[:, 8:264], w[:, :256].contiguous(), out_dtype=torch.float32)]
+
+    want = run()
+    torch.cuda.synchronize()
+    monkeypatch.setattr(library, "_entry", library._CtypesEntry())
+    monkeypatch.setattr(library, "_callables", {})
+    library._entry.handle = None
+    with torch.cuda.stream(torch.cuda.Stream()):
+        got = run()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
+    with pytest.raises(KernelError):
+        ops.linear(x, w[:, :256].contiguous())
+    with pytest.raises(KernelError):
+        ops.linear(x.cpu(), w)
+
+
 def test_allocation_leaves_other_threads_running(entry):
     """``empty`` gives up the interpreter's lock: another thread runs although the interpreter itself would not switch for a minute."""
     import _thread
