@@ -199,3 +199,29 @@ def test_gate_up_products_read_once_where_that_pays(tokens, top, ff, K, E, once,
     ids = torch.zeros(tokens, top, dtype=torch.int32, device=DEV)
     assert (ops.expert_gate_up(x, ids, w, "silu") == 0).all()
     assert called == ["dl_expert_gate_up_rows" if once else "dl_expert_gate_up"]
+
+
+@pytest.mark.parametrize("tokens,top,E,K,ff,N", [(16, 8, 64, 4096, 1024, 2048), (8, 16, 128, 1024, 1408, 4736), (16, 1, 16, 2048, 9472, 2048)])
+def test_chosen_experts_repeat_with_full_rings(tokens, top, E, K, ff, N, monkeypatch):
+    """Many entries, of several passes in the last, with every column of the instructions in use: slots are refilled the moment they are released, and 30
+    launches give the bits of the first, which are near the exact ones (a slot released before its reads are done shows as wrong columns)."""
+    from dotllm_b200.kernels import library, ops
+    monkeypatch.setattr(ops, "EXPERT_ROWS_MB", (0.0, 0.0))
+    g = torch.Generator(device=DEV).manual_seed(E)
+    make = lambda *s: (torch.randn(*s, generator=g, device=DEV) * 0.05).to(torch.bfloat16)
+    x, w_in, w_out = make(tokens, K), make(E, 2 * ff, K), make(E, N, ff)
+    ids = torch.stack([torch.randperm(E, generator=g, device=DEV)[:top] for _ in range(tokens)]).to(torch.int32)
+    weights = torch.rand(tokens, top, generator=g, device=DEV)
+    assert ops.experts_by_rows(x, ids, w_in, w_out, "silu")
+    h = ops.expert_gate_up(x, ids, w_in, "silu")
+    y = ops.expert_down(h, ids, weights, w_out, read_once=True)
+    flat = ids.flatten().tolist()
+    z = torch.stack([w_in[e].double() @ x[r // top].double() for r, e in enumerate(flat)])
+    want_h = torch.nn.functional.silu(z[:, :ff]) * z[:, ff:]
+    assert float((h.double() - want_h).norm() / want_h.norm()) < 2.0 ** -8       # rounded once to bfloat16
+    want = (weights.flatten()[:, None].double() * torch.stack([w_out[e].double() @ h[r].double() for r, e in enumerate(flat)])).view(tokens, top, N).sum(1)
+    assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -22          # float32 sums (test_sums_of_chosen_experts_keep_float32)
+    for _ in range(30):
+        again = ops.expert_gate_up(x, ids, w_in, "silu")
+        assert torch.equal(again, h) and torch.equal(ops.expert_down(again, ids, weights, w_out, read_once=True), y)
+    library.check_status()

@@ -479,19 +479,28 @@ def test_gemm_skinny(M, N, K, out_dtype, monkeypatch):
     assert torch.equal(gemm_skinny.run(x.to(DEV), w.to(DEV), out_dtype).cpu(), y.cpu())
 
 
-def test_gemm_skinny_repeats_with_full_rings(monkeypatch):
-    """16 rows make the consumer warps the slower side, so the rings stay full and every slot is
+@pytest.mark.parametrize("N,K,gated", [(4096, 4096, False), (20000, 4096, False), (4096, 14336, False), (9472, 8192, True), (2048, 8192, False), (2400, 24576, False)])
+def test_gemm_skinny_repeats_with_full_rings(N, K, gated, monkeypatch):
+    """16 rows make the consumer warps the slower side, so the rings stay full and a slot is
     refilled the moment it is released: 30 launches must give the same bits as the first (a release
-    that does not wait for the reads of the slot shows up as a few wrong output columns)."""
+    that does not wait for the reads of the slot shows up as a few wrong output columns).  By rows a warp has four chunks for its slots in the first
+    size and dozens in several passes in the next ones; the last two go by shares."""
     from dotllm_b200.kernels import gemm_skinny
     monkeypatch.setattr(gemm_skinny, "SKINNY_ROWS", gemm_skinny.KERNEL_ROWS)
+    assert gemm_skinny.plan(N, K, gated)[0] == ("shares" if (N, K) in ((2048, 8192), (2400, 24576)) else "rows")
     g = torch.Generator().manual_seed(27)
-    x = torch.randn(16, 4096, generator=g).to(torch.bfloat16).to(DEV)
-    w = (torch.randn(4096, 4096, generator=g) * 0.05).to(torch.bfloat16).to(DEV)
-    first = gemm_skinny.run(x, w, torch.float32)
-    close(first, (x.double() @ w.double().T).float(), 2e-4 * 8, 1e-5)
+    x = torch.randn(16, K, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn((2 if gated else 1) * N, K, generator=g) * 0.05).to(torch.bfloat16).to(DEV)
+    first = gemm_skinny.run(x, w, torch.float32, fuse_swiglu=gated)
+    p = x.double() @ w.double().T
+    if gated:
+        # the gating multiplies an error of the gate by at most 1.1 |up| and one of the up product by at most |gate|
+        ref, size = torch.nn.functional.silu(p[:, :N]) * p[:, N:], 1.1 * (p[:, :N].abs() + p[:, N:].abs() + 1)
+        assert ((first.double() - ref).abs() <= 2e-4 * math.sqrt(K / 64) * size + 1e-5 * ref.abs()).all()
+    else:
+        close(first, p.float(), 2e-4 * math.sqrt(K / 64), 1e-5)
     for _ in range(30):
-        assert torch.equal(gemm_skinny.run(x, w, torch.float32), first)
+        assert torch.equal(gemm_skinny.run(x, w, torch.float32, fuse_swiglu=gated), first)
 
 
 @pytest.mark.parametrize("N,K", [(16, 8), (1, 264), (17, 256), (40, 2048), (2048, 2048), (1184 * 16 + 5, 256), (9, 16384), (2368 * 2 + 16, 2048)])

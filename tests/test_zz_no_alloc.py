@@ -35,10 +35,13 @@ def _static_status(lib, stream):
 
 @pytest.mark.parametrize("M,N,K,fuse,out_dtype", [(8, 4096, 4096, 0, torch.float32), (3, 1000, 320, 0, torch.float32),
                                                   (16, 512, 2048, 1, torch.float32), (1, 6144, 512, 0, torch.float32),
-                                                  (5, 1000, 320, 0, torch.bfloat16), (16, 512, 2048, 1, torch.bfloat16)])
+                                                  (5, 1000, 320, 0, torch.bfloat16), (16, 512, 2048, 1, torch.bfloat16),
+                                                  # by shares: partial sums and counters in the scratch, which the next call finds used
+                                                  (16, 2000, 8192, 0, torch.float32), (9, 40, 12288, 0, torch.bfloat16), (8, 512, 14336, 1, torch.float32)])
 def test_static_scratch_product_matches_the_ordinary_one(M, N, K, fuse, out_dtype, monkeypatch):
     from dotllm_b200.kernels import gemm_skinny
     monkeypatch.setattr(gemm_skinny, "SKINNY_ROWS", gemm_skinny.KERNEL_ROWS)      # the same kernel on both sides, up to its 16 rows
+    assert gemm_skinny.plan(N, K, bool(fuse))[0] == ("shares" if K >= 8192 else "rows")
     lib, fn = _symbol()
     dev = torch.device("cuda", 0)
     g = torch.Generator().manual_seed(40)
@@ -71,7 +74,7 @@ def test_static_scratch_product_matches_the_ordinary_one(M, N, K, fuse, out_dtyp
 def test_static_scratch_refuses_what_does_not_fit():
     lib, fn = _symbol()
     dev = torch.device("cuda", 0)
-    M, N, K = 16, 16 * 20000, 64                             # more row tiles than the fixed scratch covers
+    M, N, K = 16, 16 * 20000, 64                             # more row tiles than the fixed scratch covers (by rows, which would need none of it, too)
     x = torch.zeros(M, K, dtype=torch.bfloat16, device=dev)
     w = torch.zeros(N, K, dtype=torch.bfloat16, device=dev)
     out = torch.zeros(M, N, dtype=torch.float32, device=dev)
