@@ -16,9 +16,11 @@
 //
 // What bounds it: the bytes of the chosen experts' matrices, and for small experts about 1.25 us an entry and product (1.8 with 16 columns): a chain of
 // the rows of x, a chunk's instructions and the hand-over of its sums.  Both products, against row by row: 8 tokens of 16 experts of 25 MB, two choices
-// each (11 distinct) 84 -> 53 us (5.2 TB/s); 32 experts of 50 MB, four choices (24 distinct) 335 -> 180 (6.7 TB/s).  Which steps go this way: kernels/ops.py.
+// each (11 distinct) 84 -> 49 us (5.6 TB/s); 32 experts of 50 MB, four choices (about 21 distinct) 280 -> 151.  Which steps go this way: kernels/ops.py.
 //
 // Every wait on an mbarrier is bounded; on expiry the kernel records a code in `status` and returns after waiting (bounded) for copies in flight.
+//
+// Rings, hand-over and producer are gemm_skinny_rows_kernel's with entries around the passes: a change to a wait or to the release of a slot belongs in both.
 #include "common.cuh"
 #include "gating.cuh"
 #include "stream_rows.cuh"

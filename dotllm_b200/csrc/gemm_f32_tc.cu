@@ -40,10 +40,10 @@
 //
 // Measured (launched one after the other, FFMA kernel in brackets): 500 x 16,384 x 2,048 in 216 us, 156 TFLOP/s (1,036); 2,048 x
 // 28,672 x 4,096 in 2.85 ms, 169 TFLOP/s (12.8); 8 rows x 28,672 x 4,096 in 122 us, 3.8 TB/s of W (528).  With 128 tokens the
-// shared memory is what bounds it: per block of 32 k the MMAs read 80 KB and as much passes through it besides, 1,250 cycles at 128
-// bytes a cycle against 770 of tensor pipe; three tensor-memory ranges of 128 columns leave no second set of accumulators, so the
-// pipe also waits for the epilogue once per run (runs of 128 k instead of 256: 5 % slower).  With a few tokens it is the MMAs' own
-// time, six per 16 KB of W, and the splitting.
+// tensor pipe is half used.  Of the 216 us, 209 are left without the splitting of W, 204 without the drain of the accumulators (three tensor-memory ranges of 128
+// columns leave no second set: the pipe waits for the epilogue once per run; runs of 128 k instead of 256: 5 % slower), 167 with a third of the MMAs: no one of them
+// bounds it alone.  Shared memory, 160 KB per block of 32 k by count, is at 22 % under ncu; the operands' way from the L2, 40 KB per block and
+// 9 TB/s over the GPU, is the likely bound.  With a few tokens it is the MMAs' own time, six per 16 KB of W, and the splitting.
 #include "common.cuh"
 #include "tma.cuh"
 #include "tcgen05.cuh"

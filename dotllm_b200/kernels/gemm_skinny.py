@@ -3,7 +3,7 @@
 Up to ``SKINNY_ROWS`` rows go to the mma.sync kernel of csrc/gemm_skinny.cu (it can take 16), more, up
 to 128, to the tcgen05 kernel of csrc/gemm_decode_tc.cu (``gemm_decode_tc.run``, same contract).  The first gives every multiprocessor
 the same rows of W, or (few sizes) cuts its work into equal shares per warp, where tiles that straddle two shares are summed through a
-scratch buffer with arrival counters.  Both are kept here per device (they are small and every launch leaves the
+scratch buffer with arrival counters (``plan`` tells).  Both are kept here per device (they are small and every launch leaves the
 counters zero).  Launches that share them must be on one stream.
 """
 from __future__ import annotations
@@ -29,10 +29,10 @@ _library.register_signatures({
 
 KERNEL_ROWS = 16         # rows the mma.sync kernel can take (two tiles of eight)
 # Rows up to which the dispatcher gives a product to the mma.sync kernel; more go the way of 17 and
-# more (the gated product to the tcgen05 kernel, the plain ones to the library).  Measured on whole
-# decode steps at the 8B shape: 9 rows 4.76 against 4.79 ms, 12 rows 5.30 against 5.24, 16 rows 6.08
-# against 5.83 - the second tile of eight rows costs the mma.sync kernel more than the library's
-# launch costs the step.
+# more (the gated product to the tcgen05 kernel, the plain ones to the library).  The line was drawn when the kernel cut every product into
+# shares (whole decode steps at the 8B shape: 9 rows 4.76 against 4.79 ms, 12 rows 5.30 against 5.24, 16 rows 6.08 against 5.83).  By rows it would
+# lie beyond 16: a step at the 1B shape of 12 rows 0.94 ms against 1.17 by the library and the tcgen05 kernel, of 16 rows 0.97 against 1.18; a gated
+# MLP of 16 rows, 8B, 59 us against 68; only the 8B attention layer's two products are about 1.5 us faster by the library.
 SKINNY_ROWS = 10
 MAX_ROWS = 128           # rows the two kernels take between them; beyond this the products are prefill products
 # Of 17 to 128 rows the gated product goes to the tcgen05 kernel (47 us against 56 for the library product plus
