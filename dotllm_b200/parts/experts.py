@@ -171,7 +171,8 @@ class RoutedExperts(FeedForward):
             return ops.experts_grouped(x, ids, weights, self.w_gate_up, self.w_down, self.activation, self.limit, self.alpha,
                                        addend=shared, row_scale=scale, addend_gate=shared_gate, identity=identity)
         h = ops.expert_gate_up(x, ids, self.w_gate_up, self.activation, self.limit, self.alpha, row_scale=scale)
-        return ops.expert_down(h, ids, weights, self.w_down, addend=shared, addend_gate=shared_gate, identity=identity, read_once=read_once)
+        once = {"read_once": True} if read_once else {}
+        return ops.expert_down(h, ids, weights, self.w_down, addend=shared, addend_gate=shared_gate, identity=identity, **once)
 
 
 register_feed_forward("routed_experts", RoutedExperts)
