@@ -147,7 +147,7 @@ __device__ __forceinline__ int ad_pages_of(int len, AdWin win) {
 // of the block's warps and its part of the output (about 3.4 us more than one segment of as many pages; a block's 11 pages of
 // 8 sequences of 1,100 to 2,000 tokens and heads of 64 take 4).  Where the pairs are no more than the blocks, a pair's pages are cut into
 // segments of at most `len` instead, a block each, as long as the longest is at most `slack` pages longer than a share would be; and not cut at
-// all if the longest pair is at most `slack` pages longer than that (parts that pass between blocks cost 3 us as well).  128 KB of
+// all if the longest pair is at most `slack` pages longer than that, and 1.25 `slack` longer than a share (parts that pass between blocks cost 3 us as well).  128 KB of
 // pages stream to a multiprocessor in that time.  An attention layer (three launches, in a graph): 8 sequences of 1,100 to 2,000 tokens, 32 heads of 64,
 // 24.4 -> 23.2 us; 8 of 280 to 500, heads of 128, 31.8 -> 29.2; 18 of 360 to 700 47.0 -> 39.6; a decode step of 16 such layers (the first) 855 -> 840.
 // Against shares alone, the attention in a chain of its own, heads of 64 (128): 18 of 360 to 700 16.0 -> 9.4 (22.1 -> 12.1), 16 of a page 6.2 -> 6.5 (7.9 -> 8.1).

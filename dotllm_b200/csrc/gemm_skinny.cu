@@ -24,8 +24,7 @@
 // By rows against by shares, each product in a graph of many, 8 rows: 3,072 x 2,048 5.5 -> 5.0 us, 2,048 x 2,048 5.1 -> 4.2, 64 x 2,048 3.8 -> 2.7, gated
 // 8,192 x 2,048 15.4 -> 13.3, 6,144 x 4,096 12.7 -> 11.1, 4,096 x 14,336 22.1 -> 20.9, gated 14,336 x 4,096 40.3 -> 38.5, 128,256 x 2,048
 // 87.0 -> 80.6 (6.5 TB/s); the small ones are a chain of latencies (start, rows of x, sums).  One tile a block leaves x at half the bytes of W again.
-// A decode step of 16 layers of the smaller
-// widths, 8 sequences at 2,000 tokens: 905 -> 849 us.  Tried: rings of half the size, so that the next product's first weights arrive under this one
+// A decode step of 16 layers of the smaller widths, 8 sequences at 2,000 tokens: 905 -> 849 us.  Tried: rings of half the size, so that the next product's first weights arrive under this one
 // (941 us), x asked for three chunks ahead (2,048 x 2,048 4.3 -> 4.7), passes of 32 rows (5,120 x 13,824, 35 rows a block: 25.5 -> 30.1).
 //
 // Two optional fusions take the add + RMSNorm between two products of a decode step into the products
@@ -742,6 +741,7 @@ gemm_skinny_rows_kernel(const __grid_constant__ CUtensorMap tmap, const GsRowsWo
 //   2,048 x 5,120   7.3 8.2 / 8.0 8.6      2,048 x 12,288 12.6 14.2 / 11.8 12.8     2,048 x 16,384  15.1 17.6 / 15.9 16.6
 //   1,536 x 14,336 12.6 14.5 / 11.1 12.2   512 x 4,096      4.5  5.3 / 5.1  5.8      512 x 14,336   10.2 12.6 / 8.0 9.1
 //   2,400 x 4,096 and less as 2,048        2,400 x 8,192  12.6 14.3 / 11.4 12.2     3,072 x 8,192   13.4 14.2 / 13.2 13.9
+//   2,368 x 12,288 13.5 15.5 / 14.3 14.8   2,368 x 16,384 16.4 18.6 / 17.3 17.8      (14 to 16 rows a block and K >= 12,288: level, 5 % either way)
 // Gated: 1,024 x 14,336 (14 rows: 7 pairs) 13.9 15.8 / 13.1 13.9, 512 x 8,192 7.6 9.0 / 6.9 8.0, 512 x 14,336 10.8 13.5 / 9.4 10.6, 64 x 14,336 9.5 12.2 / 7.7 8.8.
 static bool gs_by_rows(int N, int K, bool gated, int sms) {
     const int rows = (gated ? 2 : 1) * ((N + sms - 1) / sms);     // of W a block
@@ -773,7 +773,7 @@ static GsPlan gs_plan(int N, int K, int fuse_swiglu, int sms) {
     // A share is a whole number of chunks, so the last multiprocessors get less, or nothing: the number of warps, and the share, that leave the busiest
     // multiprocessor the fewest chunks.  Shares that do not divide a tile's chunks count six more: their warps end one tile and begin another, about 1 us
     // (1,536 x 8,192, 8 rows: seven warps of 3 of 32 chunks 8.75 us, six of 4 7.9; 1,024 x 10,240: six of 3 of 40 8.9, six of 4 8.1).  And a tile is cut
-    // into 28 parts at most, or fewer where k is long, since one warp adds them all (512 x 8,192: 32 parts 7.3 us, 16 6.3; 512 x 12,288: 24
+    // into 31 parts at most, or fewer where k is long, since one warp adds them all (512 x 8,192: 32 parts 7.3 us, 16 6.3; 512 x 12,288: 24
     // parts 7.3, 12 7.2; 16 x 16,384: 64 parts 9.0, 32 7.1, 16 6.7).  Of equals the one with more warps: they have more of the ring.
     const int least = p.cpt >= 48 ? 4 : p.cpt >= 32 ? 2 : 1;
     int best = 0;
